@@ -34,10 +34,83 @@ template <> struct Elem<BSP_U8> {
   __device__ static bool nz(T x) { return x != 0; }
 };
 
-constexpr int kWordsPerWarpIter = 4;
+// Rows that start 16-byte aligned.  A lane loads 16 bytes (VEC columns), makes
+// their VEC bits, and the G = 32 / VEC lanes of a word OR theirs together; a
+// warp takes U such loads (512 columns of FP32, 1024 of the narrower types)
+// before it stores, so 2 KB a warp are in flight.  Bound by HBM: the form
+// that built a word by one ballot of 32 scalar loads, with a 64-bit division
+// per word, read 4096x4096 FP32 at 1.5 TB/s (45 us); this one takes 13 us.
+template <int DT> struct PackVec;
+template <> struct PackVec<BSP_F32> {
+  static constexpr int VEC = 4, U = 4;
+  __device__ static uint32_t bits(const uint4& q) {
+    // x != 0 for -0.0 (no) and NaN (yes): any bit but the sign
+    return ((q.x << 1) ? 1u : 0u) | ((q.y << 1) ? 2u : 0u) | ((q.z << 1) ? 4u : 0u) | ((q.w << 1) ? 8u : 0u);
+  }
+};
+template <> struct PackVec<BSP_F16> {
+  static constexpr int VEC = 8, U = 4;
+  __device__ static uint32_t two(uint32_t x) { return ((x & 0x7fffu) ? 1u : 0u) | ((x & 0x7fff0000u) ? 2u : 0u); }
+  __device__ static uint32_t bits(const uint4& q) {
+    return two(q.x) | (two(q.y) << 2) | (two(q.z) << 4) | (two(q.w) << 6);
+  }
+};
+template <> struct PackVec<BSP_BF16> : PackVec<BSP_F16> {};
+template <> struct PackVec<BSP_U8> {
+  static constexpr int VEC = 16, U = 2;
+  // bytes 0..3 of x != 0 -> bits 0..3 (the multiply moves bit 8i to bit 24+i)
+  __device__ static uint32_t four(uint32_t x) { return ((__vcmpne4(x, 0u) & 0x01010101u) * 0x01020408u) >> 24; }
+  __device__ static uint32_t bits(const uint4& q) {
+    return four(q.x) | (four(q.y) << 4) | (four(q.z) << 8) | (four(q.w) << 12);
+  }
+};
+template <> struct PackVec<BSP_I8> : PackVec<BSP_U8> {};
 
-// One warp builds kWordsPerWarpIter words per iteration (independent loads in
-// flight), lane u < 4 stores word u.
+template <int DT>
+__global__ void __launch_bounds__(256) k_pack_rows_v16(const typename Elem<DT>::T* __restrict__ dense, int64_t M,
+                                                       int64_t K, int64_t ld, uint32_t* __restrict__ words,
+                                                       int64_t Kw, int msb) {
+  using E = Elem<DT>;
+  using V = PackVec<DT>;
+  constexpr int G = 32 / V::VEC, WPL = 32 / G;  // lanes per word, words per load of the warp
+  static_assert(V::U <= G, "a lane of every word's group for each load");
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int64_t nch = (Kw + WPL * V::U - 1) / (WPL * V::U);
+  const int64_t total = M * nch;
+  for (int64_t t = warp; t < total; t += nwarps) {
+    const int64_t r = total <= 0x7fffffff ? (int64_t)((uint32_t)t / (uint32_t)nch) : t / nch;
+    const int64_t ch = t - r * nch;
+    const typename E::T* row = dense + r * ld;
+    const int64_t c0 = ch * (32 * WPL * V::U) + lane * V::VEC;
+    uint4 q[V::U];
+#pragma unroll
+    for (int u = 0; u < V::U; u++) {
+      const int64_t c = c0 + u * (32 * WPL);
+      q[u] = make_uint4(0u, 0u, 0u, 0u);
+      if (c + V::VEC <= K) q[u] = __ldg(reinterpret_cast<const uint4*>(row + c));
+    }
+    uint32_t mine = 0;
+#pragma unroll
+    for (int u = 0; u < V::U; u++) {
+      const int64_t c = c0 + u * (32 * WPL);
+      uint32_t b = V::bits(q[u]);
+      if (c < K && c + V::VEC > K)  // the row's last columns
+        for (int i = 0; i < V::VEC; i++)
+          if (c + i < K && E::nz(row[c + i])) b |= 1u << i;
+      b <<= V::VEC * (lane % G);
+#pragma unroll
+      for (int o = 1; o < G; o <<= 1) b |= __shfl_xor_sync(kFull, b, o);
+      if (lane % G == u) mine = b;
+    }
+    const int64_t w = ch * (WPL * V::U) + (lane % G) * WPL + lane / G;
+    if (lane % G < V::U && w < Kw) words[r * Kw + w] = msb ? __brev(mine) : mine;
+  }
+}
+
+// Any alignment: a warp takes 32 words of a row, one coalesced load of 32
+// columns and one ballot per word, 8 loads in flight; lane j keeps word j.
 template <int DT>
 __global__ void __launch_bounds__(256) k_pack_rows(const typename Elem<DT>::T* __restrict__ dense,
                                                    int64_t M, int64_t K, int64_t ld,
@@ -47,27 +120,28 @@ __global__ void __launch_bounds__(256) k_pack_rows(const typename Elem<DT>::T* _
   const int lane = threadIdx.x & 31;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int64_t total = M * Kw;
-  for (int64_t base = warp * kWordsPerWarpIter; base < total; base += nwarps * kWordsPerWarpIter) {
-    bool nz[kWordsPerWarpIter];
+  const int64_t nch = (Kw + 31) / 32;
+  const int64_t total = M * nch;
+  for (int64_t t = warp; t < total; t += nwarps) {
+    const int64_t r = total <= 0x7fffffff ? (int64_t)((uint32_t)t / (uint32_t)nch) : t / nch;
+    const int64_t w0 = (t - r * nch) * 32;
+    const typename E::T* row = dense + r * ld;
+    const int nw = (int)(Kw - w0 < 32 ? Kw - w0 : 32);
+    uint32_t mine = 0;
+    for (int j0 = 0; j0 < nw; j0 += 8) {
+      bool nz[8];
 #pragma unroll
-    for (int u = 0; u < kWordsPerWarpIter; u++) {
-      const int64_t t = base + u;
-      nz[u] = false;
-      if (t < total) {
-        const int64_t r = t / Kw;
-        const int64_t c = (t - r * Kw) * 32 + lane;
-        if (c < K) nz[u] = E::nz(dense[r * ld + c]);
+      for (int j = 0; j < 8; j++) {
+        const int64_t c = (w0 + j0 + j) * 32 + lane;
+        nz[j] = c < K ? E::nz(row[c]) : false;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const uint32_t b = __ballot_sync(kFull, nz[j]);
+        if (lane == j0 + j) mine = b;
       }
     }
-    uint32_t mine = 0;
-#pragma unroll
-    for (int u = 0; u < kWordsPerWarpIter; u++) {
-      uint32_t b = __ballot_sync(kFull, nz[u]);
-      if (msb) b = __brev(b);
-      if (lane == u) mine = b;
-    }
-    if (lane < kWordsPerWarpIter && base + lane < total) words[base + lane] = mine;
+    if (lane < nw) words[r * Kw + w0 + lane] = msb ? __brev(mine) : mine;
   }
 }
 
@@ -240,16 +314,29 @@ int grid_for(int64_t warps_needed) {
 
 }  // namespace
 
+template <int DT>
+static void pack_rows_t(const void* dense, int64_t M, int64_t K, int64_t ld, uint32_t* words, int64_t Kw, int msb,
+                        cudaStream_t s) {
+  using T = typename Elem<DT>::T;
+  using V = PackVec<DT>;
+  // 16-byte loads need every row to start on 16 bytes; a row narrower than
+  // one load of the warp leaves most of its lanes idle there
+  if (is_aligned(dense, 16) && (ld * (int64_t)sizeof(T)) % 16 == 0 && K >= 32 * V::VEC)
+    k_pack_rows_v16<DT><<<grid_for(M * ceil_div(Kw, V::VEC * V::U)), 256, 0, s>>>((const T*)dense, M, K, ld, words, Kw,
+                                                                               msb);
+  else
+    k_pack_rows<DT><<<grid_for(M * ceil_div(Kw, 32)), 256, 0, s>>>((const T*)dense, M, K, ld, words, Kw, msb);
+}
+
 int launch_pack_rows(const void* dense, int dtype, int64_t M, int64_t K, int64_t ld,
                      uint32_t* words, int msb, cudaStream_t s) {
   const int64_t Kw = ceil_div(K, 32);
-  const int grid = grid_for(ceil_div(M * Kw, kWordsPerWarpIter));
   switch (dtype) {
-    case BSP_F32: k_pack_rows<BSP_F32><<<grid, 256, 0, s>>>((const float*)dense, M, K, ld, words, Kw, msb); break;
-    case BSP_F16: k_pack_rows<BSP_F16><<<grid, 256, 0, s>>>((const uint16_t*)dense, M, K, ld, words, Kw, msb); break;
-    case BSP_BF16: k_pack_rows<BSP_BF16><<<grid, 256, 0, s>>>((const uint16_t*)dense, M, K, ld, words, Kw, msb); break;
-    case BSP_I8: k_pack_rows<BSP_I8><<<grid, 256, 0, s>>>((const int8_t*)dense, M, K, ld, words, Kw, msb); break;
-    case BSP_U8: k_pack_rows<BSP_U8><<<grid, 256, 0, s>>>((const uint8_t*)dense, M, K, ld, words, Kw, msb); break;
+    case BSP_F32: pack_rows_t<BSP_F32>(dense, M, K, ld, words, Kw, msb, s); break;
+    case BSP_F16: pack_rows_t<BSP_F16>(dense, M, K, ld, words, Kw, msb, s); break;
+    case BSP_BF16: pack_rows_t<BSP_BF16>(dense, M, K, ld, words, Kw, msb, s); break;
+    case BSP_I8: pack_rows_t<BSP_I8>(dense, M, K, ld, words, Kw, msb, s); break;
+    case BSP_U8: pack_rows_t<BSP_U8>(dense, M, K, ld, words, Kw, msb, s); break;
     default: return BSP_ERR_INVALID_ARG;
   }
   BSP_LAUNCHED();

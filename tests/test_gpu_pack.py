@@ -45,6 +45,24 @@ def test_pack_rows_strided_and_special_values():
     assert np.array_equal(got, O.pack_rows(np.ascontiguousarray(base[:, 10:150])))
 
 
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16, torch.uint8])
+@pytest.mark.parametrize("K", [127, 128, 129, 255, 256, 511, 512, 513, 1023, 1024, 1057, 2051])
+@pytest.mark.parametrize("pad", [0, 1, 16])
+def test_pack_rows_vector_edges(dt, K, pad):
+    """Around one load and one task of a warp, rows 16-byte aligned (K + pad
+    a multiple of 16 bytes) and not; the padding columns are nonzero."""
+    M = 5
+    rng = np.random.default_rng(K * 3 + pad)
+    bits = rng.random((M, K)) < 0.3
+    ld = K if pad == 0 else (K + 15) // 16 * 16 + (0 if pad == 16 else 1)
+    full = np.ones((M, ld), dtype=np.float32)
+    full[:, :K] = np.where(bits, 3, 0)
+    t = torch.from_numpy(full).to(dt).cuda()[:, :K]
+    for order in (capi.LSB_FIRST, capi.MSB_FIRST):
+        exp = O.pack_rows(bits.astype(np.uint8), msb_first=order == capi.MSB_FIRST)
+        assert np.array_equal(words_host(ops.pack_rows(t, bit_order=order)), exp)
+
+
 @pytest.mark.parametrize("shape", [(1, 1), (37, 45), (64, 1024), (300, 97)])
 def test_pack_cols_and_transpose(shape):
     rng = np.random.default_rng(sum(shape))
