@@ -30,6 +30,17 @@ def test_group_rows_reference_fixture(golden):
     assert np.array_equal(words_host(g["group_mask"]), golden["group_mask_ref"])
 
 
+@pytest.mark.parametrize("G", [1, 2, 31, 32])
+@pytest.mark.parametrize("TR,M", [(31, 100), (32, 64), (33, 70), (512, 600)])
+@pytest.mark.parametrize("p", [0.0, 0.02, 0.3, 1.0])
+def test_group_rows_settled_chunks(G, TR, M, p):
+    """Chunks of 32 rows where none, some and all rows spill at once."""
+    rng = np.random.default_rng(G * TR + M)
+    bits = rng.random((M, 70)) < p
+    bits[:3, :32] = [[True] * 32, [False] * 32, [True] + [False] * 31]  # group 0 full after the first row
+    _cmp(W.pack_bits(bits), TR, G)
+
+
 @pytest.mark.parametrize("M,K,TR,G,p", [(1024, 1024, 512, 2, 0.1), (1000, 100, 64, 4, 0.05),
                                         (77, 33, 7, 1, 0.3), (2048, 256, 2048, 32, 0.02),
                                         (1, 32, 4096, 2, 0.5)])
