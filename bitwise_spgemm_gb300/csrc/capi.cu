@@ -284,11 +284,17 @@ static int run_spmm(SpmmArgs a, const bsp_plan* plan, bool vec, const TuneSched&
     return launch_spmm_tc(a, plan->occ, plan->wordsT, s, workspace, workspace_bytes,
                           TcForm{sc.tc_tps, sc.tc_tiled, sc.tc_split});
   const int64_t N = a.N, K = a.K;
-  const bool proto = plan && plan->mode == BSP_PLAN_PROTO && vec;
+  bool proto = plan && plan->mode == BSP_PLAN_PROTO;
   if (proto) {
     size_t need = 0;
     bsp_spmm_workspace(plan, N, &need);
-    if (!workspace || workspace_bytes < need) return BSP_ERR_WORKSPACE;
+    const bool room = workspace && workspace_bytes >= need;
+    if (!room && vec) return BSP_ERR_WORKSPACE;
+    // layouts without 16-byte access take the plan too where there is room
+    // for the prototype sums, and walk A's rows as they always could without
+    if (!vec) proto = room && K < (int64_t)1 << 30;
+  }
+  if (proto) {
     a.row_cluster = plan->row_cluster;
     a.delta_ptr = plan->delta_ptr;
     a.delta_idx = plan->delta_idx;
@@ -305,20 +311,21 @@ static int run_spmm(SpmmArgs a, const bsp_plan* plan, bool vec, const TuneSched&
     if (K < (int64_t)1 << 30) {
       // prototype sums, then clustered rows (register gathers, or slices
       // staged by TMA bulk copies); rows without a cluster: walk A
-      BSP_TRY(launch_proto_sums(a, s));
-      if (sc.proto_path == 1) BSP_TRY(launch_spmm_proto_bulk(a, sc.proto_variant, s));
-      else BSP_TRY(launch_spmm_proto_regs(a, sc.proto_variant, s));
+      BSP_TRY(launch_proto_sums(a, vec, s));
+      if (sc.proto_path == 1 && vec) BSP_TRY(launch_spmm_proto_bulk(a, sc.proto_variant, s));
+      else BSP_TRY(launch_spmm_proto_regs(a, sc.proto_variant, vec, s));
       if (plan->direct_rows > 0) {
         SpmmArgs d = a;
         d.row_list = plan->direct_list;
         d.n_list = plan->direct_rows;
-        BSP_TRY(launch_spmm_rows(d, false, vec, s));
+        BSP_TRY(launch_spmm_rows(d, vec, s));
       }
       return BSP_OK;
     }
-    BSP_TRY(launch_proto_sums(a, s));
+    BSP_TRY(launch_proto_sums(a, vec, s));
+    return launch_spmm_rows_wide(a, s);
   }
-  return launch_spmm_rows(a, proto, vec, s);
+  return launch_spmm_rows(a, vec, s);
 }
 
 int bsp_spmm_workspace(const bsp_plan* plan, int64_t N, size_t* bytes) {
@@ -725,7 +732,7 @@ int bsp_spmm_t(const uint32_t* A_words, int64_t M, int64_t K, const void* G, int
   a.N = N;
   a.C = dX;
   a.ldc = lddx;
-  return launch_spmm_rows(a, false, vec, s);
+  return launch_spmm_rows(a, vec, s);
 }
 
 int bsp_sddmm(const uint32_t* A_words, int64_t M, int64_t K, const void* G, int64_t ldg, const void* X,

@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(256) k_bitplane_rows(PlaneArgs a) {
     wk.init(a.planes + ((int64_t)b * a.M + row) * a.Kw, 0, (int)a.Kw, lane);
     Acc<VPL, COLS, true> acc;
     acc.zero();
-    accumulate_walk<BT, VPL, D, true>(wk, B, a.ldb, col, cvalid, acc);
+    accumulate_walk<V, VPL, D, true>(wk, B, a.ldb, col, cvalid, acc);
     const float w = plane_weight(b, a.nplanes, a.signed_top);
 #pragma unroll
     for (int v = 0; v < VPL; v++)

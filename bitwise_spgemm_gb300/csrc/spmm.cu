@@ -24,17 +24,34 @@ namespace cg = cooperative_groups;
 namespace bsp {
 namespace {
 
-// One warp per (row, column chunk of 32*VPL*COLS).  In PROTO launches, rows
-// with a cluster walk their delta list and add P[c]; every other row walks
-// A's words.  Rows with more than kCompThreshold set bits are summed with
-// TwoSum one column vector at a time, which keeps the wide path's register
-// budget unchanged.
-template <typename BT, int VPL, int D, bool PROTO>
-__global__ void __launch_bounds__(256) k_spmm_rows(SpmmArgs a) {
-  using V = Vec<BT>;
+// Walking kernel: one warp per (row, column chunk of 32*VPL*COLS).  The warp
+// first writes the columns of its row's set bits to a list in shared memory,
+// 128 words at a time (a prefix sum of the lanes' bit counts gives every lane
+// its place), and then gathers D rows of B per round, their indices read four
+// to a shared load; sums run over the list in order, so a row is added in
+// ascending column order whatever the shape.
+//
+// Bound by the L2 gather rate where there are enough warps, by the latency of
+// a row's rounds of D gathers where there are few.  A walker that took one
+// bit at a time from the words (find first set, shuffle, branch) between the
+// gathers spent about twenty dependent instructions per bit and cut every
+// round at a word: 1024x1024x256 FP32 at 10 %, 22.4 us against 9.7 now;
+// 2048x2048x1024, 155 us against 96 (17.9 TB/s of gathers, the L2 roof).  Rows with more than
+// kCompThreshold set bits, where there can be any, are summed with TwoSum one
+// vector at a time.
+constexpr int kListStep = 128;                 // entries wanted before a round of gathers
+constexpr int kListCap = kListStep + 32 * 32;  // one more group of 32 words
+
+template <typename V, int VPL, int D>
+__global__ void __launch_bounds__(256) k_spmm_list(SpmmArgs a) {
+  using BT = typename V::T;
   constexpr int COLS = V::COLS;
   constexpr int CW = 32 * VPL * COLS;
+  constexpr int GROUPS = 4;  // word groups (of 32) loaded at a time
+  static_assert(kListStep % D == 0 && D % 4 == 0 && D <= 32, "whole rounds");
+  __shared__ __align__(16) uint32_t lists[8][kListCap];
   const int lane = threadIdx.x & 31;
+  uint32_t* list = lists[threadIdx.x >> 5];
   int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (a.row_list) {
     if (row >= a.n_list) return;
@@ -42,6 +59,230 @@ __global__ void __launch_bounds__(256) k_spmm_rows(SpmmArgs a) {
   } else if (row >= a.M) {
     return;
   }
+  const BT* __restrict__ B = static_cast<const BT*>(a.B);
+  const uint32_t* arow = a.A + row * a.Kw;
+  const int Kw = (int)a.Kw;
+  const bool comp = a.K > kCompThreshold && row_popcount(arow, Kw, lane) > kCompThreshold;
+  for (int64_t n0 = (int64_t)blockIdx.y * CW; n0 < a.N; n0 += (int64_t)gridDim.y * CW) {
+    int col[VPL];
+    bool cvalid[VPL];
+#pragma unroll
+    for (int v = 0; v < VPL; v++) {
+      const int64_t c = n0 + (v * 32 + lane) * COLS;
+      cvalid[v] = c < a.N;
+      col[v] = cvalid[v] ? (int)c : 0;
+    }
+    float* crow = a.C + row * a.ldc;
+    if (comp) {
+      for (int v = 0; v < VPL; v++) {
+        BitWalker wk;
+        wk.init(arow, 0, Kw, lane);
+        Acc<1, COLS, true> acc;
+        acc.zero();
+        int c1[1] = {col[v]};
+        bool ok[1] = {cvalid[v]};
+        accumulate_walk<V, 1, 4, true>(wk, B, a.ldb, c1, ok, acc);
+        store_vecs<1, COLS, true>(crow, c1, ok, acc, nullptr);
+      }
+      continue;
+    }
+    Acc<VPL, COLS, false> acc;
+    acc.zero();
+    auto gather = [&](int i, int n) {  // list entries [i, i + n), n <= D (uniform)
+      uint32_t idx[D];
+#pragma unroll
+      for (int s = 0; s < D; s += 4) {
+        const uint4 q = *reinterpret_cast<const uint4*>(list + i + s);
+        idx[s] = q.x;
+        idx[s + 1] = q.y;
+        idx[s + 2] = q.z;
+        idx[s + 3] = q.w;
+      }
+      typename V::Raw raw[D][VPL];
+#pragma unroll
+      for (int s = 0; s < D; s++) {
+        const BT* brow = B + (int64_t)idx[s] * a.ldb;
+#pragma unroll
+        for (int v = 0; v < VPL; v++)
+          if (s < n && cvalid[v]) raw[s][v] = V::load(brow + col[v]);
+      }
+#pragma unroll
+      for (int s = 0; s < D; s++) {
+        if (s >= n) break;
+#pragma unroll
+        for (int v = 0; v < VPL; v++) {
+          if (!cvalid[v]) continue;
+          float f[COLS];
+          V::cvt(raw[s][v], f);
+#pragma unroll
+          for (int j = 0; j < COLS; j++) acc.add(v, j, f[j]);
+        }
+      }
+    };
+    uint32_t wx[GROUPS];
+#pragma unroll
+    for (int g = 0; g < GROUPS; g++) wx[g] = g * 32 + lane < Kw ? __ldg(arow + g * 32 + lane) : 0u;
+    int n = 0;  // entries in the list
+    for (int w0 = 0; w0 < Kw; w0 += GROUPS * 32) {
+      uint32_t wn[GROUPS];
+#pragma unroll
+      for (int g = 0; g < GROUPS; g++) {
+        const int w = w0 + (GROUPS + g) * 32 + lane;
+        wn[g] = w < Kw ? __ldg(arow + w) : 0u;
+      }
+#pragma unroll
+      for (int g = 0; g < GROUPS; g++) {
+        if (w0 + g * 32 >= Kw) break;
+        uint32_t x = wx[g];
+        const int c = __popc(x);
+        int incl = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(kFull, incl, o);
+          if (lane >= o) incl += y;
+        }
+        int pos = n + incl - c;
+        const uint32_t k0 = (uint32_t)(w0 + g * 32 + lane) * 32u;
+        while (x) {
+          list[pos++] = k0 + (uint32_t)(__ffs(x) - 1);
+          x &= x - 1;
+        }
+        n += __shfl_sync(kFull, incl, 31);
+        const bool last = w0 + (g + 1) * 32 >= Kw;
+        if (n < kListStep && !last) continue;
+        __syncwarp();
+        int i = 0;
+        for (; i + D <= n; i += D) gather(i, D);
+        n -= i;
+        if (last) {
+          if (n > 0) gather(i, n);
+        } else if (i > 0) {  // the rest (less than D entries) starts the next round
+          const uint32_t rest = lane < n ? list[i + lane] : 0u;
+          __syncwarp();
+          if (lane < n) list[lane] = rest;
+        }
+        __syncwarp();
+      }
+#pragma unroll
+      for (int g = 0; g < GROUPS; g++) wx[g] = wn[g];
+    }
+    store_vecs<VPL, COLS, false>(crow, col, cvalid, acc, nullptr);
+    __syncwarp();
+  }
+}
+
+// A few long rows: a CTA per (row, column chunk).  Its 8 warps write the row's
+// column list (8192 columns at a time), gather 16 rows of B each into shared
+// memory, and then every thread adds its own column over the 128 staged rows
+// in list order — the sum the walking kernel forms.  One row of 427 bits cost
+// the walking kernel a chain of gathers of 115 us behind the clustered 8192x8192x512
+// product, more than the product; here it has 4 rounds and adds 3 us.
+constexpr int kCoopSlots = 16;                  // rows in flight per warp
+constexpr int kCoopBatch = 8 * kCoopSlots;
+constexpr int kCoopWords = 256;                 // words listed at a time, one per thread
+
+template <typename V, int VPL>
+struct CoopSmem {
+  static constexpr int CW = 32 * VPL * V::COLS;
+  typename V::Raw stage[kCoopBatch][VPL][32];
+  uint16_t list[kCoopWords * 32];
+  int scan[32];
+};
+
+template <typename V, int VPL>
+__global__ void __launch_bounds__(256) k_spmm_coop(SpmmArgs a) {
+  using BT = typename V::T;
+  using Smem = CoopSmem<V, VPL>;
+  constexpr int COLS = V::COLS, CW = Smem::CW;
+  static_assert(CW <= 256, "one thread per column");
+  extern __shared__ __align__(16) uint8_t coop_raw[];
+  Smem& sm = *reinterpret_cast<Smem*>(coop_raw);
+  ptx::griddep_launch_dependents();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t row = a.row_list ? (int64_t)__ldg(a.row_list + blockIdx.x) : (int64_t)blockIdx.x;
+  const BT* __restrict__ B = static_cast<const BT*>(a.B);
+  const uint32_t* arow = a.A + row * a.Kw;
+  const int Kw = (int)a.Kw;
+  const int64_t n0 = (int64_t)blockIdx.y * CW;
+  const BT* bcol[VPL];
+  bool cvalid[VPL];
+#pragma unroll
+  for (int v = 0; v < VPL; v++) {
+    const int64_t c = n0 + (v * 32 + lane) * COLS;
+    cvalid[v] = c < a.N;
+    bcol[v] = B + (cvalid[v] ? c : 0);
+  }
+  bool comp = false;
+  if (a.K > kCompThreshold) {
+    int c = 0;
+    for (int w = tid; w < Kw; w += 256) c += __popc(__ldg(arow + w));
+    int total;
+    block_exclusive_scan(c, sm.scan, &total);
+    comp = total > kCompThreshold;
+  }
+  float s = 0.f, e = 0.f;
+  const BT* mine = reinterpret_cast<const BT*>(&sm.stage[0][0][0]) + tid;  // column tid of slot 0
+  for (int w0 = 0; w0 < Kw; w0 += kCoopWords) {
+    uint32_t x = w0 + tid < Kw ? __ldg(arow + w0 + tid) : 0u;
+    int total;
+    int pos = block_exclusive_scan(__popc(x), sm.scan, &total);
+    while (x) {
+      sm.list[pos++] = (uint16_t)(tid * 32 + __ffs(x) - 1);
+      x &= x - 1;
+    }
+    __syncthreads();
+    typename V::Raw raw[kCoopSlots][VPL];
+    auto load = [&](int b0) {
+#pragma unroll
+      for (int u = 0; u < kCoopSlots; u++) {
+        const int i = b0 + warp * kCoopSlots + u;
+        if (i >= total) break;
+        const int64_t k = (int64_t)w0 * 32 + sm.list[i];
+#pragma unroll
+        for (int v = 0; v < VPL; v++)
+          if (cvalid[v]) raw[u][v] = V::load(bcol[v] + k * a.ldb);
+      }
+    };
+    load(0);
+    for (int b0 = 0; b0 < total; b0 += kCoopBatch) {
+      const int cnt = min(kCoopBatch, total - b0);
+#pragma unroll
+      for (int u = 0; u < kCoopSlots; u++)
+#pragma unroll
+        for (int v = 0; v < VPL; v++) sm.stage[warp * kCoopSlots + u][v][lane] = raw[u][v];
+      __syncthreads();
+      load(b0 + kCoopBatch);
+      if (tid < CW) {
+        if (comp) {
+          for (int i = 0; i < cnt; i++) {
+            const float f = to_f32(mine[i * CW]);
+            const float t = s + f, bp = t - s;
+            e += (s - (t - bp)) + (f - bp);
+            s = t;
+          }
+        } else {
+#pragma unroll 8
+          for (int i = 0; i < cnt; i++) s += to_f32(mine[i * CW]);
+        }
+      }
+      __syncthreads();
+    }
+  }
+  if (tid < CW && n0 + tid < a.N) a.C[row * a.ldc + n0 + tid] = comp ? s + e : s;
+  ptx::griddep_wait();  // this grid ends after the one it may overlap
+}
+
+// Plans of A with 2^30 or more columns: one warp per (row, column chunk).
+// Rows with a cluster walk their delta list and add P[c]; every other row
+// walks A's words.
+template <typename BT, int VPL, int D>
+__global__ void __launch_bounds__(256) k_spmm_rows_wide(SpmmArgs a) {
+  using V = Vec<BT>;
+  constexpr int COLS = V::COLS;
+  constexpr int CW = 32 * VPL * COLS;
+  const int lane = threadIdx.x & 31;
+  const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= a.M) return;
   const int n0 = (int)blockIdx.y * CW;
   const BT* __restrict__ B = static_cast<const BT*>(a.B);
   int col[VPL];
@@ -52,37 +293,33 @@ __global__ void __launch_bounds__(256) k_spmm_rows(SpmmArgs a) {
     cvalid[v] = col[v] < a.N;
   }
   float* crow = a.C + row * a.ldc;
-  if (PROTO) {
-    const int cl = __ldg(a.row_cluster + row);
-    if (cl >= 0) {
-      ListWalker wk;
-      wk.init(a.delta_idx, __ldg(a.delta_ptr + row), __ldg(a.delta_ptr + row + 1), lane);
-      Acc<VPL, COLS, false> acc;
-      acc.zero();
-      accumulate_walk<BT, VPL, D, false>(wk, B, a.ldb, col, cvalid, acc);
-      store_vecs<VPL, COLS, false>(crow, col, cvalid, acc, a.P + (int64_t)cl * a.ldp);
-      return;
-    }
-  }
-  const uint32_t* arow = a.A + row * a.Kw;
-  const int nnz = row_popcount(arow, (int)a.Kw, lane);
-  if (nnz <= kCompThreshold) {
-    BitWalker wk;
-    wk.init(arow, 0, (int)a.Kw, lane);
+  const int cl = __ldg(a.row_cluster + row);
+  if (cl >= 0) {
+    ListWalker wk;
+    wk.init(a.delta_idx, __ldg(a.delta_ptr + row), __ldg(a.delta_ptr + row + 1), lane);
     Acc<VPL, COLS, false> acc;
     acc.zero();
-    accumulate_walk<BT, VPL, D, false>(wk, B, a.ldb, col, cvalid, acc);
-    store_vecs<VPL, COLS, false>(crow, col, cvalid, acc, nullptr);
-  } else {
-    for (int v = 0; v < VPL; v++) {
-      BitWalker wk;
-      wk.init(arow, 0, (int)a.Kw, lane);
+    accumulate_walk<V, VPL, D, false>(wk, B, a.ldb, col, cvalid, acc);
+    store_vecs<VPL, COLS, false>(crow, col, cvalid, acc, a.P + (int64_t)cl * a.ldp);
+    return;
+  }
+  const uint32_t* arow = a.A + row * a.Kw;
+  const bool comp = row_popcount(arow, (int)a.Kw, lane) > kCompThreshold;
+  for (int v = 0; v < VPL; v++) {
+    BitWalker wk;
+    wk.init(arow, 0, (int)a.Kw, lane);
+    int c1[1] = {col[v]};
+    bool ok[1] = {cvalid[v]};
+    if (comp) {
       Acc<1, COLS, true> acc;
       acc.zero();
-      int c1[1] = {col[v]};
-      bool ok[1] = {cvalid[v]};
-      accumulate_walk<BT, 1, 4, true>(wk, B, a.ldb, c1, ok, acc);
+      accumulate_walk<V, 1, 4, true>(wk, B, a.ldb, c1, ok, acc);
       store_vecs<1, COLS, true>(crow, c1, ok, acc, nullptr);
+    } else {
+      Acc<1, COLS, false> acc;
+      acc.zero();
+      accumulate_walk<V, 1, 4, false>(wk, B, a.ldb, c1, ok, acc);
+      store_vecs<1, COLS, false>(crow, c1, ok, acc, nullptr);
     }
   }
 }
@@ -96,12 +333,13 @@ __global__ void __launch_bounds__(256) k_spmm_rows(SpmmArgs a) {
 // arithmetic (M < 2^31, checked on the host) they keep the 8-blocks-per-SM
 // shape within its 32 registers without spilling (a 12-byte spill cost the
 // clustered 8192²×512 step 3 µs).
-template <typename BT, int VPL, int D, int MINB, bool OFF32, bool FULL, bool SLOT>
+template <typename V, int VPL, int D, int MINB, bool OFF32, bool FULL, bool SLOT>
 __global__ void __launch_bounds__(256, MINB) k_spmm_proto_regs(SpmmArgs a) {
-  using V = Vec<BT>;
+  using BT = typename V::T;
   constexpr int COLS = V::COLS;
   constexpr int CW = 32 * VPL * COLS;
   const int lane = threadIdx.x & 31;
+  ptx::griddep_launch_dependents();  // the direct rows' kernel, if there is one
   int row, cl;
   uint32_t slot = 0u;
   if (SLOT) {
@@ -130,13 +368,13 @@ __global__ void __launch_bounds__(256, MINB) k_spmm_proto_regs(SpmmArgs a) {
     if (SLOT) {
       SlotWalker wk;
       wk.init(slot, a.delta_idx, lane);
-      if (OFF32) accumulate_walk<BT, VPL, D, false>(wk, B, (uint32_t)a.ldb, col, cvalid, acc);
-      else accumulate_walk<BT, VPL, D, false>(wk, B, a.ldb, col, cvalid, acc);
+      if (OFF32) accumulate_walk<V, VPL, D, false>(wk, B, (uint32_t)a.ldb, col, cvalid, acc);
+      else accumulate_walk<V, VPL, D, false>(wk, B, a.ldb, col, cvalid, acc);
     } else {
       ListWalker wk;
       wk.init(a.delta_idx, __ldg(a.delta_ptr + row), __ldg(a.delta_ptr + row + 1), lane);
-      if (OFF32) accumulate_walk<BT, VPL, D, false>(wk, B, (uint32_t)a.ldb, col, cvalid, acc);
-      else accumulate_walk<BT, VPL, D, false>(wk, B, a.ldb, col, cvalid, acc);
+      if (OFF32) accumulate_walk<V, VPL, D, false>(wk, B, (uint32_t)a.ldb, col, cvalid, acc);
+      else accumulate_walk<V, VPL, D, false>(wk, B, a.ldb, col, cvalid, acc);
     }
     ptx::griddep_wait();
     store_vecs<VPL, COLS, false>(a.C + (int64_t)row * a.ldc, col, cvalid, acc, a.P + (int64_t)cl * a.ldp);
@@ -145,43 +383,14 @@ __global__ void __launch_bounds__(256, MINB) k_spmm_proto_regs(SpmmArgs a) {
   }
 }
 
-// Scalar fallback for unaligned or ragged layouts: lane = column.
-template <typename BT>
-__global__ void __launch_bounds__(256) k_spmm_rows_scalar(SpmmArgs a) {
-  const int lane = threadIdx.x & 31;
-  const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (row >= a.M) return;
-  const BT* __restrict__ B = static_cast<const BT*>(a.B);
-  const uint32_t* arow = a.A + row * a.Kw;
-  const int nnz = row_popcount(arow, (int)a.Kw, lane);
-  const bool comp = nnz > kCompThreshold;
-  for (int64_t n0 = (int64_t)blockIdx.y * 32; n0 < a.N; n0 += (int64_t)gridDim.y * 32) {
-    const int64_t j = n0 + lane;
-    float s = 0.f, c = 0.f;
-    BitWalker wk;
-    wk.init(arow, 0, (int)a.Kw, lane);
-    for (uint32_t k = wk.next(); k != kEnd; k = wk.next()) {
-      const float x = j < a.N ? to_f32(B[(int64_t)k * a.ldb + j]) : 0.f;
-      if (comp) {
-        const float t = s + x, bp = t - s;
-        c += (s - (t - bp)) + (x - bp);
-        s = t;
-      } else {
-        s += x;
-      }
-    }
-    if (j < a.N) a.C[row * a.ldc + j] = comp ? s + c : s;
-  }
-}
-
 // P[c][n0 .. n0+32*COLS) for one prototype per CTA row: warp w walks the
 // prototype's words [w*Kw/W, (w+1)*Kw/W), partial sums meet in shared memory
 // and are added in warp order.  COMP (the densest prototype has more than
 // 4096 set bits): each warp keeps a TwoSum pair (sum, error) and the pairs
 // are added with TwoSum too; P = sum + error.
-template <typename BT, int D, bool COMP, bool OFF32>
+template <typename V, int D, bool COMP, bool OFF32>
 __global__ void __launch_bounds__(512) k_proto_sums(SpmmArgs a) {
-  using V = Vec<BT>;
+  using BT = typename V::T;
   constexpr int COLS = V::COLS;
   constexpr int CW = 32 * COLS;
   extern __shared__ float part[];  // [W][CW] sums, then (COMP) [W][CW] errors
@@ -198,8 +407,8 @@ __global__ void __launch_bounds__(512) k_proto_sums(SpmmArgs a) {
   wk.init(cw, w0, w1, lane);
   Acc<1, COLS, COMP> acc;
   acc.zero();
-  if (OFF32) accumulate_walk<BT, 1, D, COMP>(wk, B, (uint32_t)a.ldb, col, cvalid, acc);
-  else accumulate_walk<BT, 1, D, COMP>(wk, B, a.ldb, col, cvalid, acc);
+  if (OFF32) accumulate_walk<V, 1, D, COMP>(wk, B, (uint32_t)a.ldb, col, cvalid, acc);
+  else accumulate_walk<V, 1, D, COMP>(wk, B, a.ldb, col, cvalid, acc);
 #pragma unroll
   for (int j = 0; j < COLS; j++) {
     part[wid * CW + lane * COLS + j] = acc.s[0][j];
@@ -232,9 +441,9 @@ __global__ void __launch_bounds__(512) k_proto_sums(SpmmArgs a) {
 // order; rank 0 adds the 8 CTA partials in rank order through distributed
 // shared memory (all loads issued first), so P is the same on every run.
 constexpr int kSumCluster = 8;
-template <typename BT, int VPL, bool OFF32>
+template <typename V, int VPL, bool OFF32>
 __global__ void __cluster_dims__(kSumCluster, 1, 1) __launch_bounds__(256) k_proto_sums_list(SpmmArgs a) {
-  using V = Vec<BT>;
+  using BT = typename V::T;
   constexpr int COLS = V::COLS;
   constexpr int CW = 32 * VPL * COLS;
   constexpr int PARTS = kSumCluster * 8;
@@ -260,8 +469,8 @@ __global__ void __cluster_dims__(kSumCluster, 1, 1) __launch_bounds__(256) k_pro
   Acc<VPL, COLS, false> acc;
   acc.zero();
   const BT* __restrict__ B = static_cast<const BT*>(a.B);
-  if (OFF32) accumulate_walk<BT, VPL, 1, false>(wk, B, (uint32_t)a.ldb, col, cvalid, acc);
-  else accumulate_walk<BT, VPL, 1, false>(wk, B, a.ldb, col, cvalid, acc);
+  if (OFF32) accumulate_walk<V, VPL, 1, false>(wk, B, (uint32_t)a.ldb, col, cvalid, acc);
+  else accumulate_walk<V, VPL, 1, false>(wk, B, a.ldb, col, cvalid, acc);
   float* w = reinterpret_cast<float*>(&wp[wid][0]);
 #pragma unroll
   for (int v = 0; v < VPL; v++)
@@ -299,34 +508,65 @@ __global__ void __cluster_dims__(kSumCluster, 1, 1) __launch_bounds__(256) k_pro
   cluster.sync();
 }
 
+template <typename V, int VPL, int D>
+int launch_list_s(const SpmmArgs& a, int64_t rows, cudaStream_t s) {
+  const int64_t gy = ceil_div(a.N, 32 * VPL * V::COLS);
+  k_spmm_list<V, VPL, D><<<dim3((unsigned)ceil_div(rows, 8), (unsigned)(gy < 65535 ? gy : 65535)), 256, 0, s>>>(a);
+  BSP_LAUNCHED();
+  return BSP_OK;
+}
+
+template <typename V, int VPL>
+int launch_coop_s(const SpmmArgs& a, int64_t rows, cudaStream_t s) {
+  constexpr int smem = (int)sizeof(CoopSmem<V, VPL>);
+  auto kern = k_spmm_coop<V, VPL>;
+  static bool configured[64] = {};
+  int dev = 0;
+  BSP_CUDA(cudaGetDevice(&dev));
+  if (dev >= 64 || !configured[dev]) {
+    BSP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    if (dev < 64) configured[dev] = true;
+  }
+  // A programmatic dependent of the prototype rows' kernel: it reads only A
+  // and B and writes its own rows of C, so it may run beside that kernel's
+  // last CTAs (alone in its stream the attribute changes nothing).
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)rows, (unsigned)ceil_div(a.N, CoopSmem<V, VPL>::CW));
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = a.row_list ? 1 : 0;
+  BSP_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
+  return BSP_OK;
+}
+
+template <typename V>
+int launch_rows_t(const SpmmArgs& a, cudaStream_t s) {
+  constexpr int VPL = V::COLS == 1 ? 4 : 1;
+  const int64_t rows = a.row_list ? a.n_list : a.M;
+  if (rows == 0) return BSP_OK;
+  const int64_t sms = num_sms(), chunks = ceil_div(a.N, 32 * VPL * V::COLS), tasks = rows * chunks;
+  // One (row, chunk) per SM at most: a chain of gathers per row would be all
+  // that runs (one row, 8192 columns at 5 %, N = 512: 9.1 us against 15.2;
+  // from a few hundred tasks on the two are equal, 117 rows 21.5 and 20.0).
+  if (tasks <= sms && a.K >= 1024 && chunks <= 65535) return launch_coop_s<V, VPL>(a, rows, s);
+  // One vector per lane: more warps beat wider slices at every size measured
+  // (2048x2048x1024 FP32, 10 %: 96 us, two vectors 106, four 112).  With 12
+  // or more warps an SM, 8 gathers in flight each (1024x1024x256: 9.7 us, 16
+  // in flight 11.2; 2048x2048x1024: 96 and 123); with fewer, 16 (300x4000x512
+  // at 2 %: 6.7 us, 8 in flight 7.7; 512x512x64: 4.3 and 5.2).
+  if (V::COLS == 1 || tasks >= 12 * sms) return launch_list_s<V, VPL, 8>(a, rows, s);
+  return launch_list_s<V, VPL, 16>(a, rows, s);
+}
+
 template <typename BT>
-int launch_rows_t(const SpmmArgs& a, bool proto, bool vec, cudaStream_t s) {
-  constexpr int COLS = Vec<BT>::COLS;
-  const unsigned gx = (unsigned)ceil_div(a.row_list ? a.n_list : a.M, 8);
-  if (gx == 0) return BSP_OK;
-  if (!vec) {
-    if (proto) return BSP_ERR_INTERNAL;
-    const int64_t gy = ceil_div(a.N, 32) < 65535 ? ceil_div(a.N, 32) : 65535;
-    k_spmm_rows_scalar<BT><<<dim3(gx, (unsigned)gy), 256, 0, s>>>(a);
-    BSP_LAUNCHED();
-    return BSP_OK;
-  }
-  // columns per warp: up to 4 vectors per lane for FP32, 2 for 16-bit B
-  constexpr int VPL_MAX = COLS == 4 ? 4 : 2;
-  const int64_t per1 = 32 * COLS;
-  if (a.N <= per1) {
-    const dim3 g(gx, (unsigned)ceil_div(a.N, per1));
-    if (proto) k_spmm_rows<BT, 1, 16, true><<<g, 256, 0, s>>>(a);
-    else k_spmm_rows<BT, 1, 16, false><<<g, 256, 0, s>>>(a);
-  } else if (a.N <= 2 * per1 || VPL_MAX == 2) {
-    const dim3 g(gx, (unsigned)ceil_div(a.N, 2 * per1));
-    if (proto) k_spmm_rows<BT, 2, 8, true><<<g, 256, 0, s>>>(a);
-    else k_spmm_rows<BT, 2, 8, false><<<g, 256, 0, s>>>(a);
-  } else {
-    const dim3 g(gx, (unsigned)ceil_div(a.N, 4 * per1));
-    if (proto) k_spmm_rows<BT, 4, 4, true><<<g, 256, 0, s>>>(a);
-    else k_spmm_rows<BT, 4, 4, false><<<g, 256, 0, s>>>(a);
-  }
+int launch_rows_wide_t(const SpmmArgs& a, cudaStream_t s) {
+  const dim3 g((unsigned)ceil_div(a.M, 8), (unsigned)ceil_div(a.N, 32 * Vec<BT>::COLS));
+  k_spmm_rows_wide<BT, 1, 8><<<g, 256, 0, s>>>(a);
   BSP_LAUNCHED();
   return BSP_OK;
 }
@@ -341,9 +581,9 @@ bool slot_lists_enabled() {
   return on;
 }
 
-template <typename BT, int VPL, int D, int MINB>
+template <typename V, int VPL, int D, int MINB>
 int launch_proto_regs_t(const SpmmArgs& a, cudaStream_t s) {
-  constexpr int CW = 32 * VPL * Vec<BT>::COLS;
+  constexpr int CW = 32 * VPL * V::COLS;
   cudaLaunchConfig_t cfg = {};
   const bool off32 = a.K * a.ldb < ((int64_t)1 << 31), full = a.N % CW == 0;
   const bool slot = off32 && a.delta_pad && a.n_slot > 0 && slot_lists_enabled();
@@ -357,40 +597,42 @@ int launch_proto_regs_t(const SpmmArgs& a, cudaStream_t s) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   if (slot && full)
-    BSP_CUDA(cudaLaunchKernelEx(&cfg, k_spmm_proto_regs<BT, VPL, D, MINB, true, true, true>, a));
+    BSP_CUDA(cudaLaunchKernelEx(&cfg, k_spmm_proto_regs<V, VPL, D, MINB, true, true, true>, a));
   else if (slot)
-    BSP_CUDA(cudaLaunchKernelEx(&cfg, k_spmm_proto_regs<BT, VPL, D, MINB, true, false, true>, a));
+    BSP_CUDA(cudaLaunchKernelEx(&cfg, k_spmm_proto_regs<V, VPL, D, MINB, true, false, true>, a));
   else if (off32 && full)
-    BSP_CUDA(cudaLaunchKernelEx(&cfg, k_spmm_proto_regs<BT, VPL, D, MINB, true, true, false>, a));
+    BSP_CUDA(cudaLaunchKernelEx(&cfg, k_spmm_proto_regs<V, VPL, D, MINB, true, true, false>, a));
   else if (off32)
-    BSP_CUDA(cudaLaunchKernelEx(&cfg, k_spmm_proto_regs<BT, VPL, D, MINB, true, false, false>, a));
+    BSP_CUDA(cudaLaunchKernelEx(&cfg, k_spmm_proto_regs<V, VPL, D, MINB, true, false, false>, a));
   else
-    BSP_CUDA(cudaLaunchKernelEx(&cfg, k_spmm_proto_regs<BT, VPL, D, MINB, false, false, false>, a));
+    BSP_CUDA(cudaLaunchKernelEx(&cfg, k_spmm_proto_regs<V, VPL, D, MINB, false, false, false>, a));
   return BSP_OK;
 }
 
 template <typename BT>
-int launch_proto_regs_v(const SpmmArgs& a, int variant, cudaStream_t s) {
+int launch_proto_regs_v(const SpmmArgs& a, int variant, bool vec, cudaStream_t s) {
+  if (!vec) return launch_proto_regs_t<Elem1<BT>, 4, 4, 4>(a, s);
   constexpr bool F32 = Vec<BT>::COLS == 4;
   // variants: columns per warp (VPL vectors per lane), gathers in flight (D), min blocks/SM
-  if (a.N <= 32 * Vec<BT>::COLS) return launch_proto_regs_t<BT, 1, 16, 3>(a, s);
+  if (a.N <= 32 * Vec<BT>::COLS) return launch_proto_regs_t<Vec<BT>, 1, 16, 3>(a, s);
   switch (variant) {
-    case 1: return launch_proto_regs_t<BT, 2, 4, 4>(a, s);
-    case 2: return launch_proto_regs_t<BT, (F32 ? 4 : 2), 1, 5>(a, s);
-    case 3: return launch_proto_regs_t<BT, 2, 2, 6>(a, s);
-    case 4: return launch_proto_regs_t<BT, 2, 1, 8>(a, s);
-    case 5: return launch_proto_regs_t<BT, 1, 4, 8>(a, s);
-    case 6: return launch_proto_regs_t<BT, 2, 2, 5>(a, s);
-    case 7: return launch_proto_regs_t<BT, (F32 ? 4 : 2), 1, 6>(a, s);
-    case 8: return launch_proto_regs_t<BT, (F32 ? 4 : 2), 3, 3>(a, s);
-    default: return launch_proto_regs_t<BT, (F32 ? 4 : 2), 2, 4>(a, s);
+    case 1: return launch_proto_regs_t<Vec<BT>, 2, 4, 4>(a, s);
+    case 2: return launch_proto_regs_t<Vec<BT>, (F32 ? 4 : 2), 1, 5>(a, s);
+    case 3: return launch_proto_regs_t<Vec<BT>, 2, 2, 6>(a, s);
+    case 4: return launch_proto_regs_t<Vec<BT>, 2, 1, 8>(a, s);
+    case 5: return launch_proto_regs_t<Vec<BT>, 1, 4, 8>(a, s);
+    case 6: return launch_proto_regs_t<Vec<BT>, 2, 2, 5>(a, s);
+    case 7: return launch_proto_regs_t<Vec<BT>, (F32 ? 4 : 2), 1, 6>(a, s);
+    case 8: return launch_proto_regs_t<Vec<BT>, (F32 ? 4 : 2), 3, 3>(a, s);
+    default: return launch_proto_regs_t<Vec<BT>, (F32 ? 4 : 2), 2, 4>(a, s);
   }
 }
 
-template <typename BT>
+template <typename V>
 int launch_proto_t(const SpmmArgs& a, cudaStream_t s) {
-  constexpr int VPL = Vec<BT>::COLS == 4 ? 2 : 1;
-  constexpr int CWL = 32 * VPL * Vec<BT>::COLS;
+  using BT = typename V::T;
+  constexpr int VPL = V::COLS == 1 ? 8 : V::COLS == 4 ? 2 : 1;
+  constexpr int CWL = 32 * VPL * V::COLS;
   const bool comp = a.proto_max_nnz > kCompThreshold;
   // From the column lists, B slices staged by bulk copies when B's rows are
   // 16-byte aligned (BSP_SUMS_BULK = -1 selects the cluster form below, n >=
@@ -405,20 +647,20 @@ int launch_proto_t(const SpmmArgs& a, cudaStream_t s) {
   }
   if (a.cons_idx && !comp && a.n_proto <= 65535 && ceil_div(a.N, CWL) * kSumCluster <= 0x7fffffff) {
     const dim3 g((unsigned)(ceil_div(a.N, CWL) * kSumCluster), (unsigned)a.n_proto);
-    if (a.K * a.ldb < ((int64_t)1 << 31)) k_proto_sums_list<BT, VPL, true><<<g, 256, 0, s>>>(a);
-    else k_proto_sums_list<BT, VPL, false><<<g, 256, 0, s>>>(a);
+    if (a.K * a.ldb < ((int64_t)1 << 31)) k_proto_sums_list<V, VPL, true><<<g, 256, 0, s>>>(a);
+    else k_proto_sums_list<V, VPL, false><<<g, 256, 0, s>>>(a);
     BSP_LAUNCHED();
     return BSP_OK;
   }
-  constexpr int CW = 32 * Vec<BT>::COLS;
+  constexpr int CW = 32 * V::COLS;
   const int threads = 512;
   const size_t smem = (size_t)(threads / 32) * CW * sizeof(float) * (comp ? 2 : 1);
   const dim3 g((unsigned)a.n_proto, (unsigned)ceil_div(a.N, CW));
   const bool off32 = a.K * a.ldb < ((int64_t)1 << 31);
-  if (comp && off32) k_proto_sums<BT, 8, true, true><<<g, threads, smem, s>>>(a);
-  else if (comp) k_proto_sums<BT, 8, true, false><<<g, threads, smem, s>>>(a);
-  else if (off32) k_proto_sums<BT, 8, false, true><<<g, threads, smem, s>>>(a);
-  else k_proto_sums<BT, 8, false, false><<<g, threads, smem, s>>>(a);
+  if (comp && off32) k_proto_sums<V, 8, true, true><<<g, threads, smem, s>>>(a);
+  else if (comp) k_proto_sums<V, 8, true, false><<<g, threads, smem, s>>>(a);
+  else if (off32) k_proto_sums<V, 8, false, true><<<g, threads, smem, s>>>(a);
+  else k_proto_sums<V, 8, false, false><<<g, threads, smem, s>>>(a);
   BSP_LAUNCHED();
   return BSP_OK;
 }
@@ -467,32 +709,42 @@ int launch_sddmm_rows(const uint32_t* A, int64_t M, int64_t K, const void* G, in
   return BSP_OK;
 }
 
-int launch_spmm_rows(const SpmmArgs& a, bool proto, bool vec, cudaStream_t s) {
+int launch_spmm_rows(const SpmmArgs& a, bool vec, cudaStream_t s) {
   if (a.M == 0 || a.N == 0) return BSP_OK;
   switch (a.bdt) {
-    case BSP_F32: return launch_rows_t<float>(a, proto, vec, s);
-    case BSP_BF16: return launch_rows_t<__nv_bfloat16>(a, proto, vec, s);
-    case BSP_F16: return launch_rows_t<__half>(a, proto, vec, s);
+    case BSP_F32: return vec ? launch_rows_t<Vec<float>>(a, s) : launch_rows_t<Elem1<float>>(a, s);
+    case BSP_BF16: return vec ? launch_rows_t<Vec<__nv_bfloat16>>(a, s) : launch_rows_t<Elem1<__nv_bfloat16>>(a, s);
+    case BSP_F16: return vec ? launch_rows_t<Vec<__half>>(a, s) : launch_rows_t<Elem1<__half>>(a, s);
     default: return BSP_ERR_UNSUPPORTED;
   }
 }
 
-int launch_spmm_proto_regs(const SpmmArgs& a, int variant, cudaStream_t s) {
+int launch_spmm_rows_wide(const SpmmArgs& a, cudaStream_t s) {
   if (a.M == 0 || a.N == 0) return BSP_OK;
   switch (a.bdt) {
-    case BSP_F32: return launch_proto_regs_v<float>(a, variant, s);
-    case BSP_BF16: return launch_proto_regs_v<__nv_bfloat16>(a, variant, s);
-    case BSP_F16: return launch_proto_regs_v<__half>(a, variant, s);
+    case BSP_F32: return launch_rows_wide_t<float>(a, s);
+    case BSP_BF16: return launch_rows_wide_t<__nv_bfloat16>(a, s);
+    case BSP_F16: return launch_rows_wide_t<__half>(a, s);
     default: return BSP_ERR_UNSUPPORTED;
   }
 }
 
-int launch_proto_sums(const SpmmArgs& a, cudaStream_t s) {
+int launch_spmm_proto_regs(const SpmmArgs& a, int variant, bool vec, cudaStream_t s) {
+  if (a.M == 0 || a.N == 0) return BSP_OK;
+  switch (a.bdt) {
+    case BSP_F32: return launch_proto_regs_v<float>(a, variant, vec, s);
+    case BSP_BF16: return launch_proto_regs_v<__nv_bfloat16>(a, variant, vec, s);
+    case BSP_F16: return launch_proto_regs_v<__half>(a, variant, vec, s);
+    default: return BSP_ERR_UNSUPPORTED;
+  }
+}
+
+int launch_proto_sums(const SpmmArgs& a, bool vec, cudaStream_t s) {
   if (a.n_proto == 0 || a.N == 0) return BSP_OK;
   switch (a.bdt) {
-    case BSP_F32: return launch_proto_t<float>(a, s);
-    case BSP_BF16: return launch_proto_t<__nv_bfloat16>(a, s);
-    case BSP_F16: return launch_proto_t<__half>(a, s);
+    case BSP_F32: return vec ? launch_proto_t<Vec<float>>(a, s) : launch_proto_t<Elem1<float>>(a, s);
+    case BSP_BF16: return vec ? launch_proto_t<Vec<__nv_bfloat16>>(a, s) : launch_proto_t<Elem1<__nv_bfloat16>>(a, s);
+    case BSP_F16: return vec ? launch_proto_t<Vec<__half>>(a, s) : launch_proto_t<Elem1<__half>>(a, s);
     default: return BSP_ERR_UNSUPPORTED;
   }
 }

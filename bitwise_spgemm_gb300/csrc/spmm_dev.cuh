@@ -12,12 +12,14 @@ constexpr int kCompThreshold = 4096;  // set bits above which rows use TwoSum
 // ---- vector loads of B ----------------------------------------------------
 template <typename BT> struct Vec;
 template <> struct Vec<float> {
+  using T = float;
   static constexpr int COLS = 4;
   using Raw = float4;
   __device__ static Raw load(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
   __device__ static void cvt(const Raw& r, float* o) { o[0] = r.x; o[1] = r.y; o[2] = r.z; o[3] = r.w; }
 };
 template <> struct Vec<__nv_bfloat16> {
+  using T = __nv_bfloat16;
   static constexpr int COLS = 8;
   using Raw = uint4;
   __device__ static Raw load(const __nv_bfloat16* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
@@ -31,6 +33,7 @@ template <> struct Vec<__nv_bfloat16> {
   }
 };
 template <> struct Vec<__half> {
+  using T = __half;
   static constexpr int COLS = 8;
   using Raw = uint4;
   __device__ static Raw load(const __half* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
@@ -44,6 +47,17 @@ template <> struct Vec<__half> {
       o[2 * j + 1] = f.y;
     }
   }
+};
+
+// One element at a time, for operands whose rows do not start on 16 bytes or
+// whose width is no multiple of a vector: lane = column, neighbouring lanes
+// neighbouring columns.
+template <typename BT> struct Elem1 {
+  using T = BT;
+  static constexpr int COLS = 1;
+  using Raw = BT;
+  __device__ static Raw load(const BT* p) { return __ldg(p); }
+  __device__ static void cvt(const Raw& r, float* o) { o[0] = to_f32(r); }
 };
 
 // ---- index streams --------------------------------------------------------
@@ -164,11 +178,11 @@ struct Acc {
 
 // Gathers D rows of B at a time (this lane's VPL vectors of each) and adds
 // them in stream order; entries with bit 31 set are subtracted.
-template <typename BT, int VPL, int D, bool COMP, typename Walker, typename LD = int64_t>
-__device__ __forceinline__ void accumulate_walk(Walker& wk, const BT* __restrict__ B, LD ldb,
+template <typename V, int VPL, int D, bool COMP, typename Walker, typename LD = int64_t>
+__device__ __forceinline__ void accumulate_walk(Walker& wk, const typename V::T* __restrict__ B, LD ldb,
                                                 const int* col, const bool* cvalid,
-                                                Acc<VPL, Vec<BT>::COLS, COMP>& acc) {
-  using V = Vec<BT>;
+                                                Acc<VPL, V::COLS, COMP>& acc) {
+  using BT = typename V::T;
   while (true) {
     uint32_t idx[D];
 #pragma unroll
@@ -217,16 +231,20 @@ __device__ __forceinline__ void store_vecs(float* __restrict__ crow, const int* 
     float o[COLS];
 #pragma unroll
     for (int j = 0; j < COLS; j++) o[j] = acc.result(v, j);
-    if (prow) {
+    if constexpr (COLS == 1) {
+      crow[col[v]] = prow ? o[0] + prow[col[v]] : o[0];
+    } else {
+      if (prow) {
 #pragma unroll
-      for (int j = 0; j < COLS; j += 4) {
-        const float4 p = *reinterpret_cast<const float4*>(prow + col[v] + j);
-        o[j] += p.x; o[j + 1] += p.y; o[j + 2] += p.z; o[j + 3] += p.w;
+        for (int j = 0; j < COLS; j += 4) {
+          const float4 p = *reinterpret_cast<const float4*>(prow + col[v] + j);
+          o[j] += p.x; o[j + 1] += p.y; o[j + 2] += p.z; o[j + 3] += p.w;
+        }
       }
-    }
 #pragma unroll
-    for (int j = 0; j < COLS; j += 4)
-      *reinterpret_cast<float4*>(crow + col[v] + j) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
+      for (int j = 0; j < COLS; j += 4)
+        *reinterpret_cast<float4*>(crow + col[v] + j) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
+    }
   }
 }
 

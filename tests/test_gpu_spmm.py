@@ -140,6 +140,55 @@ def test_heavy_rows_compensated():
     assert np.abs(C - C64).max() < 0.5 * np.abs(C32 - C64).max()
 
 
+@pytest.mark.parametrize("copies", [1, 40])  # a CTA per row / a warp per row
+@pytest.mark.parametrize("N", [132, 133])     # 16-byte vectors / single elements
+def test_walk_list_edges(copies, N):
+    """Row lengths around a round of gathers, the list's refill step and the
+    compensated sums' threshold, over more than 8192 columns: ascending FP32
+    sums, bit for bit, up to 4096 set bits."""
+    rng = np.random.default_rng(N + copies)
+    K = 9001
+    lens = [0, 1, 7, 8, 9, 15, 16, 17, 127, 128, 129, 143, 255, 256, 1151, 1152, 1153, 4095, 4096, 4097, 9001]
+    bits = np.zeros((len(lens), K), dtype=bool)
+    for i, n in enumerate(lens):
+        # the long rows spread out, the short ones in the last words
+        bits[i, rng.choice(K if n > 150 else np.arange(K - 200, K), n, replace=False)] = True
+    bits = np.tile(bits, (copies, 1))
+    words = W.pack_bits(bits)
+    Bf = rng.standard_normal((K, N)).astype(np.float32)
+    C = ops.spmm(words_dev(words), K, torch.from_numpy(Bf).cuda()).cpu().numpy()
+    short = bits.sum(1) <= 4096
+    ref = O.spmm_f32(words, K, Bf)
+    assert np.array_equal(C[short], ref[short])
+    _check_f64(C, words, K, Bf)
+    assert torch.equal(torch.from_numpy(C[:21]), torch.from_numpy(C[-21:]))
+
+
+@pytest.mark.parametrize("bdt", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("N", [1, 127, 129, 333])
+def test_prototype_plan_unaligned_columns(N, bdt):
+    """A prototype plan on layouts without 16-byte access, rows without a
+    cluster among them: exact on integers, and nothing written past N."""
+    rng = np.random.default_rng(N)
+    K = 3001
+    A, _, _ = W.clustered_bits(600, K, n_proto=6, p_proto=0.08, p_flip=0.004, seed_proto=N, seed_rows=N + 1)
+    A[::67] = rng.random((A[::67].shape[0], K)) < 0.05
+    words = W.pack_bits(A)
+    wd = words_dev(words)
+    plan = ops.Plan(wd, K, mode=capi.PLAN_PROTO)
+    assert plan.info()["mode"] == capi.PLAN_PROTO and plan.info()["direct_rows"] > 0
+    dt = dict(f32=torch.float32, bf16=torch.bfloat16, f16=torch.float16)[bdt]
+    Bi = rng.integers(-8, 9, (K, N)).astype(np.float32)
+    out = torch.full((600, N + 3), 7.0, device="cuda")
+    ops.spmm(wd, K, torch.from_numpy(Bi).to(dt).cuda(), plan=plan, out=out[:, :N])
+    assert np.array_equal(out[:, :N].cpu().numpy().astype(np.float64), O.spmm_f64(words, K, Bi))
+    assert torch.all(out[:, N:] == 7.0)
+    B = torch.from_numpy(rng.standard_normal((K, N)).astype(np.float32)).to(dt)
+    C = ops.spmm(wd, K, B.cuda(), plan=plan).cpu().numpy()
+    _check_f64(C, words, K, B.float().numpy())
+    assert capi.device_status() == 0
+
+
 def test_dense_prototypes_compensated():
     """Prototypes with more than 4096 set bits: their sums P[c] are formed
     with TwoSum pairs, so clustered rows stay as close to FP64 as the
