@@ -275,6 +275,33 @@ static TuneSched default_schedule(const bsp_plan* plan, int64_t N, int esz, bool
   return t;
 }
 
+// Room for a copy of B with 16-byte rows.
+static int64_t align_cols(int64_t N, int esz) { return ceil_div(N, 16 / esz) * (16 / esz); }
+static size_t align_b_bytes(int64_t K, int64_t N, int esz) {
+  return (size_t)K * (size_t)align_cols(N, esz) * (size_t)esz + 512;
+}
+
+// B in a layout that 16-byte loads can read, copied behind the first `used`
+// bytes of the workspace if it is not one already; false where there is no
+// room.  The single-element kernels gather at 3.5 TB/s, the vector ones at
+// 17, so a copy of K rows (read and written once) pays from about 1.8 set bits
+// per column on: taken as 64 rows where the set bits are not known
+// (2000x3001x333 FP32 at 5 %: 116 us without the copy, 41 with it, 3.5 of them for the copy).
+static bool align_operands(SpmmArgs* a, const bsp_plan* plan, void* workspace, size_t bytes, size_t used,
+                           cudaStream_t s) {
+  const int esz = dtype_size(a->bdt);
+  if (is_aligned(a->B, 16) && (a->ldb * esz) % 16 == 0 && (a->N * esz) % 16 == 0) return true;  // C alone is not
+  if (!workspace || bytes < used + align_b_bytes(a->K, a->N, esz)) return false;
+  if (plan ? plan->nnz < 2 * plan->K : a->M < 64) return false;
+  void* out = reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(workspace) + used + 255) & ~uintptr_t(255));
+  const int64_t Nb = align_cols(a->N, esz);
+  if (launch_align_b(a->B, a->bdt, a->K, a->N, a->ldb, out, Nb, s) != BSP_OK) return false;
+  a->B = out;
+  a->ldb = Nb;
+  a->Nb = Nb;
+  return true;
+}
+
 // Runs the SpMM with a given schedule (arguments already validated).
 static int run_spmm(SpmmArgs a, const bsp_plan* plan, bool vec, const TuneSched& sc, void* workspace,
                     size_t workspace_bytes, cudaStream_t s) {
@@ -284,15 +311,23 @@ static int run_spmm(SpmmArgs a, const bsp_plan* plan, bool vec, const TuneSched&
     return launch_spmm_tc(a, plan->occ, plan->wordsT, s, workspace, workspace_bytes,
                           TcForm{sc.tc_tps, sc.tc_tiled, sc.tc_split});
   const int64_t N = a.N, K = a.K;
+  int path = sc.proto_path;
   bool proto = plan && plan->mode == BSP_PLAN_PROTO;
+  size_t need = 0;
   if (proto) {
-    size_t need = 0;
     bsp_spmm_workspace(plan, N, &need);
     const bool room = workspace && workspace_bytes >= need;
     if (!room && vec) return BSP_ERR_WORKSPACE;
     // layouts without 16-byte access take the plan too where there is room
     // for the prototype sums, and walk A's rows as they always could without
-    if (!vec) proto = room && K < (int64_t)1 << 30;
+    if (!vec) {
+      proto = room && K < (int64_t)1 << 30;
+      if (!proto) need = 0;
+    }
+  }
+  if (!vec) {
+    path = 0;  // the staged rows copy whole slices: natural layouts only
+    vec = align_operands(&a, plan, workspace, workspace_bytes, need, s);
   }
   if (proto) {
     a.row_cluster = plan->row_cluster;
@@ -312,7 +347,7 @@ static int run_spmm(SpmmArgs a, const bsp_plan* plan, bool vec, const TuneSched&
       // prototype sums, then clustered rows (register gathers, or slices
       // staged by TMA bulk copies); rows without a cluster: walk A
       BSP_TRY(launch_proto_sums(a, vec, s));
-      if (sc.proto_path == 1 && vec) BSP_TRY(launch_spmm_proto_bulk(a, sc.proto_variant, s));
+      if (path == 1 && vec) BSP_TRY(launch_spmm_proto_bulk(a, sc.proto_variant, s));
       else BSP_TRY(launch_spmm_proto_regs(a, sc.proto_variant, vec, s));
       if (plan->direct_rows > 0) {
         SpmmArgs d = a;
@@ -340,9 +375,24 @@ int bsp_spmm_workspace(const bsp_plan* plan, int64_t N, size_t* bytes) {
 int bsp_spmm_workspace_preferred(const bsp_plan* plan, int64_t N, size_t* bytes) {
   BSP_TRY(bsp_spmm_workspace(plan, N, bytes));
   if (plan) {
+    // an odd width needs the aligned copy of B behind the prototype sums
+    if (N % 8 != 0) *bytes += align_b_bytes(plan->K, N, N % 4 != 0 ? 4 : 2);
     const size_t tc = tc_preferred_bytes(plan->M, N, plan->K);
     if (tc > *bytes) *bytes = tc;
   }
+  return BSP_OK;
+}
+
+int bsp_spmm_workspace_layout(const bsp_plan* plan, int64_t K, int64_t N, const void* B, int b_dtype, int64_t ldb,
+                              size_t* bytes) {
+  if (K < 0 || (b_dtype != BSP_F32 && b_dtype != BSP_BF16 && b_dtype != BSP_F16)) return BSP_ERR_INVALID_ARG;
+  BSP_TRY(bsp_spmm_workspace_preferred(plan, N, bytes));
+  const int esz = dtype_size(b_dtype);
+  if (is_aligned(B, 16) && (ldb * esz) % 16 == 0 && (N * esz) % 16 == 0) return BSP_OK;
+  size_t base = 0;
+  BSP_TRY(bsp_spmm_workspace(plan, N, &base));
+  const size_t copy = base + align_b_bytes(K, N, esz);
+  if (copy > *bytes) *bytes = copy;
   return BSP_OK;
 }
 
@@ -379,6 +429,8 @@ static int prepare_spmm(const uint32_t* A_words, int64_t M, int64_t K, const voi
   a->N = N;
   a->C = C;
   a->ldc = ldc;
+  a->Nb = N;
+  a->c_vec = is_aligned(C, 16) && ldc % 4 == 0 && N % 4 == 0;
   *tc_ok = plan && *vec && b_dtype != BSP_F32 && N % 8 == 0 && plan->K <= tc_max_reduction();
   *esz_out = esz;
   return BSP_OK;
@@ -732,7 +784,9 @@ int bsp_spmm_t(const uint32_t* A_words, int64_t M, int64_t K, const void* G, int
   a.N = N;
   a.C = dX;
   a.ldc = lddx;
-  return launch_spmm_rows(a, vec, s);
+  a.Nb = N;
+  a.c_vec = layout16(dX, lddx, 4, N, 4);
+  return launch_spmm_rows(a, vec || layout16(G, ldg, esz, N, vcols), s);
 }
 
 int bsp_sddmm(const uint32_t* A_words, int64_t M, int64_t K, const void* G, int64_t ldg, const void* X,

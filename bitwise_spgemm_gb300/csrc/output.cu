@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(256) k_bitplane_rows(PlaneArgs a) {
 #pragma unroll
       for (int j = 0; j < COLS; j++) tot.s[v][j] += w * acc.result(v, j);
   }
-  store_vecs<VPL, COLS, false>(a.C + row * a.ldc, col, cvalid, tot, nullptr);
+  store_vecs<VPL, COLS, false>(a.C + row * a.ldc, col, cvalid, tot, nullptr, true, a.N);
 }
 
 // Any layout: one warp per (row, 32 columns), a lane per column.

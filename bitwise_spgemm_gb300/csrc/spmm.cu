@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(256) k_spmm_list(SpmmArgs a) {
 #pragma unroll
     for (int v = 0; v < VPL; v++) {
       const int64_t c = n0 + (v * 32 + lane) * COLS;
-      cvalid[v] = c < a.N;
+      cvalid[v] = c < a.Nb;
       col[v] = cvalid[v] ? (int)c : 0;
     }
     float* crow = a.C + row * a.ldc;
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(256) k_spmm_list(SpmmArgs a) {
         int c1[1] = {col[v]};
         bool ok[1] = {cvalid[v]};
         accumulate_walk<V, 1, 4, true>(wk, B, a.ldb, c1, ok, acc);
-        store_vecs<1, COLS, true>(crow, c1, ok, acc, nullptr);
+        store_vecs<1, COLS, true>(crow, c1, ok, acc, nullptr, a.c_vec, a.N);
       }
       continue;
     }
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(256) k_spmm_list(SpmmArgs a) {
 #pragma unroll
       for (int g = 0; g < GROUPS; g++) wx[g] = wn[g];
     }
-    store_vecs<VPL, COLS, false>(crow, col, cvalid, acc, nullptr);
+    store_vecs<VPL, COLS, false>(crow, col, cvalid, acc, nullptr, a.c_vec, a.N);
     __syncwarp();
   }
 }
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(256) k_spmm_coop(SpmmArgs a) {
 #pragma unroll
   for (int v = 0; v < VPL; v++) {
     const int64_t c = n0 + (v * 32 + lane) * COLS;
-    cvalid[v] = c < a.N;
+    cvalid[v] = c < a.Nb;
     bcol[v] = B + (cvalid[v] ? c : 0);
   }
   bool comp = false;
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(256) k_spmm_rows_wide(SpmmArgs a) {
     Acc<VPL, COLS, false> acc;
     acc.zero();
     accumulate_walk<V, VPL, D, false>(wk, B, a.ldb, col, cvalid, acc);
-    store_vecs<VPL, COLS, false>(crow, col, cvalid, acc, a.P + (int64_t)cl * a.ldp);
+    store_vecs<VPL, COLS, false>(crow, col, cvalid, acc, a.P + (int64_t)cl * a.ldp, a.c_vec, a.N);
     return;
   }
   const uint32_t* arow = a.A + row * a.Kw;
@@ -314,12 +314,12 @@ __global__ void __launch_bounds__(256) k_spmm_rows_wide(SpmmArgs a) {
       Acc<1, COLS, true> acc;
       acc.zero();
       accumulate_walk<V, 1, 4, true>(wk, B, a.ldb, c1, ok, acc);
-      store_vecs<1, COLS, true>(crow, c1, ok, acc, nullptr);
+      store_vecs<1, COLS, true>(crow, c1, ok, acc, nullptr, a.c_vec, a.N);
     } else {
       Acc<1, COLS, false> acc;
       acc.zero();
       accumulate_walk<V, 1, 4, false>(wk, B, a.ldb, c1, ok, acc);
-      store_vecs<1, COLS, false>(crow, c1, ok, acc, nullptr);
+      store_vecs<1, COLS, false>(crow, c1, ok, acc, nullptr, a.c_vec, a.N);
     }
   }
 }
@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(256, MINB) k_spmm_proto_regs(SpmmArgs a) {
 #pragma unroll
     for (int v = 0; v < VPL; v++) {
       col[v] = n0 + (v * 32 + lane) * COLS;
-      cvalid[v] = FULL || col[v] < (int)a.N;
+      cvalid[v] = FULL || col[v] < (int)a.Nb;
     }
     Acc<VPL, COLS, false> acc;
     acc.zero();
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(256, MINB) k_spmm_proto_regs(SpmmArgs a) {
       else accumulate_walk<V, VPL, D, false>(wk, B, a.ldb, col, cvalid, acc);
     }
     ptx::griddep_wait();
-    store_vecs<VPL, COLS, false>(a.C + (int64_t)row * a.ldc, col, cvalid, acc, a.P + (int64_t)cl * a.ldp);
+    store_vecs<VPL, COLS, false>(a.C + (int64_t)row * a.ldc, col, cvalid, acc, a.P + (int64_t)cl * a.ldp, a.c_vec, a.N);
   } else {
     ptx::griddep_wait();
   }
@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(512) k_proto_sums(SpmmArgs a) {
   const int64_t n0 = (int64_t)blockIdx.y * CW;
   const BT* __restrict__ B = static_cast<const BT*>(a.B);
   int col[1] = {(int)n0 + lane * COLS};
-  bool cvalid[1] = {col[0] < a.N};
+  bool cvalid[1] = {col[0] < a.Nb};
   ptx::griddep_launch_dependents();
   const uint32_t* cw = a.cons + c * a.Kw;
   const int w0 = (int)(a.Kw * wid / W), w1 = (int)(a.Kw * (wid + 1) / W);
@@ -460,7 +460,7 @@ __global__ void __cluster_dims__(kSumCluster, 1, 1) __launch_bounds__(256) k_pro
 #pragma unroll
   for (int v = 0; v < VPL; v++) {
     col[v] = n0 + (v * 32 + lane) * COLS;
-    cvalid[v] = col[v] < (int)a.N;
+    cvalid[v] = col[v] < (int)a.Nb;
   }
   const int s0 = __ldg(a.cons_ptr + c), len = __ldg(a.cons_ptr + c + 1) - s0;
   const int p = rank * 8 + wid;
@@ -585,7 +585,7 @@ template <typename V, int VPL, int D, int MINB>
 int launch_proto_regs_t(const SpmmArgs& a, cudaStream_t s) {
   constexpr int CW = 32 * VPL * V::COLS;
   cudaLaunchConfig_t cfg = {};
-  const bool off32 = a.K * a.ldb < ((int64_t)1 << 31), full = a.N % CW == 0;
+  const bool off32 = a.K * a.ldb < ((int64_t)1 << 31), full = a.Nb % CW == 0;
   const bool slot = off32 && a.delta_pad && a.n_slot > 0 && slot_lists_enabled();
   cfg.gridDim = dim3((unsigned)ceil_div(slot ? a.n_slot : a.M, 8), (unsigned)ceil_div(a.N, CW));
   cfg.blockDim = dim3(256);
@@ -641,7 +641,7 @@ int launch_proto_t(const SpmmArgs& a, cudaStream_t s) {
   static const int sv = getenv("BSP_SUMS_BULK") ? atoi(getenv("BSP_SUMS_BULK")) : (sizeof(BT) == 4 ? 1 : 8);
   const int esz = (int)sizeof(BT);
   if (sv >= 0 && a.cons_idx && !comp && a.n_proto <= 65535 && reinterpret_cast<uintptr_t>(a.B) % 16 == 0 &&
-      (a.ldb * esz) % 16 == 0 && (a.N * esz) % 16 == 0) {
+      (a.ldb * esz) % 16 == 0 && (a.Nb * esz) % 16 == 0) {
     const int rc = launch_proto_sums_bulk(a, sv, s);
     if (rc != BSP_ERR_UNSUPPORTED) return rc;  // a shape too large for this B type: the cluster form
   }
@@ -663,6 +663,28 @@ int launch_proto_t(const SpmmArgs& a, cudaStream_t s) {
   else k_proto_sums<V, 8, false, false><<<g, threads, smem, s>>>(a);
   BSP_LAUNCHED();
   return BSP_OK;
+}
+
+// An aligned copy of B for layouts without 16-byte access: a warp takes 256
+// columns of a row, 8 loads in flight.
+template <typename T>
+__global__ void __launch_bounds__(256) k_align_b(const T* __restrict__ B, int64_t K, int64_t N, int64_t ldb,
+                                                 T* __restrict__ out, int64_t Nb) {
+  const int lane = threadIdx.x & 31;
+  const int64_t nch = (Nb + 255) / 256, total = K * nch;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; t < total; t += nwarps) {
+    const int64_t k = total <= 0x7fffffff ? (int64_t)((uint32_t)t / (uint32_t)nch) : t / nch;
+    const int64_t c0 = (t - k * nch) * 256 + lane;
+    const T* src = B + k * ldb;
+    T* dst = out + k * Nb;
+    T v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) v[u] = c0 + 32 * u < N ? __ldg(src + c0 + 32 * u) : T(0);
+#pragma unroll
+    for (int u = 0; u < 8; u++)
+      if (c0 + 32 * u < Nb) dst[c0 + 32 * u] = v[u];
+  }
 }
 
 // SDDMM on CUDA cores: warp per row i of A; the row of dA is zeroed, then for
@@ -693,6 +715,16 @@ __global__ void __launch_bounds__(256) k_sddmm_rows(const uint32_t* __restrict__
 }
 
 }  // namespace
+
+int launch_align_b(const void* B, int bdt, int64_t K, int64_t N, int64_t ldb, void* out, int64_t Nb, cudaStream_t s) {
+  if (K == 0 || Nb == 0) return BSP_OK;
+  const int64_t blocks = ceil_div(K * ceil_div(Nb, 256), 8), cap = (int64_t)num_sms() * 8;
+  const unsigned grid = (unsigned)(blocks < cap ? blocks : cap);
+  if (dtype_size(bdt) == 4) k_align_b<<<grid, 256, 0, s>>>((const uint32_t*)B, K, N, ldb, (uint32_t*)out, Nb);
+  else k_align_b<<<grid, 256, 0, s>>>((const uint16_t*)B, K, N, ldb, (uint16_t*)out, Nb);
+  BSP_LAUNCHED();
+  return BSP_OK;
+}
 
 int launch_sddmm_rows(const uint32_t* A, int64_t M, int64_t K, const void* G, int64_t ldg, const void* X,
                       int64_t ldx, int dt, int64_t N, float* dA, int64_t ldda, cudaStream_t s) {

@@ -37,8 +37,10 @@ struct SpmmArgs {
   const void* B;      // [K][ldb] of bdt
   int bdt;
   int64_t ldb, N;
+  int64_t Nb;         // columns of B that may be read: N, or N rounded up to a vector in an aligned copy of B
   float* C;           // [M][ldc]
   int64_t ldc;
+  bool c_vec;         // C's rows take 16-byte stores (else element by element)
   // prototype mode (plan)
   const int32_t* row_cluster;  // [M], -1 = walk A's row
   const int32_t* delta_ptr;    // [M+1]
@@ -58,7 +60,9 @@ struct SpmmArgs {
   int64_t n_list;
 };
 
-// vec = B/C layouts allow 16-byte vector access (else lane-per-column path)
+// B [K][N] (row stride ldb, any alignment) -> out [K][Nb], columns N..Nb-1 zero
+int launch_align_b(const void* B, int bdt, int64_t K, int64_t N, int64_t ldb, void* out, int64_t Nb, cudaStream_t s);
+// vec = B's layout allows 16-byte vector access (else lane-per-column path)
 int launch_spmm_rows(const SpmmArgs& a, bool vec, cudaStream_t s);
 // prototype plans of A with 2^30 or more columns (vec layouts only)
 int launch_spmm_rows_wide(const SpmmArgs& a, cudaStream_t s);

@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_proto_sums_bulk(SpmmArgs a) {
 
   const int n0 = (int)blockIdx.x * CW;
   const int64_t c = blockIdx.y;
-  const int ncols = min(CW, (int)(a.N - n0));
+  const int ncols = min(CW, (int)(a.Nb - n0));
   const uint32_t bytes = (uint32_t)ncols * (uint32_t)sizeof(BT);
   const BT* Bn = static_cast<const BT*>(a.B) + n0;
   const int s0 = __ldg(a.cons_ptr + c), len = __ldg(a.cons_ptr + c + 1) - s0;
@@ -369,7 +369,7 @@ int launch_sums_bulk_t(const SpmmArgs& a, cudaStream_t st) {
     BSP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kTotal));
     configured[dev] = true;
   }
-  const int64_t chunks = ceil_div(a.N, L::kCW);
+  const int64_t chunks = ceil_div(a.Nb, L::kCW);
   if (chunks > 0x7fffffff || a.n_proto > 65535) return BSP_ERR_CAPACITY;
   kern<<<dim3((unsigned)chunks, (unsigned)a.n_proto), WARPS * 32, L::kTotal, st>>>(a);
   BSP_LAUNCHED();

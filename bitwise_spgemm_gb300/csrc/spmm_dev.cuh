@@ -224,7 +224,7 @@ __device__ __forceinline__ int row_popcount(const uint32_t* __restrict__ row, in
 template <int VPL, int COLS, bool COMP>
 __device__ __forceinline__ void store_vecs(float* __restrict__ crow, const int* col,
                                            const bool* cvalid, const Acc<VPL, COLS, COMP>& acc,
-                                           const float* __restrict__ prow) {
+                                           const float* __restrict__ prow, bool c_vec, int64_t N) {
 #pragma unroll
   for (int v = 0; v < VPL; v++) {
     if (!cvalid[v]) continue;
@@ -232,6 +232,8 @@ __device__ __forceinline__ void store_vecs(float* __restrict__ crow, const int* 
 #pragma unroll
     for (int j = 0; j < COLS; j++) o[j] = acc.result(v, j);
     if constexpr (COLS == 1) {
+      (void)c_vec;
+      (void)N;
       crow[col[v]] = prow ? o[0] + prow[col[v]] : o[0];
     } else {
       if (prow) {
@@ -241,9 +243,15 @@ __device__ __forceinline__ void store_vecs(float* __restrict__ crow, const int* 
           o[j] += p.x; o[j + 1] += p.y; o[j + 2] += p.z; o[j + 3] += p.w;
         }
       }
+      if (c_vec) {
 #pragma unroll
-      for (int j = 0; j < COLS; j += 4)
-        *reinterpret_cast<float4*>(crow + col[v] + j) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
+        for (int j = 0; j < COLS; j += 4)
+          *reinterpret_cast<float4*>(crow + col[v] + j) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < COLS; j++)
+          if (col[v] + j < N) crow[col[v] + j] = o[j];
+      }
     }
   }
 }

@@ -173,15 +173,22 @@ def spmm(words, K, B, plan=None, out=None, workspace=None):
     ldc = _rowmajor(out, "out")
     h = plan.handle if plan is not None else None
     ws_ptr, ws_n = None, 0
+    # a caller's workspace is used if it holds the minimum; without one, the
+    # preferred size is allocated (room for the tensor-core split, and for a
+    # copy of B where its rows do not take 16-byte loads)
+    have = workspace.numel() * workspace.element_size() if workspace is not None else 0
     if plan is not None:
-        # a caller's workspace is used if it holds the minimum; without one,
-        # the preferred size (room for the tensor-core split) is allocated
-        have = workspace.numel() * workspace.element_size() if workspace is not None else 0
-        if workspace is None or have < plan.workspace_bytes(N, preferred=False):
-            need = plan.workspace_bytes(N)
-            workspace = torch.empty(max(need, 1), dtype=torch.uint8, device=B.device) if need else None
-        if workspace is not None:
-            ws_ptr, ws_n = _p(workspace), workspace.numel() * workspace.element_size()
+        fits = workspace is not None and have >= plan.workspace_bytes(N, preferred=False)
+    else:
+        e = B.element_size()
+        fits = workspace is not None or (N * e % 16 == 0 and ldb * e % 16 == 0 and B.data_ptr() % 16 == 0)
+    if not fits:
+        n = C.c_size_t()
+        call("bsp_spmm_workspace_layout", h, K, N, _p(B), _DT[B.dtype], ldb, C.byref(n))
+        workspace = torch.empty(n.value, dtype=torch.uint8, device=B.device) if n.value else None
+        have = n.value
+    if workspace is not None:
+        ws_ptr, ws_n = _p(workspace), have
     call("bsp_spmm", _p(words), M, K, _p(B), _DT[B.dtype], ldb, N, _p(out), ldc, h, ws_ptr, ws_n,
          _stream())
     return out

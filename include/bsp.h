@@ -219,6 +219,13 @@ int bsp_spmm_workspace(const bsp_plan* plan, int64_t N, size_t* bytes);
  * bsp_spmm_t uses its own workspace the same way when it is large enough. */
 int bsp_spmm_workspace_preferred(const bsp_plan* plan, int64_t N, size_t* bytes);
 
+/* Workspace for these operands: the above and, where B's rows do not take
+ * 16-byte loads (B, ldb or N not a multiple of 16 bytes; plan may be NULL),
+ * room for a copy of B that does.  A smaller workspace only turns the copy
+ * off (results are identical).  B is looked at as an address, not read.     */
+int bsp_spmm_workspace_layout(const bsp_plan* plan, int64_t K, int64_t N, const void* B, int b_dtype,
+                              int64_t ldb, size_t* bytes);
+
 /* C[M×N] (FP32, row stride ldc) = A·B, A given by its packed words and,
  * optionally, a plan built from the same words (NULL = walk every row's set
  * bits).  B is K×N of b_dtype ∈ {F32, F16, BF16}, row stride ldb elements;
