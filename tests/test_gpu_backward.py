@@ -85,6 +85,31 @@ def test_sddmm(kind, tc, M, K, N, p, monkeypatch):
     assert np.allclose(vals, full[bits], rtol=0, atol=1e-9 * max(1.0, np.abs(full).max()))
 
 
+@pytest.mark.parametrize("kind", ["f32", "bf16"])
+@pytest.mark.parametrize("M,K,N,p,pad", [(3, 2111, 1, 0.5, 0), (40, 1500, 129, 0.3, 0), (40, 1500, 132, 0.3, 4),
+                                         (2500, 70, 8, 0.9, 0), (5, 9000, 260, 0.02, 1)])
+def test_sddmm_rows_lists_and_parts(kind, M, K, N, p, pad, monkeypatch):
+    """Rows cut into parts, lists across their refill step, dot products in
+    rounds of 8 with a remainder, a last partial vector, unaligned rows."""
+    monkeypatch.setenv("BSP_TC", "0")
+    rng = np.random.default_rng(M + K + N)
+    bits = rng.random((M, K)) < p
+    bits[0, :] = False
+    bits[1, :] = True
+    words = W.pack_bits(bits)
+    G, Gx = _operand(rng.standard_normal((M, N + pad)).astype(np.float32), kind)
+    X, Xx = _operand(rng.standard_normal((K, N + pad)).astype(np.float32), kind)
+    out = torch.full((M, K + 3), 7.0, device="cuda")
+    ops.sddmm(words_dev(words), M, K, G[:, :N], X[:, :N], out=out[:, :K])
+    dA = out[:, :K].cpu().numpy()
+    Gx, Xx = Gx[:, :N].astype(np.float64), Xx[:, :N].astype(np.float64)
+    scale = np.abs(Gx) @ np.abs(Xx).T
+    assert np.all(dA[~bits] == 0)
+    assert torch.all(out[:, K:] == 7.0)
+    # FP32 dot products of N terms: N/32 roundings a lane, 5 in the reduction
+    assert _scaled_max((dA - Gx @ Xx.T)[bits], scale[bits]) <= TOL
+
+
 def _loss64(A, X, G):
     return float(((A @ X) * G).sum())
 
