@@ -244,9 +244,11 @@ __device__ __forceinline__ void store_vecs(float* __restrict__ crow, const int* 
         }
       }
       if (c_vec) {
+        // (a vector of 8 may end 4 columns past N, in an aligned copy of B)
 #pragma unroll
         for (int j = 0; j < COLS; j += 4)
-          *reinterpret_cast<float4*>(crow + col[v] + j) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
+          if (j == 0 || col[v] + j < N)
+            *reinterpret_cast<float4*>(crow + col[v] + j) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
       } else {
 #pragma unroll
         for (int j = 0; j < COLS; j++)

@@ -165,7 +165,24 @@ def test_walk_list_edges(copies, N):
 
 
 @pytest.mark.parametrize("bdt", ["f32", "bf16", "f16"])
-@pytest.mark.parametrize("N", [1, 127, 129, 333])
+@pytest.mark.parametrize("N", [4, 12, 130, 132, 180])
+def test_walk_aligned_copy_of_b(N, bdt):
+    """Widths that are no multiple of a vector, 4 columns past one among them,
+    with C's rows back to back: no row's store reaches into the next."""
+    rng = np.random.default_rng(N)
+    M, K = 200, 700
+    words = W.pack_bits(rng.random((M, K)) < 0.1)
+    dt = dict(f32=torch.float32, bf16=torch.bfloat16, f16=torch.float16)[bdt]
+    Bi = rng.integers(-8, 9, (K, N)).astype(np.float32)
+    for ld in (N, N + 4, N + 5):
+        B = torch.zeros((K, ld), dtype=dt, device="cuda")
+        B[:, :N] = torch.from_numpy(Bi).to(dt)
+        C = ops.spmm(words_dev(words), K, B[:, :N]).cpu().numpy()
+        assert np.array_equal(C.astype(np.float64), O.spmm_f64(words, K, Bi))
+
+
+@pytest.mark.parametrize("bdt", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("N", [1, 127, 129, 132, 333])
 def test_prototype_plan_unaligned_columns(N, bdt):
     """A prototype plan on layouts without 16-byte access, rows without a
     cluster among them: exact on integers, and nothing written past N."""
