@@ -10,6 +10,7 @@
 #include "plan.cuh"
 #include "tune.h"
 #include "spmm.cuh"
+#include "ts.cuh"
 
 namespace bsp {
 
@@ -226,11 +227,14 @@ static int64_t proto_ldp(int64_t N) { return (N + 7) / 8 * 8; }
 // Cost model of the tensor-core decision, in seconds: dense BF16 work on the
 // occupied (128 x 32) tiles at ~1.2 PFLOP/s against the B-row gathers of the
 // CUDA-core schedule at ~8 TB/s (rates measured on GB300).
-static bool use_tensor_cores(const bsp_plan* plan, int64_t N, int esize) {
+// Layouts without 16-byte access pay for a flag, B's tile order and the walk
+// that stands by for it: about 8 us of launches (4093x495x102 BF16 behind a new
+// plan: 10 us slower on the tensor cores than without).
+static bool use_tensor_cores(const bsp_plan* plan, int64_t N, int esize, bool vec) {
   if (plan->K > tc_max_reduction()) return false;
   const char* e = getenv("BSP_TC");
   if (e) return e[0] == '1';
-  const double tc = (double)plan->occ_tiles * 128.0 * 32.0 * (double)N * 2.0 / 1.2e15;
+  const double tc = (double)plan->occ_tiles * 128.0 * 32.0 * (double)N * 2.0 / 1.2e15 + (vec ? 0.0 : 8e-6);
   double gathers = (double)plan->nnz;
   if (plan->mode == BSP_PLAN_PROTO)
     gathers = (double)(plan->proto_nnz + plan->delta_nnz + plan->direct_nnz + plan->M);
@@ -267,9 +271,9 @@ static int proto_variant(int esz) {
 // Default schedule: the cost model for the engine (BSP_TC=0/1 forces it),
 // the measured default shape of the prototype kernels (BSP_PROTO_PATH /
 // BSP_PROTO_VARIANT override them).
-static TuneSched default_schedule(const bsp_plan* plan, int64_t N, int esz, bool tc_ok) {
+static TuneSched default_schedule(const bsp_plan* plan, int64_t N, int esz, bool tc_ok, bool vec) {
   TuneSched t;
-  t.engine = (tc_ok && use_tensor_cores(plan, N, esz)) ? 1 : 2;
+  t.engine = (tc_ok && use_tensor_cores(plan, N, esz, vec)) ? 1 : 2;
   t.proto_path = proto_path();
   t.proto_variant = proto_variant(esz);
   return t;
@@ -307,9 +311,14 @@ static int run_spmm(SpmmArgs a, const bsp_plan* plan, bool vec, const TuneSched&
                     size_t workspace_bytes, cudaStream_t s) {
   // Tensor cores for 16-bit B when the occupied bit tiles make a dense
   // contraction cheaper than gathering B rows.
-  if (sc.engine == 1)
-    return launch_spmm_tc(a, plan->occ, plan->wordsT, s, workspace, workspace_bytes,
-                          TcForm{sc.tc_tps, sc.tc_tiled, sc.tc_split});
+  if (sc.engine == 1) {
+    const int* skipped = nullptr;
+    BSP_TRY(launch_spmm_tc(a, plan->occ, plan->wordsT, vec, s, workspace, workspace_bytes,
+                           TcForm{sc.tc_tps, sc.tc_tiled, sc.tc_split}, &skipped));
+    if (!skipped) return BSP_OK;
+    a.run_if = skipped;
+    return launch_spmm_rows(a, vec, s);
+  }
   const int64_t N = a.N, K = a.K;
   int path = sc.proto_path;
   bool proto = plan && plan->mode == BSP_PLAN_PROTO;
@@ -400,8 +409,8 @@ int bsp_spmm_workspace_layout(const bsp_plan* plan, int64_t K, int64_t N, const 
 // product is empty (C already written or nothing to write).
 constexpr int kDone = 1;
 static int prepare_spmm(const uint32_t* A_words, int64_t M, int64_t K, const void* B, int b_dtype, int64_t ldb,
-                        int64_t N, float* C, int64_t ldc, const bsp_plan* plan, cudaStream_t s, SpmmArgs* a,
-                        bool* vec, bool* tc_ok, int* esz_out) {
+                        int64_t N, float* C, int64_t ldc, const bsp_plan* plan, const void* workspace,
+                        size_t workspace_bytes, cudaStream_t s, SpmmArgs* a, bool* vec, bool* tc_ok, int* esz_out) {
   BSP_TRY(check_dims(M, K));
   if (N < 0 || N > kMaxCols) return BSP_ERR_INVALID_ARG;
   if (b_dtype != BSP_F32 && b_dtype != BSP_BF16 && b_dtype != BSP_F16) return BSP_ERR_UNSUPPORTED;
@@ -431,7 +440,9 @@ static int prepare_spmm(const uint32_t* A_words, int64_t M, int64_t K, const voi
   a->ldc = ldc;
   a->Nb = N;
   a->c_vec = is_aligned(C, 16) && ldc % 4 == 0 && N % 4 == 0;
-  *tc_ok = plan && *vec && b_dtype != BSP_F32 && N % 8 == 0 && plan->K <= tc_max_reduction();
+  // 16-bit B by TMA boxes, or copied into tile order where its rows take none
+  *tc_ok = plan && b_dtype != BSP_F32 && plan->K <= tc_max_reduction() &&
+           (*vec || (workspace && workspace_bytes >= tc_tiled_b_bytes(K, N)));
   *esz_out = esz;
   return BSP_OK;
 }
@@ -443,11 +454,12 @@ int bsp_spmm(const uint32_t* A_words, int64_t M, int64_t K, const void* B, int b
   SpmmArgs a;
   bool vec = false, tc_ok = false;
   int esz = 4;
-  const int rc = prepare_spmm(A_words, M, K, B, b_dtype, ldb, N, C, ldc, plan, s, &a, &vec, &tc_ok, &esz);
+  const int rc = prepare_spmm(A_words, M, K, B, b_dtype, ldb, N, C, ldc, plan, workspace, workspace_bytes, s, &a, &vec,
+                              &tc_ok, &esz);
   if (rc != BSP_OK) return rc == kDone ? BSP_OK : rc;
   // A measured schedule for this shape bucket (bsp_tune) replaces the cost
   // model, unless the environment forces a choice.
-  TuneSched sc = default_schedule(plan, N, esz, tc_ok);
+  TuneSched sc = default_schedule(plan, N, esz, tc_ok, vec);
   TuneSched tuned;
   if (plan && !getenv("BSP_TC") && !getenv("BSP_PROTO_PATH") && !getenv("BSP_PROTO_VARIANT") &&
       tune_lookup(plan, N, b_dtype, &tuned) && (tuned.engine == 2 || tc_ok))
@@ -463,26 +475,26 @@ int bsp_tune(const uint32_t* A_words, int64_t M, int64_t K, const void* B, int b
   SpmmArgs a;
   bool vec = false, tc_ok = false;
   int esz = 4;
-  const int rc = prepare_spmm(A_words, M, K, B, b_dtype, ldb, N, C, ldc, plan, s, &a, &vec, &tc_ok, &esz);
+  const int rc = prepare_spmm(A_words, M, K, B, b_dtype, ldb, N, C, ldc, plan, workspace, workspace_bytes, s, &a, &vec,
+                              &tc_ok, &esz);
   if (rc == kDone) return BSP_ERR_INVALID_ARG;  // nothing to time
   BSP_TRY(rc);
-  // candidates: the tensor cores in each tile form (2 or 3 K tiles per
-  // stage, B by boxes or pre-tiled, split-K by the rule or never); every
+  // candidates: the tensor cores in each tile form (B by boxes or pre-tiled,
+  // split-K by the rule or never; one stage form); every
   // prototype-kernel shape on both CUDA-core paths; the plain walk when the
   // plan has no prototypes
-  TuneSched cand[8 + 9 + 8];
+  TuneSched cand[4 + 9 + 8];
   int nc = 0;
   if (tc_ok)
-    for (int tps = 2; tps <= 3; tps++)
-      for (int tiled = 0; tiled <= 1; tiled++)
-        for (int split = -1; split <= 0; split++) {
-          TuneSched t;
-          t.engine = 1;
-          t.tc_tps = tps;
-          t.tc_tiled = tiled;
-          t.tc_split = split;
-          cand[nc++] = t;
-        }
+    for (int tiled = 0; tiled <= 1; tiled++)
+      for (int split = -1; split <= 0; split++) {
+        TuneSched t;
+        t.engine = 1;
+        t.tc_tps = 2;
+        t.tc_tiled = tiled;
+        t.tc_split = split;
+        cand[nc++] = t;
+      }
   if (plan->mode == BSP_PLAN_PROTO && vec) {
     for (int v = 0; v <= 8; v++) cand[nc++] = TuneSched{2, 0, v, 0.0};
     for (int v = 0; v <= 7; v++) cand[nc++] = TuneSched{2, 1, v, 0.0};
@@ -819,11 +831,12 @@ int bsp_sddmm(const uint32_t* A_words, int64_t M, int64_t K, const void* G, int6
 
 int bsp_device_status(int* status, int clear) {
   if (!status) return BSP_ERR_INVALID_ARG;
-  int a = 0, b = 0, c = 0;
+  int a = 0, b = 0, c = 0, d = 0;
   BSP_TRY(bulk_device_error(&a, clear != 0));
   BSP_TRY(tc_device_error(&b, clear != 0));
   BSP_TRY(batched_device_error(&c, clear != 0));
-  *status = a ? a : (b ? b : c);
+  BSP_TRY(ts_device_error(&d, clear != 0));
+  *status = a ? a : (b ? b : (c ? c : d));
   return BSP_OK;
 }
 

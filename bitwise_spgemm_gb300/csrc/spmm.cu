@@ -52,6 +52,7 @@ __global__ void __launch_bounds__(256) k_spmm_list(SpmmArgs a) {
   __shared__ __align__(16) uint32_t lists[8][kListCap];
   const int lane = threadIdx.x & 31;
   uint32_t* list = lists[threadIdx.x >> 5];
+  if (a.run_if && !__ldg(a.run_if)) return;
   int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (a.row_list) {
     if (row >= a.n_list) return;
@@ -198,6 +199,7 @@ __global__ void __launch_bounds__(256) k_spmm_coop(SpmmArgs a) {
   extern __shared__ __align__(16) uint8_t coop_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(coop_raw);
   ptx::griddep_launch_dependents();
+  if (a.run_if && !__ldg(a.run_if)) return;  // (never with a row list)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t row = a.row_list ? (int64_t)__ldg(a.row_list + blockIdx.x) : (int64_t)blockIdx.x;
   const BT* __restrict__ B = static_cast<const BT*>(a.B);

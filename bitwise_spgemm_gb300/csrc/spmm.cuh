@@ -41,6 +41,7 @@ struct SpmmArgs {
   float* C;           // [M][ldc]
   int64_t ldc;
   bool c_vec;         // C's rows take 16-byte stores (else element by element)
+  const int* run_if;  // device flag: zero = do nothing (walking kernels only); null = run
   // prototype mode (plan)
   const int32_t* row_cluster;  // [M], -1 = walk A's row
   const int32_t* delta_ptr;    // [M+1]
@@ -102,8 +103,12 @@ int launch_occupancy(const uint32_t* A, int64_t M, int64_t K, uint32_t* occ, uin
 struct TcForm {
   int tps = 0, tiled = -1, split = -1;
 };
-int launch_spmm_tc(const SpmmArgs& a, const uint32_t* occ, const uint32_t* At, cudaStream_t s, void* ws = nullptr,
-                   size_t ws_bytes = 0, TcForm form = TcForm{});
+// vec = false (layouts without 16-byte access): B has to fit the workspace in
+// tile order, and *skipped becomes a device flag that is nonzero when the
+// product was left to the walking kernels (infinities or NaN in B, which a
+// dense product would spread over rows that do not hold their column).
+int launch_spmm_tc(const SpmmArgs& a, const uint32_t* occ, const uint32_t* At, bool vec, cudaStream_t s, void* ws,
+                   size_t ws_bytes, TcForm form, const int** skipped);
 int launch_transpose_words(const uint32_t* words, int64_t M, int64_t Kw, uint32_t* At, cudaStream_t s);
 int tc_split_count(int64_t out_rows, int64_t out_cols, int64_t red_tiles);
 size_t tc_split_bytes(int64_t out_rows, int64_t out_cols, int64_t red_tiles);

@@ -1,35 +1,27 @@
-// spmm_tc.cu — tensor-core bitmap SpMM for 16-bit B (tcgen05, TMEM).
+// spmm_tc.cu — tensor-core kernels with both operands in shared memory
+// (tcgen05, TMEM accumulators) and the host side of the tensor-core products.
 //
-// For matrices whose bits come in dense blocks (or are dense enough that a
-// dense contraction beats per-bit adds), C = A·B runs on the 5th-generation
-// tensor cores: each 32-column bit tile of A is expanded to 0/1 BF16/FP16
-// operands in shared memory (the idea of the reference's tSparse kernel,
-// source/src/mm.cu:123-145, which expanded 8x8 bitmap tiles into 0/1 half
-// wmma fragments) and multiplied by the matching 32 rows of B.
+// k_spmm_tc runs the SDDMM dA = (G·Xᵀ) ⊙ A, dense over N with a masked store,
+// and the CTA-per-item forms of the batched products (forward, Aᵀ·G and
+// SDDMM).  The single forward product and Aᵀ·G run on the persistent kernel of
+// spmm_ts.cu, launched from here.
 //
 // CTA tile: 256 rows x 256 columns of C as two 128-row halves, each with its
 // FP32 accumulator in TMEM (2 x 256 columns); both halves multiply the same
-// B stage, so every B byte brought into shared memory feeds 256 rows.  K
-// advances over the 32-column tiles where either 128-row block has a set bit
-// (the plan's occupancy bitmap); a half without bits in a tile skips its
-// MMAs.  A stage carries TPS tiles (2 tiles x 3 stages, or 3 x 2 where many
-// row blocks share B); per CTA:
-//   256·TPS producer threads (one row of one tile each): load the tile's
-//     words (column-major copy in the plan: one 128-byte run per warp),
-//     expand them into the A operand (K-major core matrices, 2.0 per set
-//     bit) and arrive on the stage's "full" mbarrier; after the last stage
-//     16 of these warps read the accumulators back (tcgen05.ld), scale by
-//     0.5 and store C through a 32x32 staging tile per warp;
-//   a TMA warp: B rows of the stage's tiles, either as one bulk copy of 16
-//     KB per tile from B already in tile order (k_tile_b) or as four 64x32
-//     tensor boxes (128-byte swizzle, MN-major);
+// B stage, so every B byte brought into shared memory feeds 256 rows.  Per
+// CTA:
+//   256·TPS producer threads (one row of one tile each; batched bit operands):
+//     load the tile's words, expand them into the A operand (K-major core
+//     matrices, 2.0 per set bit; the idea of the reference's tSparse kernel,
+//     source/src/mm.cu:123-145) and arrive on the stage's "full" mbarrier;
+//     after the last stage 16 of these warps read the accumulators back
+//     (tcgen05.ld), scale by 0.5 and store C through a 32x32 staging tile per
+//     warp;
+//   a TMA warp: the dense operands' boxes (128-byte swizzle);
 //   an MMA warp: allocates TMEM; its lane 0 issues two tcgen05.mma (K=16) per
 //     occupied half per tile and commits the stage to its "empty" mbarrier.
-// An mbarrier hand-off costs 200-500 cycles on GB300, and the tensor pipe
-// queues about one MMA beyond the running one, so the design keeps the
-// MMA thread's work between stages minimal and carries several tiles per
-// hand-off.  Every mbarrier wait is bounded (timeout -> error 3 in
-// g_tc_error, the CTA skips its stores and frees its TMEM).
+// Every mbarrier wait is bounded (timeout -> error 3 in g_tc_error, the CTA
+// skips its stores and frees its TMEM).
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -40,6 +32,7 @@
 #include "ptx.cuh"
 #include "spmm_dev.cuh"
 #include "tc_common.cuh"
+#include "ts.cuh"
 
 namespace bsp {
 
@@ -79,11 +72,11 @@ constexpr int kEpiWarps = 16;  // 4 TMEM lane quarters x 2 accumulators x 2 colu
 using tc::kLbo;
 using tc::kSbo;
 using tc::kLayoutSw128;
-constexpr int kFwd = 0, kTrans = 1, kSddmm = 2, kBatch = 3, kBatchT = 4, kBatchS = 5;
+constexpr int kSddmm = 2, kBatch = 3, kBatchT = 4, kBatchS = 5;
 // kBatch / kBatchT / kBatchS: the forward product, Aᵀ·G and the SDDMM of a
 // batch, CTA b running work item b with its problem's record
 __host__ __device__ constexpr bool batched_mode(int m) { return m == kBatch || m == kBatchT || m == kBatchS; }
-__host__ __device__ constexpr bool trans_mode(int m) { return m == kTrans || m == kBatchT; }
+__host__ __device__ constexpr bool trans_mode(int m) { return m == kBatchT; }
 __host__ __device__ constexpr bool sddmm_mode(int m) { return m == kSddmm || m == kBatchS; }
 // B (fwd) / G (trans) tile: four TMA boxes of 64 columns x 32 reduction rows,
 // 128-byte swizzle, kBox bytes apart (the LBO); 8-row groups 1 KB apart (SBO).
@@ -122,31 +115,19 @@ struct TcArgs {
   int64_t N;
   float* C;           // fwd: C [M][ldc]; trans: dX [K][ldc]; sddmm: dA [M][ldc]
   int64_t ldc;
-  const uint32_t* occ;  // fwd / trans occupancy bitmap (unused by sddmm)
-  int occ_words;
   int bdt;
-  // split-K (gridDim.z > 1): CTA z sums list slice z into part + z*part_stride
-  // (row stride ldp); a reduction kernel adds the slices into C
-  float* part;
-  int64_t ldp, part_stride;
-  // fwd / trans: B (or G) already in shared-memory order (k_tile_b), one
-  // 16 KB block per (32-row tile, 256-column block), bt_cb blocks per tile
-  // row; nullptr = B by TMA tensor boxes
-  const uint8_t* bt;
-  int64_t bt_cb;
   // batched form (kBatch): CTA b runs work item b of the batch
   const BatchProblemTc* bprobs;
-  // fwd / trans: A's words column by column ([Kw][M]) for coalesced loads, or null
-  const uint32_t* At;
   const int4* items;  // {problem, 256-row block, 256-column block, K tiles}
 };
 
-// One kernel, three products (MODE):
-//   kFwd   C[M,N]  = A · B        A bits K-major from A's words, B MN-major
-//   kTrans C[K,N]  = Aᵀ · G       Aᵀ MN-major built from A's row words (no
-//                                 transposed copy), G MN-major
-//   kSddmm dA[M,K] = (G · Xᵀ) ⊙ A  G and X K-major (TMA, 64-byte swizzle),
-//                                 dense over N, masked store
+// MODE:
+//   kSddmm   dA[M,K] = (G · Xᵀ) ⊙ A  G and X K-major (TMA, 128-byte swizzle),
+//                                    dense over N, masked store
+//   kBatch   C[M,N]  = A · B         A bits K-major from A's words, B MN-major
+//   kBatchT  C[K,N]  = Aᵀ · G        Aᵀ MN-major built from A's row words (no
+//                                    transposed copy), G MN-major
+//   kBatchS  the SDDMM per problem
 // The bit operands are expanded into core matrices (LBO = 128 B along the
 // reduction, SBO = 512 B along M/N); the dense 16-bit operands come by TMA
 // in swizzled layouts.  The modes differ only in the producers, the
@@ -167,7 +148,7 @@ __global__ void __launch_bounds__(tc_threads(TPS), 1) k_spmm_tc(TcArgs a, const 
   TcSmem& sm = *reinterpret_cast<TcSmem*>(
       smem_raw + ((kSmemAlign - (ptx::smem_addr(smem_raw) & (kSmemAlign - 1))) & (kSmemAlign - 1)));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  constexpr bool kFwdLike = MODE == kFwd || MODE == kBatch;
+  constexpr bool kFwdLike = MODE == kBatch;
   // the CTA's problem: the launch's (fwd / trans / sddmm) or its work item's (batch)
   const uint32_t* gA = a.A;
   int64_t gM = a.M, gK = a.K, gKw = a.Kw, gldc = a.ldc;
@@ -225,51 +206,6 @@ __global__ void __launch_bounds__(tc_threads(TPS), 1) k_spmm_tc(TcArgs a, const 
       sm.seen = ntot > 0 ? dense_halves : 0;
     }
   }
-  if ((MODE == kFwd || MODE == kTrans) && warp == 0) {
-    // List the occupied K tiles of the two 128-row blocks (ascending), with
-    // the halves that have bits in each; the launcher guarantees that the
-    // list fits (at most kListMax reduction tiles).
-    const int nblk = (int)((out_rows + kTcM - 1) / kTcM);
-    const uint32_t* occ0 = a.occ + (int64_t)blockIdx.x * kHalves * a.occ_words;
-    const bool has1 = (int)blockIdx.x * kHalves + 1 < nblk;
-    int n = 0;
-    for (int ow0 = 0; ow0 < a.occ_words; ow0 += 32) {
-      const int ow = ow0 + lane;
-      const uint32_t b0 = ow < a.occ_words ? __ldg(occ0 + ow) : 0u;
-      const uint32_t b1 = (has1 && ow < a.occ_words) ? __ldg(occ0 + a.occ_words + ow) : 0u;
-      uint32_t bits = b0 | b1;
-      const int c = __popc(bits);
-      int incl = c;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int y = __shfl_up_sync(kFull, incl, d);
-        if (lane >= d) incl += y;
-      }
-      int pos = n + incl - c;
-      while (bits) {
-        const int b = __ffs(bits) - 1;
-        bits &= bits - 1;
-        if (pos < kListMax)
-          sm.list[pos] = (ow * 32 + b) | (int)((((b0 >> b) & 1u) | (((b1 >> b) & 1u) << 1)) << 28);
-        pos++;
-      }
-      n += __shfl_sync(kFull, incl, 31);
-    }
-    // this CTA's slice of the list (all of it without split-K) and the
-    // halves that slice touches
-    __syncwarp();
-    const int ntot = min(n, kListMax);
-    const int lo = (int)((int64_t)ntot * blockIdx.z / gridDim.z);
-    const int hi = (int)((int64_t)ntot * (blockIdx.z + 1) / gridDim.z);
-    uint32_t hs = 0;
-    for (int k = lo + lane; k < hi; k += 32) hs |= ((uint32_t)sm.list[k] >> 28) & 3u;
-    hs = __reduce_or_sync(kFull, hs);
-    if (lane == 0) {
-      sm.lo = lo;
-      sm.nlist = hi - lo;
-      sm.seen = (int)hs;
-    }
-  }
   // SDDMM: a block of A without set bits needs no product at all
   if (kSd) {
     uint32_t acc = 0;
@@ -308,12 +244,12 @@ __global__ void __launch_bounds__(tc_threads(TPS), 1) k_spmm_tc(TcArgs a, const 
         if (kFwdLike) {
           const int64_t arow = row0 + r;
           if (arow >= gM) return 0u;
-          return (!kBat && a.At) ? __ldg(a.At + (int64_t)t * gM + arow) : __ldg(gA + arow * gKw + t);
+          return __ldg(gA + arow * gKw + t);
         }
         const int64_t arow = (int64_t)t * kTcK + (r & 31);
         const int64_t wcol = row0 / 32 + (r >> 5);
         if (arow >= gM || wcol >= gKw) return 0u;
-        return (!kBat && a.At) ? __ldg(a.At + wcol * gM + arow) : __ldg(gA + arow * gKw + wcol);
+        return __ldg(gA + arow * gKw + wcol);
       };
       uint32_t wq[kWordAhead];
 #pragma unroll
@@ -382,16 +318,6 @@ __global__ void __launch_bounds__(tc_threads(TPS), 1) k_spmm_tc(TcArgs a, const 
         const int k0 = kTilesPerStage * i;
         const int cnt = min(kTilesPerStage, n - k0);  // tiles in this stage
         ptx::mbar_arrive_expect_tx(&sm.full[s], cnt * nbox * kBox);
-        if (!kBat && a.bt) {
-          // tiled B: each tile's first nbox atoms are one contiguous copy
-#pragma unroll
-          for (int u = 0; u < kTilesPerStage; u++)
-            if (u < cnt)
-              ptx::bulk_g2s(sm.b + s * kStageBytes + u * kBTile,
-                            a.bt + ((int64_t)(lst[k0 + u] & 0x0fffffff) * a.bt_cb + blockIdx.y) * kBTile,
-                            nbox * kBox, &sm.full[s]);
-          continue;
-        }
 #pragma unroll
         for (int u = 0; u < kTilesPerStage; u++) {
           if (u >= cnt) break;
@@ -501,9 +427,8 @@ __global__ void __launch_bounds__(tc_threads(TPS), 1) k_spmm_tc(TcArgs a, const 
     const bool wlive = __all_sync(kFull, ok && !*(volatile int*)&sm.abort);
     const int64_t rbase = row0 + h * kTcM + q * 32;  // the warp's first row
     const int64_t row = rbase + lane;
-    const bool split = gridDim.z > 1;
-    float* cbase = split ? a.part + (int64_t)blockIdx.z * a.part_stride : gC;
-    const int64_t cld = split ? a.ldp : gldc;
+    float* cbase = gC;
+    const int64_t cld = gldc;
     const int cspan = nbox * (kBoxCols / 2);      // live columns per column half (a multiple of 32)
     const int64_t ccol = col0 + cg * cspan;         // the warp's first column
     const bool live = row < out_rows && wlive;
@@ -584,11 +509,17 @@ __global__ void __launch_bounds__(tc_threads(TPS), 1) k_spmm_tc(TcArgs a, const 
 // of 4 KB; in atom j, row r occupies 128 bytes whose 16-byte chunk c sits at
 // position c ^ (r % 8) (the 128-byte swizzle, as a TMA load into a
 // 1024-byte aligned stage writes it).  Rows past R and columns past N are
-// zero.  One thread per 16-byte chunk: a warp reads 512 contiguous bytes of
-// one row and writes four 128-byte runs.
+// zero.
+// One thread per 16-byte chunk: a warp reads 512 contiguous bytes of one row
+// and writes four 128-byte runs.  VEC: B's rows take 16-byte loads; otherwise
+// the elements are read one by one, and `flag` is set if any of them is an
+// infinity or a NaN (exp_mask: the type's exponent bits).
+template <bool VEC>
 __global__ void __launch_bounds__(256) k_tile_b(const uint8_t* __restrict__ B, int64_t R, int64_t N, int64_t ldb,
-                                                int64_t ntiles, int64_t ncb, uint4* __restrict__ bt) {
+                                                int64_t ntiles, int64_t ncb, uint4* __restrict__ bt, uint32_t exp_mask,
+                                                int* flag) {
   const int64_t total = ntiles * ncb * (kBTile / 16);
+  bool bad = false;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t blk = e >> 10;
     const int in = (int)(e & 1023);
@@ -596,9 +527,21 @@ __global__ void __launch_bounds__(256) k_tile_b(const uint8_t* __restrict__ B, i
     const int64_t t = blk / ncb, cb = blk - t * ncb;
     const int64_t row = t * kTcK + r, col = cb * kTcN + j * kBoxCols + c * 8;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (row < R && col < N) v = __ldg(reinterpret_cast<const uint4*>(B + (row * ldb + col) * 2));
+    if (VEC) {
+      if (row < R && col < N) v = __ldg(reinterpret_cast<const uint4*>(B + (row * ldb + col) * 2));
+    } else if (row < R && col < N) {
+      const uint16_t* p = reinterpret_cast<const uint16_t*>(B) + row * ldb + col;
+      uint32_t w[8];
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        w[i] = col + i < N ? (uint32_t)__ldg(p + i) : 0u;
+        bad |= (w[i] & exp_mask) == exp_mask;
+      }
+      v = make_uint4(w[0] | (w[1] << 16), w[2] | (w[3] << 16), w[4] | (w[5] << 16), w[6] | (w[7] << 16));
+    }
     bt[blk * 1024 + j * 256 + r * 8 + (c ^ (r & 7))] = v;
   }
+  if (!VEC && bad) *flag = 1;
 }
 
 // Both occupancy bitmaps in one pass over A's words.  A block of 4 warps
@@ -650,7 +593,8 @@ int64_t tc_max_reduction() { return (int64_t)kListMax * kTcK; }
 int tc_occupancy_t_words(int64_t M) { return (int)ceil_div(ceil_div(M, 32), 32); }
 
 // words [M][Kw] -> At [Kw][M] through 32x32 shared-memory tiles (coalesced
-// on both sides).
+// on both sides), every word unshuffled (tc_common.cuh), as the persistent
+// kernel's producers take it.
 __global__ void __launch_bounds__(256) k_transpose_words(const uint32_t* __restrict__ w, int64_t M, int64_t Kw,
                                                          uint32_t* __restrict__ At) {
   __shared__ uint32_t tile[32][33];
@@ -663,7 +607,7 @@ __global__ void __launch_bounds__(256) k_transpose_words(const uint32_t* __restr
   __syncthreads();
   for (int k = ty; k < 32; k += 8) {
     const int64_t c = c0 + k, r = r0 + tx;
-    if (c < Kw && r < M) At[c * M + r] = tile[tx][k];
+    if (c < Kw && r < M) At[c * M + r] = tc::unshuffle32(tile[tx][k]);
   }
 }
 
@@ -743,11 +687,11 @@ int launch_mode(const TcArgs& a, const CUtensorMap& ma, const CUtensorMap& mb, d
 }
 
 // C = Σ_z part[z] in ascending z (deterministic), four columns per thread
-// (the tensor-core path needs N % 8 == 0 and 16-byte aligned C rows).
+// (part's rows are a multiple of four floats; c_vec: C's take 16-byte stores).
 __global__ void __launch_bounds__(256) k_split_reduce(const float* __restrict__ part, int64_t ldp, int64_t stride,
                                                       int splits, int64_t rows, int64_t cols, float* __restrict__ C,
-                                                      int64_t ldc) {
-  const int64_t q = cols / 4, total = rows * q;
+                                                      int64_t ldc, bool c_vec) {
+  const int64_t q = (cols + 3) / 4, total = rows * q;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = e / q, c = (e - r * q) * 4;
     float4 acc = __ldg(reinterpret_cast<const float4*>(part + r * ldp + c));
@@ -758,18 +702,26 @@ __global__ void __launch_bounds__(256) k_split_reduce(const float* __restrict__ 
       acc.z += v.z;
       acc.w += v.w;
     }
-    *reinterpret_cast<float4*>(C + r * ldc + c) = acc;
+    float* o = C + r * ldc + c;
+    if (c_vec) {
+      *reinterpret_cast<float4*>(o) = acc;
+    } else {
+      o[0] = acc.x;
+      if (c + 1 < cols) o[1] = acc.y;
+      if (c + 2 < cols) o[2] = acc.z;
+      if (c + 3 < cols) o[3] = acc.w;
+    }
   }
 }
 
 }  // namespace
 
-// Split-K for the tensor-core products: when the output has fewer CTA tiles
+// Split-K for the tensor-core products: when the output has fewer items
 // than half the SMs, the reduction (list of occupied tiles) is cut into S
 // slices, up to 8 and at least 16 reduction tiles each, so that about one CTA
 // per SM runs; every slice's FP32 partial needs rows x round4(cols) floats.
 int tc_split_count(int64_t out_rows, int64_t out_cols, int64_t red_tiles) {
-  const int64_t tiles = ceil_div(out_rows, kCtaM) * ceil_div(out_cols, kTcN);
+  const int64_t tiles = ceil_div(out_rows, ts_item_rows()) * ceil_div(out_cols, ts_item_cols());
   const int64_t sms = num_sms();
   if (tiles == 0 || tiles * 2 > sms) return 1;
   int64_t S = sms / tiles;
@@ -785,34 +737,24 @@ size_t tc_split_bytes(int64_t out_rows, int64_t out_cols, int64_t red_tiles) {
 
 // B (or G) in tile order: every (32-row tile, 256-column block) is 16 KB.
 size_t tc_tiled_b_bytes(int64_t red_rows, int64_t cols) {
-  return (size_t)ceil_div(red_rows, kTcK) * (size_t)ceil_div(cols, kTcN) * kBTile + 1024;
+  return (size_t)ceil_div(red_rows, kTcK) * (size_t)ceil_div(cols, kTcN) * kBTile + 2048;
 }
 
 // Tiling B costs a read and a write of it; it pays where many row blocks
-// read every B tile (measured on GB300: 16384 rows, 64 blocks, 0.84 -> 0.80
-// ms; 4096 rows, 16 blocks, forward + backward 0.76 -> 0.79 ms).
-constexpr int64_t kTiledMinRowBlocks = 32;
+// read every B tile.  Copy included, against boxes: 64 row blocks
+// (16384x16384x2048) 556 and 652 us, 32 (8192x8192x512) 52 and 58, 16
+// (4096x4096x8192) 180 and 186, 8 (2048x2048x1024) 20.3 and 18.6, 4 13.8 and
+// 12.5.
+constexpr int64_t kTiledMinRowBlocks = 16;
 
-bool tc_tiles_b(int64_t out_rows) { return ceil_div(out_rows, kCtaM) >= kTiledMinRowBlocks; }
+bool tc_tiles_b(int64_t out_rows) { return ceil_div(out_rows, ts_item_rows()) >= kTiledMinRowBlocks; }
 
 size_t tc_preferred_bytes(int64_t out_rows, int64_t out_cols, int64_t red_rows) {
   return tc_split_bytes(out_rows, out_cols, ceil_div(red_rows, kTcK)) +
-         (tc_tiles_b(out_rows) ? tc_tiled_b_bytes(red_rows, out_cols) : 0);
+         (tc_tiles_b(out_rows) || out_cols % 8 != 0 ? tc_tiled_b_bytes(red_rows, out_cols) : 0);
 }
 
 namespace {
-
-// Three K tiles per stage (two stages) where the output has this many row
-// blocks; BSP_TC_TPS=2 or 3 forces one form.
-constexpr int64_t kThreeTileMinRowBlocks = 32;
-bool three_tiles(int64_t out_rows) {
-  static const int force = [] {
-    const char* e = getenv("BSP_TC_TPS");
-    return e && *e ? atoi(e) : 0;
-  }();
-  if (force == 2 || force == 3) return force == 3;
-  return ceil_div(out_rows, kCtaM) >= kThreeTileMinRowBlocks;
-}
 
 // BSP_TC_TILED_B=0 keeps B on tensor boxes even with room for the tiled copy.
 bool tiled_b_enabled() {
@@ -823,116 +765,111 @@ bool tiled_b_enabled() {
   return on;
 }
 
-template <int MODE>
-int launch_tc(TcArgs a, cudaStream_t s, void* ws = nullptr, size_t ws_bytes = 0, TcForm form = TcForm{}) {
-  const int64_t rows = MODE == kTrans ? a.K : a.M;
-  const int64_t cols = MODE == kSddmm ? a.K : a.N;
+// C = A·B (trans: dX = Aᵀ·G) on the persistent kernel: split-K and B in tile
+// order as far as the workspace goes.
+int launch_product(TsArgs a, const void* B, int64_t ldb, bool vec, bool trans, cudaStream_t s, void* ws,
+                   size_t ws_bytes, TcForm form, const int** skipped) {
+  const int64_t rows = trans ? a.K : a.M, cols = a.N, red_rows = trans ? a.M : a.K;
   if (rows == 0 || cols == 0) return BSP_OK;
+  if (a.bdt != BSP_BF16 && a.bdt != BSP_F16) return BSP_ERR_UNSUPPORTED;
+  if (a.N > INT32_MAX || a.M > INT32_MAX || a.K > INT32_MAX) return BSP_ERR_CAPACITY;
+  // an item's tile list holds every reduction tile (fwd: K, trans: M)
+  if (ceil_div(red_rows, kTcK) > kListMax) return BSP_ERR_CAPACITY;
+  const size_t tiled_bytes = tc_tiled_b_bytes(red_rows, cols);
+  if (!vec && (!ws || ws_bytes < tiled_bytes)) return BSP_ERR_WORKSPACE;
   int splits = 1;
   size_t used = 0;
-  if (MODE != kSddmm && ws && form.split != 0) {
-    const int64_t red_tiles = ceil_div(MODE == kFwd ? a.K : a.M, kTcK);
+  if (ws && form.split != 0) {
+    const int64_t red_tiles = ceil_div(red_rows, kTcK);
     const int S = tc_split_count(rows, cols, red_tiles);
-    if (S > 1 && ws_bytes >= tc_split_bytes(rows, cols, red_tiles)) {
+    const size_t bytes = tc_split_bytes(rows, cols, red_tiles);
+    if (S > 1 && ws_bytes >= bytes + (vec ? 0 : tiled_bytes)) {
       splits = S;
       a.part = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(ws) + 255) & ~(uintptr_t)255);
       a.ldp = ceil_div(cols, 4) * 4;
       a.part_stride = rows * a.ldp;
-      used = tc_split_bytes(rows, cols, red_tiles);
+      used = bytes;
     }
   }
   // B in tile order when the rest of the workspace holds it (else tensor boxes)
-  const int64_t red_rows = MODE == kFwd ? a.K : a.M;
-  const bool room = MODE != kSddmm && ws && ws_bytes >= used + tc_tiled_b_bytes(red_rows, cols);
-  const bool tiled = room && (form.tiled >= 0 ? form.tiled == 1 : tc_tiles_b(rows) && tiled_b_enabled());
-  const dim3 grid((unsigned)ceil_div(rows, kCtaM), (unsigned)ceil_div(cols, kTcN), (unsigned)splits);
-  if (ceil_div(cols, kTcN) > 65535 || ceil_div(rows, kCtaM) > 0x7fffffff) return BSP_ERR_CAPACITY;
-  if (a.N > INT32_MAX || a.M > INT32_MAX || a.K > INT32_MAX) return BSP_ERR_CAPACITY;
-  // the tile list of a CTA holds every reduction tile (fwd: K, trans: M)
-  if (MODE != kSddmm && ceil_div(MODE == kFwd ? a.K : a.M, kTcK) > kListMax) return BSP_ERR_CAPACITY;
-  CUtensorMap ma, mb;
-  memset(&ma, 0, sizeof(ma));
-  if (MODE == kSddmm) {
-    BSP_TRY(make_map(&ma, a.G, a.bdt, a.M, a.N, a.ldg, kSdK, kCtaM, CU_TENSOR_MAP_SWIZZLE_128B));  // G [M][N]
-    BSP_TRY(make_map(&mb, a.B, a.bdt, a.K, a.N, a.ldb, kSdK, kTcN, CU_TENSOR_MAP_SWIZZLE_128B));   // X [K][N]
-  } else {
-    // B [K][N] (fwd) or G [M][N] (trans), 64 columns x 32 reduction rows per box
-    BSP_TRY(make_map(&mb, a.B, a.bdt, MODE == kFwd ? a.K : a.M, a.N, a.ldb, kBoxCols, kTcK,
-                     CU_TENSOR_MAP_SWIZZLE_128B));
-  }
+  const bool room = ws && ws_bytes >= used + tiled_bytes;
+  const bool tiled = !vec || (room && (form.tiled >= 0 ? form.tiled == 1 : tc_tiles_b(rows) && tiled_b_enabled()));
+  CUtensorMap map;
+  memset(&map, 0, sizeof(map));
   if (tiled) {
+    // the blocks of tile order, behind a head that holds the flag
     const int64_t ntiles = ceil_div(red_rows, kTcK), ncb = ceil_div(cols, kTcN);
     uint8_t* bt = reinterpret_cast<uint8_t*>(
-        (reinterpret_cast<uintptr_t>(static_cast<char*>(ws) + used) + 1023) & ~(uintptr_t)1023);
+        (reinterpret_cast<uintptr_t>(static_cast<char*>(ws) + used) + 256 + 1023) & ~(uintptr_t)1023);
+    int* flag = reinterpret_cast<int*>(bt - 256);
     const int64_t work = ntiles * ncb * (kBTile / 16);
     const int64_t cap = (int64_t)num_sms() * 16;
-    k_tile_b<<<(unsigned)(ceil_div(work, 256) < cap ? ceil_div(work, 256) : cap), 256, 0, s>>>(
-        static_cast<const uint8_t*>(a.B), red_rows, cols, a.ldb, ntiles, ncb, reinterpret_cast<uint4*>(bt));
+    const unsigned grid = (unsigned)(ceil_div(work, 256) < cap ? ceil_div(work, 256) : cap);
+    if (vec) {
+      k_tile_b<true><<<grid, 256, 0, s>>>(static_cast<const uint8_t*>(B), red_rows, cols, ldb, ntiles, ncb,
+                                          reinterpret_cast<uint4*>(bt), 0u, nullptr);
+    } else {
+      BSP_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), s));
+      k_tile_b<false><<<grid, 256, 0, s>>>(static_cast<const uint8_t*>(B), red_rows, cols, ldb, ntiles, ncb,
+                                           reinterpret_cast<uint4*>(bt), a.bdt == BSP_BF16 ? 0x7f80u : 0x7c00u, flag);
+      a.skip_if = flag;
+      *skipped = flag;
+    }
     BSP_LAUNCHED();
     a.bt = bt;
     a.bt_cb = ncb;
+  } else {
+    // B [K][N] (fwd) or G [M][N] (trans), 64 columns x 32 reduction rows per box
+    BSP_TRY(make_map(&map, B, a.bdt, red_rows, a.N, ldb, kBoxCols, kTcK, CU_TENSOR_MAP_SWIZZLE_128B));
   }
-  if (a.bdt != BSP_BF16 && a.bdt != BSP_F16) return BSP_ERR_UNSUPPORTED;
-  bool launched = false;
-  if constexpr (MODE != kSddmm) {  // (the SDDMM has one stage form)
-    if (form.tps ? form.tps == 3 : three_tiles(rows)) {
-      if (a.bdt == BSP_BF16) BSP_TRY((launch_mode<__nv_bfloat16, MODE, 3>(a, ma, mb, grid, s)));
-      else BSP_TRY((launch_mode<__half, MODE, 3>(a, ma, mb, grid, s)));
-      launched = true;
-    }
-  }
-  if (!launched) {
-    if (a.bdt == BSP_BF16) BSP_TRY((launch_mode<__nv_bfloat16, MODE, 2>(a, ma, mb, grid, s)));
-    else BSP_TRY((launch_mode<__half, MODE, 2>(a, ma, mb, grid, s)));
-  }
+  BSP_TRY(launch_ts(a, map, trans, splits, s));
   if (splits > 1) {
-    const int64_t work = rows * (cols / 4);
+    const int64_t work = rows * ceil_div(cols, 4);
     const int64_t cap = (int64_t)num_sms() * 8;
     k_split_reduce<<<(unsigned)(ceil_div(work, 256) < cap ? ceil_div(work, 256) : cap), 256, 0, s>>>(
-        a.part, a.ldp, a.part_stride, splits, rows, cols, a.C, a.ldc);
+        a.part, a.ldp, a.part_stride, splits, rows, cols, a.C, a.ldc, a.c_vec);
     BSP_LAUNCHED();
   }
   return BSP_OK;
 }
 }  // namespace
 
-int launch_spmm_tc(const SpmmArgs& sa, const uint32_t* occ, const uint32_t* At, cudaStream_t s, void* ws,
-                   size_t ws_bytes, TcForm form) {
-  TcArgs a = {};
+int launch_spmm_tc(const SpmmArgs& sa, const uint32_t* occ, const uint32_t* At, bool vec, cudaStream_t s, void* ws,
+                   size_t ws_bytes, TcForm form, const int** skipped) {
+  TsArgs a = {};
   a.At = At;
   a.A = sa.A;
   a.M = sa.M;
   a.K = sa.K;
   a.Kw = sa.Kw;
-  a.B = sa.B;
-  a.ldb = sa.ldb;
   a.N = sa.N;
   a.C = sa.C;
   a.ldc = sa.ldc;
+  a.c_vec = sa.c_vec;
   a.occ = occ;
   a.occ_words = tc_occupancy_words(sa.K);
   a.bdt = sa.bdt;
-  return launch_tc<kFwd>(a, s, ws, ws_bytes, form);
+  return launch_product(a, sa.B, sa.ldb, vec, false, s, ws, ws_bytes, form, skipped);
 }
 
 int launch_spmm_t_tc(const uint32_t* A, int64_t M, int64_t K, const void* G, int gdt, int64_t ldg, int64_t N,
                      float* dX, int64_t lddx, const uint32_t* occT, const uint32_t* At, cudaStream_t s, void* ws,
                      size_t ws_bytes) {
-  TcArgs a = {};
+  TsArgs a = {};
   a.At = At;
   a.A = A;
   a.M = M;
   a.K = K;
   a.Kw = ceil_div(K, 32);
-  a.B = G;
-  a.ldb = ldg;
   a.N = N;
   a.C = dX;
   a.ldc = lddx;
+  a.c_vec = is_aligned(dX, 16) && lddx % 4 == 0 && N % 4 == 0;
   a.occ = occT;
   a.occ_words = tc_occupancy_t_words(M);
   a.bdt = gdt;
-  return launch_tc<kTrans>(a, s, ws, ws_bytes);
+  const int* skipped = nullptr;  // (only vector layouts come here)
+  return launch_product(a, G, ldg, true, true, s, ws, ws_bytes, TcForm{}, &skipped);
 }
 
 int launch_sddmm_tc(const uint32_t* A, int64_t M, int64_t K, const void* G, int64_t ldg, const void* X,
@@ -950,7 +887,16 @@ int launch_sddmm_tc(const uint32_t* A, int64_t M, int64_t K, const void* G, int6
   a.C = dA;
   a.ldc = ldda;
   a.bdt = dt;
-  return launch_tc<kSddmm>(a, s);
+  if (M == 0 || K == 0) return BSP_OK;
+  if (dt != BSP_BF16 && dt != BSP_F16) return BSP_ERR_UNSUPPORTED;
+  const dim3 grid((unsigned)ceil_div(M, kCtaM), (unsigned)ceil_div(K, kTcN));
+  if (ceil_div(K, kTcN) > 65535 || ceil_div(M, kCtaM) > 0x7fffffff) return BSP_ERR_CAPACITY;
+  if (N > INT32_MAX || M > INT32_MAX || K > INT32_MAX) return BSP_ERR_CAPACITY;
+  CUtensorMap ma, mb;
+  BSP_TRY(make_map(&ma, G, dt, M, N, ldg, kSdK, kCtaM, CU_TENSOR_MAP_SWIZZLE_128B));  // G [M][N]
+  BSP_TRY(make_map(&mb, X, dt, K, N, ldx, kSdK, kTcN, CU_TENSOR_MAP_SWIZZLE_128B));   // X [K][N]
+  return dt == BSP_BF16 ? launch_mode<__nv_bfloat16, kSddmm, 2>(a, ma, mb, grid, s)
+                        : launch_mode<__half, kSddmm, 2>(a, ma, mb, grid, s);
 }
 
 int make_batch_map(CUtensorMap* m, const void* B, int bdt, int64_t K, int64_t N, int64_t ldb) {

@@ -1,0 +1,35 @@
+// ts.cuh — the persistent tensor-core kernel's launcher (spmm_ts.cu).
+#pragma once
+#include <cuda.h>
+
+#include "bsp_internal.cuh"
+
+namespace bsp {
+
+struct TsArgs {
+  const uint32_t* A;   // packed rows [M][Kw]
+  const uint32_t* At;  // A's words column by column ([Kw][M], launch_transpose_words), or null
+  int64_t M, K, Kw;
+  int64_t N;
+  float* C;            // [M][ldc]; trans: dX [K][ldc]
+  int64_t ldc;
+  bool c_vec;          // C's rows take 16-byte stores
+  const uint32_t* occ; // occupancy bitmap of 128-row blocks (trans: of 128-column blocks)
+  int occ_words;
+  int bdt;
+  // split-K: slice z of an item's tile list goes to part + z*part_stride (row stride ldp)
+  float* part;
+  int64_t ldp, part_stride;
+  // B (or G) in tile order, bt_cb blocks of 256 columns per 32-row tile; null = TMA boxes through the map
+  const uint8_t* bt;
+  int64_t bt_cb;
+  const int* skip_if;  // device flag: nonzero = leave C alone; null = run
+};
+
+// rows and columns of the output per work item
+int64_t ts_item_rows();
+int64_t ts_item_cols();
+int launch_ts(const TsArgs& a, const CUtensorMap& map, bool trans, int splits, cudaStream_t s);
+int ts_device_error(int* out, bool clear);
+
+}  // namespace bsp

@@ -178,6 +178,57 @@ def _t_workspaces(M, K, N):
 
 
 @pytest.mark.parametrize("kind", ["bf16", "f16"])
+@pytest.mark.parametrize("M,K,N", [(1, 32, 8), (127, 31, 64), (128, 33, 72), (129, 96, 128), (256, 128, 136),
+                                   (257, 160, 192), (385, 300, 264), (5000, 200, 1500), (200, 5000, 1500)])
+def test_tc_items_and_stages(force_tc, kind, M, K, N):
+    """Edges of the 256x128 items and of the stages of four K tiles, empty
+    tiles and halves, one item and many per CTA: exact on integers, both ways."""
+    rng = np.random.default_rng(M + K + N)
+    bits = rng.random((M, K)) < 0.2
+    bits[128:256] = False          # a half without bits
+    bits[:, 32:64] = False         # a K tile without bits
+    bits[: M // 2, K // 2:] = False
+    words = W.pack_bits(bits)
+    wd = words_dev(words)
+    plan = ops.Plan(wd, K)
+    Bi, Bie = _b16(rng.integers(-8, 9, (K, N)).astype(np.float32), kind)
+    C = ops.spmm(wd, K, Bi, plan=plan).cpu().numpy()
+    assert np.array_equal(C.astype(np.float64), O.spmm_f64(words, K, Bie))
+    Gi, Gie = _b16(rng.integers(-8, 9, (M, N)).astype(np.float32), kind)
+    dX = ops.spmm_t(wd, M, K, Gi, plan=plan).cpu().numpy()
+    assert np.array_equal(dX.astype(np.float64), O.spmm_t_f64(words, M, K, Gie))
+    assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("kind", ["bf16", "f16"])
+@pytest.mark.parametrize("M,K,N", [(300, 200, 1), (700, 3000, 133), (600, 4000, 500), (128, 8192, 129)])
+def test_tc_unaligned_columns(force_tc, kind, M, K, N):
+    """Widths without 16-byte rows go through tile order (with and without
+    split-K); nothing is written past N, and a value that is not finite
+    reaches only the rows that hold its column."""
+    rng = np.random.default_rng(M + K + N)
+    bits = rng.random((M, K)) < 0.3
+    words = W.pack_bits(bits)
+    wd = words_dev(words)
+    plan = ops.Plan(wd, K)
+    Bi, Bie = _b16(rng.integers(-8, 9, (K, N)).astype(np.float32), kind)
+    ref = O.spmm_f64(words, K, Bie)
+    out = torch.full((M, N + 3), 7.0, device="cuda")
+    ops.spmm(wd, K, Bi, plan=plan, out=out[:, :N])
+    assert np.array_equal(out[:, :N].cpu().numpy().astype(np.float64), ref)
+    assert torch.all(out[:, N:] == 7.0)
+    for bad in (float("inf"), float("nan")):
+        B = Bi.clone()
+        B[5, N // 2] = bad
+        C = ops.spmm(wd, K, B, plan=plan).cpu().numpy()
+        hit = np.zeros((M, N), dtype=bool)
+        hit[bits[:, 5], N // 2] = True
+        assert np.array_equal(~np.isfinite(C), hit)
+        assert np.array_equal(C[~hit].astype(np.float64), ref[~hit])
+    assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("kind", ["bf16", "f16"])
 @pytest.mark.parametrize("M,K,N,p", [(8200, 1000, 264, 0.05), (8448, 3000, 64, 0.01)])
 def test_three_tile_stages(force_tc, kind, M, K, N, p):
     # 32+ row blocks: stages of three K tiles (two stages in flight); list
