@@ -288,15 +288,20 @@ static size_t align_b_bytes(int64_t K, int64_t N, int esz) {
 // B in a layout that 16-byte loads can read, copied behind the first `used`
 // bytes of the workspace if it is not one already; false where there is no
 // room.  The single-element kernels gather at 3.5 TB/s, the vector ones at
-// 17, so a copy of K rows (read and written once) pays from about 1.8 set bits
-// per column on: taken as 64 rows where the set bits are not known
-// (2000x3001x333 FP32 at 5 %: 116 us without the copy, 41 with it, 3.5 of them for the copy).
+// 17; the copy and its launch cost 8 us of a small call (50x184x9 BF16: 11.5
+// and 19 us), so it is made where the gathers alone would take that long, 27
+// MB (5 % of the matrix where the set bits are not known; 2000x3001x333 FP32
+// at 5 %: 116 us without the copy, 41 with it, 3.5 of them for the copy).
+static bool align_pays(const bsp_plan* plan, int64_t M, int64_t K, int64_t N, int esz) {
+  const double bits = plan ? (double)plan->nnz : 0.05 * (double)M * (double)K;
+  return bits * (double)N * (double)esz >= 27e6 && bits >= 2.0 * (double)K;
+}
 static bool align_operands(SpmmArgs* a, const bsp_plan* plan, void* workspace, size_t bytes, size_t used,
                            cudaStream_t s) {
   const int esz = dtype_size(a->bdt);
   if (is_aligned(a->B, 16) && (a->ldb * esz) % 16 == 0 && (a->N * esz) % 16 == 0) return true;  // C alone is not
   if (!workspace || bytes < used + align_b_bytes(a->K, a->N, esz)) return false;
-  if (plan ? plan->nnz < 2 * plan->K : a->M < 64) return false;
+  if (!align_pays(plan, a->M, a->K, a->N, esz)) return false;
   void* out = reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(workspace) + used + 255) & ~uintptr_t(255));
   const int64_t Nb = align_cols(a->N, esz);
   if (launch_align_b(a->B, a->bdt, a->K, a->N, a->ldb, out, Nb, s) != BSP_OK) return false;

@@ -69,6 +69,10 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
   return false;
 }
 
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
 // Named barrier `id` (1..15) of `threads` threads, whole warps.
 __device__ __forceinline__ void bar_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
@@ -99,13 +103,8 @@ __device__ __forceinline__ void bulk_g2s_u32(uint32_t dst_smem, const void* src_
       : "memory");
 }
 
-// Bulk copy shared -> global (multiples of 16 bytes) in this thread's current
-// bulk group; wait until the groups' reads of shared memory, or all of them, are done.
-__device__ __forceinline__ void bulk_s2g(void* dst_gmem, const void* src_smem, uint32_t bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst_gmem), "r"(smem_addr(src_smem)),
-               "r"(bytes)
-               : "memory");
-}
+// Close this thread's current bulk group of stores; wait until the groups'
+// reads of shared memory, or all of them, are done.
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
@@ -277,6 +276,14 @@ __device__ __forceinline__ void tma_load_2d(void* dst_smem, const void* map, int
           smem_addr(dst_smem)),
       "l"(map), "r"(x), "r"(y), "r"(smem_addr(bar))
       : "memory");
+}
+
+// 3-D TMA tensor copy shared -> global of one box, in this thread's current
+// bulk group; what lies past the tensor is not written.
+__device__ __forceinline__ void tma_store_3d(const void* map, int x, int y, int z, const void* src_smem) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(map), "r"(x),
+               "r"(y), "r"(z), "r"(smem_addr(src_smem))
+               : "memory");
 }
 
 // Acquire a tensor map that was written through the generic proxy (here: by

@@ -11,7 +11,7 @@ namespace bsp {
 // and C.
 struct BatchProblemTc {
   CUtensorMap map;   // forward: B [K][N]; Aᵀ·G: G [M][N] (64x32 boxes); SDDMM: G [M][N] (64x256 boxes)
-  CUtensorMap map2;  // SDDMM: X [K][N] (64x256 boxes); otherwise unused
+  CUtensorMap map2;  // SDDMM: X [K][N] (64x256 boxes); forward, Aᵀ·G: C, dX (make_out_map)
   CUtensorMap map3;  // SDDMM: G [M][N] in 64x128 boxes (the persistent batched SDDMM); otherwise unused
   const uint32_t* A;
   int64_t M, K, Kw;
@@ -25,6 +25,10 @@ int make_batch_map(CUtensorMap* m, const void* B, int bdt, int64_t K, int64_t N,
 // 256-row boxes.
 int make_batch_map_sddmm(CUtensorMap* m, const void* T, int bdt, int64_t rows, int64_t N, int64_t ld,
                          int box_rows = 256);
+// Tensor map of an FP32 output [rows][cols] (row stride ld floats, 16-byte
+// aligned), `splits` of them split_stride floats apart: 32x32 boxes, 128-byte
+// swizzle.
+int make_out_map(CUtensorMap* m, float* C, int64_t rows, int64_t cols, int64_t ld, int splits, int64_t split_stride);
 // Work item b = {problem, 256-row block, 256-column block, reduction tiles}:
 // one CTA each.  kind 0 = forward C = A·B, 1 = dX = Aᵀ·G (rows: K),
 // 2 = dA = (G·Xᵀ) ⊙ A (columns: K).

@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(tc_threads(TPS), 1) k_spmm_tc(TcArgs a, const 
   // column tile loads, multiplies and stores only those (MMA N = 64·nbox)
   const int nbox = kSd ? kTcN / kBoxCols
                                   : (int)min((int64_t)(kTcN / kBoxCols), (out_cols - col0 + kBoxCols - 1) / kBoxCols);
-  const int dense_halves = row0 + kTcM < out_rows ? 3 : 1;
+  const int dense_halves = __any_sync(kFull, row0 + kTcM < out_rows) ? 3 : 1;
 
   if (tid == 0) {
     for (int s = 0; s < kStages; s++) {
@@ -223,8 +223,8 @@ __global__ void __launch_bounds__(tc_threads(TPS), 1) k_spmm_tc(TcArgs a, const 
   ptx::tc_fence_before_sync();
   __syncthreads();
   ptx::tc_fence_after_sync();
-  const uint32_t tmem = sm.tmem_addr;
-  const int n = sm.nlist;
+  const uint32_t tmem = __reduce_max_sync(kFull, sm.tmem_addr);  // (uniform to the compiler, as is n)
+  const int n = __reduce_max_sync(kFull, sm.nlist);
   const int* lst = sm.list + sm.lo;  // this CTA's occupied tiles (fwd / trans)
   // stage i: list entries 2i and 2i+1 (fwd / trans) or N columns [64i, 64i+64) (SDDMM)
   const int nstages = kSd ? n : (n + kTilesPerStage - 1) / kTilesPerStage;
@@ -292,47 +292,60 @@ __global__ void __launch_bounds__(tc_threads(TPS), 1) k_spmm_tc(TcArgs a, const 
         wq[kWordAhead - 1] = wnew;
       }
     }
-  } else if (warp == kTmaWarp && lane == 0) {
+  } else if (warp == kTmaWarp) {
     // ---------------- TMA issuer ----------------
-    // Shared-memory addresses are formed once; a stage adds its offset.
+    // (this warp and the next run whole, with one elected lane to issue: see
+    // ptx::mbar_wait_warp)
+    const bool leader = ptx::elect_one();
     const uint32_t a0 = ptx::smem_addr(sm.a), b0 = ptx::smem_addr(sm.b), f0 = ptx::smem_addr(&sm.full[0]);
-    if (kBat) {  // written by the host into global memory
+    if (kBat && leader) {  // written by the host into global memory
       ptx::tensormap_acquire(bmap);
       if (kSd) ptx::tensormap_acquire(amap);
     }
+    __syncwarp();
+    uint32_t s = 0, ph = 1;  // stage, and the parity its emptying completes (the first round passes at once)
     for (int i = 0; i < nstages; i++) {
-      const int s = i % kStages;
-      if (i >= kStages && !ptx::mbar_wait(&sm.empty[s], ((i / kStages) - 1) & 1)) {
-        atomicCAS(&g_tc_error, 0, 3);
-        sm.abort = 1;
+      if (!ptx::mbar_wait_warp(&sm.empty[s], ph)) {
+        if (leader) {
+          atomicCAS(&g_tc_error, 0, 3);
+          sm.abort = 1;
+        }
         break;
       }
-      const uint32_t fb = f0 + s * 8, as = a0 + s * kStageBytes, bs = b0 + s * kStageBytes;
-      if (kSd) {
-        // G rows row0.. and X rows col0.. (256 each), N columns i*64..
-        ptx::mbar_arrive_expect_tx(&sm.full[s], 2 * kSdTile);
-        ptx::tma_load_2d_u32(as, amap, i * kSdK, (int)row0, fb);
-        ptx::tma_load_2d_u32(bs, bmap, i * kSdK, (int)col0, fb);
-      } else {
-        // B (fwd) / G (trans) rows t*32.. of the stage's tiles, columns col0 + 64*j
-        const int k0 = kTilesPerStage * i;
-        const int cnt = min(kTilesPerStage, n - k0);  // tiles in this stage
-        ptx::mbar_arrive_expect_tx(&sm.full[s], cnt * nbox * kBox);
+      if (leader) {
+        const uint32_t fb = f0 + s * 8, as = a0 + s * kStageBytes, bs = b0 + s * kStageBytes;
+        if (kSd) {
+          // G rows row0.. and X rows col0.. (256 each), N columns i*64..
+          ptx::mbar_arrive_expect_tx(&sm.full[s], 2 * kSdTile);
+          ptx::tma_load_2d_u32(as, amap, i * kSdK, (int)row0, fb);
+          ptx::tma_load_2d_u32(bs, bmap, i * kSdK, (int)col0, fb);
+        } else {
+          // B (fwd) / G (trans) rows t*32.. of the stage's tiles, columns col0 + 64*j
+          const int k0 = kTilesPerStage * i;
+          const int cnt = min(kTilesPerStage, n - k0);  // tiles in this stage
+          ptx::mbar_arrive_expect_tx(&sm.full[s], cnt * nbox * kBox);
 #pragma unroll
-        for (int u = 0; u < kTilesPerStage; u++) {
-          if (u >= cnt) break;
-          const int t = lst[k0 + u] & 0x0fffffff;
+          for (int u = 0; u < kTilesPerStage; u++) {
+            if (u >= cnt) break;
+            const int t = lst[k0 + u] & 0x0fffffff;
 #pragma unroll
-          for (int j = 0; j < kTcN / kBoxCols; j++)
-            if (j < nbox)
-              ptx::tma_load_2d_u32(bs + u * kBTile + j * kBox, bmap, (int)col0 + j * kBoxCols, t * kTcK, fb);
+            for (int j = 0; j < kTcN / kBoxCols; j++)
+              if (j < nbox)
+                ptx::tma_load_2d_u32(bs + u * kBTile + j * kBox, bmap, (int)col0 + j * kBoxCols, t * kTcK, fb);
+          }
         }
       }
+      __syncwarp();
+      if (++s == kStages) {
+        s = 0;
+        ph ^= 1u;
+      }
     }
-  } else if (warp == kMmaWarp && lane == 0) {
+  } else if (warp == kMmaWarp) {
     // ---------------- MMA issuer ----------------
     // Descriptors of stage 0 are built once; every MMA adds a compile-time
     // offset (plus the stage's) to the 14-bit start-address field (>> 4).
+    const bool leader = ptx::elect_one();
     const uint32_t ab = std::is_same<BT, __nv_bfloat16>::value ? 1u : 0u;
     const uint32_t idesc = tc::idesc_f16(ab, kTr ? 1u : 0u, kSd ? 0u : 1u,
                                          (uint32_t)(nbox * kBoxCols), kTcM);
@@ -341,67 +354,58 @@ __global__ void __launch_bounds__(tc_threads(TPS), 1) k_spmm_tc(TcArgs a, const 
                                           : ptx::smem_desc_noswizzle_u32(a0, kLbo, kSbo);
     const uint64_t bdesc = kSd ? ptx::smem_desc_noswizzle_u32(b0, 16, kSdSbo) | ((uint64_t)kLayoutSw128 << 61)
                                           : ptx::smem_desc_noswizzle_u32(b0, kBox, 1024) | ((uint64_t)kLayoutSw128 << 61);
-    // The tensor pipe queues about one MMA beyond the one it runs, so every
-    // cycle this thread spends between stages is idle tensor time: the next
-    // stage's halves are read from the list while this stage issues, and the
-    // abort flag is not polled here either.
-    auto halves = [&](int st, int (&hv)[kTilesPerStage]) {
-#pragma unroll
-      for (int u = 0; u < kTilesPerStage; u++) {
-        const int k = kTilesPerStage * st + u;
-        hv[u] = kSd ? (u == 0 ? dense_halves : 0)
-                               : (st < nstages && k < n ? (lst[k] >> 28) & 3 : 0);
-      }
-    };
-    uint32_t started = 0;
+    // (a batch's list names every tile of its rows, with the halves that hold rows)
+    uint32_t s = 0, ph = 0;
     int i = 0;
-    int hn[kTilesPerStage];
-    halves(0, hn);
     for (; i < nstages; i++) {
-      const int s = i % kStages;
-      int hv[kTilesPerStage];
-#pragma unroll
-      for (int u = 0; u < kTilesPerStage; u++) hv[u] = hn[u];
-      halves(i + 1, hn);
-      const int hv0 = hv[0];
-      if (!ptx::mbar_wait(&sm.full[s], (i / kStages) & 1)) {
-        atomicCAS(&g_tc_error, 0, 3);
-        sm.abort = 1;
+      if (!ptx::mbar_wait_warp(&sm.full[s], ph)) {
+        if (leader) {
+          atomicCAS(&g_tc_error, 0, 3);
+          sm.abort = 1;
+        }
         break;
       }
       ptx::tc_fence_after_sync();
       const uint64_t soff = (uint64_t)((s * kStageBytes) >> 4);
       const uint64_t as = adesc + soff, bs = bdesc + soff;
-      if (kSd) {
-#pragma unroll
-        for (int h = 0; h < kHalves; h++) {
-          if (!((hv0 >> h) & 1)) continue;
-#pragma unroll
-          for (int j = 0; j < kSdK / 16; j++)  // K step j starts 32 B into the 128-byte rows
-            ptx::tc_mma_f16(tmem + (uint32_t)(h * kTcN), as + (uint64_t)((h * kTcM * 128 + j * 32) >> 4),
-                            bs + (uint64_t)((j * 32) >> 4), idesc, ((started >> h) & 1u) || j > 0);
-          started |= 1u << h;
-        }
-      } else {
-#pragma unroll
-        for (int u = 0; u < kTilesPerStage; u++) {
-          const int hu = hv[u];
+      if (leader) {
+        if (kSd) {
 #pragma unroll
           for (int h = 0; h < kHalves; h++) {
-            if (!((hu >> h) & 1)) continue;
+            if (!((dense_halves >> h) & 1)) break;
 #pragma unroll
-            for (int j = 0; j < 2; j++)  // K half j: A two core-matrix columns on, B two 8-row groups on
-              ptx::tc_mma_f16(tmem + (uint32_t)(h * kTcN),
-                              as + (uint64_t)((u * kATile + h * kAHalf + j * 2 * kLbo) >> 4),
-                              bs + (uint64_t)((u * kBTile + j * 2 * 1024) >> 4), idesc, ((started >> h) & 1u) || j > 0);
-            started |= 1u << h;
+            for (int j = 0; j < kSdK / 16; j++)  // K step j starts 32 B into the 128-byte rows
+              ptx::tc_mma_f16(tmem + (uint32_t)(h * kTcN), as + (uint64_t)((h * kTcM * 128 + j * 32) >> 4),
+                              bs + (uint64_t)((j * 32) >> 4), idesc, i > 0 || j > 0);
+          }
+        } else {
+#pragma unroll
+          for (int u = 0; u < kTilesPerStage; u++) {
+            if (kTilesPerStage * i + u >= n) break;
+#pragma unroll
+            for (int h = 0; h < kHalves; h++) {
+              if (!((dense_halves >> h) & 1)) break;
+#pragma unroll
+              for (int j = 0; j < 2; j++)  // K half j: A two core-matrix columns on, B two 8-row groups on
+                ptx::tc_mma_f16(tmem + (uint32_t)(h * kTcN),
+                                as + (uint64_t)((u * kATile + h * kAHalf + j * 2 * kLbo) >> 4),
+                                bs + (uint64_t)((u * kBTile + j * 2 * 1024) >> 4), idesc, i > 0 || u > 0 || j > 0);
+            }
           }
         }
+        ptx::tc_commit(&sm.empty[s]);
       }
-      ptx::tc_commit(&sm.empty[s]);
+      __syncwarp();
+      if (++s == kStages) {
+        s = 0;
+        ph ^= 1u;
+      }
     }
-    if (i > 0) ptx::tc_commit(&sm.done);
-    else ptx::mbar_arrive(&sm.done);
+    if (leader) {
+      if (i > 0) ptx::tc_commit(&sm.done);
+      else ptx::mbar_arrive(&sm.done);
+    }
+    __syncwarp();
   }
 
   // ---------------- epilogue (producer warps) ----------------
@@ -906,6 +910,19 @@ int make_batch_map(CUtensorMap* m, const void* B, int bdt, int64_t K, int64_t N,
 int make_batch_map_sddmm(CUtensorMap* m, const void* T, int bdt, int64_t rows, int64_t N, int64_t ld,
                          int box_rows) {
   return make_map(m, T, bdt, rows, N, ld, kSdK, (uint32_t)box_rows, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+int make_out_map(CUtensorMap* m, float* C, int64_t rows, int64_t cols, int64_t ld, int splits, int64_t split_stride) {
+  PFN_cuTensorMapEncodeTiled_v12000 enc = encode_tiled();
+  if (!enc) return BSP_ERR_UNSUPPORTED;
+  const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)splits};
+  const cuuint64_t strides[2] = {(cuuint64_t)ld * 4, (cuuint64_t)split_stride * 4};
+  const cuuint32_t box[3] = {32, 32, 1};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, C, dims, strides, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? BSP_OK : BSP_ERR_ALIGNMENT;
 }
 
 int launch_batched_tc(const BatchProblemTc* probs, const int4* items, int n_items, int64_t N, int bdt,

@@ -37,12 +37,13 @@
 //   warps 17-18 MMAs (128x128x16), one warp per half, by an elected lane; the
 //               first also holds the CTA's TMEM;
 //   warp 19     takes items and lists their occupied K tiles;
-//   warps 20-27 epilogue: TMEM -> registers -> staging rows -> C.
+//   warps 20-27 epilogue: TMEM -> registers -> staging boxes -> C (TMA).
 // Stage and item counters run over the whole launch, so every mbarrier phase
 // follows from a counter.  Every wait is bounded: on timeout the role records
 // error 5 in g_ts_error and stops; the others' bounded waits then end.
 #include <cuda.h>
 
+#include <cstring>
 #include <type_traits>
 
 #include "ptx.cuh"
@@ -75,20 +76,20 @@ constexpr int kAhead = 2;                       // tiles of its own a group load
 constexpr int kListPad = kTps * (kAhead + 1);   // entries past the list that may be read
 constexpr int kListMax = 4096;                  // K tiles of an item
 constexpr int kEpiCols = 64;                    // columns of an epilogue warp
-constexpr int kEpiStride = kEpiCols + 4;        // its staging rows' distance in floats (16-byte aligned, conflict-free)
+constexpr int kEpiBox = 32 * 32 * 4;            // its staging: two boxes of 32 rows x 32 columns (128-byte swizzle)
 constexpr int kErr = 5;
 constexpr uint32_t kTmemCols = 512;
 static_assert(kATmem + kAStages * kTps * kATile <= kTmemCols, "TMEM");
 
 struct Item {
   int n;          // K tiles, -1 = no more items
-  int x, y, z;    // row block, column block, split
+  int x, y, z;    // row block, column block, split (batch: problem)
   int seen;       // halves with tiles
 };
 
 struct __align__(1024) Smem {
   uint8_t b[kStages * kBStage];
-  float epi[kEpiWarps][32 * kEpiStride];
+  uint8_t epi[kEpiWarps][2 * kEpiBox];
   __align__(16) uint16_t list[kItems][kListMax + kListPad];  // tile index | halves << 12, then zeros
   uint64_t full[kStages];   // the producers' warps and B's bytes
   uint64_t done[kStages];   // the stage's MMAs
@@ -134,14 +135,29 @@ struct Transpose32 {
   }
 };
 
+// The matrix of an item: the launch's, or its problem's.
+struct Matrix {
+  const uint32_t* A;
+  int64_t M, K, Kw;
+};
+
 // TR: dX[K][N] = Aᵀ·G (output rows: columns of A, K tiles: 32 rows of A).
-template <typename BT, bool TR>
-__global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_constant__ CUtensorMap mapB) {
+// BAT: CTA x of the grid is work item x of a batch (problem, 256-row block,
+// 128-column block, K tiles), all of whose tiles are multiplied (a batch has
+// no occupancy plan) and whose words come from A's rows.
+template <typename BT, bool TR, bool BAT>
+__global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_constant__ CUtensorMap mapB,
+                                                         const __grid_constant__ CUtensorMap mapC) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(
       smem_raw + ((kSmemAlign - (ptx::smem_addr(smem_raw) & (kSmemAlign - 1))) & (kSmemAlign - 1)));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int64_t out_rows = TR ? a.K : a.M;
+  auto matrix = [&](int z) -> Matrix {
+    if (!BAT) return Matrix{a.A, a.M, a.K, a.Kw};
+    const BatchProblemTc& p = a.probs[z];
+    return Matrix{p.A, p.M, p.K, p.Kw};
+  };
+  ptx::griddep_launch_dependents();  // a batch's SDDMM may start on SMs this grid has left
   if (a.skip_if && __ldg(a.skip_if)) return;  // uniform over the grid
   if (tid == 0) {
     for (int s = 0; s < kStages; s++) {
@@ -189,7 +205,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
     if (TR) transpose.init(lane);
     // Aᵀ·G: lane p takes the A row that bit p of the transposed word stands for
     const uint32_t trow = (uint32_t)tc::unshuffled_column(lane);
-    const uint32_t M = (uint32_t)a.M;
     uint32_t g = 0, s2 = kStages - kAStages, p2 = 1u;  // stage, and the barrier and parity of the stage two before it
     for (int j = 0;; j++) {
       const int qs = j & (kItems - 1);
@@ -200,25 +215,28 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
       const int n = sm.item[qs].n;
       if (n < 0) break;
       const uint16_t* lst = sm.list[qs];
+      const Matrix m = matrix(sm.item[qs].z);
+      const uint32_t M = (uint32_t)m.M;
       // forward: the lane's row in each half; Aᵀ·G: the warp's word column in each half
       uint32_t at[2];
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         const int64_t r = (int64_t)sm.item[qs].x * kRows + h * kM + q * 32;
-        at[h] = TR ? (uint32_t)min(r / 32, a.Kw - 1) : (uint32_t)min(r + lane, a.M - 1);
+        at[h] = TR ? (uint32_t)min(r / 32, m.Kw - 1) : (uint32_t)min(r + lane, m.M - 1);
       }
       auto load_words = [&](int k, uint32_t (&w)[2]) {
         const uint32_t t = lst[k] & (kListMax - 1);
         const uint32_t r = TR ? min(t * kK + trow, M - 1) : 0u;
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-          if (a.At) w[h] = __ldg(a.At + (TR ? at[h] * M + r : t * M + at[h]));
-          else w[h] = tc::unshuffle32(__ldg(a.A + (TR ? (int64_t)r * a.Kw + at[h] : (int64_t)at[h] * a.Kw + t)));
+          if (!BAT && a.At) w[h] = __ldg(a.At + (TR ? at[h] * M + r : t * M + at[h]));
+          else w[h] = tc::unshuffle32(__ldg(m.A + (TR ? (int64_t)r * m.Kw + at[h] : (int64_t)at[h] * m.Kw + t)));
         }
       };
       uint32_t wq[kAhead][2];
 #pragma unroll
-      for (int d = 0; d < kAhead; d++) load_words(kTps * d + grp, wq[d]);
+      for (int d = 0; d < kAhead; d++)
+        if (n > 0) load_words(kTps * d + grp, wq[d]);
       bool ok = true;
       for (int k = grp; k - grp < n; k += kTps, g++) {
         uint32_t e[32];
@@ -273,6 +291,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
       const uint32_t tile_bytes = (uint32_t)nbox * kBox;
       // 256-column blocks of four 64-column atoms; this item's are two neighbours
       const uint8_t* bt = a.bt + (int64_t)(y >> 1) * (4 * (int)kBox) + (y & 1) * kBTile;
+      const void* map = &mapB;
+      if (BAT) {
+        map = &a.probs[__reduce_max_sync(kFull, *(volatile int*)&sm.item[qs].z)].map;
+        if (leader) ptx::tensormap_acquire(map);  // written by the host into global memory
+        __syncwarp();
+      }
       bool ok = true;
       for (int k0 = 0; k0 < n; k0 += kTps) {
         if (!ptx::mbar_wait_warp<64>(&sm.done[s], ph)) {
@@ -287,11 +311,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
             if (u >= cnt) break;
             const int t = lst[k0 + u] & (kListMax - 1);
             const uint32_t dst = b0 + s * kBStage + (uint32_t)u * kBTile;
-            if (a.bt) {
+            if (!BAT && a.bt) {
               ptx::bulk_g2s_u32(dst, bt + (int64_t)t * a.bt_cb * (4 * (int)kBox), tile_bytes, f0 + s * 8u);
             } else {
               for (int b = 0; b < nbox; b++)
-                ptx::tma_load_2d_u32(dst + (uint32_t)b * kBox, &mapB, y * kN + b * 64, t * kK, f0 + s * 8u);
+                ptx::tma_load_2d_u32(dst + (uint32_t)b * kBox, map, y * kN + b * 64, t * kK, f0 + s * 8u);
             }
           }
         }
@@ -311,8 +335,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
   } else if (warp == kMmaWarp || warp == kMmaWarp + 1) {
     // ---------------- MMA issuers ----------------
     // One warp per half: a stage is a wait, eight MMAs and a commit for each.
-    // (One warp for both took 1210 cycles a stage to issue what the tensor
-    // pipe runs in 1024.)
     const int h = warp - kMmaWarp;
     const bool leader = ptx::elect_one();
     const uint32_t ab = std::is_same<BT, __nv_bfloat16>::value ? 1u : 0u;
@@ -399,7 +421,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
   } else if (warp == kSchedWarp) {
     // ---------------- items and their lists ----------------
     uint32_t x = blockIdx.x, y = blockIdx.y, z = blockIdx.z;
-    const int nblk = (int)((out_rows + kM - 1) / kM);
+    const int nblk = BAT ? 0 : (int)(((TR ? a.K : a.M) + kM - 1) / kM);
     bool more = true;
     for (int j = 0;; j++) {
       if (lane == 0 && more) {  // ask for the next item while this one is listed
@@ -418,6 +440,25 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
         }
         break;
       }
+      if (BAT) {
+        const int4 it = __ldg(a.items + x);
+        const Matrix m = matrix(it.x);
+        const uint32_t hv = (int64_t)it.y * kRows + kM < (TR ? m.K : m.M) ? 3u : 1u;
+        const int n = it.w;
+        // the item's first words, on their way to L2 before its producers ask
+        if (n > 0) {
+          const int64_t w0 = TR ? (int64_t)it.y * (kRows / 32) : 0;
+          const int64_t r0 = TR ? 0 : (int64_t)it.y * kRows;
+          for (int64_t r = r0 + lane; r < min(m.M, r0 + kRows); r += 32) ptx::prefetch_l2(m.A + r * m.Kw + w0);
+        }
+        for (int k = lane; k < n; k += 32) sm.list[qs][k] = (uint16_t)((uint32_t)k | (hv << 12));
+        if (lane < kListPad) sm.list[qs][n + lane] = 0;
+        __syncwarp();
+        if (lane == 0) {
+          sm.item[qs] = Item{n, it.y, it.z, it.x, n > 0 ? (int)hv : 0};
+          ptx::mbar_arrive(&sm.qfull[qs]);
+        }
+      } else {
       // occupied tiles of the two 128-row blocks (ascending), this split's
       // share of them; the launcher guarantees that they fit
       const uint32_t* occ0 = a.occ + (int64_t)x * 2 * a.occ_words;
@@ -456,6 +497,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
         sm.item[qs] = Item{n, (int)x, (int)y, (int)z, (int)hs};
         ptx::mbar_arrive(&sm.qfull[qs]);
       }
+      }
       // the answer
       if (!ptx::mbar_wait_warp<256>(&sm.clc, (uint32_t)j & 1u)) {
         if (lane == 0) fail();
@@ -468,14 +510,20 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
   } else {
     // ---------------- epilogue ----------------
     // Every half is read back by all eight warps, a lane quarter and 64 columns
-    // each, into a staging block of the warp's own, and handed back at once (590
-    // cycles a half); its rows are stored from there (1700) while the next
-    // item's MMAs begin.
+    // each, into two boxes of the warp's own, and handed back at once (590
+    // cycles a half); the boxes leave by TMA while the next half is read.
+    // Stores from registers took another 1700 cycles a half and kept the second
+    // half's accumulator waiting (1024-column products 20.3 -> 18.6 us, a batch
+    // of 128 problems of 64..2048 rows and columns with both gradients 114 ->
+    // 111).
     const int ew = warp - kEpiWarp0, q = warp & 3;  // the TMEM lane quarter this warp may access
     const int cw = (ew >> 2) * kEpiCols;            // (ew & 3 runs over the quarters too)
-    float* tile = sm.epi[ew];
-    // the row of its 32 that a TMEM lane holds (Aᵀ·G: the column at the lane's bit of an unshuffled word)
-    float* mine = tile + (TR ? tc::unshuffled_column(lane) : lane) * kEpiStride;
+    const bool leader = ptx::elect_one();
+    uint8_t* box = sm.epi[ew];
+    // the row of its 32 that a TMEM lane holds (Aᵀ·G: the column at the lane's
+    // bit of an unshuffled word); 16-byte chunk u of row r sits at u ^ (r % 8)
+    const uint32_t mr = (uint32_t)(TR ? tc::unshuffled_column(lane) : lane);
+    uint8_t* mine = box + mr * 128;
     // one warp polls, the others wait for it at a hardware barrier
     auto epi_wait = [&](uint64_t* bar, uint32_t parity) -> bool {
       if (ew == 0 && !ptx::mbar_wait_warp(bar, parity) && lane == 0) *(volatile int*)&sm.gave_up = 1;
@@ -490,10 +538,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
       }
       const Item it = sm.item[qs];
       if (it.n < 0) break;
-      const bool split = gridDim.z > 1;
-      float* cbase = split ? a.part + (int64_t)it.z * a.part_stride : a.C;
-      const int64_t cld = split ? a.ldp : a.ldc;
-      const bool cvec = split || a.c_vec;
+      const Matrix m = matrix(it.z);
+      const int64_t out_rows = TR ? m.K : m.M;
+      const void* cmap = &mapC;
+      if (BAT) {
+        cmap = &a.probs[it.z].map2;
+        if (leader) ptx::tensormap_acquire(cmap);  // written by the host into global memory
+        __syncwarp();
+      }
       const int64_t gcol = (int64_t)it.y * kN + cw;
       const int cols = (int)max((int64_t)0, min((int64_t)kEpiCols, a.N - gcol));  // live columns of this warp
       bool ok = true;
@@ -507,47 +559,50 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
         const int64_t rbase = (int64_t)it.x * kRows + h * kM + q * 32;  // the warp's first row
         const bool have = (it.seen >> h) & 1;
         const bool live = rbase < out_rows && cols > 0;
+        if (leader) ptx::bulk_wait_read();  // the half before has left the boxes
+        __syncwarp();
         if (live) {
           const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + h * kN + (uint32_t)cw;
 #pragma unroll
-          for (int c = 0; c < kEpiCols; c += 32) {
+          for (int c = 0; c < 2; c++) {
             uint32_t v[32];
             if (have) {
-              ptx::tmem_ld_32x32b_x32(tb + (uint32_t)c, v);
+              ptx::tmem_ld_32x32b_x32(tb + (uint32_t)(c * 32), v);
               ptx::tmem_wait_ld();
             }
 #pragma unroll
-            for (int u = 0; u < 32; u += 4)
-              *reinterpret_cast<float4*>(mine + c + u) =
-                  have ? make_float4(__uint_as_float(v[u]) * tc::kTwoScale, __uint_as_float(v[u + 1]) * tc::kTwoScale,
-                                     __uint_as_float(v[u + 2]) * tc::kTwoScale, __uint_as_float(v[u + 3]) * tc::kTwoScale)
+            for (int u = 0; u < 8; u++)
+              *reinterpret_cast<float4*>(mine + c * kEpiBox + ((u ^ (mr & 7)) << 4)) =
+                  have ? make_float4(__uint_as_float(v[4 * u]) * tc::kTwoScale, __uint_as_float(v[4 * u + 1]) * tc::kTwoScale,
+                                     __uint_as_float(v[4 * u + 2]) * tc::kTwoScale, __uint_as_float(v[4 * u + 3]) * tc::kTwoScale)
                        : make_float4(0.f, 0.f, 0.f, 0.f);
           }
         }
         ptx::tc_fence_before_sync();
+        ptx::fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(&sm.tempty[h]);
         if (!live) continue;
-        if (cvec) {
-          // 16 lanes per row: two rows of 256 bytes per store
-          const int c4 = (lane & 15) * 4;
-          const float* src = tile + (lane >> 4) * kEpiStride + c4;
-          float* dst = cbase + (rbase + (lane >> 4)) * cld + gcol + c4;
-          const int nr = c4 < cols ? (int)min((int64_t)32, out_rows - rbase) - (lane >> 4) : 0;
-#pragma unroll 8
-          for (int r = 0; r < 32; r += 2)
-            if (r < nr) *reinterpret_cast<float4*>(dst + (int64_t)r * cld) = *reinterpret_cast<const float4*>(src + r * kEpiStride);
-          __syncwarp();
+        if (BAT || a.c_map) {  // rows and columns past the output are clipped
+          if (leader) {
+            for (int c = 0; c * 32 < cols; c++)
+              ptx::tma_store_3d(cmap, (int)gcol + c * 32, (int)rbase, BAT ? 0 : it.z, box + c * kEpiBox);
+            ptx::bulk_commit();
+          }
         } else {
           const int nr = (int)min((int64_t)32, out_rows - rbase);
           for (int r = 0; r < nr; r++)
-            for (int c = lane; c < cols; c += 32) cbase[(rbase + r) * cld + gcol + c] = tile[r * kEpiStride + c];
+            for (int c = lane; c < cols; c += 32)
+              a.C[(rbase + r) * a.ldc + gcol + c] = *reinterpret_cast<const float*>(
+                  box + (c >> 5) * kEpiBox + r * 128 + ((((c & 31) >> 2) ^ (r & 7)) << 4) + (c & 3) * 4);
           __syncwarp();
         }
       }
       if (!ok) break;
       if (lane == 0) ptx::mbar_arrive(&sm.qempty[qs]);
     }
+    if (leader) ptx::bulk_wait_all();
+    __syncwarp();
   }
   ptx::tc_fence_before_sync();
   __syncthreads();
@@ -557,10 +612,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
   }
 }
 
-template <typename BT, bool TR>
-int launch_t(const TsArgs& a, const CUtensorMap& map, dim3 grid, cudaStream_t s) {
+template <typename BT, bool TR, bool BAT>
+int launch_t(const TsArgs& a, const CUtensorMap& map, const CUtensorMap& mapc, dim3 grid, cudaStream_t s) {
   constexpr size_t smem = sizeof(Smem) + kSmemAlign;
-  auto kern = k_spmm_ts<BT, TR>;
+  auto kern = k_spmm_ts<BT, TR, BAT>;
   static bool configured[64] = {};
   int dev = 0;
   BSP_CUDA(cudaGetDevice(&dev));
@@ -568,7 +623,7 @@ int launch_t(const TsArgs& a, const CUtensorMap& map, dim3 grid, cudaStream_t s)
     BSP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     if (dev < 64) configured[dev] = true;
   }
-  kern<<<grid, kThreads, smem, s>>>(a, map);
+  kern<<<grid, kThreads, smem, s>>>(a, map, mapc);
   BSP_LAUNCHED();
   return BSP_OK;
 }
@@ -578,13 +633,46 @@ int launch_t(const TsArgs& a, const CUtensorMap& map, dim3 grid, cudaStream_t s)
 int64_t ts_item_rows() { return kRows; }
 int64_t ts_item_cols() { return kN; }
 
-int launch_ts(const TsArgs& a, const CUtensorMap& map, bool trans, int splits, cudaStream_t s) {
+int launch_ts(TsArgs a, const CUtensorMap& map, bool trans, int splits, cudaStream_t s) {
   const int64_t gx = ceil_div(trans ? a.K : a.M, kRows), gy = ceil_div(a.N, kN);
   if (gy > 65535 || gx > 0x7fffffff) return BSP_ERR_CAPACITY;
   const dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)splits);
+  // C (or the splits' partials) by TMA, where its rows start on 16 bytes
+  CUtensorMap mapc;
+  memset(&mapc, 0, sizeof(mapc));
+  const int64_t rows = trans ? a.K : a.M;
+  if (splits > 1) {
+    BSP_TRY(make_out_map(&mapc, a.part, rows, a.N, a.ldp, splits, a.part_stride));
+    a.c_map = true;
+  } else if (a.c_vec) {
+    BSP_TRY(make_out_map(&mapc, a.C, rows, a.N, a.ldc, 1, rows * a.ldc));
+    a.c_map = true;
+  }
   if (a.bdt == BSP_BF16)
-    return trans ? launch_t<__nv_bfloat16, true>(a, map, grid, s) : launch_t<__nv_bfloat16, false>(a, map, grid, s);
-  if (a.bdt == BSP_F16) return trans ? launch_t<__half, true>(a, map, grid, s) : launch_t<__half, false>(a, map, grid, s);
+    return trans ? launch_t<__nv_bfloat16, true, false>(a, map, mapc, grid, s)
+                 : launch_t<__nv_bfloat16, false, false>(a, map, mapc, grid, s);
+  if (a.bdt == BSP_F16)
+    return trans ? launch_t<__half, true, false>(a, map, mapc, grid, s) : launch_t<__half, false, false>(a, map, mapc, grid, s);
+  return BSP_ERR_UNSUPPORTED;
+}
+
+int launch_ts_batch(const BatchProblemTc* probs, const int4* items, int n_items, int64_t N, int bdt, bool trans,
+                    cudaStream_t s) {
+  if (n_items == 0 || N == 0) return BSP_OK;
+  TsArgs a = {};
+  a.N = N;
+  a.bdt = bdt;
+  a.c_vec = true;
+  a.probs = probs;
+  a.items = items;
+  CUtensorMap unused;
+  memset(&unused, 0, sizeof(unused));
+  const dim3 grid((unsigned)n_items);
+  if (bdt == BSP_BF16)
+    return trans ? launch_t<__nv_bfloat16, true, true>(a, unused, unused, grid, s)
+                 : launch_t<__nv_bfloat16, false, true>(a, unused, unused, grid, s);
+  if (bdt == BSP_F16)
+    return trans ? launch_t<__half, true, true>(a, unused, unused, grid, s) : launch_t<__half, false, true>(a, unused, unused, grid, s);
   return BSP_ERR_UNSUPPORTED;
 }
 

@@ -3,6 +3,7 @@
 #include <cuda.h>
 
 #include "bsp_internal.cuh"
+#include "spmm.cuh"
 
 namespace bsp {
 
@@ -13,7 +14,8 @@ struct TsArgs {
   int64_t N;
   float* C;            // [M][ldc]; trans: dX [K][ldc]
   int64_t ldc;
-  bool c_vec;          // C's rows take 16-byte stores
+  bool c_vec;          // C's rows start on 16 bytes
+  bool c_map;          // (set by the launcher) the output leaves by TMA
   const uint32_t* occ; // occupancy bitmap of 128-row blocks (trans: of 128-column blocks)
   int occ_words;
   int bdt;
@@ -23,13 +25,19 @@ struct TsArgs {
   // B (or G) in tile order, bt_cb blocks of 256 columns per 32-row tile; null = TMA boxes through the map
   const uint8_t* bt;
   int64_t bt_cb;
+  // batch: work items (problem, 256-row block, 128-column block, K tiles) and the problems' records
+  const BatchProblemTc* probs;
+  const int4* items;
   const int* skip_if;  // device flag: nonzero = leave C alone; null = run
 };
 
 // rows and columns of the output per work item
 int64_t ts_item_rows();
 int64_t ts_item_cols();
-int launch_ts(const TsArgs& a, const CUtensorMap& map, bool trans, int splits, cudaStream_t s);
+int launch_ts(TsArgs a, const CUtensorMap& map, bool trans, int splits, cudaStream_t s);
+// Every item of a batch: C = A·B of its problem (trans: dX = Aᵀ·G), longest items first.
+int launch_ts_batch(const BatchProblemTc* probs, const int4* items, int n_items, int64_t N, int bdt, bool trans,
+                    cudaStream_t s);
 int ts_device_error(int* out, bool clear);
 
 }  // namespace bsp

@@ -180,8 +180,10 @@ def spmm(words, K, B, plan=None, out=None, workspace=None):
     if plan is not None:
         fits = workspace is not None and have >= plan.workspace_bytes(N, preferred=False)
     else:
+        # (below 540 MB of matrix x width the library makes no copy)
         e = B.element_size()
-        fits = workspace is not None or (N * e % 16 == 0 and ldb * e % 16 == 0 and B.data_ptr() % 16 == 0)
+        fits = (workspace is not None or M * K * N * e < 540e6
+                or (N * e % 16 == 0 and ldb * e % 16 == 0 and B.data_ptr() % 16 == 0))
     if not fits:
         n = C.c_size_t()
         call("bsp_spmm_workspace_layout", h, K, N, _p(B), _DT[B.dtype], ldb, C.byref(n))
@@ -412,9 +414,9 @@ def csr_to_tiled(row_ptr, col_idx, M, K, tile_rows, tile_cols, values=None):
 
 class Batch:
     """Many independent C_i = A_i·B_i (16-bit B, shared N) in one tensor-core
-    launch: for N ≤ 128 a persistent kernel (a CTA per SM, 256-row items from
-    a device work queue), otherwise a CTA per 256x256 item.  Runs of one
-    batch must not overlap on the GPU (they share the queue and the C buffers).  ``problems``: list of (words, K, B, C) tensors; the
+    launch of the persistent kernel (a CTA per SM, items of 256 rows x 128
+    columns).  Runs of one batch must not overlap on the GPU (they share the
+    C buffers).  ``problems``: list of (words, K, B, C) tensors; the
     tensors are referenced by the batch and must outlive it."""
 
     def __init__(self, problems):
@@ -441,9 +443,8 @@ class Batch:
         call("bsp_batched_spmm", self._h, _stream())
 
     def tune(self):
-        """Time the persistent kernel's shapes on this batch (runs it four
-        times per shape), keep the fastest for later runs; returns (shape,
-        ms)."""
+        """Time the batch (runs it four times); returns (shape, ms) — one
+        kernel shape is built."""
         shape, ms = C.c_int(), C.c_float()
         call("bsp_batch_tune", self._h, _stream(), C.byref(shape), C.byref(ms))
         return shape.value, ms.value

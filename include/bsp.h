@@ -270,19 +270,14 @@ int bsp_batch_create(const bsp_problem* problems, int n, int64_t N,
 int bsp_batch_destroy(bsp_batch* batch);
 /* Every problem of the batch in one tensor-core launch, with no host
  * synchronisation and no allocation; it can be captured in a CUDA graph.
- * For N ≤ 128 the launch is persistent: a CTA per SM takes items from a
- * work queue in the batch's device memory, which a memset in the same stream
- * resets first.  For wider N it is one CTA per work item.  Runs of one batch
- * must not overlap on the GPU: they share the queue and the C buffers.     */
+ * The launch is persistent: a CTA per SM takes over the items of CTAs that
+ * have not started.  Runs of one batch must not overlap on the GPU: they
+ * share the C buffers.                                                      */
 int bsp_batched_spmm(const bsp_batch* batch, bsp_stream_t stream);
-/* Times the persistent kernel's shapes (pipeline stages, epilogue warps, A
- * words loaded ahead) on this batch — each once to warm up, then three runs
- * — keeps the fastest in the batch for later bsp_batched_spmm calls and
- * returns its index and ms per run.  It runs the batch (writes its C
- * buffers) four times per shape and synchronises the stream.  Batches of
- * N > 128 have
- * one shape (index 0); a gradient batch is refused (BSP_ERR_INVALID_ARG).
- * On an error the batch keeps its previous shape.                         */
+/* Times the batch — once to warm up, then three runs — and returns the index
+ * of the kernel shape that bsp_batched_spmm uses (one is built: 0) and its ms
+ * per run.  It runs the batch (writes its C buffers) four times and
+ * synchronises the stream; a gradient batch is refused (BSP_ERR_INVALID_ARG). */
 int bsp_batch_tune(bsp_batch* batch, bsp_stream_t stream, int* shape, float* ms);
 
 /* One problem of a batched backward pass of Y = A·X (A a 0/1 mask, packed
@@ -317,13 +312,13 @@ typedef struct bsp_problem_grad {
 int bsp_batch_grad_create(const bsp_problem_grad* problems, int n, int64_t N,
                           int dtype, bsp_batch** batch, bsp_stream_t stream);
 /* Every dX and dA of a gradient batch: two tensor-core launches, no host
- * synchronisation, no allocation.  dX (for N ≤ 128 one persistent launch,
- * else a CTA per work item) sums every 32-row tile of A (a batch has no
- * occupancy plan); dA is one persistent
- * launch (a CTA per SM taking items from a work queue in the batch's
- * device memory, reset by a memset in the same stream) that writes zeros
- * off A's set bits.  Runs of one batch must not overlap on the GPU: they
- * share the queue and write the same dX and dA buffers.                    */
+ * synchronisation, no allocation.  dX (one persistent launch) sums every
+ * 32-row tile of A (a batch has no occupancy plan); dA is one persistent
+ * launch (a CTA per SM taking items from a work queue in the batch's device
+ * memory, reset by a memset in the same stream) that writes zeros off A's set
+ * bits and may run beside dX's last items: dX and dA must not overlap in
+ * memory.  Runs of one batch must not overlap on the GPU: they share the queue
+ * and write the same dX and dA buffers.                                     */
 int bsp_batched_spmm_grad(const bsp_batch* batch, bsp_stream_t stream);
 
 /* ======================================================================== */
