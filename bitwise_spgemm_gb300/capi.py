@@ -106,6 +106,10 @@ SIGNATURES = {
     "bsp_bitplanes_rows": [_P, _I64, _I64, _I64, _I, _P, _P],
     "bsp_stack_planes_b": [_P, _I, _I64, _I64, _I64, _I, _I, _P, _I64, _P],
     "bsp_spmm_i8": [_P, _I64, _I64, _I64, _P, _I, _I64, _I64, _P, _I64, _P, _SZ, _P],
+    "bsp_i8_tiles_bytes": [_I64, _I64, C.POINTER(_SZ)],
+    "bsp_i8_tiles": [_P, _I64, _I64, _I64, _P, _P],
+    "bsp_spmm_i8_tiles_workspace": [_I64, _I64, _I64, C.POINTER(_SZ)],
+    "bsp_spmm_i8_tiles": [_P, _I64, _I64, _P, _I, _I64, _I64, _P, _I64, _P, _SZ, _P],
     "bsp_tiles8_workspace": [_I64, _I64, C.POINTER(_SZ)],
     "bsp_rows_to_tiles8": [_P, _I64, _I64, _P, _P, _P, _P, _P, _P, _SZ, _P],
     "bsp_tiles8_to_rows": [_P, _P, _P, _I64, _I64, _I64, _P, _P],

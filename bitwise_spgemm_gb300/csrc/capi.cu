@@ -677,6 +677,44 @@ int bsp_spmm_i8(const int8_t* A, int64_t M, int64_t K, int64_t lda, const void* 
   return bsp_bitplane_spmm(planes, 8, 1, M, K, B, b_dtype, ldb, N, C, ldc, stream);
 }
 
+int bsp_i8_tiles_bytes(int64_t M, int64_t K, size_t* bytes) {
+  if (!bytes || M < 0 || K < 0) return BSP_ERR_INVALID_ARG;
+  *bytes = i8_tiles_bytes(M, K);
+  return BSP_OK;
+}
+
+int bsp_i8_tiles(const int8_t* A, int64_t M, int64_t K, int64_t lda, int8_t* tiles, bsp_stream_t stream) {
+  BSP_TRY(check_dims(M, K));
+  if (lda < K) return BSP_ERR_INVALID_ARG;
+  if (M == 0 || K == 0) return BSP_OK;
+  if (!A || !tiles) return BSP_ERR_INVALID_ARG;
+  if (!is_aligned(tiles, 16)) return BSP_ERR_ALIGNMENT;
+  return launch_i8_tiles(A, M, K, lda, tiles, (cudaStream_t)stream);
+}
+
+int bsp_spmm_i8_tiles_workspace(int64_t M, int64_t K, int64_t N, size_t* bytes) {
+  if (!bytes || M < 0 || K < 0 || N < 0) return BSP_ERR_INVALID_ARG;
+  *bytes = tc_preferred_bytes(M, N, K);
+  return BSP_OK;
+}
+
+int bsp_spmm_i8_tiles(const int8_t* tiles, int64_t M, int64_t K, const void* B, int b_dtype, int64_t ldb, int64_t N,
+                      float* C, int64_t ldc, void* workspace, size_t workspace_bytes, bsp_stream_t stream) {
+  BSP_TRY(check_dims(M, K));
+  if (N < 0 || N > kMaxCols || ldb < N || ldc < N) return BSP_ERR_INVALID_ARG;
+  if (b_dtype != BSP_BF16 && b_dtype != BSP_F16) return BSP_ERR_UNSUPPORTED;
+  if (K > tc_max_reduction()) return BSP_ERR_CAPACITY;
+  if (M == 0 || N == 0) return BSP_OK;
+  if (!C || (K > 0 && (!tiles || !B))) return BSP_ERR_INVALID_ARG;
+  if (!layout16(B, ldb, 2, N, 8) || !layout16(C, ldc, 4, N, 4) || !is_aligned(tiles, 16)) return BSP_ERR_ALIGNMENT;
+  const cudaStream_t s = (cudaStream_t)stream;
+  if (K == 0) {
+    BSP_CUDA(cudaMemset2DAsync(C, sizeof(float) * ldc, 0, sizeof(float) * N, M, s));
+    return BSP_OK;
+  }
+  return launch_spmm_i8_tc(tiles, M, K, B, b_dtype, ldb, N, C, ldc, workspace, workspace_bytes, s);
+}
+
 int bsp_tiles8_workspace(int64_t M, int64_t K, size_t* bytes) {
   if (!bytes || M < 0 || K < 0) return BSP_ERR_INVALID_ARG;
   *bytes = tiles8_workspace_bytes(M, K) + 256;

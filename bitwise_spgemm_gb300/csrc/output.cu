@@ -364,7 +364,53 @@ __global__ void __launch_bounds__(256) k_stack_planes_b(const BT* __restrict__ B
   }
 }
 
+// int8 A [M][K] -> [ceil(K/32)][M][32], zeros past K: the order in which the
+// tensor-core product's producers read it (a lane's 32 bytes of a tile next to
+// its neighbour row's), and behind it one bit per 128 x 32 tile that holds a
+// nonzero.  A thread takes 4 columns of a row; runs once per weight matrix.
+template <bool VEC>
+__global__ void __launch_bounds__(256) k_i8_tiles(const int8_t* __restrict__ A, int64_t M, int64_t K, int64_t lda,
+                                                  int64_t Kw, uint32_t* __restrict__ tiles, uint32_t* occ,
+                                                  int occ_words) {
+  const int64_t q = Kw * 8;
+  for (int64_t r = blockIdx.y; r < M; r += gridDim.y) {
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < q; e += (int64_t)gridDim.x * blockDim.x) {
+      const int64_t c = e * 4, t = e >> 3;
+      uint32_t w = 0u;
+      if (VEC && c + 4 <= K) {
+        w = __ldg(reinterpret_cast<const uint32_t*>(A + r * lda + c));
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+          if (c + i < K) w |= (uint32_t)(uint8_t)A[r * lda + c + i] << (8 * i);
+      }
+      tiles[(t * M + r) * 8 + (e & 7)] = w;
+      uint32_t* o = occ + (r >> 7) * occ_words + (t >> 5);
+      const uint32_t bit = 1u << (t & 31);
+      if (w && !(*reinterpret_cast<volatile uint32_t*>(o) & bit)) atomicOr(o, bit);
+    }
+  }
+}
+
 }  // namespace
+
+size_t i8_values_bytes(int64_t M, int64_t K) { return (size_t)M * (size_t)ceil_div(K, 32) * 32; }
+
+size_t i8_tiles_bytes(int64_t M, int64_t K) {
+  return i8_values_bytes(M, K) + (size_t)ceil_div(M, 128) * tc_occupancy_words(K) * sizeof(uint32_t);
+}
+
+int launch_i8_tiles(const int8_t* A, int64_t M, int64_t K, int64_t lda, int8_t* tiles, cudaStream_t s) {
+  const int64_t Kw = ceil_div(K, 32);
+  const dim3 grid((unsigned)(ceil_div(Kw * 8, 256) < 64 ? ceil_div(Kw * 8, 256) : 64), (unsigned)(M < 65535 ? M : 65535));
+  uint32_t* occ = reinterpret_cast<uint32_t*>(tiles + i8_values_bytes(M, K));
+  BSP_CUDA(cudaMemsetAsync(occ, 0, i8_tiles_bytes(M, K) - i8_values_bytes(M, K), s));
+  const bool vec = lda % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 4 == 0;
+  (vec ? k_i8_tiles<true> : k_i8_tiles<false>)<<<grid, 256, 0, s>>>(A, M, K, lda, Kw, (uint32_t*)tiles, occ,
+                                                                    tc_occupancy_words(K));
+  BSP_LAUNCHED();
+  return BSP_OK;
+}
 
 int launch_stack_planes_b(const void* B, int bdt, int64_t ldb, int64_t K, int64_t N, int nplanes, int signed_top,
                           void* out, int64_t ldo, cudaStream_t s) {

@@ -124,6 +124,13 @@ size_t tc_preferred_bytes(int64_t out_rows, int64_t out_cols, int64_t red_rows);
 // dX[K][N] = Aᵀ·G on the tensor cores, Aᵀ read from A's row words
 int launch_spmm_t_tc(const uint32_t* A, int64_t M, int64_t K, const void* G, int gdt, int64_t ldg, int64_t N,
                      float* dX, int64_t lddx, const uint32_t* occT, const uint32_t* At, cudaStream_t s, void* ws = nullptr, size_t ws_bytes = 0);
+// C = A·B for int8 A in the order of launch_i8_tiles (values [ceil(K/32)][M][32], then a bit per 128 x 32
+// tile with a nonzero), 16-bit B, vector layouts
+size_t i8_values_bytes(int64_t M, int64_t K);
+size_t i8_tiles_bytes(int64_t M, int64_t K);
+int launch_spmm_i8_tc(const void* tiles, int64_t M, int64_t K, const void* B, int bdt, int64_t ldb, int64_t N, float* C,
+                      int64_t ldc, void* ws, size_t ws_bytes, cudaStream_t s);
+int launch_i8_tiles(const int8_t* A, int64_t M, int64_t K, int64_t lda, int8_t* tiles, cudaStream_t s);
 // dA[M][K] = (G·Xᵀ) at A's set bits, 0 elsewhere, on the tensor cores
 int launch_sddmm_tc(const uint32_t* A, int64_t M, int64_t K, const void* G, int64_t ldg, const void* X,
                     int64_t ldx, int dt, int64_t N, float* dA, int64_t ldda, cudaStream_t s);

@@ -751,6 +751,13 @@ size_t tc_tiled_b_bytes(int64_t red_rows, int64_t cols) {
 // 12.5.
 constexpr int64_t kTiledMinRowBlocks = 16;
 
+// Not of a small product, where the copy's launch costs more than it saves
+// (10 % bits, BF16, tiled and not: 16384x1024x256 14.3 and 13.7 us,
+// 4096x4096x256 18.5 and 17.5, x512 24.6 and 24.3, x1024 31.2 and 32.3), nor
+// of int8 values, whose producers bound the kernel (4096x4096x256 20.8 and
+// 18.7 us, x1024 41.3 and 37.6, x4096 144.9 and 131.7).
+constexpr double kTiledMinWork = 6e9;  // rows x columns x reduction
+
 bool tc_tiles_b(int64_t out_rows) { return ceil_div(out_rows, ts_item_rows()) >= kTiledMinRowBlocks; }
 
 size_t tc_preferred_bytes(int64_t out_rows, int64_t out_cols, int64_t red_rows) {
@@ -797,7 +804,10 @@ int launch_product(TsArgs a, const void* B, int64_t ldb, bool vec, bool trans, c
   }
   // B in tile order when the rest of the workspace holds it (else tensor boxes)
   const bool room = ws && ws_bytes >= used + tiled_bytes;
-  const bool tiled = !vec || (room && (form.tiled >= 0 ? form.tiled == 1 : tc_tiles_b(rows) && tiled_b_enabled()));
+  const bool tiled = !vec || (room && (form.tiled >= 0 ? form.tiled == 1
+                                                            : tc_tiles_b(rows) && tiled_b_enabled() &&
+                                                                  !a.tiles &&
+                                                                  (double)rows * (double)cols * (double)red_rows >= kTiledMinWork));
   CUtensorMap map;
   memset(&map, 0, sizeof(map));
   if (tiled) {
@@ -874,6 +884,24 @@ int launch_spmm_t_tc(const uint32_t* A, int64_t M, int64_t K, const void* G, int
   a.bdt = gdt;
   const int* skipped = nullptr;  // (only vector layouts come here)
   return launch_product(a, G, ldg, true, true, s, ws, ws_bytes, TcForm{}, &skipped);
+}
+
+int launch_spmm_i8_tc(const void* tiles, int64_t M, int64_t K, const void* B, int bdt, int64_t ldb, int64_t N, float* C,
+                      int64_t ldc, void* ws, size_t ws_bytes, cudaStream_t s) {
+  TsArgs a = {};
+  a.tiles = static_cast<const uint4*>(tiles);
+  a.occ = reinterpret_cast<const uint32_t*>(static_cast<const uint8_t*>(tiles) + i8_values_bytes(M, K));
+  a.occ_words = tc_occupancy_words(K);
+  a.M = M;
+  a.K = K;
+  a.Kw = ceil_div(K, 32);
+  a.N = N;
+  a.C = C;
+  a.ldc = ldc;
+  a.c_vec = true;
+  a.bdt = bdt;
+  const int* skipped = nullptr;
+  return launch_product(a, B, ldb, true, false, s, ws, ws_bytes, TcForm{}, &skipped);
 }
 
 int launch_sddmm_tc(const uint32_t* A, int64_t M, int64_t K, const void* G, int64_t ldg, const void* X,

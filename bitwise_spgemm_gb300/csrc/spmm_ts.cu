@@ -135,19 +135,54 @@ struct Transpose32 {
   }
 };
 
+constexpr int kModeBits = 0, kModeTrans = 1, kModeBatch = 2, kModeBatchTrans = 3, kModeI8 = 4;
+
 // The matrix of an item: the launch's, or its problem's.
 struct Matrix {
   const uint32_t* A;
   int64_t M, K, Kw;
 };
 
+// int8 values as pairs of 16-bit floats (exact): 4 bytes of w -> 2 pairs.
+// BF16: 128 + (low 7 bits) and 128 or 256 by the sign bit are bit patterns,
+// their difference the value; FP16: 1024 + (value + 128) less 1152.
+template <typename BT>
+__device__ __forceinline__ uint32_t i8_pair(uint32_t p) {  // bytes 0 and 2 of p
+  if constexpr (std::is_same<BT, __nv_bfloat16>::value) {
+    const uint32_t a = (p & 0x007f007fu) | 0x43004300u, b = (p & 0x00800080u) | 0x43004300u;
+    const __nv_bfloat162 d = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
+    return *reinterpret_cast<const uint32_t*>(&d);
+  } else {
+    const uint32_t a = (p ^ 0x00800080u) | 0x64006400u, b = 0x64806480u;
+    const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
+    return *reinterpret_cast<const uint32_t*>(&d);
+  }
+}
+template <typename BT>
+__device__ __forceinline__ void i8_pairs(const uint4& q, uint32_t* v) {  // 16 values
+  const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    v[2 * i] = i8_pair<BT>(__byte_perm(w[i], 0u, 0x4140));
+    v[2 * i + 1] = i8_pair<BT>(__byte_perm(w[i], 0u, 0x4342));
+  }
+}
+
+// I8: A is int8, [K tile][row][32] (bsp_i8_tiles), its values the MMA's operand
+// (exact in 16 bits): one product over K where the planes' bits take eight,
+// with weighted copies of B stacked first (4096x4096x256 BF16, 5 %: planes
+// 29 us to stack B, 57 to multiply, 6 to reduce; values 19 in all).  Bound by
+// the producers' loads and conversions (4096^3: 132 us, 1.04 PFLOP/s).
 // TR: dX[K][N] = Aᵀ·G (output rows: columns of A, K tiles: 32 rows of A).
 // BAT: CTA x of the grid is work item x of a batch (problem, 256-row block,
 // 128-column block, K tiles), all of whose tiles are multiplied (a batch has
 // no occupancy plan) and whose words come from A's rows.
-template <typename BT, bool TR, bool BAT>
+template <typename BT, int MODE>
 __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_constant__ CUtensorMap mapB,
                                                          const __grid_constant__ CUtensorMap mapC) {
+  constexpr bool TR = MODE == kModeTrans || MODE == kModeBatchTrans, BAT = MODE == kModeBatch || MODE == kModeBatchTrans;
+  constexpr bool I8 = MODE == kModeI8;
+  constexpr float kScale = I8 ? 1.f : tc::kTwoScale;  // a set bit is expanded to 2.0
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(
       smem_raw + ((kSmemAlign - (ptx::smem_addr(smem_raw) & (kSmemAlign - 1))) & (kSmemAlign - 1)));
@@ -234,19 +269,39 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
         }
       };
       uint32_t wq[kAhead][2];
+      uint4 vq[2][2];  // int8: the coming tile's 32 bytes of each half
+      auto load_bytes = [&](int k) {
+        const uint32_t t = lst[k] & (kListMax - 1);
 #pragma unroll
-      for (int d = 0; d < kAhead; d++)
-        if (n > 0) load_words(kTps * d + grp, wq[d]);
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+          for (int b = 0; b < 2; b++) vq[h][b] = __ldg(a.tiles + ((int64_t)t * m.M + at[h]) * 2 + b);
+      };
+      if (I8) {
+        if (n > 0) load_bytes(grp);
+      } else {
+#pragma unroll
+        for (int d = 0; d < kAhead; d++)
+          if (n > 0) load_words(kTps * d + grp, wq[d]);
+      }
       bool ok = true;
       for (int k = grp; k - grp < n; k += kTps, g++) {
         uint32_t e[32];
+        if (I8) {
 #pragma unroll
-        for (int h = 0; h < 2; h++) tc::expand_pairs(TR ? transpose(wq[0][h]) : wq[0][h], e + 16 * h);
+          for (int h = 0; h < 2; h++)
 #pragma unroll
-        for (int d = 0; d + 1 < kAhead; d++)
+            for (int b = 0; b < 2; b++) i8_pairs<BT>(vq[h][b], e + 16 * h + 8 * b);
+          load_bytes(min(k + kTps, n));
+        } else {
 #pragma unroll
-          for (int h = 0; h < 2; h++) wq[d][h] = wq[d + 1][h];
-        load_words(min(k + kTps * kAhead, n), wq[kAhead - 1]);
+          for (int h = 0; h < 2; h++) tc::expand_pairs(TR ? transpose(wq[0][h]) : wq[0][h], e + 16 * h);
+#pragma unroll
+          for (int d = 0; d + 1 < kAhead; d++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) wq[d][h] = wq[d + 1][h];
+          load_words(min(k + kTps * kAhead, n), wq[kAhead - 1]);
+        }
         if (!ptx::mbar_wait_warp(&sm.done[s2], p2)) {
           ok = false;
           break;
@@ -573,8 +628,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
 #pragma unroll
             for (int u = 0; u < 8; u++)
               *reinterpret_cast<float4*>(mine + c * kEpiBox + ((u ^ (mr & 7)) << 4)) =
-                  have ? make_float4(__uint_as_float(v[4 * u]) * tc::kTwoScale, __uint_as_float(v[4 * u + 1]) * tc::kTwoScale,
-                                     __uint_as_float(v[4 * u + 2]) * tc::kTwoScale, __uint_as_float(v[4 * u + 3]) * tc::kTwoScale)
+                  have ? make_float4(__uint_as_float(v[4 * u]) * kScale, __uint_as_float(v[4 * u + 1]) * kScale,
+                                     __uint_as_float(v[4 * u + 2]) * kScale, __uint_as_float(v[4 * u + 3]) * kScale)
                        : make_float4(0.f, 0.f, 0.f, 0.f);
           }
         }
@@ -612,10 +667,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
   }
 }
 
-template <typename BT, bool TR, bool BAT>
+template <typename BT, int MODE>
 int launch_t(const TsArgs& a, const CUtensorMap& map, const CUtensorMap& mapc, dim3 grid, cudaStream_t s) {
   constexpr size_t smem = sizeof(Smem) + kSmemAlign;
-  auto kern = k_spmm_ts<BT, TR, BAT>;
+  auto kern = k_spmm_ts<BT, MODE>;
   static bool configured[64] = {};
   int dev = 0;
   BSP_CUDA(cudaGetDevice(&dev));
@@ -648,11 +703,16 @@ int launch_ts(TsArgs a, const CUtensorMap& map, bool trans, int splits, cudaStre
     BSP_TRY(make_out_map(&mapc, a.C, rows, a.N, a.ldc, 1, rows * a.ldc));
     a.c_map = true;
   }
+  if (a.tiles) {
+    if (a.bdt == BSP_BF16) return launch_t<__nv_bfloat16, kModeI8>(a, map, mapc, grid, s);
+    if (a.bdt == BSP_F16) return launch_t<__half, kModeI8>(a, map, mapc, grid, s);
+    return BSP_ERR_UNSUPPORTED;
+  }
   if (a.bdt == BSP_BF16)
-    return trans ? launch_t<__nv_bfloat16, true, false>(a, map, mapc, grid, s)
-                 : launch_t<__nv_bfloat16, false, false>(a, map, mapc, grid, s);
+    return trans ? launch_t<__nv_bfloat16, kModeTrans>(a, map, mapc, grid, s)
+                 : launch_t<__nv_bfloat16, kModeBits>(a, map, mapc, grid, s);
   if (a.bdt == BSP_F16)
-    return trans ? launch_t<__half, true, false>(a, map, mapc, grid, s) : launch_t<__half, false, false>(a, map, mapc, grid, s);
+    return trans ? launch_t<__half, kModeTrans>(a, map, mapc, grid, s) : launch_t<__half, kModeBits>(a, map, mapc, grid, s);
   return BSP_ERR_UNSUPPORTED;
 }
 
@@ -669,10 +729,10 @@ int launch_ts_batch(const BatchProblemTc* probs, const int4* items, int n_items,
   memset(&unused, 0, sizeof(unused));
   const dim3 grid((unsigned)n_items);
   if (bdt == BSP_BF16)
-    return trans ? launch_t<__nv_bfloat16, true, true>(a, unused, unused, grid, s)
-                 : launch_t<__nv_bfloat16, false, true>(a, unused, unused, grid, s);
+    return trans ? launch_t<__nv_bfloat16, kModeBatchTrans>(a, unused, unused, grid, s)
+                 : launch_t<__nv_bfloat16, kModeBatch>(a, unused, unused, grid, s);
   if (bdt == BSP_F16)
-    return trans ? launch_t<__half, true, true>(a, unused, unused, grid, s) : launch_t<__half, false, true>(a, unused, unused, grid, s);
+    return trans ? launch_t<__half, kModeBatchTrans>(a, unused, unused, grid, s) : launch_t<__half, kModeBatch>(a, unused, unused, grid, s);
   return BSP_ERR_UNSUPPORTED;
 }
 

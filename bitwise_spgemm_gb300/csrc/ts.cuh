@@ -25,6 +25,7 @@ struct TsArgs {
   // B (or G) in tile order, bt_cb blocks of 256 columns per 32-row tile; null = TMA boxes through the map
   const uint8_t* bt;
   int64_t bt_cb;
+  const uint4* tiles;  // int8 A in [K tile][row][32] order instead of words; null = words
   // batch: work items (problem, 256-row block, 128-column block, K tiles) and the problems' records
   const BatchProblemTc* probs;
   const int4* items;

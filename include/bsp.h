@@ -461,6 +461,22 @@ int bsp_stack_planes_b(const void* B, int b_dtype, int64_t ldb, int64_t K,
                        int64_t N, int n_planes, int is_signed, void* B_out,
                        int64_t ld_out, bsp_stream_t stream);
 
+/* A third form, for a dense weight matrix A that is reused with 16-bit B: the
+ * int8 values themselves as the tensor cores' operand (exact in BF16 and FP16),
+ * one product over K instead of one per plane.  bsp_i8_tiles lays A out as
+ * tiles[ceil(K/32)][M][32], zeros past K, and a bit per 128 x 32 tile with a
+ * nonzero behind it (bsp_i8_tiles_bytes in all, 16-byte aligned);
+ * bsp_spmm_i8_tiles is C = A·B in FP32 from it, for B and C rows that take
+ * 16-byte access and N a multiple of 8 (BSP_ERR_ALIGNMENT) and K up to 131072
+ * (BSP_ERR_CAPACITY); the workspace (may be smaller or NULL) only speeds it
+ * up.  Same reference product as bsp_bitplane_spmm.                          */
+int bsp_i8_tiles_bytes(int64_t M, int64_t K, size_t* bytes);
+int bsp_i8_tiles(const int8_t* A, int64_t M, int64_t K, int64_t lda, int8_t* tiles, bsp_stream_t stream);
+int bsp_spmm_i8_tiles_workspace(int64_t M, int64_t K, int64_t N, size_t* bytes);
+int bsp_spmm_i8_tiles(const int8_t* tiles, int64_t M, int64_t K, const void* B, int b_dtype, int64_t ldb,
+                      int64_t N, float* C, int64_t ldc, void* workspace, size_t workspace_bytes,
+                      bsp_stream_t stream);
+
 int bsp_spmm_i8_workspace(int64_t M, int64_t K, size_t* bytes);
 int bsp_spmm_i8(const int8_t* A, int64_t M, int64_t K, int64_t lda,
                 const void* B, int b_dtype, int64_t ldb, int64_t N, float* C,

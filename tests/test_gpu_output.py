@@ -152,3 +152,30 @@ def test_int8_planes_along_k(kind, M, K, N, d, monkeypatch):
         mat.close()
         ms, _, mn = O.rel_errors(C, C64, Cabs)
         assert ms <= tol, (tc, ms, mn)
+
+
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("M,K,N", [(128, 64, 8), (129, 33, 136), (300, 1000, 264), (1000, 3001, 520), (64, 8192, 128),
+                                   (5000, 257, 2048), (2400, 5000, 2304)])
+def test_int8_values_on_tensor_cores(M, K, N, dt):
+    """The product of int8 values kept in the tensor cores' order: every byte
+    value, empty tiles, row and column remainders, split reductions, tiled B.
+    Integer operands with |sum| <= 4 * 128 * nnz(row) < 2^24: exact in FP32."""
+    rng = np.random.default_rng(M + K + N)
+    A = (rng.integers(-128, 128, (M, K)) * (rng.random((M, K)) < 0.3)).astype(np.int8)
+    A[:, 32:64] = 0
+    A[0, :min(K, 256)] = np.arange(-128, 128)[:min(K, 256)]
+    B = rng.integers(-4, 5, (K, N))
+    mat = ops.Int8Matrix(dev(A))
+    assert mat.tiles is not None
+    Bt = torch.from_numpy(B).cuda().to(torch.bfloat16 if dt == "bf16" else torch.float16)
+    got = mat.matmul(Bt).cpu().numpy()
+    out = torch.full((M, N + 8), 7.0, device="cuda")
+    mat.matmul(Bt, out=out[:, :N])
+    wide = torch.zeros((K, N + 1), dtype=Bt.dtype, device="cuda")  # rows off the 16-byte grid: as planes
+    wide[:, :N] = Bt
+    planes = mat.matmul(wide[:, :N]).cpu().numpy()
+    mat.close()
+    want = A.astype(np.float64) @ B.astype(np.float64)
+    assert np.array_equal(got, want) and np.array_equal(out[:, :N].cpu().numpy(), want)
+    assert (out[:, N:] == 7.0).all() and np.array_equal(planes, want)
