@@ -97,6 +97,7 @@ SIGNATURES = {
     "bsp_spmm_i8_workspace": [_I64, _I64, C.POINTER(_SZ)],
     "bsp_spmm_workspace_layout": [_P, _I64, _I64, _P, _I, _I64, C.POINTER(_SZ)],
     "bsp_spmm_workspace_preferred": [_P, _I64, C.POINTER(_SZ)],
+    "bsp_spmm_t_workspace_layout": [_P, _I64, _I64, _I64, _I, C.POINTER(_SZ)],
     "bsp_spmm_t_workspace_preferred": [_I64, _I64, _I64, C.POINTER(_SZ)],
     "bsp_tune": [_P, _I64, _I64, _P, _I, _I64, _I64, _P, _I64, _P, _P, _SZ, _P, C.POINTER(Schedule)],
     "bsp_tune_cache_load": [C.c_char_p, C.POINTER(_I)],

@@ -88,7 +88,7 @@ int launch_pack_rows(const void* dense, int dtype, int64_t M, int64_t K, int64_t
 int launch_pack_cols(const void* dense, int dtype, int64_t M, int64_t K, int64_t ld,
                      uint32_t* words_t, int msb, cudaStream_t s);
 int launch_transpose_bits(const uint32_t* words, int64_t M, int64_t K, uint32_t* words_t,
-                          cudaStream_t s);
+                          cudaStream_t s, const int* run_if = nullptr);
 int launch_unpack_rows(const uint32_t* words, int64_t M, int64_t K, void* dense, int dtype,
                        int64_t ld, int msb, cudaStream_t s);
 // rows_layout: words[M][planes][Kw] (planes of a row side by side) instead

@@ -230,7 +230,34 @@ static int64_t proto_ldp(int64_t N) { return (N + 7) / 8 * 8; }
 // Layouts without 16-byte access pay for a flag, B's tile order and the walk
 // that stands by for it: about 8 us of launches (4093x495x102 BF16 behind a new
 // plan: 10 us slower on the tensor cores than without).
+// FP32 B goes there as three BF16 parts, exact in B, where the dense products
+// cost less than the walk's gathers at their 17 TB/s and the parts' traffic
+// (10 bytes per value of B, 32 of C) and launches (walk and parts in us:
+// 512x512x256 at 10 % 4.7 and 21.5, 1024x1024x1024 at 5 % 19.6 and 28,
+// 2048x2048x256 at 10 % 29 and 27, 2048x2048x1024 at 2 % 31 and 48, at 5 % 57
+// and 49, at 10 % 97 and 49; the rule picks the smaller one each time).  B
+// whose values span too many octaves is left to the walk on the device
+// (k_split_b), and so is a reduction of more than 4096 rows: the walk sums
+// longer rows with compensation.
+constexpr int64_t kPartsMaxReduction = 4096;
+constexpr size_t kPartsMaxBytes = (size_t)4 << 30;
+static bool parts_pay(double tiles, double gathers, int64_t out_rows, int64_t N, int64_t red_rows) {
+  if (red_rows > kPartsMaxReduction || N > (int64_t)1 << 21) return false;
+  if (tc_parts_bytes(out_rows, N, red_rows) > kPartsMaxBytes) return false;
+  const char* e = getenv("BSP_TC");
+  if (e) return e[0] == '1';
+  const double n = (double)N;
+  const double tc = tiles * 8192.0 * 3.0 * n / 1.2e15 + ((double)red_rows * 10.0 + (double)out_rows * 32.0) * n / 8e12;
+  return tc + 12e-6 < gathers * n * 4.0 / 17e12;
+}
+
 static bool use_tensor_cores(const bsp_plan* plan, int64_t N, int esize, bool vec) {
+  if (esize == 4) {
+    double g = (double)plan->nnz;
+    if (plan->mode == BSP_PLAN_PROTO)
+      g = (double)(plan->proto_nnz + plan->delta_nnz + plan->direct_nnz + plan->M);
+    return parts_pay((double)plan->occ_tiles, g, plan->M, N, plan->K);
+  }
   if (plan->K > tc_max_reduction()) return false;
   const char* e = getenv("BSP_TC");
   if (e) return e[0] == '1';
@@ -318,6 +345,12 @@ static int run_spmm(SpmmArgs a, const bsp_plan* plan, bool vec, const TuneSched&
   // contraction cheaper than gathering B rows.
   if (sc.engine == 1) {
     const int* skipped = nullptr;
+    if (a.bdt == BSP_F32) {
+      BSP_TRY(launch_spmm_parts(a.A, a.M, a.K, plan->occ, plan->wordsT, static_cast<const float*>(a.B), a.ldb, a.N,
+                                a.C, a.ldc, false, s, workspace, workspace_bytes, &skipped));
+      a.run_if = skipped;
+      return launch_spmm_rows(a, vec, s);
+    }
     BSP_TRY(launch_spmm_tc(a, plan->occ, plan->wordsT, vec, s, workspace, workspace_bytes,
                            TcForm{sc.tc_tps, sc.tc_tiled, sc.tc_split}, &skipped));
     if (!skipped) return BSP_OK;
@@ -402,6 +435,10 @@ int bsp_spmm_workspace_layout(const bsp_plan* plan, int64_t K, int64_t N, const 
   if (K < 0 || (b_dtype != BSP_F32 && b_dtype != BSP_BF16 && b_dtype != BSP_F16)) return BSP_ERR_INVALID_ARG;
   BSP_TRY(bsp_spmm_workspace_preferred(plan, N, bytes));
   const int esz = dtype_size(b_dtype);
+  if (plan && b_dtype == BSP_F32 && N > 0 && use_tensor_cores(plan, N, esz, true)) {
+    const size_t parts = tc_parts_bytes(plan->M, N, plan->K);
+    if (parts > *bytes) *bytes = parts;
+  }
   if (is_aligned(B, 16) && (ldb * esz) % 16 == 0 && (N * esz) % 16 == 0) return BSP_OK;
   size_t base = 0;
   BSP_TRY(bsp_spmm_workspace(plan, N, &base));
@@ -448,6 +485,9 @@ static int prepare_spmm(const uint32_t* A_words, int64_t M, int64_t K, const voi
   // 16-bit B by TMA boxes, or copied into tile order where its rows take none
   *tc_ok = plan && b_dtype != BSP_F32 && plan->K <= tc_max_reduction() &&
            (*vec || (workspace && workspace_bytes >= tc_tiled_b_bytes(K, N)));
+  // FP32 as parts, where there is room for them
+  if (plan && b_dtype == BSP_F32 && K <= kPartsMaxReduction && N <= (int64_t)1 << 21)
+    *tc_ok = workspace && workspace_bytes >= tc_parts_bytes(M, N, K);
   *esz_out = esz;
   return BSP_OK;
 }
@@ -490,7 +530,12 @@ int bsp_tune(const uint32_t* A_words, int64_t M, int64_t K, const void* B, int b
   // plan has no prototypes
   TuneSched cand[4 + 9 + 8];
   int nc = 0;
-  if (tc_ok)
+  if (tc_ok && b_dtype == BSP_F32) {
+    TuneSched t;
+    t.engine = 1;
+    t.tc_tps = 2;
+    cand[nc++] = t;
+  } else if (tc_ok)
     for (int tiled = 0; tiled <= 1; tiled++)
       for (int split = -1; split <= 0; split++) {
         TuneSched t;
@@ -785,6 +830,20 @@ int bsp_spmm_t_workspace_preferred(int64_t M, int64_t K, int64_t N, size_t* byte
   return BSP_OK;
 }
 
+int bsp_spmm_t_workspace_layout(const bsp_plan* plan, int64_t M, int64_t K, int64_t N, int g_dtype, size_t* bytes) {
+  if (g_dtype != BSP_F32 && g_dtype != BSP_BF16 && g_dtype != BSP_F16) return BSP_ERR_INVALID_ARG;
+  BSP_TRY(bsp_spmm_t_workspace_preferred(M, K, N, bytes));
+  if (plan && (plan->M != M || plan->K != K)) return BSP_ERR_INVALID_ARG;
+  if (plan && g_dtype == BSP_F32 && M > 0 && K > 0 && N > 0 &&
+      parts_pay((double)plan->occT_tiles, (double)plan->nnz, K, N, M)) {
+    size_t need = 0;
+    BSP_TRY(bsp_spmm_t_workspace(M, K, &need));
+    need += tc_parts_bytes(K, N, M);
+    if (need > *bytes) *bytes = need;
+  }
+  return BSP_OK;
+}
+
 int bsp_spmm_t_workspace(int64_t M, int64_t K, size_t* bytes) {
   if (!bytes || M < 0 || K < 0) return BSP_ERR_INVALID_ARG;
   *bytes = sizeof(uint32_t) * (size_t)K * (size_t)ceil_div(M, 32) + 256;
@@ -823,11 +882,17 @@ int bsp_spmm_t(const uint32_t* A_words, int64_t M, int64_t K, const void* G, int
                               workspace_bytes);
   }
   // CUDA cores: transpose the bits into the workspace, then walk the rows of Aᵀ
+  // (after FP32 parts on the tensor cores: only if they left dX alone)
   size_t need = 0;
   bsp_spmm_t_workspace(M, K, &need);
   if (!workspace || workspace_bytes < need) return BSP_ERR_WORKSPACE;
   uint32_t* At = reinterpret_cast<uint32_t*>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~uintptr_t(255));
-  BSP_TRY(launch_transpose_bits(A_words, M, K, At, s));
+  const int* skipped = nullptr;
+  if (plan && g_dtype == BSP_F32 && parts_pay((double)plan->occT_tiles, (double)plan->nnz, K, N, M) &&
+      workspace_bytes >= need + tc_parts_bytes(K, N, M))
+    BSP_TRY(launch_spmm_parts(A_words, M, K, plan->occT, plan->wordsT, static_cast<const float*>(G), ldg, N, dX, lddx,
+                              true, s, static_cast<char*>(workspace) + need, workspace_bytes - need, &skipped));
+  BSP_TRY(launch_transpose_bits(A_words, M, K, At, s, skipped));
   SpmmArgs a = {};
   a.A = At;
   a.M = K;
@@ -841,6 +906,7 @@ int bsp_spmm_t(const uint32_t* A_words, int64_t M, int64_t K, const void* G, int
   a.ldc = lddx;
   a.Nb = N;
   a.c_vec = layout16(dX, lddx, 4, N, 4);
+  a.run_if = skipped;
   return launch_spmm_rows(a, vec || layout16(G, ldg, esz, N, vcols), s);
 }
 

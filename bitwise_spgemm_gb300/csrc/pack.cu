@@ -179,7 +179,9 @@ __global__ void __launch_bounds__(256) k_pack_cols(const typename Elem<DT>::T* _
 // j across lanes is column 32w+j of the transpose.
 __global__ void __launch_bounds__(256) k_transpose_bits(const uint32_t* __restrict__ words,
                                                         int64_t M, int64_t Kw, int64_t K,
-                                                        uint32_t* __restrict__ words_t, int64_t Mw) {
+                                                        uint32_t* __restrict__ words_t, int64_t Mw,
+                                                        const int* __restrict__ run_if) {
+  if (run_if && !__ldg(run_if)) return;
   const int lane = threadIdx.x & 31;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -360,9 +362,9 @@ int launch_pack_cols(const void* dense, int dtype, int64_t M, int64_t K, int64_t
 }
 
 int launch_transpose_bits(const uint32_t* words, int64_t M, int64_t K, uint32_t* words_t,
-                          cudaStream_t s) {
+                          cudaStream_t s, const int* run_if) {
   const int64_t Kw = ceil_div(K, 32), Mw = ceil_div(M, 32);
-  k_transpose_bits<<<grid_for(Mw * Kw), 256, 0, s>>>(words, M, Kw, K, words_t, Mw);
+  k_transpose_bits<<<grid_for(Mw * Kw), 256, 0, s>>>(words, M, Kw, K, words_t, Mw, run_if);
   BSP_LAUNCHED();
   return BSP_OK;
 }

@@ -121,6 +121,14 @@ size_t tc_split_bytes(int64_t out_rows, int64_t out_cols, int64_t red_tiles);
 // both splits the reduction (when it would) and tiles B.
 size_t tc_tiled_b_bytes(int64_t red_rows, int64_t cols);
 size_t tc_preferred_bytes(int64_t out_rows, int64_t out_cols, int64_t red_rows);
+// FP32 B (any layout) on the tensor cores as three exact BF16 parts: C = A·B, or
+// dX = Aᵀ·G with occT; the workspace must hold tc_parts_bytes(output rows, N,
+// reduction rows).  *skipped: a device flag, nonzero when C was left to the
+// walking kernels (values outside the parts' range).
+size_t tc_parts_bytes(int64_t out_rows, int64_t N, int64_t red_rows);
+int launch_spmm_parts(const uint32_t* A, int64_t M, int64_t K, const uint32_t* occ, const uint32_t* At, const float* B,
+                      int64_t ldb, int64_t N, float* C, int64_t ldc, bool trans, cudaStream_t s, void* ws,
+                      size_t ws_bytes, const int** skipped);
 // dX[K][N] = Aᵀ·G on the tensor cores, Aᵀ read from A's row words
 int launch_spmm_t_tc(const uint32_t* A, int64_t M, int64_t K, const void* G, int gdt, int64_t ldg, int64_t N,
                      float* dX, int64_t lddx, const uint32_t* occT, const uint32_t* At, cudaStream_t s, void* ws = nullptr, size_t ws_bytes = 0);

@@ -548,6 +548,145 @@ __global__ void __launch_bounds__(256) k_tile_b(const uint8_t* __restrict__ B, i
   if (!VEC && bad) *flag = 1;
 }
 
+// FP32 B [R][N] as three BF16 parts in tile order: part p of column c is column
+// p*Np + c of the tiles (Np = N rounded up to 8).  x = h + m + l exactly: each
+// part takes the next 8 bits of the significand, rounded, and what is left of
+// 24 bits after two of them fits the third, as long as no part leaves BF16's
+// normal range.  The flag is set by any x that is not 0 or in [2^-100, 2^100),
+// infinities and NaN among them, and where the largest exponent is more than
+// kPartsOctaves above the mean one: the tensor cores' sums truncate, which
+// costs nothing while the first parts' 8 bits add up exactly in 24, as they do
+// for values of about one size (normal values: 3.5 octaves).  Rows past R are
+// zero; columns past 3 Np stay as they are (each column of a product depends
+// on its own alone).  Bound by memory: 4 bytes in, 6 out per value.
+constexpr int kPartsOctaves = 6;
+struct PartsStats {  // zeroed before the kernel
+  int flag, max_exp;
+  unsigned blocks_done, pad;
+  unsigned long long nonzeros, exp_sum;
+};
+template <bool VEC>
+__global__ void __launch_bounds__(256) k_split_b(const float* __restrict__ B, int64_t R, int64_t N, int64_t ldb,
+                                                 int64_t ntiles, int64_t ncb, uint4* __restrict__ bt,
+                                                 PartsStats* st) {
+  const uint32_t q = (uint32_t)((N + 7) / 8);
+  const int64_t rows = ntiles * kTcK;
+  bool bad = false;
+  int top = 0;
+  unsigned long long nonzeros = 0, exps = 0;
+  for (int64_t row = blockIdx.y; row < rows; row += gridDim.y) {
+    for (uint32_t c8 = blockIdx.x * blockDim.x + threadIdx.x; c8 < q; c8 += gridDim.x * blockDim.x) {
+      const int64_t col = (int64_t)c8 * 8;
+      float x[8];
+#pragma unroll
+      for (int i = 0; i < 8; i++) x[i] = 0.f;
+      if (row < R) {
+        const float* p = B + row * ldb + col;
+        if (VEC && col + 8 <= N) {
+          const float4 u = __ldg(reinterpret_cast<const float4*>(p)), v = __ldg(reinterpret_cast<const float4*>(p) + 1);
+          x[0] = u.x, x[1] = u.y, x[2] = u.z, x[3] = u.w;
+          x[4] = v.x, x[5] = v.y, x[6] = v.z, x[7] = v.w;
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; i++)
+            if (col + i < N) x[i] = __ldg(p + i);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const uint32_t e = (__float_as_uint(x[i]) >> 23) & 255u;
+        bad |= x[i] != 0.f && (e < 27u || e >= 227u);
+        top = max(top, (int)e);
+        nonzeros += x[i] != 0.f;
+        exps += e;
+      }
+#pragma unroll
+      for (int part = 0; part < 3; part++) {
+        uint32_t w[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const __nv_bfloat162 b = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
+          w[i] = *reinterpret_cast<const uint32_t*>(&b);
+          x[2 * i] -= __low2float(b);
+          x[2 * i + 1] -= __high2float(b);
+        }
+        const int64_t c = ((int64_t)part * q + c8) * 8, cb = c / kTcN;
+        const int in = (int)(c - cb * kTcN), j = in / kBoxCols, ch = (in % kBoxCols) / 8, r = (int)(row % kTcK);
+        bt[((row / kTcK) * ncb + cb) * 1024 + j * 256 + r * 8 + (ch ^ (r & 7))] = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+    }
+  }
+  // the block's figures, and the verdict by the block that comes last
+  __shared__ unsigned long long s_n[8], s_e[8];
+  __shared__ int s_top[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    nonzeros += __shfl_xor_sync(kFull, nonzeros, o);
+    exps += __shfl_xor_sync(kFull, exps, o);
+  }
+  top = __reduce_max_sync(kFull, top);
+  if (lane == 0) s_n[warp] = nonzeros, s_e[warp] = exps, s_top[warp] = top;
+  bad = __syncthreads_or(bad);
+  if (threadIdx.x != 0) return;
+  for (unsigned w = 1; w < blockDim.x / 32; w++) {
+    nonzeros += s_n[w];
+    exps += s_e[w];
+    top = max(top, s_top[w]);
+  }
+  if (bad) atomicExch(&st->flag, 1);
+  atomicMax(&st->max_exp, top);
+  atomicAdd(&st->nonzeros, nonzeros);
+  atomicAdd(&st->exp_sum, exps);
+  __threadfence();
+  if (atomicAdd(&st->blocks_done, 1u) + 1u == gridDim.x * gridDim.y) {
+    __threadfence();
+    const unsigned long long n = atomicAdd(&st->nonzeros, 0ull), e = atomicAdd(&st->exp_sum, 0ull);
+    const unsigned long long m = (unsigned long long)atomicMax(&st->max_exp, 0);
+    if (m * n > e + (unsigned long long)kPartsOctaves * n) atomicExch(&st->flag, 1);
+  }
+}
+
+// C = (Σ_z l + Σ_z m) + Σ_z h over the splits z (ascending), from the three
+// parts' products side by side (rows of 3 Np floats); four columns per thread.
+__global__ void __launch_bounds__(256) k_join_parts(const float* __restrict__ part, int64_t Np, int64_t stride,
+                                                    int splits, int64_t rows, int64_t cols, float* __restrict__ C,
+                                                    int64_t ldc, bool c_vec, const int* __restrict__ skip_if) {
+  if (__ldg(skip_if)) return;
+  const uint32_t q = (uint32_t)((cols + 3) / 4);
+  for (int64_t r = blockIdx.y; r < rows; r += gridDim.y) {
+    for (uint32_t c4 = blockIdx.x * blockDim.x + threadIdx.x; c4 < q; c4 += gridDim.x * blockDim.x) {
+      const int64_t c = (int64_t)c4 * 4;
+      float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int p = 2; p >= 0; p--) {
+        const float* at = part + r * 3 * Np + p * Np + c;
+        float4 acc = __ldg(reinterpret_cast<const float4*>(at));
+        for (int z = 1; z < splits; z++) {
+          const float4 v = __ldg(reinterpret_cast<const float4*>(at + z * stride));
+          acc.x += v.x;
+          acc.y += v.y;
+          acc.z += v.z;
+          acc.w += v.w;
+        }
+        sum.x += acc.x;
+        sum.y += acc.y;
+        sum.z += acc.z;
+        sum.w += acc.w;
+      }
+      float* o = C + r * ldc + c;
+      if (c_vec) {
+        *reinterpret_cast<float4*>(o) = sum;
+      } else {
+        o[0] = sum.x;
+        if (c + 1 < cols) o[1] = sum.y;
+        if (c + 2 < cols) o[2] = sum.z;
+        if (c + 3 < cols) o[3] = sum.w;
+      }
+    }
+  }
+}
+
 // Both occupancy bitmaps in one pass over A's words.  A block of 4 warps
 // covers 128 rows x 32 word columns: thread (warp j, lane l) ORs the 32 rows
 // of row tile 4·blockIdx.y + j in word column 32·blockIdx.x + l (coalesced
@@ -847,6 +986,85 @@ int launch_product(TsArgs a, const void* B, int64_t ldb, bool vec, bool trans, c
   return BSP_OK;
 }
 }  // namespace
+
+// The room that an FP32 product on the tensor cores takes: the parts' products, B's parts in tile order.
+static int64_t parts_cols(int64_t N) { return ceil_div(N, 8) * 8; }
+size_t tc_parts_bytes(int64_t out_rows, int64_t N, int64_t red_rows) {
+  const int64_t n3 = 3 * parts_cols(N);
+  const int S = tc_split_count(out_rows, n3, ceil_div(red_rows, kTcK));
+  return (size_t)S * (size_t)out_rows * (size_t)n3 * sizeof(float) + 256 + tc_tiled_b_bytes(red_rows, n3);
+}
+
+// C = A·B (trans: dX = Aᵀ·G) for FP32 B on the tensor cores, exact in B: its
+// three BF16 parts are multiplied as 3N columns, each with accumulators of its
+// own, and joined afterwards.  2048x2048x1024 at 10 %: walk 97 us, here 49
+// (Aᵀ·G 99 and 51); 4096x4096x2048 at 5 % 389 and 188.  Bound there by the
+// tensor kernel's producers, below about 1024x1024x1024 by its five launches.
+// Errors against FP64, relative in the Frobenius norm, walk and here:
+// normal values 2.6e-7 and 2.7e-8, their magnitudes 2.2e-7 and 3.5e-8
+// (512x512x256 9.7e-8 and 2.5e-8, 1024x4096x512 3.7e-7 and 2.8e-8): the first
+// part's 8 bits add up nearly exactly.
+static int launch_parts(TsArgs a, const float* B, int64_t ldb, int64_t N, float* C, int64_t ldc, bool trans,
+                        cudaStream_t s, void* ws, size_t ws_bytes, const int** skipped) {
+  const int64_t rows = trans ? a.K : a.M, red_rows = trans ? a.M : a.K;
+  if (a.M > INT32_MAX || a.K > INT32_MAX || N > INT32_MAX / 4) return BSP_ERR_CAPACITY;
+  if (ceil_div(red_rows, kTcK) > kListMax) return BSP_ERR_CAPACITY;
+  if (!ws || ws_bytes < tc_parts_bytes(rows, N, red_rows)) return BSP_ERR_WORKSPACE;
+  const int64_t Np = parts_cols(N), n3 = 3 * Np, ntiles = ceil_div(red_rows, kTcK), ncb = ceil_div(n3, kTcN);
+  const int splits = tc_split_count(rows, n3, ntiles);
+  float* part = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(ws) + 255) & ~(uintptr_t)255);
+  uint8_t* bt = reinterpret_cast<uint8_t*>(
+      (reinterpret_cast<uintptr_t>(part + (int64_t)splits * rows * n3) + 256 + 1023) & ~(uintptr_t)1023);
+  PartsStats* stats = reinterpret_cast<PartsStats*>(bt - 256);
+  int* flag = &stats->flag;
+  BSP_CUDA(cudaMemsetAsync(stats, 0, sizeof(PartsStats), s));
+  const int64_t q = Np / 8;
+  const unsigned t = q >= 256 ? 256 : (unsigned)(ceil_div(q, 32) * 32);
+  const unsigned gx = (unsigned)(ceil_div(q, t) < 1024 ? ceil_div(q, t) : 1024);
+  const int64_t blocks = ceil_div((int64_t)num_sms() * 8, gx);
+  const int64_t gy = blocks < ntiles * kTcK ? blocks : ntiles * kTcK;
+  const bool vec = is_aligned(B, 16) && ldb % 4 == 0;
+  (vec ? k_split_b<true> : k_split_b<false>)<<<dim3(gx, (unsigned)(gy < 65535 ? gy : 65535)), t, 0, s>>>(
+      B, red_rows, N, ldb, ntiles, ncb, reinterpret_cast<uint4*>(bt), stats);
+  BSP_LAUNCHED();
+  a.N = n3;
+  a.bdt = BSP_BF16;
+  a.bt = bt;
+  a.bt_cb = ncb;
+  a.C = part;
+  a.ldc = n3;
+  a.c_vec = true;
+  a.part = part;
+  a.ldp = n3;
+  a.part_stride = rows * n3;
+  a.skip_if = flag;
+  CUtensorMap map;
+  memset(&map, 0, sizeof(map));
+  BSP_TRY(launch_ts(a, map, trans, splits, s));
+  const int64_t q4 = ceil_div(N, 4);
+  const unsigned t4 = q4 >= 256 ? 256 : (unsigned)(ceil_div(q4, 32) * 32);
+  const unsigned gx4 = (unsigned)(ceil_div(q4, t4) < 1024 ? ceil_div(q4, t4) : 1024);
+  const bool c_vec = is_aligned(C, 16) && ldc % 4 == 0 && N % 4 == 0;
+  k_join_parts<<<dim3(gx4, (unsigned)(rows < 65535 ? rows : 65535)), t4, 0, s>>>(part, Np, rows * n3, splits, rows, N,
+                                                                               C, ldc, c_vec, flag);
+  BSP_LAUNCHED();
+  *skipped = flag;
+  return BSP_OK;
+}
+
+int launch_spmm_parts(const uint32_t* A, int64_t M, int64_t K, const uint32_t* occ, const uint32_t* At, const float* B,
+                      int64_t ldb, int64_t N, float* C, int64_t ldc, bool trans, cudaStream_t s, void* ws,
+                      size_t ws_bytes, const int** skipped) {
+  TsArgs a = {};
+  a.At = At;
+  a.A = A;
+  a.M = M;
+  a.K = K;
+  a.Kw = ceil_div(K, 32);
+  a.occ = occ;
+  a.occ_words = trans ? tc_occupancy_t_words(M) : tc_occupancy_words(K);
+  return launch_parts(a, B, ldb, N, C, ldc, trans, s, ws, ws_bytes, skipped);
+}
 
 int launch_spmm_tc(const SpmmArgs& sa, const uint32_t* occ, const uint32_t* At, bool vec, cudaStream_t s, void* ws,
                    size_t ws_bytes, TcForm form, const int** skipped) {

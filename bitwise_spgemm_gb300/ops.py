@@ -205,7 +205,8 @@ def spmm_t(words, M, K, G, plan=None, out=None, workspace=None):
         out = torch.empty((K, N), dtype=torch.float32, device=G.device)
     n_min, n_pref = C.c_size_t(), C.c_size_t()
     call("bsp_spmm_t_workspace", M, K, C.byref(n_min))
-    call("bsp_spmm_t_workspace_preferred", M, K, N, C.byref(n_pref))
+    call("bsp_spmm_t_workspace_layout", plan.handle if plan is not None else None, M, K, N, _DT[G.dtype],
+         C.byref(n_pref))
     # a caller's workspace is used if it holds the minimum; else the preferred size
     if workspace is None or workspace.numel() * workspace.element_size() < n_min.value:
         workspace = torch.empty(n_pref.value, dtype=torch.uint8, device=G.device)
@@ -243,7 +244,9 @@ def tune(words, K, B, plan, out=None, workspace=None):
         out = torch.empty((M, N), dtype=torch.float32, device=B.device)
     need = plan.workspace_bytes(N)
     if workspace is None or workspace.numel() * workspace.element_size() < need:
-        workspace = torch.empty(max(need, 1), dtype=torch.uint8, device=B.device)
+        n = C.c_size_t()
+        call("bsp_spmm_workspace_layout", plan.handle, K, N, _p(B), _DT[B.dtype], ldb, C.byref(n))
+        workspace = torch.empty(max(n.value, 1), dtype=torch.uint8, device=B.device)
     best = capi.Schedule()
     call("bsp_tune", _p(words), M, K, _p(B), _DT[B.dtype], ldb, N, _p(out), out.stride(0), plan.handle,
          _p(workspace), workspace.numel() * workspace.element_size(), _stream(), C.byref(best))

@@ -221,8 +221,11 @@ int bsp_spmm_workspace_preferred(const bsp_plan* plan, int64_t N, size_t* bytes)
 
 /* Workspace for these operands: the above and, where B's rows do not take
  * 16-byte loads (B, ldb or N not a multiple of 16 bytes; plan may be NULL),
- * room for a copy of B that does.  A smaller workspace only turns the copy
- * off (results are identical).  B is looked at as an address, not read.     */
+ * room for a copy of B that does; for FP32 B whose product is cheaper on the
+ * tensor cores, room for its three BF16 parts (exact: x = h + m + l) and their
+ * products.  A smaller workspace only turns these off (the copy changes no
+ * result, the parts change the order of the FP32 sums).  B is looked at as an
+ * address, not read.                                                        */
 int bsp_spmm_workspace_layout(const bsp_plan* plan, int64_t K, int64_t N, const void* B, int b_dtype,
                               int64_t ldb, size_t* bytes);
 
@@ -369,7 +372,8 @@ int bsp_tune_cache_size(int* entries);
 /* ======================================================================== */
 
 /* dX[K×N] (FP32, row stride lddx) = Aᵀ·G for G[M×N] of g_dtype (row stride
- * ldg).  With a plan and 16-bit G the tensor cores read Aᵀ's bit tiles
+ * ldg).  With a plan, 16-bit G, or FP32 G and room for its parts, the tensor
+ * cores read Aᵀ's bit tiles
  * straight from A's row words (no transposed copy is made); otherwise the
  * bits are transposed into the workspace (bsp_spmm_t_workspace bytes) and
  * walked like bsp_spmm.  The backward of the forward SpMM; no reference
@@ -377,6 +381,9 @@ int bsp_tune_cache_size(int* entries);
 int bsp_spmm_t_workspace(int64_t M, int64_t K, size_t* bytes);
 /* ... and with room for the tensor-core reduction split (as for bsp_spmm). */
 int bsp_spmm_t_workspace_preferred(int64_t M, int64_t K, int64_t N, size_t* bytes);
+/* ... for these operands: also with the room that FP32 G takes on the tensor
+ * cores where the plan makes that the faster way (plan may be NULL).        */
+int bsp_spmm_t_workspace_layout(const bsp_plan* plan, int64_t M, int64_t K, int64_t N, int g_dtype, size_t* bytes);
 int bsp_spmm_t(const uint32_t* A_words, int64_t M, int64_t K, const void* G,
                int g_dtype, int64_t ldg, int64_t N, float* dX, int64_t lddx,
                const bsp_plan* plan, void* workspace, size_t workspace_bytes,

@@ -247,3 +247,50 @@ def test_three_tile_stages(force_tc, kind, M, K, N, p):
     C = ops.spmm(wd, K, B, plan=plan).cpu().numpy()
     mx, _, _ = O.rel_errors(C, O.spmm_f64(words, K, Bexact), O.spmm_abs_f64(words, K, Bexact))
     assert mx <= TOL
+
+
+@pytest.mark.parametrize("M,K,N,p", [(1, 33, 1, 0.5), (128, 64, 8, 0.3), (257, 129, 43, 0.2), (300, 1000, 201, 0.2),
+                                     (64, 4096, 256, 0.3), (4096, 64, 40, 0.3), (1000, 3000, 520, 0.1)])
+def test_f32_parts(force_tc, M, K, N, p):
+    """FP32 operands as three BF16 parts: exact where the sums are (integers of
+    13 bits, |sum| < 2^24), otherwise within the bound of truncating sums of 16
+    products each; a value outside the parts' range, or values of very different
+    sizes, leave the whole product to the walk."""
+    rng = np.random.default_rng(M + K + N)
+    bits = rng.random((M, K)) < p
+    words = W.pack_bits(bits)
+    wd = words_dev(words)
+    plan = ops.Plan(wd, K)
+    pad = 3 if N % 2 else 0
+    mk = lambda a: torch.nn.functional.pad(torch.from_numpy(a), (0, pad)).cuda()[:, :N]
+    B, G = rng.integers(-4000, 4001, (K, N)).astype(np.float32), rng.integers(-4000, 4001, (M, N)).astype(np.float32)
+    out = torch.full((M, N + 5), 7.0, device="cuda")
+    ops.spmm(wd, K, mk(B), plan=plan, out=out[:, :N])
+    assert np.array_equal(out[:, :N].cpu().numpy().astype(np.float64), O.spmm_f64(words, K, B))
+    assert torch.all(out[:, N:] == 7.0)
+    dX = ops.spmm_t(wd, M, K, mk(G), plan=plan).cpu().numpy()
+    assert np.array_equal(dX.astype(np.float64), O.spmm_t_f64(words, M, K, G))
+    B, G = rng.standard_normal((K, N)).astype(np.float32), rng.standard_normal((M, N)).astype(np.float32)
+    C = ops.spmm(wd, K, mk(B), plan=plan).cpu().numpy()
+    err = np.abs(C - O.spmm_f64(words, K, B))
+    # each of ceil(K/16) steps loses at most 2 units of 2^-23 of the sum so far
+    assert np.all(err <= (-(-K // 16) + 4) * 2.0**-22 * O.spmm_abs_f64(words, K, B) + 1e-30)
+    dX = ops.spmm_t(wd, M, K, mk(G), plan=plan).cpu().numpy()
+    assert np.all(np.abs(dX - O.spmm_t_f64(words, M, K, G))
+                  <= (-(-M // 16) + 4) * 2.0**-22 * (bits.T.astype(np.float64) @ np.abs(G)) + 1e-30)
+    heavy = np.exp(6 * rng.standard_normal(max(M, K) * N)).astype(np.float32)  # sums that lose bits by truncation
+    for bad in (float("inf"), float("nan"), 1e38, 1e-38, None):
+        if bad is None:
+            if min(M, K) * N < 1000:
+                continue
+            B, G = heavy[:K * N].reshape(K, N), heavy[:M * N].reshape(M, N)
+        else:
+            B[K // 2, N // 2] = bad
+            G[M // 2, N // 2] = bad
+        got = ops.spmm(wd, K, mk(B), plan=plan), ops.spmm_t(wd, M, K, mk(G), plan=plan)
+        os.environ["BSP_TC"] = "0"
+        want = ops.spmm(wd, K, mk(B), plan=plan), ops.spmm_t(wd, M, K, mk(G), plan=plan)
+        os.environ["BSP_TC"] = "1"
+        for g, w in zip(got, want):
+            assert torch.equal(g.view(torch.int32), w.view(torch.int32))
+    assert capi.device_status() == 0
