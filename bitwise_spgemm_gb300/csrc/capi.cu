@@ -910,6 +910,17 @@ int bsp_spmm_t(const uint32_t* A_words, int64_t M, int64_t K, const void* G, int
   return launch_spmm_rows(a, vec || layout16(G, ldg, esz, N, vcols), s);
 }
 
+// FP32 products with X staged for 32 rows of A pay where those rows share its
+// rows, the sooner the more columns a staged row has (staged and walk in us:
+// 2048x2048, N = 1024: 2 % 55 and 56, 3 % 60 and 77, 10 % 95 and 206; N = 256,
+// 5 % 28 and 34; N = 128, 5 % 26 and 27; 512x512, N = 64, 10 % 9.8 and 12.1;
+// 128x128, N = 128, 10 % 5.7 and 5.3).
+static bool staged_pays(const bsp_plan* plan, int64_t N) {
+  const double rows = plan->M < 32 ? (double)plan->M : 32.0;
+  const double density = (double)plan->nnz / ((double)plan->M * (double)plan->K);
+  return (double)plan->nnz * (double)N >= 1e6 && rows * density >= 32.0 * (0.02 + 4.0 / (double)N);
+}
+
 int bsp_sddmm(const uint32_t* A_words, int64_t M, int64_t K, const void* G, int64_t ldg, const void* X,
               int64_t ldx, int dtype, int64_t N, float* dA, int64_t ldda, const bsp_plan* plan,
               bsp_stream_t stream) {
@@ -935,17 +946,22 @@ int bsp_sddmm(const uint32_t* A_words, int64_t M, int64_t K, const void* G, int6
     tc = dense < cores;
   }
   if (tc) return launch_sddmm_tc(A_words, M, K, G, ldg, X, ldx, dtype, N, dA, ldda, s);
+  if (dtype == BSP_F32 && plan && N > 0 && M <= INT32_MAX && K <= INT32_MAX - 32 && N <= INT32_MAX / 2 &&
+      is_aligned(G, 16) && ldg % 4 == 0 && is_aligned(X, 16) && ldx % 4 == 0 && staged_pays(plan, N))
+    return launch_sddmm_staged(A_words, M, K, static_cast<const float*>(G), ldg, static_cast<const float*>(X), ldx, N,
+                               dA, ldda, s);
   return launch_sddmm_rows(A_words, M, K, G, ldg, X, ldx, dtype, N, dA, ldda, s);
 }
 
 int bsp_device_status(int* status, int clear) {
   if (!status) return BSP_ERR_INVALID_ARG;
-  int a = 0, b = 0, c = 0, d = 0;
+  int a = 0, b = 0, c = 0, d = 0, e = 0;
   BSP_TRY(bulk_device_error(&a, clear != 0));
   BSP_TRY(tc_device_error(&b, clear != 0));
   BSP_TRY(batched_device_error(&c, clear != 0));
   BSP_TRY(ts_device_error(&d, clear != 0));
-  *status = a ? a : (b ? b : (c ? c : d));
+  BSP_TRY(sddmm_staged_device_error(&e, clear != 0));
+  *status = a ? a : (b ? b : (c ? c : (d ? d : e)));
   return BSP_OK;
 }
 

@@ -29,6 +29,8 @@ int make_batch_map_sddmm(CUtensorMap* m, const void* T, int bdt, int64_t rows, i
 // aligned), `splits` of them split_stride floats apart: 32x32 boxes, 128-byte
 // swizzle.
 int make_out_map(CUtensorMap* m, float* C, int64_t rows, int64_t cols, int64_t ld, int splits, int64_t split_stride);
+// Rows of FP32 X in plain boxes (16-byte rows): zeros past the matrix.
+int make_rows_map_f32(CUtensorMap* m, const float* X, int64_t rows, int64_t cols, int64_t ld, int box_cols, int box_rows);
 // Work item b = {problem, 256-row block, 256-column block, reduction tiles}:
 // one CTA each.  kind 0 = forward C = A·B, 1 = dX = Aᵀ·G (rows: K),
 // 2 = dA = (G·Xᵀ) ⊙ A (columns: K).
@@ -143,6 +145,10 @@ int launch_i8_tiles(const int8_t* A, int64_t M, int64_t K, int64_t lda, int8_t* 
 int launch_sddmm_tc(const uint32_t* A, int64_t M, int64_t K, const void* G, int64_t ldg, const void* X,
                     int64_t ldx, int dt, int64_t N, float* dA, int64_t ldda, cudaStream_t s);
 // same on CUDA cores (any dtype / layout): warp per row, one dot product per set bit
+// FP32, 16-byte rows of G and X: X staged in shared memory for 32 rows of A at a time.
+int launch_sddmm_staged(const uint32_t* A, int64_t M, int64_t K, const float* G, int64_t ldg, const float* X,
+                        int64_t ldx, int64_t N, float* dA, int64_t ldda, cudaStream_t s);
+int sddmm_staged_device_error(int* out, bool clear);
 int launch_sddmm_rows(const uint32_t* A, int64_t M, int64_t K, const void* G, int64_t ldg, const void* X,
                       int64_t ldx, int dt, int64_t N, float* dA, int64_t ldda, cudaStream_t s);
 int tc_device_error(int* out, bool clear);

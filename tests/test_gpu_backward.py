@@ -110,6 +110,36 @@ def test_sddmm_rows_lists_and_parts(kind, M, K, N, p, pad, monkeypatch):
     assert _scaled_max((dA - Gx @ Xx.T)[bits], scale[bits]) <= TOL
 
 
+@pytest.mark.parametrize("M,K,N,p", [(33, 100, 400, 0.9), (300, 1000, 200, 0.2), (31, 3001, 517, 0.4), (1000, 333, 129, 0.3),
+                                     (257, 129, 1100, 0.9), (20, 40000, 64, 0.3)])
+def test_sddmm_staged(M, K, N, p):
+    """X staged for 32 rows of A at a time: slices of N with a remainder, rows
+    and columns past the last block, words of every count, parts of a row;
+    infinities and NaN in X reach the set bits of their row alone."""
+    rng = np.random.default_rng(M + K + N)
+    bits = rng.random((M, K)) < p
+    bits[0, :] = False
+    bits[1, :] = True
+    words = W.pack_bits(bits)
+    plan = ops.Plan(words_dev(words), K)
+    ld = -(-N // 4) * 4
+    mk = lambda a: torch.nn.functional.pad(torch.from_numpy(a), (0, ld - N), value=float("nan")).cuda()[:, :N]
+    G, X = rng.integers(-50, 51, (M, N)).astype(np.float32), rng.integers(-50, 51, (K, N)).astype(np.float32)
+    out = torch.full((M, K + 3), 7.0, device="cuda")
+    ops.sddmm(words_dev(words), M, K, mk(G), mk(X), plan=plan, out=out[:, :K])
+    # |sums| <= 2500 N < 2^24: exact in FP32, in any order
+    want = (G.astype(np.float64) @ X.astype(np.float64).T) * bits
+    assert np.array_equal(out[:, :K].cpu().numpy().astype(np.float64), want)
+    assert torch.all(out[:, K:] == 7.0)
+    X[K // 2, N // 2], X[K // 3, N - 1] = float("inf"), float("nan")
+    G[:, N // 2] = 1.0
+    dA = ops.sddmm(words_dev(words), M, K, mk(G), mk(X), plan=plan).cpu().numpy()
+    hit = np.zeros((M, K), dtype=bool)
+    hit[:, K // 2], hit[:, K // 3] = bits[:, K // 2], bits[:, K // 3]
+    assert np.array_equal(~np.isfinite(dA), hit)
+    assert capi.device_status() == 0
+
+
 def _loss64(A, X, G):
     return float(((A @ X) * G).sum())
 
