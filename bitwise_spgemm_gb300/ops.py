@@ -17,11 +17,13 @@ _DT = {torch.float32: capi.F32, torch.float16: capi.F16, torch.bfloat16: capi.BF
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # The current stream's handle without the Stream object around it: a small
+    # product is bound by the host (64x96x16 FP32: 10.3 us with it, 5.9 without).
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _p(t):
-    return C.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 def _rowmajor(t, name):
