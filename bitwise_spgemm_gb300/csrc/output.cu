@@ -16,6 +16,7 @@
 //    row, sums each plane in FP32 (TwoSum compensated) and adds it, scaled by
 //    its power-of-two weight (exact), to the row's total.
 #include <climits>
+#include <type_traits>
 
 #include "ptx.cuh"
 #include "spmm_dev.cuh"
@@ -66,54 +67,65 @@ __global__ void __launch_bounds__(256) k_symbolic_rows(const uint32_t* __restric
 }
 
 // ---- symbolic masks through a prototype plan ------------------------------
-// For a row i of cluster c, the number of A_i's columns k whose B mask has
-// column j set is  n_c[j] + #adds_i with j − #removes_i with j, where n_c
-// counts over the cluster's consensus columns: every removed column is in
-// the consensus, so the running count never goes below zero, and the mask
-// bit is n > 0 — exact.  Counts are kept bit-sliced: plane p of a word holds
-// bit p of its 32 columns' counts (16 planes: counts < 65536, which K <
-// 65536 guarantees), so adding or removing one row's mask word is a ripple
-// carry or borrow over the planes.  A row then reads its cluster's planes
-// and its delta rows' masks (≈16 for the clustered workload) instead of the
-// mask of every set bit (≈425).
+// Row i of cluster c holds the cluster's consensus columns without those that
+// it removes, and the columns that it adds.  Bit j of its mask is set if an
+// added column's B mask has it, or if more of the consensus columns' masks
+// have it than of the removed ones' (every removed column is in the
+// consensus) — exact.  Counts are kept bit-sliced: plane p of a word holds
+// bit p of its 32 columns' counts (16 planes: counts < 65536, which K < 65536
+// guarantees).  Eight masks are counted at a time by full adders over whole
+// words (two three-input operations each), and a count is compared with
+// another by one such operation per plane.  A row then reads its cluster's
+// planes in use and its delta rows' masks (≈16 for the clustered workload)
+// instead of the mask of every set bit (≈425).
 constexpr int kSymPlanes = 16;
 constexpr int kSymCWords = 64;   // output words per CTA of the plane kernel
 constexpr int kSymCGroups = 8;   // consensus parts per CTA of the plane kernel
+constexpr int kSymRows = 8;      // rows per CTA of the planned row kernel
 constexpr int kSymPWords = 2;    // output words per lane of the planned row kernel (64 per warp)
 
-__device__ __forceinline__ void planes_add(uint32_t (&pl)[kSymPlanes], uint32_t x) {
-#pragma unroll
-  for (int p = 0; p < kSymPlanes; p++) {
-    const uint32_t carry = pl[p] & x;
-    pl[p] ^= x;
-    x = carry;
-    if (!x) break;
-  }
+// a + b + c of every bit: the sum's low bit, the carry
+__device__ __forceinline__ void full_add(uint32_t a, uint32_t b, uint32_t c, uint32_t* sum, uint32_t* carry) {
+  *sum = a ^ b ^ c;
+  *carry = (a & b) | (a & c) | (b & c);
 }
-__device__ __forceinline__ void planes_sub(uint32_t (&pl)[kSymPlanes], uint32_t x) {
+
+// pl += the number of masks among x[0..8) that have the bit
+template <int P>
+__device__ __forceinline__ void planes_add8(uint32_t (&pl)[P], const uint32_t (&x)[8]) {
+  uint32_t s1, s2, s3, c1, c2, c3, c4, t1, d1, d2, e;
+  full_add(x[0], x[1], x[2], &s1, &c1);
+  full_add(x[3], x[4], x[5], &s2, &c2);
+  full_add(x[6], x[7], pl[0], &s3, &c3);
+  full_add(s1, s2, s3, &pl[0], &c4);
+  full_add(c1, c2, c3, &t1, &d1);
+  full_add(t1, c4, pl[1], &pl[1], &d2);
+  full_add(d1, d2, pl[2], &pl[2], &e);
 #pragma unroll
-  for (int p = 0; p < kSymPlanes; p++) {
-    const uint32_t borrow = ~pl[p] & x;
-    pl[p] ^= x;
-    x = borrow;
-    if (!x) break;
+  for (int p = 3; p < P; p++) {
+    if (!e) break;
+    const uint32_t carry = pl[p] & e;
+    pl[p] ^= e;
+    e = carry;
   }
 }
 
 // planes[c][p][w] for cluster c = blockIdx.x, words w of chunk blockIdx.y:
 // thread (g, wl) counts its word's column bits over part g of the consensus
-// columns (bit-sliced, 8 masks in flight), the parts meet as per-column
-// counts in shared memory, and 64 threads write the planes of the total.
+// columns (8 masks in flight), and the parts' planes are added up through
+// shared memory.  Bound by the latency of the masks' gathers; one ripple of
+// carries per mask, with the parts joined as counts of single columns by
+// shared-memory atomics, took 27 us at 66 clusters x 8192 columns, this
+// takes 17.
 __global__ void __launch_bounds__(kSymCWords * kSymCGroups) k_sym_cluster_planes(
     const uint32_t* __restrict__ cons, int64_t Kw, int64_t K, const uint32_t* __restrict__ Bw, int64_t Nw,
     uint32_t* __restrict__ planes, int* __restrict__ top) {
-  __shared__ int cnt[32][kSymCWords];
+  static_assert(kSymDepth == 8, "planes_add8");
+  __shared__ uint32_t part[kSymCGroups][kSymPlanes][kSymCWords];
   const int lane = threadIdx.x & 31;
   const int g = threadIdx.x / kSymCWords, wl = threadIdx.x % kSymCWords;
   const int64_t c = blockIdx.x;
   const int64_t w = (int64_t)blockIdx.y * kSymCWords + wl;
-  for (int i = threadIdx.x; i < 32 * kSymCWords; i += blockDim.x) (&cnt[0][0])[i] = 0;
-  __syncthreads();
   uint32_t pl[kSymPlanes];
 #pragma unroll
   for (int p = 0; p < kSymPlanes; p++) pl[p] = 0u;
@@ -127,40 +139,41 @@ __global__ void __launch_bounds__(kSymCWords * kSymCGroups) k_sym_cluster_planes
 #pragma unroll
     for (int s = 0; s < kSymDepth; s++)
       v[s] = (idx[s] != kEnd && (int64_t)idx[s] < K && w < Nw) ? __ldg(Bw + (int64_t)idx[s] * Nw + w) : 0u;
-#pragma unroll
-    for (int s = 0; s < kSymDepth; s++) planes_add(pl, v[s]);
+    planes_add8(pl, v);
     if (idx[kSymDepth - 1] == kEnd) break;
   }
-  int np = 0;  // this thread's planes in use
 #pragma unroll
-  for (int p = 0; p < kSymPlanes; p++)
-    if (pl[p]) np = p + 1;
-  if (np) {
-    for (int b = 0; b < 32; b++) {
-      int n = 0;
-      for (int p = 0; p < np; p++) n |= (int)((pl[p] >> b) & 1u) << p;
-      if (n) atomicAdd(&cnt[b][wl], n);
-    }
-  }
+  for (int p = 0; p < kSymPlanes; p++) part[g][p][wl] = pl[p];
   __syncthreads();
-  if (g == 0 && w < Nw) {
-    int mx = 0;  // the largest count of this word's columns
-    for (int b = 0; b < 32; b++) mx = max(mx, cnt[b][wl]);
-    const int used = mx ? 32 - __clz(mx) : 0;  // planes up to the highest nonzero one
+  // (whole warps: two of the first group)
+  if (g == 0) {
+    int used = 0;  // planes up to the highest nonzero one
+    uint32_t carry[kSymCGroups - 1];
+#pragma unroll
+    for (int h = 0; h + 1 < kSymCGroups; h++) carry[h] = 0u;
+#pragma unroll
     for (int p = 0; p < kSymPlanes; p++) {
-      uint32_t word = 0u;
-      if (p < used)
-        for (int b = 0; b < 32; b++) word |= (uint32_t)((cnt[b][wl] >> p) & 1) << b;
-      planes[(c * kSymPlanes + p) * Nw + w] = word;
+      uint32_t sum = pl[p];
+#pragma unroll
+      for (int h = 1; h < kSymCGroups; h++) full_add(sum, part[h][p][wl], carry[h - 1], &sum, &carry[h - 1]);
+      if (w < Nw) {
+        planes[(c * kSymPlanes + p) * Nw + w] = sum;
+        if (sum) used = p + 1;
+      }
     }
-    const int cu = __reduce_max_sync(__activemask(), used);
-    if ((threadIdx.x & 31) == __ffs(__activemask()) - 1 && cu) atomicMax(top + c, cu);
+    used = __reduce_max_sync(kFull, used);
+    if (lane == 0 && used) atomicMax(top + c, used);
   }
 }
 
-// One warp per (row of C, 64-word chunk): clustered rows start from their
-// cluster's planes and apply their delta rows; other rows OR the masks of
-// their set bits.
+// One warp per (row of C, 64-word chunk): clustered rows count their removed
+// columns' masks, compare with their cluster's planes and OR their added
+// columns'; a row without a cluster is the OR of its set bits' masks, by the
+// whole block: one warp's chain of gathers for such a row, 433 bits long, made
+// all of 8192x8192x8192 take 66 us (45 now; 53 with the words of a lane apart
+// and a walker over the list).  Bound by the issue of the counting and by the
+// latency of the gathers.
+template <bool PAIR>
 __global__ void __launch_bounds__(256, 4) k_sym_rows_planned(const uint32_t* __restrict__ A, int64_t M, int64_t K,
                                                           int64_t Kw, const uint32_t* __restrict__ Bw, int64_t Nw,
                                                           const int32_t* __restrict__ row_cluster,
@@ -168,80 +181,125 @@ __global__ void __launch_bounds__(256, 4) k_sym_rows_planned(const uint32_t* __r
                                                           const uint32_t* __restrict__ delta_idx,
                                                           const uint32_t* __restrict__ planes,
                                                           const int* __restrict__ top, uint32_t* __restrict__ Cw) {
+  static_assert(kSymPWords == 2, "PAIR");
   const int lane = threadIdx.x & 31;
-  const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (row >= M) return;
+  const int warp = threadIdx.x >> 5;
+  const int64_t row0 = (int64_t)blockIdx.x * kSymRows, row = row0 + warp;
   const int64_t w0 = (int64_t)blockIdx.y * (32 * kSymPWords);
   int64_t wq[kSymPWords];
   bool wv[kSymPWords];
 #pragma unroll
   for (int q = 0; q < kSymPWords; q++) {
-    wq[q] = w0 + q * 32 + lane;
+    wq[q] = w0 + (PAIR ? lane * 2 + q : q * 32 + lane);
     wv[q] = wq[q] < Nw;
   }
-  const int cl = __ldg(row_cluster + row);
+  const int cl = row < M ? __ldg(row_cluster + row) : 0;
   uint32_t out[kSymPWords];
-  if (cl < 0) {
 #pragma unroll
-    for (int q = 0; q < kSymPWords; q++) out[q] = 0u;
-    BitWalker wk;
-    wk.init(A + row * Kw, 0, (int)Kw, lane);
-    while (true) {
-      uint32_t idx[kSymDepth];
+  for (int q = 0; q < kSymPWords; q++) out[q] = 0u;
+  // rows without a cluster: the whole block walks each, an eighth a warp
+  if (__syncthreads_or(cl < 0)) {
+    __shared__ uint32_t masks[kSymRows][32 * kSymPWords];
+    for (int i = threadIdx.x; i < kSymRows * 32 * kSymPWords; i += blockDim.x) (&masks[0][0])[i] = 0u;
+    __syncthreads();
+    for (int r = 0; r < kSymRows; r++) {
+      if (row0 + r >= M || __ldg(row_cluster + row0 + r) >= 0) continue;
+      uint32_t got[kSymPWords];
 #pragma unroll
-      for (int s = 0; s < kSymDepth; s++) idx[s] = wk.next();
-      if (idx[0] == kEnd) break;
+      for (int q = 0; q < kSymPWords; q++) got[q] = 0u;
+      BitWalker wk;
+      wk.init(A + (row0 + r) * Kw, (int)(Kw * warp / kSymRows), (int)(Kw * (warp + 1) / kSymRows), lane);
+      while (true) {
+        uint32_t idx[kSymDepth];
 #pragma unroll
-      for (int s = 0; s < kSymDepth; s++)
+        for (int s = 0; s < kSymDepth; s++) idx[s] = wk.next();
+        if (idx[0] == kEnd) break;
 #pragma unroll
-        for (int q = 0; q < kSymPWords; q++)
-          out[q] |= (idx[s] != kEnd && (int64_t)idx[s] < K && wv[q]) ? __ldg(Bw + (int64_t)idx[s] * Nw + wq[q]) : 0u;
-      if (idx[kSymDepth - 1] == kEnd) break;
+        for (int s = 0; s < kSymDepth; s++)
+#pragma unroll
+          for (int q = 0; q < kSymPWords; q++)
+            got[q] |= (idx[s] != kEnd && (int64_t)idx[s] < K && wv[q]) ? __ldg(Bw + (int64_t)idx[s] * Nw + wq[q]) : 0u;
+        if (idx[kSymDepth - 1] == kEnd) break;
+      }
+#pragma unroll
+      for (int q = 0; q < kSymPWords; q++)
+        if (got[q]) atomicOr(&masks[r][q * 32 + lane], got[q]);
     }
-  } else {
-    // planes this row's counts can reach: the cluster's counts are below
-    // 2^top, and the row adds at most one per delta entry
+    __syncthreads();
+    if (cl < 0)
+#pragma unroll
+      for (int q = 0; q < kSymPWords; q++) out[q] = masks[warp][q * 32 + lane];
+  }
+  if (row >= M) return;
+  if (cl >= 0) {
     const int d0 = __ldg(delta_ptr + row), d1 = __ldg(delta_ptr + row + 1);
-    const uint32_t bound = ((1u << __ldg(top + cl)) - 1u) + (uint32_t)(d1 - d0);
-    const int np = bound ? min(kSymPlanes, 32 - __clz(bound)) : 0;
-    uint32_t pl[kSymPWords][kSymPlanes];
+    const int np = __ldg(top + cl);  // the removed ones' counts are within the cluster's
+    const uint32_t nw = (uint32_t)Nw;
     const uint32_t* pc = planes + (int64_t)cl * kSymPlanes * Nw;
+    // P planes of the removed columns' counts: five for lists below 32 entries
+    // (16 of two words each cost the registers that keep four blocks on an SM)
+    auto apply = [&](auto count) {
+      constexpr int P = decltype(count)::value;
+      uint32_t pl[kSymPWords][P];
 #pragma unroll
-    for (int q = 0; q < kSymPWords; q++)
+      for (int q = 0; q < kSymPWords; q++)
 #pragma unroll
-      for (int p = 0; p < kSymPlanes; p++) pl[q][p] = (wv[q] && p < np) ? __ldg(pc + (int64_t)p * Nw + wq[q]) : 0u;
-    ListWalker wk;
-    wk.init(delta_idx, d0, d1, lane);
-    while (true) {
-      uint32_t idx[kSymDepth];
+        for (int p = 0; p < P; p++) pl[q][p] = 0u;
+      for (int d = d0; d < d1; d += 32) {
+        const int n = min(32, d1 - d);
+        const uint32_t mine = lane < n ? __ldg(delta_idx + d + lane) : 0u;
+        for (int e = 0; e < n; e += 8) {
+          uint32_t idx[8], v[kSymPWords][8];
 #pragma unroll
-      for (int s = 0; s < kSymDepth; s++) idx[s] = wk.next();
-      if (idx[0] == kEnd) break;
-      uint32_t v[kSymDepth][kSymPWords];
+          for (int s = 0; s < 8; s++) idx[s] = __shfl_sync(kFull, mine, e + s);
 #pragma unroll
-      for (int s = 0; s < kSymDepth; s++)
+          for (int s = 0; s < 8; s++) {
+            const uint64_t at = (uint64_t)(idx[s] & 0x7fffffffu) * nw;
+            if (PAIR) {
+              uint2 x = make_uint2(0u, 0u);
+              if (e + s < n && wv[0]) x = __ldg(reinterpret_cast<const uint2*>(Bw + wq[0] + at));
+              v[0][s] = x.x;
+              v[1][s] = x.y;
+            } else {
 #pragma unroll
-        for (int q = 0; q < kSymPWords; q++)
-          v[s][q] = (idx[s] != kEnd && wv[q]) ? __ldg(Bw + (int64_t)(idx[s] & 0x7fffffffu) * Nw + wq[q]) : 0u;
+              for (int q = 0; q < kSymPWords; q++) v[q][s] = (e + s < n && wv[q]) ? __ldg(Bw + wq[q] + at) : 0u;
+            }
+          }
 #pragma unroll
-      for (int s = 0; s < kSymDepth; s++) {
-        if (idx[s] == kEnd) continue;
-        const bool sub = (idx[s] >> 31) != 0u;
+          for (int s = 0; s < 8; s++) {
+            const uint32_t sub = (uint32_t)((int32_t)idx[s] >> 31);  // all ones: removed
 #pragma unroll
-        for (int q = 0; q < kSymPWords; q++) {
-          if (sub) planes_sub(pl[q], v[s][q]);
-          else planes_add(pl[q], v[s][q]);
+            for (int q = 0; q < kSymPWords; q++) {
+              out[q] |= v[q][s] & ~sub;
+              v[q][s] &= sub;
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < kSymPWords; q++) planes_add8(pl[q], v[q]);
         }
       }
-      if (idx[kSymDepth - 1] == kEnd) break;
-    }
+      // count of the cluster > count of the removed, from the lowest plane up
+      uint32_t more[kSymPWords];
 #pragma unroll
-    for (int q = 0; q < kSymPWords; q++) {
-      uint32_t m = 0u;
+      for (int q = 0; q < kSymPWords; q++) more[q] = 0u;
 #pragma unroll
-      for (int p = 0; p < kSymPlanes; p++) m |= pl[q][p];
-      out[q] = m;
-    }
+      for (int p = 0; p < P; p++) {
+        if (p >= np) break;
+#pragma unroll
+        for (int q = 0; q < kSymPWords; q++) {
+          const uint32_t n = wv[q] ? __ldg(pc + (int64_t)p * Nw + wq[q]) : 0u, r = ~pl[q][p];
+          more[q] = (n & r) | (n & more[q]) | (r & more[q]);
+        }
+      }
+#pragma unroll 1
+      for (int p = P; p < np; p++)  // (the removed ones' counts have none there)
+#pragma unroll
+        for (int q = 0; q < kSymPWords; q++) more[q] |= wv[q] ? __ldg(pc + (int64_t)p * Nw + wq[q]) : 0u;
+#pragma unroll
+      for (int q = 0; q < kSymPWords; q++) out[q] |= more[q];
+    };
+    if (d1 - d0 < 32) apply(std::integral_constant<int, 5>());
+    else apply(std::integral_constant<int, kSymPlanes>());
   }
 #pragma unroll
   for (int q = 0; q < kSymPWords; q++)
@@ -464,7 +522,10 @@ int launch_symbolic_planned(const uint32_t* A, int64_t M, int64_t K, const uint3
     k_sym_cluster_planes<<<dim3((unsigned)n_proto, (unsigned)gpy), kSymCWords * kSymCGroups, 0, s>>>(cons, Kw, K, Bw,
                                                                                                     Nw, planes, top);
   }
-  k_sym_rows_planned<<<dim3((unsigned)ceil_div(M, 8), (unsigned)gry), 256, 0, s>>>(
+  // a lane's two words side by side where every row starts on 8 bytes
+  const bool pair = Nw % 2 == 0 && is_aligned(Bw, 8);
+  auto rows = pair ? k_sym_rows_planned<true> : k_sym_rows_planned<false>;
+  rows<<<dim3((unsigned)ceil_div(M, kSymRows), (unsigned)gry), kSymRows * 32, 0, s>>>(
       A, M, K, Kw, Bw, Nw, row_cluster, delta_ptr, delta_idx, planes, top, Cw);
   BSP_LAUNCHED();
   return BSP_OK;

@@ -154,6 +154,30 @@ def test_int8_planes_along_k(kind, M, K, N, d, monkeypatch):
         assert ms <= tol, (tc, ms, mn)
 
 
+@pytest.mark.parametrize("flips", [0.004, 0.03])
+@pytest.mark.parametrize("N,pb", [(33, 0.5), (64, 0.01), (2080, 0.02), (4100, 0.3)])
+def test_symbolic_planned_counts(N, pb, flips):
+    """Delta lists within and past 32 entries, counts of one and of many
+    planes, rows without a cluster among clustered ones, rows past the last
+    block, odd and even numbers of words: the same bits as without a plan."""
+    rng = np.random.default_rng(N)
+    M, K = 1003, 2000
+    protos = rng.random((3, K)) < 0.1
+    bits = protos[rng.integers(0, 3, M)] ^ (rng.random((M, K)) < flips)
+    bits[[0, 500, 501, 1002]] = rng.random((4, K)) < 0.1
+    bits[700] = False
+    a = words_dev(W.pack_bits(bits))
+    B = rng.random((K, N)) < pb
+    b = words_dev(W.pack_bits(B))
+    plan = ops.Plan(a, K, mode=2, min_cluster_rows=8)
+    info = plan.info()
+    assert info["n_proto"] >= 1 and info["direct_rows"] >= 1
+    got = ops.symbolic_rows(a, K, b, N, plan=plan)
+    want = W.pack_bits((bits.astype(np.float32) @ B.astype(np.float32)) > 0)
+    assert np.array_equal(words_host(got), want)
+    assert torch.equal(got, ops.symbolic_rows(a, K, b, N))
+
+
 @pytest.mark.parametrize("dt", ["bf16", "f16"])
 @pytest.mark.parametrize("M,K,N", [(128, 64, 8), (129, 33, 136), (300, 1000, 264), (1000, 3001, 520), (64, 8192, 128),
                                    (5000, 257, 2048), (2400, 5000, 2304)])
