@@ -18,8 +18,8 @@
 //     (tcgen05.ld), scale by 0.5 and store C through a 32x32 staging tile per
 //     warp;
 //   a TMA warp: the dense operands' boxes (128-byte swizzle);
-//   an MMA warp: allocates TMEM; its lane 0 issues two tcgen05.mma (K=16) per
-//     occupied half per tile and commits the stage to its "empty" mbarrier.
+//   an MMA warp: allocates TMEM; an elected lane issues two tcgen05.mma (K=16)
+//     per occupied half per tile and commits the stage to its "empty" mbarrier.
 // Every mbarrier wait is bounded (timeout -> error 3 in g_tc_error, the CTA
 // skips its stores and frees its TMEM).
 #include <cuda.h>
@@ -48,10 +48,9 @@ constexpr int kTcK = 32;                  // one packed word of A per row and K 
 constexpr int kATile = kCtaM * kTcK * 2;  // 16 KB: both halves of one K tile
 constexpr int kAHalf = kTcM * kTcK * 2;   // 8 KB
 constexpr int kBTile = kTcK * kTcN * 2;   // 16 KB
-// Each operand has a 96 KB ring of stages.  A stage carries TPS occupied K
-// tiles (a kernel template parameter): 2 tiles in 3 stages of 32 KB, or 3
-// tiles in 2 stages of 48 KB (a third fewer hand-offs per MMA, one stage
-// less in flight).  The SDDMM runs 3 stages of one 32 KB box per operand.
+// Each operand has a 96 KB ring of stages.  A stage carries TPS K tiles (a
+// kernel template parameter): 2 tiles in 3 stages of 32 KB.  The SDDMM runs 3
+// stages of one 32 KB box per operand.
 constexpr int kRingBytes = 96 * 1024;
 constexpr int kMaxStages = 3;
 // Producers: one group of 256 threads (one per row of the CTA tile) per tile

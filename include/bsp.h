@@ -210,7 +210,7 @@ int bsp_plan_get_info(const bsp_plan* plan, bsp_plan_info* info);
 int bsp_spmm_workspace(const bsp_plan* plan, int64_t N, size_t* bytes);
 
 /* Workspace (bytes, ≥ the above) with which the tensor-core path (16-bit
- * B) also (1) splits the reduction: when the output has fewer 256x256 tiles
+ * B) also (1) splits the reduction: when the output has fewer 256x128 items
  * than half the SMs, up to 8 slices of the occupied K tiles run on separate
  * CTAs and their FP32 partials (kept in the workspace) are added in a fixed
  * order; and (2) copies B into tile order first (ceil(K/32)·ceil(N/256)
