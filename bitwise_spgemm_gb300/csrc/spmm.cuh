@@ -145,6 +145,10 @@ int launch_i8_tiles(const int8_t* A, int64_t M, int64_t K, int64_t lda, int8_t* 
 int launch_sddmm_tc(const uint32_t* A, int64_t M, int64_t K, const void* G, int64_t ldg, const void* X,
                     int64_t ldx, int dt, int64_t N, float* dA, int64_t ldda, cudaStream_t s);
 // same on CUDA cores (any dtype / layout): warp per row, one dot product per set bit
+// 16-bit dA = (G·Xᵀ) ⊙ A on the persistent batched kernel: one problem, layouts as for launch_sddmm_tc, which
+// calls it for outputs of few tiles
+int launch_sddmm_persist(const uint32_t* A, int64_t M, int64_t K, const void* G, int64_t ldg, const void* X,
+                         int64_t ldx, int dt, int64_t N, float* dA, int64_t ldda, cudaStream_t s);
 // FP32, 16-byte rows of G and X: X staged in shared memory for 32 rows of A at a time.
 int launch_sddmm_staged(const uint32_t* A, int64_t M, int64_t K, const float* G, int64_t ldg, const float* X,
                         int64_t ldx, int64_t N, float* dA, int64_t ldda, cudaStream_t s);

@@ -95,15 +95,25 @@ struct __align__(1024) SddmmSmem {
 };
 static_assert(sizeof(SddmmSmem) + kPSmemAlign <= 232448, "persistent SDDMM: shared memory");
 
-template <typename BT>
+// SINGLE: one problem, whose record comes as an argument; its items are dealt
+// to the CTAs in turn (rows fastest), and those without a bit in A are neither
+// loaded nor multiplied.
+constexpr int kSdSkip = 1 << 30;
+
+template <typename BT, bool SINGLE>
 __global__ void __launch_bounds__(kSdThreads, 1)
     k_batched_sddmm_persist(const BatchProblemTc* __restrict__ probs, const int4* __restrict__ items, int n_items,
-                            int* next_item, int64_t N) {
+                            int* next_item, int64_t N, const __grid_constant__ BatchProblemTc one) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   SddmmSmem& sm = *reinterpret_cast<SddmmSmem*>(
       smem_raw + ((kPSmemAlign - (ptx::smem_addr(smem_raw) & (kPSmemAlign - 1))) & (kPSmemAlign - 1)));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nst = (int)((N + kSdStep - 1) / kSdStep);  // stages of an item (every item reduces all of N)
+  auto item = [&](int it) -> int4 {
+    if (!SINGLE) return __ldg(items + it);
+    const int nrb = (int)((one.M + kSdRows - 1) / kSdRows);
+    return make_int4(0, it % nrb, it / nrb, 0);
+  };
   if (tid == 0) {
     for (int s = 0; s < kSdStages; s++) {
       ptx::mbar_init(&sm.full[s], 1);   // the TMA transaction arrival
@@ -140,16 +150,38 @@ __global__ void __launch_bounds__(kSdThreads, 1)
         break;
       }
       int it = 0;
-      if (leader) {
-        it = atomicAdd(next_item, 1);
-        sm.qitem[q] = it < n_items ? it : -1;
-        ptx::mbar_arrive(&sm.qfull[q]);
+      if (SINGLE) {
+        it = (int)blockIdx.x + j * (int)gridDim.x;
+        bool skip = false;
+        if (it < n_items) {
+          const int4 b = item(it);
+          uint32_t any = 0u;
+#pragma unroll
+          for (int r = 0; r < kSdRows / 4; r++) {  // lanes 8 r' + w: word w of row 4 r + r'
+            const int64_t row = (int64_t)b.y * kSdRows + r * 4 + (lane >> 3), w = (int64_t)b.z * (kSdCols / 32) + (lane & 7);
+            if (row < one.M && w < one.Kw) any |= __ldg(one.A + row * one.Kw + w);
+          }
+          skip = !__any_sync(kFull, any != 0u);
+        }
+        if (leader) {
+          sm.qitem[q] = it >= n_items ? -1 : (skip ? it | kSdSkip : it);
+          ptx::mbar_arrive(&sm.qfull[q]);
+        }
+        __syncwarp();
+        if (it >= n_items) break;
+        if (skip) continue;
+      } else {
+        if (leader) {
+          it = atomicAdd(next_item, 1);
+          sm.qitem[q] = it < n_items ? it : -1;
+          ptx::mbar_arrive(&sm.qfull[q]);
+        }
+        it = __reduce_max_sync(kFull, it);
+        if (it >= n_items) break;
       }
-      it = __reduce_max_sync(kFull, it);
-      if (it >= n_items) break;
-      const int4 w4 = __ldg(items + it);
-      const BatchProblemTc* p = probs + w4.x;
-      if (leader) {
+      const int4 w4 = item(it);
+      const BatchProblemTc* p = SINGLE ? &one : probs + w4.x;
+      if (!SINGLE && leader) {
         ptx::tensormap_acquire(&p->map3);  // written by the host into global memory
         ptx::tensormap_acquire(&p->map2);
       }
@@ -191,7 +223,9 @@ __global__ void __launch_bounds__(kSdThreads, 1)
         if (leader) persist_fail();
         break;
       }
-      if (__reduce_max_sync(kFull, *(volatile const int*)&sm.qitem[j % kPQ]) < 0) break;
+      const int it = __reduce_max_sync(kFull, *(volatile const int*)&sm.qitem[j % kPQ]);
+      if (it < 0) break;
+      const int n = SINGLE && (it & kSdSkip) ? 0 : nst;
       const int set = j & 1;
       if (!ptx::mbar_wait_warp(&sm.tempty[set], ((uint32_t)(j >> 1) & 1u) ^ 1u)) {
         if (leader) persist_fail();
@@ -200,7 +234,7 @@ __global__ void __launch_bounds__(kSdThreads, 1)
       ptx::tc_fence_after_sync();
       const uint32_t dset = tmem + (uint32_t)(set * kSdCols);
       bool ok = true;
-      for (int i = 0; i < nst; i++) {
+      for (int i = 0; i < n; i++) {
         if (!ptx::mbar_wait_warp(&sm.full[s], ph)) {
           ok = false;
           break;
@@ -224,7 +258,7 @@ __global__ void __launch_bounds__(kSdThreads, 1)
         break;
       }
       if (leader) {
-        if (nst > 0) ptx::tc_commit(&sm.tfull[set]);
+        if (n > 0) ptx::tc_commit(&sm.tfull[set]);
         else ptx::mbar_arrive(&sm.tfull[set]);
       }
       __syncwarp();
@@ -242,8 +276,8 @@ __global__ void __launch_bounds__(kSdThreads, 1)
         break;
       }
       if (it < 0) break;
-      const int4 w4 = __ldg(items + it);
-      const BatchProblemTc* p = probs + w4.x;
+      const int4 w4 = item(SINGLE ? it & (kSdSkip - 1) : it);
+      const BatchProblemTc* p = SINGLE ? &one : probs + w4.x;
       const int64_t M = p->M, K = p->K, Kw = p->Kw, ldc = p->ldc;
       float* C = p->C;
       const int64_t rbase = (int64_t)w4.y * kSdRows + q4 * 32;  // the warp's first row
@@ -316,7 +350,7 @@ int launch_sddmm_persist_t(const BatchProblemTc* probs, const int4* items, int n
   int dev = 0;
   BSP_CUDA(cudaGetDevice(&dev));
   if (dev >= 64 || !configured[dev]) {
-    BSP_CUDA(cudaFuncSetAttribute(k_batched_sddmm_persist<BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    BSP_CUDA(cudaFuncSetAttribute(k_batched_sddmm_persist<BT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     if (dev < 64) configured[dev] = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -329,11 +363,46 @@ int launch_sddmm_persist_t(const BatchProblemTc* probs, const int4* items, int n
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = overlap ? 1 : 0;
-  BSP_CUDA(cudaLaunchKernelEx(&cfg, k_batched_sddmm_persist<BT>, probs, items, n_items, counter, N));
+  BSP_CUDA(cudaLaunchKernelEx(&cfg, k_batched_sddmm_persist<BT, false>, probs, items, n_items, counter, N, BatchProblemTc{}));
+  return BSP_OK;
+}
+
+template <typename BT>
+int launch_sddmm_one_t(const BatchProblemTc& one, int n_items, int64_t N, cudaStream_t st) {
+  constexpr size_t smem = sizeof(SddmmSmem) + kPSmemAlign;
+  static bool configured[64] = {false};
+  int dev = 0;
+  BSP_CUDA(cudaGetDevice(&dev));
+  if (dev >= 64 || !configured[dev]) {
+    BSP_CUDA(cudaFuncSetAttribute(k_batched_sddmm_persist<BT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (dev < 64) configured[dev] = true;
+  }
+  k_batched_sddmm_persist<BT, true><<<(unsigned)std::min(num_sms(), n_items), kSdThreads, smem, st>>>(
+      nullptr, nullptr, n_items, nullptr, N, one);
+  BSP_LAUNCHED();
   return BSP_OK;
 }
 
 }  // namespace
+
+int launch_sddmm_persist(const uint32_t* A, int64_t M, int64_t K, const void* G, int64_t ldg, const void* X,
+                         int64_t ldx, int dt, int64_t N, float* dA, int64_t ldda, cudaStream_t s) {
+  const int64_t items = ceil_div(M, kSdRows) * ceil_div(K, kSdCols);
+  if (items == 0) return BSP_OK;
+  if (items >= kSdSkip - num_sms() || N > INT32_MAX || M > INT32_MAX || K > INT32_MAX) return BSP_ERR_CAPACITY;
+  BatchProblemTc one = {};
+  BSP_TRY(make_batch_map_sddmm(&one.map3, G, dt, M, N, ldg, kSdRows));
+  BSP_TRY(make_batch_map_sddmm(&one.map2, X, dt, K, N, ldx, kSdCols));
+  one.A = A;
+  one.M = M;
+  one.K = K;
+  one.Kw = ceil_div(K, 32);
+  one.C = dA;
+  one.ldc = ldda;
+  if (dt == BSP_BF16) return launch_sddmm_one_t<__nv_bfloat16>(one, (int)items, N, s);
+  if (dt == BSP_F16) return launch_sddmm_one_t<__half>(one, (int)items, N, s);
+  return BSP_ERR_UNSUPPORTED;
+}
 
 
 }  // namespace bsp

@@ -1141,6 +1141,13 @@ int launch_sddmm_tc(const uint32_t* A, int64_t M, int64_t K, const void* G, int6
   const dim3 grid((unsigned)ceil_div(M, kCtaM), (unsigned)ceil_div(K, kTcN));
   if (ceil_div(K, kTcN) > 65535 || ceil_div(M, kCtaM) > 0x7fffffff) return BSP_ERR_CAPACITY;
   if (N > INT32_MAX || M > INT32_MAX || K > INT32_MAX) return BSP_ERR_CAPACITY;
+  // Outputs of at most half as many 256x256 tiles as SMs: 128x256 items, so that
+  // twice the SMs work (2048x2048x2048 26.7 us as tiles, 17.6 as items,
+  // 1024x1024x1024 17.9 and 12.5, 512x512x512 13.0 and 9.9).  Beyond that the
+  // larger tile wins, for it brings in two thirds of the bytes per product
+  // (3072x3072x1024 19.4 and 21.7, 1024x8192x4096 48 and 72, 4096x4096x8192
+  // 167 and 236).
+  if ((int64_t)grid.x * grid.y * 2 <= num_sms()) return launch_sddmm_persist(A, M, K, G, ldg, X, ldx, dt, N, dA, ldda, s);
   CUtensorMap ma, mb;
   BSP_TRY(make_map(&ma, G, dt, M, N, ldg, kSdK, kCtaM, CU_TENSOR_MAP_SWIZZLE_128B));  // G [M][N]
   BSP_TRY(make_map(&mb, X, dt, K, N, ldx, kSdK, kTcN, CU_TENSOR_MAP_SWIZZLE_128B));   // X [K][N]

@@ -140,6 +140,26 @@ def test_sddmm_staged(M, K, N, p):
     assert capi.device_status() == 0
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,K,N,p", [(1, 8, 8, 0.5), (129, 264, 64, 0.5), (300, 1000, 200, 0.2), (257, 136, 1104, 0.9),
+                                     (2300, 1800, 72, 0.05), (1500, 3000, 136, 0.0002), (2560, 2048, 128, 0.1)])
+def test_sddmm_small_outputs_on_tensor_cores(M, K, N, p, dt, monkeypatch):
+    """128x256 items of few output tiles and, in the last case, 256x256 tiles:
+    row, column and reduction remainders, items without a bit.  |sums| <= 64 N
+    < 2^24: exact in FP32."""
+    monkeypatch.setenv("BSP_TC", "1")
+    rng = np.random.default_rng(M + K + N)
+    bits = rng.random((M, K)) < p
+    bits[:256, :512] = False
+    wd = words_dev(W.pack_bits(bits))
+    G, X = rng.integers(-8, 9, (M, N)).astype(np.float32), rng.integers(-8, 9, (K, N)).astype(np.float32)
+    out = torch.full((M, K + 4), 7.0, device="cuda")
+    ops.sddmm(wd, M, K, torch.from_numpy(G).cuda().to(dt), torch.from_numpy(X).cuda().to(dt), out=out[:, :K])
+    assert np.array_equal(out[:, :K].cpu().numpy().astype(np.float64), (G.astype(np.float64) @ X.astype(np.float64).T) * bits)
+    assert torch.all(out[:, K:] == 7.0)
+    assert capi.device_status() == 0
+
+
 def _loss64(A, X, G):
     return float(((A @ X) * G).sum())
 
