@@ -45,7 +45,7 @@ class BitmapMatmul(torch.autograd.Function):
         G = dY.contiguous().to(X.dtype)
         dmask = dX = None
         if ctx.needs_input_grad[1]:
-            dX = ops.spmm_t(words, M, K, G, plan=plan).to(X.dtype)
+            dX = ops.spmm_t(words, M, K, G, plan=plan, dtype=X.dtype)
         if ctx.needs_input_grad[0]:
             dA = ops.sddmm(words, M, K, G, X, plan=plan)
             dmask = dA if ctx.mask_dtype == torch.float32 else dA.to(ctx.mask_dtype)

@@ -10,6 +10,7 @@ import os
 from . import build as _build
 
 BSP_OK = 0
+BSP_ERR_UNSUPPORTED = -4
 STATUS = {
     0: "BSP_OK", -1: "BSP_ERR_INVALID_ARG", -2: "BSP_ERR_ALIGNMENT", -3: "BSP_ERR_WORKSPACE",
     -4: "BSP_ERR_UNSUPPORTED", -5: "BSP_ERR_CUDA", -6: "BSP_ERR_DEVICE_TIMEOUT",
@@ -97,6 +98,7 @@ SIGNATURES = {
     "bsp_spmm_i8_workspace": [_I64, _I64, C.POINTER(_SZ)],
     "bsp_spmm_workspace_layout": [_P, _I64, _I64, _P, _I, _I64, C.POINTER(_SZ)],
     "bsp_spmm_workspace_preferred": [_P, _I64, C.POINTER(_SZ)],
+    "bsp_spmm_t_as": [_P, _I64, _I64, _P, _I, _I64, _I64, _P, _I, _I64, _P, _P, _SZ, _P],
     "bsp_spmm_t_workspace_layout": [_P, _I64, _I64, _I64, _I, C.POINTER(_SZ)],
     "bsp_spmm_t_workspace_preferred": [_I64, _I64, _I64, C.POINTER(_SZ)],
     "bsp_tune": [_P, _I64, _I64, _P, _I, _I64, _I64, _P, _I64, _P, _P, _SZ, _P, C.POINTER(Schedule)],

@@ -854,6 +854,35 @@ static bool layout16(const void* p, int64_t ld, int esz, int64_t N, int vcols) {
   return is_aligned(p, 16) && ((ld * esz) % 16 == 0) && (N % vcols == 0);
 }
 
+// 16-bit G against gathers of its rows, as use_tensor_cores.
+static bool trans_on_tensor_cores(const bsp_plan* plan, int64_t N) {
+  const char* e = getenv("BSP_TC");
+  if (e) return e[0] == '1';
+  const double tc = (double)plan->occT_tiles * 128.0 * 32.0 * (double)N * 2.0 / 1.2e15;
+  const double cc = (double)plan->nnz * (double)N * 2.0 / 8e12;
+  return tc < cc;
+}
+
+int bsp_spmm_t_as(const uint32_t* A_words, int64_t M, int64_t K, const void* G, int g_dtype, int64_t ldg, int64_t N,
+                  void* dX, int dx_dtype, int64_t lddx, const bsp_plan* plan, void* workspace, size_t workspace_bytes,
+                  bsp_stream_t stream) {
+  if (dx_dtype == BSP_F32)
+    return bsp_spmm_t(A_words, M, K, G, g_dtype, ldg, N, static_cast<float*>(dX), lddx, plan, workspace,
+                      workspace_bytes, stream);
+  BSP_TRY(check_dims(M, K));
+  if (N < 0 || N > kMaxCols || ldg < N || lddx < N) return BSP_ERR_INVALID_ARG;
+  if (plan && (plan->M != M || plan->K != K || plan->device != current_device())) return BSP_ERR_INVALID_ARG;
+  // rounded in the epilogue of one pass over the whole reduction, or not here
+  if (!plan || g_dtype == BSP_F32 || dx_dtype != g_dtype || M == 0 || K == 0 || N == 0 || M > tc_max_reduction() ||
+      tc_split_count(K, N, ceil_div(M, 32)) > 1 || !trans_on_tensor_cores(plan, N))
+    return BSP_ERR_UNSUPPORTED;
+  if (!dX || !A_words || !G) return BSP_ERR_INVALID_ARG;
+  if (!is_aligned(A_words, 4)) return BSP_ERR_ALIGNMENT;
+  if (!layout16(G, ldg, 2, N, 8) || !layout16(dX, lddx, 2, N, 8)) return BSP_ERR_UNSUPPORTED;
+  return launch_spmm_t_tc(A_words, M, K, G, g_dtype, ldg, N, dX, true, lddx, plan->occT, plan->wordsT,
+                          (cudaStream_t)stream, workspace, workspace_bytes);
+}
+
 int bsp_spmm_t(const uint32_t* A_words, int64_t M, int64_t K, const void* G, int g_dtype, int64_t ldg,
                int64_t N, float* dX, int64_t lddx, const bsp_plan* plan, void* workspace,
                size_t workspace_bytes, bsp_stream_t stream) {
@@ -874,11 +903,8 @@ int bsp_spmm_t(const uint32_t* A_words, int64_t M, int64_t K, const void* G, int
   const int vcols = g_dtype == BSP_F32 ? 4 : 8;
   const bool vec = layout16(G, ldg, esz, N, vcols) && layout16(dX, lddx, 4, N, 4);
   if (plan && vec && g_dtype != BSP_F32 && M <= tc_max_reduction()) {
-    const char* e = getenv("BSP_TC");
-    const double tc = (double)plan->occT_tiles * 128.0 * 32.0 * (double)N * 2.0 / 1.2e15;
-    const double cc = (double)plan->nnz * (double)N * (double)esz / 8e12;
-    if (e ? e[0] == '1' : tc < cc)
-      return launch_spmm_t_tc(A_words, M, K, G, g_dtype, ldg, N, dX, lddx, plan->occT, plan->wordsT, s, workspace,
+    if (trans_on_tensor_cores(plan, N))
+      return launch_spmm_t_tc(A_words, M, K, G, g_dtype, ldg, N, dX, false, lddx, plan->occT, plan->wordsT, s, workspace,
                               workspace_bytes);
   }
   // CUDA cores: transpose the bits into the workspace, then walk the rows of Aᵀ

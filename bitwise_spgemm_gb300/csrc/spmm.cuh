@@ -29,6 +29,8 @@ int make_batch_map_sddmm(CUtensorMap* m, const void* T, int bdt, int64_t rows, i
 // aligned), `splits` of them split_stride floats apart: 32x32 boxes, 128-byte
 // swizzle.
 int make_out_map(CUtensorMap* m, float* C, int64_t rows, int64_t cols, int64_t ld, int splits, int64_t split_stride);
+// The same of a 16-bit output: 64 x 32 boxes.
+int make_out_map16(CUtensorMap* m, void* C, int dt, int64_t rows, int64_t cols, int64_t ld);
 // Rows of FP32 X in plain boxes (16-byte rows): zeros past the matrix.
 int make_rows_map_f32(CUtensorMap* m, const float* X, int64_t rows, int64_t cols, int64_t ld, int box_cols, int box_rows);
 // Work item b = {problem, 256-row block, 256-column block, reduction tiles}:
@@ -133,7 +135,8 @@ int launch_spmm_parts(const uint32_t* A, int64_t M, int64_t K, const uint32_t* o
                       size_t ws_bytes, const int** skipped);
 // dX[K][N] = Aᵀ·G on the tensor cores, Aᵀ read from A's row words
 int launch_spmm_t_tc(const uint32_t* A, int64_t M, int64_t K, const void* G, int gdt, int64_t ldg, int64_t N,
-                     float* dX, int64_t lddx, const uint32_t* occT, const uint32_t* At, cudaStream_t s, void* ws = nullptr, size_t ws_bytes = 0);
+                     void* dX, bool out16, int64_t lddx, const uint32_t* occT, const uint32_t* At, cudaStream_t s,
+                     void* ws, size_t ws_bytes);
 // C = A·B for int8 A in the order of launch_i8_tiles (values [ceil(K/32)][M][32], then a bit per 128 x 32
 // tile with a nonzero), 16-bit B, vector layouts
 size_t i8_values_bytes(int64_t M, int64_t K);

@@ -1084,8 +1084,8 @@ int launch_spmm_tc(const SpmmArgs& sa, const uint32_t* occ, const uint32_t* At, 
 }
 
 int launch_spmm_t_tc(const uint32_t* A, int64_t M, int64_t K, const void* G, int gdt, int64_t ldg, int64_t N,
-                     float* dX, int64_t lddx, const uint32_t* occT, const uint32_t* At, cudaStream_t s, void* ws,
-                     size_t ws_bytes) {
+                     void* dX, bool out16, int64_t lddx, const uint32_t* occT, const uint32_t* At, cudaStream_t s,
+                     void* ws, size_t ws_bytes) {
   TsArgs a = {};
   a.At = At;
   a.A = A;
@@ -1093,8 +1093,9 @@ int launch_spmm_t_tc(const uint32_t* A, int64_t M, int64_t K, const void* G, int
   a.K = K;
   a.Kw = ceil_div(K, 32);
   a.N = N;
-  a.C = dX;
+  a.C = static_cast<float*>(dX);
   a.ldc = lddx;
+  a.out16 = out16;
   a.c_vec = is_aligned(dX, 16) && lddx % 4 == 0 && N % 4 == 0;
   a.occ = occT;
   a.occ_words = tc_occupancy_t_words(M);
@@ -1162,6 +1163,19 @@ int make_batch_map(CUtensorMap* m, const void* B, int bdt, int64_t K, int64_t N,
 int make_batch_map_sddmm(CUtensorMap* m, const void* T, int bdt, int64_t rows, int64_t N, int64_t ld,
                          int box_rows) {
   return make_map(m, T, bdt, rows, N, ld, kSdK, (uint32_t)box_rows, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+int make_out_map16(CUtensorMap* m, void* C, int dt, int64_t rows, int64_t cols, int64_t ld) {
+  PFN_cuTensorMapEncodeTiled_v12000 enc = encode_tiled();
+  if (!enc) return BSP_ERR_UNSUPPORTED;
+  const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, 1};
+  const cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)ld * 2 * (cuuint64_t)rows};
+  const cuuint32_t box[3] = {64, 32, 1};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = enc(m, dt == BSP_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, C,
+                         dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                         CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? BSP_OK : BSP_ERR_ALIGNMENT;
 }
 
 int make_rows_map_f32(CUtensorMap* m, const float* X, int64_t rows, int64_t cols, int64_t ld, int box_cols, int box_rows) {

@@ -15,6 +15,7 @@ struct TsArgs {
   float* C;            // [M][ldc]; trans: dX [K][ldc]
   int64_t ldc;
   bool c_vec;          // C's rows start on 16 bytes
+  bool out16;          // trans: dX in G's 16-bit type (C and ldc in its elements, 16-byte rows, no splits)
   bool c_map;          // (set by the launcher) the output leaves by TMA
   const uint32_t* occ; // occupancy bitmap of 128-row blocks (trans: of 128-column blocks)
   int occ_words;

@@ -199,10 +199,14 @@ def spmm(words, K, B, plan=None, out=None, workspace=None):
     return out
 
 
-def spmm_t(words, M, K, G, plan=None, out=None, workspace=None):
-    """dX = Aᵀ·G (FP32 [K, N]).  A: packed rows [M, ceil(K/32)], G: [M, N]."""
+def spmm_t(words, M, K, G, plan=None, out=None, workspace=None, dtype=torch.float32):
+    """dX = Aᵀ·G (FP32 [K, N]).  A: packed rows [M, ceil(K/32)], G: [M, N].
+    Without ``out``, ``dtype`` is dX's type: the FP32 sums are rounded to it."""
     ldg = _rowmajor(G, "G")
     N = G.shape[1]
+    if out is None and dtype != torch.float32:
+        dX = _spmm_t_as(words, M, K, G, plan, workspace, dtype) if dtype == G.dtype and plan is not None else None
+        return dX if dX is not None else spmm_t(words, M, K, G, plan, None, workspace).to(dtype)
     if out is None:
         out = torch.empty((K, N), dtype=torch.float32, device=G.device)
     n_min, n_pref = C.c_size_t(), C.c_size_t()
@@ -215,6 +219,25 @@ def spmm_t(words, M, K, G, plan=None, out=None, workspace=None):
     call("bsp_spmm_t", _p(words), M, K, _p(G), _DT[G.dtype], ldg, N, _p(out), out.stride(0),
          plan.handle if plan is not None else None, _p(workspace),
          workspace.numel() * workspace.element_size(), _stream())
+    return out
+
+
+def _spmm_t_as(words, M, K, G, plan, workspace, dtype):
+    """dX in G's 16-bit type from the product's own epilogue, or None where
+    the library has no such pass."""
+    N = G.shape[1]
+    n = C.c_size_t()
+    call("bsp_spmm_t_workspace_preferred", M, K, N, C.byref(n))
+    if workspace is None or workspace.numel() * workspace.element_size() < n.value:
+        workspace = torch.empty(n.value, dtype=torch.uint8, device=G.device)
+    out = torch.empty((K, N), dtype=dtype, device=G.device)
+    st = capi.lib().bsp_spmm_t_as(_p(words), M, K, _p(G), _DT[G.dtype], G.stride(0), N, _p(out), _DT[dtype],
+                                  out.stride(0), plan.handle, _p(workspace),
+                                  workspace.numel() * workspace.element_size(), _stream())
+    if st == capi.BSP_ERR_UNSUPPORTED:
+        return None
+    if st != capi.BSP_OK:
+        raise capi.BspError(st, "bsp_spmm_t_as")
     return out
 
 

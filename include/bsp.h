@@ -389,6 +389,15 @@ int bsp_spmm_t(const uint32_t* A_words, int64_t M, int64_t K, const void* G,
                const bsp_plan* plan, void* workspace, size_t workspace_bytes,
                bsp_stream_t stream);
 
+/* The same with dX in dx_dtype: F32 as above, or G's 16-bit type, the FP32 sum
+ * rounded once where it leaves the tensor cores.  BSP_ERR_UNSUPPORTED, with
+ * nothing launched, where the 16-bit form has no such pass (no plan, another
+ * engine, a split reduction, rows without 16-byte access): take dX in FP32.  */
+int bsp_spmm_t_as(const uint32_t* A_words, int64_t M, int64_t K, const void* G,
+                  int g_dtype, int64_t ldg, int64_t N, void* dX, int dx_dtype,
+                  int64_t lddx, const bsp_plan* plan, void* workspace,
+                  size_t workspace_bytes, bsp_stream_t stream);
+
 /* Straight-through mask gradient: dA[M×K] (FP32, row stride ldda) =
  * Σ_j G[i][j]·X[k][j] where A has bit (i,k) set, 0 elsewhere — the SDDMM of
  * G[M×N] and X[K×N] (same dtype).  16-bit operands run on the tensor cores

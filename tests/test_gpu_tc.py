@@ -294,3 +294,26 @@ def test_f32_parts(force_tc, M, K, N, p):
         for g, w in zip(got, want):
             assert torch.equal(g.view(torch.int32), w.view(torch.int32))
     assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("kind", ["bf16", "f16"])
+@pytest.mark.parametrize("M,K,N,direct", [(300, 2600, 1000, True), (129, 10000, 264, True), (64, 20000, 8, True),
+                                          (700, 500, 200, True), (2000, 500, 200, False),
+                                          (300, 2600, 1001, False)])
+def test_spmm_t_in_16_bits(force_tc, kind, M, K, N, direct):
+    """dX in G's type: the FP32 result rounded once, whether the epilogue rounds
+    it or (split reductions, unaligned rows) a cast afterwards; row and column
+    remainders of the boxes, blocks of dX without a bit."""
+    rng = np.random.default_rng(M + K + N)
+    bits = rng.random((M, K)) < 0.1
+    bits[:, 256:640] = False
+    wd = words_dev(W.pack_bits(bits))
+    plan = ops.Plan(wd, K)
+    G, _ = _b16(rng.standard_normal((M, N)).astype(np.float32), kind)
+    want = ops.spmm_t(wd, M, K, G, plan=plan).to(G.dtype)
+    got = ops._spmm_t_as(wd, M, K, G, plan, None, G.dtype)
+    assert (got is not None) == direct
+    if direct:
+        assert torch.equal(got, want)
+    assert torch.equal(ops.spmm_t(wd, M, K, G, plan=plan, dtype=G.dtype), want)
+    assert capi.device_status() == 0
