@@ -366,9 +366,10 @@ static int run_spmm(SpmmArgs a, const bsp_plan* plan, bool vec, const TuneSched&
     const bool room = workspace && workspace_bytes >= need;
     if (!room && vec) return BSP_ERR_WORKSPACE;
     // layouts without 16-byte access take the plan too where there is room
-    // for the prototype sums, and walk A's rows as they always could without
+    // for the prototype sums (and a grid of their 32-column blocks), and walk
+    // A's rows as they always could without
     if (!vec) {
-      proto = room && K < (int64_t)1 << 30;
+      proto = room && K < (int64_t)1 << 30 && N <= (int64_t)65535 * 32;
       if (!proto) need = 0;
     }
   }
@@ -484,7 +485,7 @@ static int prepare_spmm(const uint32_t* A_words, int64_t M, int64_t K, const voi
   a->c_vec = is_aligned(C, 16) && ldc % 4 == 0 && N % 4 == 0;
   // 16-bit B by TMA boxes, or copied into tile order where its rows take none
   *tc_ok = plan && b_dtype != BSP_F32 && plan->K <= tc_max_reduction() &&
-           (*vec || (workspace && workspace_bytes >= tc_tiled_b_bytes(K, N)));
+           (*vec || (workspace && workspace_bytes >= tc_tiled_b_bytes(K, N) && N <= ts_max_cols()));
   // FP32 as parts, where there is room for them
   if (plan && b_dtype == BSP_F32 && K <= kPartsMaxReduction && N <= (int64_t)1 << 21)
     *tc_ok = workspace && workspace_bytes >= tc_parts_bytes(M, N, K);

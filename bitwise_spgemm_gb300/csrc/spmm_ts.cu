@@ -488,6 +488,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
   } else if (warp == kSchedWarp) {
     // ---------------- items and their lists ----------------
     uint32_t x = blockIdx.x, y = blockIdx.y, z = blockIdx.z;
+    [[maybe_unused]] const uint32_t row_blocks = BAT ? 0u : (uint32_t)(((TR ? a.K : a.M) + kRows - 1) / kRows);
+    // the grid's x runs over row blocks, then over column blocks (gridDim.y is 1)
+    auto place = [&]() {
+      if (BAT) return;
+      y = x / row_blocks;
+      x -= y * row_blocks;
+    };
+    place();
     const int nblk = BAT ? 0 : (int)(((TR ? a.K : a.M) + kM - 1) / kM);
     bool more = true;
     for (int j = 0;; j++) {
@@ -571,6 +579,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
         break;
       }
       more = ptx::clc_query(ptx::smem_addr(sm.clc_result), &x, &y, &z);
+      place();
       __syncwarp();
       ptx::fence_proxy_async_smem();  // the answer is read before the next one is written
     }
@@ -716,11 +725,12 @@ int launch_t(const TsArgs& a, const CUtensorMap& map, const CUtensorMap& mapc, d
 
 int64_t ts_item_rows() { return kRows; }
 int64_t ts_item_cols() { return kN; }
+int64_t ts_max_cols() { return (int64_t)65535 * 256; }
 
 int launch_ts(TsArgs a, const CUtensorMap& map, bool trans, int splits, cudaStream_t s) {
   const int64_t gx = ceil_div(trans ? a.K : a.M, kRows), gy = ceil_div(a.N, kN);
-  if (gy > 65535 || gx > 0x7fffffff) return BSP_ERR_CAPACITY;
-  const dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)splits);
+  if (a.N > ts_max_cols() || gx * gy > 0x7fffffff) return BSP_ERR_CAPACITY;
+  const dim3 grid((unsigned)(gx * gy), 1, (unsigned)splits);
   // C (or the splits' partials) by TMA, where its rows start on 16 bytes
   CUtensorMap mapc;
   memset(&mapc, 0, sizeof(mapc));

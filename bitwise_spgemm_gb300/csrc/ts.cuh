@@ -36,6 +36,7 @@ struct TsArgs {
 // rows and columns of the output per work item
 int64_t ts_item_rows();
 int64_t ts_item_cols();
+int64_t ts_max_cols();  // widest output that launch_ts takes
 int launch_ts(TsArgs a, const CUtensorMap& map, bool trans, int splits, cudaStream_t s);
 // Every item of a batch: C = A·B of its problem (trans: dX = Aᵀ·G), longest items first.
 int launch_ts_batch(const BatchProblemTc* probs, const int4* items, int n_items, int64_t N, int bdt, bool trans,

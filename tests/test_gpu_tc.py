@@ -317,3 +317,34 @@ def test_spmm_t_in_16_bits(force_tc, kind, M, K, N, direct):
         assert torch.equal(got, want)
     assert torch.equal(ops.spmm_t(wd, M, K, G, plan=plan, dtype=G.dtype), want)
     assert capi.device_status() == 0
+
+
+def test_widths_past_65535_column_blocks(force_tc):
+    """More blocks of 128 columns than a grid's y holds: the product, Aᵀ·G and,
+    for rows without 16-byte access, the prototype plan and the walk."""
+    N = 65535 * 128 + 136
+    rng = np.random.default_rng(3)
+    bits = rng.random((3, 40)) < 0.4
+    bits[:, 7] = True
+    wd = words_dev(W.pack_bits(bits))
+    plan = ops.Plan(wd, 40)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    A = torch.from_numpy(bits.astype(np.float32)).cuda()
+    B = torch.randint(-8, 9, (40, N), device="cuda", generator=g).bfloat16()
+    assert torch.equal(ops.spmm(wd, 40, B, plan=plan), A @ B.float())
+    dX = ops.spmm_t(wd, 3, 40, B[:3], plan=plan)
+    assert torch.equal(dX, A.T @ B[:3].float())
+    del B, dX
+    rows = np.repeat(rng.random((1, 64)) < 0.5, 8, 0)
+    rows[3, 11] ^= True
+    wd = words_dev(W.pack_bits(rows))
+    plan = ops.Plan(wd, 64, mode=capi.PLAN_PROTO)
+    assert plan.info()["mode"] == capi.PLAN_PROTO
+    A = torch.from_numpy(rows.astype(np.float32)).cuda()
+    Bf = torch.randint(-8, 9, (64, N + 1), device="cuda", generator=g).float()
+    out = torch.full((8, N + 1), 7.0, device="cuda")
+    os.environ["BSP_TC"] = "0"
+    ops.spmm(wd, 64, Bf, plan=plan, out=out)
+    os.environ["BSP_TC"] = "1"
+    assert torch.equal(out, A @ Bf)
+    assert capi.device_status() == 0
