@@ -306,6 +306,13 @@ static TuneSched default_schedule(const bsp_plan* plan, int64_t N, int esz, bool
   return t;
 }
 
+// Octaves from the mean to the largest exponent of a column within which a
+// prototype's sum loses no more than the walk's own rounding: 8 are 3.6 bits
+// over the 4.4 by which the sum of 400 values of one size outgrows them, and
+// the prototypes' sums, 64 short ones, are 2 bits better than the walk's one
+// chain.  (Normal values: 3; one of 100 among them: 8 to 9.)
+constexpr int kProtoOctaves = 8;
+
 // Room for a copy of B with 16-byte rows.
 static int64_t align_cols(int64_t N, int esz) { return ceil_div(N, 16 / esz) * (16 / esz); }
 static size_t align_b_bytes(int64_t K, int64_t N, int esz) {
@@ -361,21 +368,38 @@ static int run_spmm(SpmmArgs a, const bsp_plan* plan, bool vec, const TuneSched&
   int path = sc.proto_path;
   bool proto = plan && plan->mode == BSP_PLAN_PROTO;
   size_t need = 0;
+  ColStats stats = {};
+  const bool plain = vec;
   if (proto) {
     bsp_spmm_workspace(plan, N, &need);
     const bool room = workspace && workspace_bytes >= need;
     if (!room && vec) return BSP_ERR_WORKSPACE;
-    // layouts without 16-byte access take the plan too where there is room
+    // Layouts without 16-byte access take the plan too where there is room
     // for the prototype sums (and a grid of their 32-column blocks), and walk
-    // A's rows as they always could without
+    // A's rows as they always could without.  A prototype's sum holds columns
+    // that a row of it may not: what is not finite there, or large enough to
+    // push the row's own values out of the sum, must not reach that row, so
+    // such values leave the product to the walk, on the device.
     if (!vec) {
-      proto = room && K < (int64_t)1 << 30 && N <= (int64_t)65535 * 32;
-      if (!proto) need = 0;
+      proto = workspace && workspace_bytes >= need + col_stats_bytes(N) && N <= (int64_t)65535 * 32 &&
+              K <= kStatMaxRows;
+      if (proto) {
+        BSP_TRY(launch_col_stats(a.B, a.bdt, K, N, a.ldb, static_cast<char*>(workspace) + need, kProtoOctaves, &stats,
+                                 s));
+        need += col_stats_bytes(N);
+      } else {
+        need = 0;
+      }
     }
   }
+  SpmmArgs walk = a;
+  walk.run_if = stats.flag;
   if (!vec) {
     path = 0;  // the staged rows copy whole slices: natural layouts only
     vec = align_operands(&a, plan, workspace, workspace_bytes, need, s);
+    walk.B = a.B;
+    walk.ldb = a.ldb;
+    walk.Nb = a.Nb;
   }
   if (proto) {
     a.row_cluster = plan->row_cluster;
@@ -403,7 +427,7 @@ static int run_spmm(SpmmArgs a, const bsp_plan* plan, bool vec, const TuneSched&
         d.n_list = plan->direct_rows;
         BSP_TRY(launch_spmm_rows(d, vec, s));
       }
-      return BSP_OK;
+      return plain ? BSP_OK : launch_spmm_rows(walk, vec, s);
     }
     BSP_TRY(launch_proto_sums(a, vec, s));
     return launch_spmm_rows_wide(a, s);
@@ -423,8 +447,12 @@ int bsp_spmm_workspace(const bsp_plan* plan, int64_t N, size_t* bytes) {
 int bsp_spmm_workspace_preferred(const bsp_plan* plan, int64_t N, size_t* bytes) {
   BSP_TRY(bsp_spmm_workspace(plan, N, bytes));
   if (plan) {
-    // an odd width needs the aligned copy of B behind the prototype sums
-    if (N % 8 != 0) *bytes += align_b_bytes(plan->K, N, N % 4 != 0 ? 4 : 2);
+    // an odd width needs the aligned copy of B behind the prototype sums, and
+    // the columns' sizes between them
+    if (N % 8 != 0) {
+      *bytes += align_b_bytes(plan->K, N, N % 4 != 0 ? 4 : 2);
+      if (plan->mode == BSP_PLAN_PROTO) *bytes += col_stats_bytes(N);
+    }
     const size_t tc = tc_preferred_bytes(plan->M, N, plan->K);
     if (tc > *bytes) *bytes = tc;
   }
@@ -443,7 +471,7 @@ int bsp_spmm_workspace_layout(const bsp_plan* plan, int64_t K, int64_t N, const 
   if (is_aligned(B, 16) && (ldb * esz) % 16 == 0 && (N * esz) % 16 == 0) return BSP_OK;
   size_t base = 0;
   BSP_TRY(bsp_spmm_workspace(plan, N, &base));
-  const size_t copy = base + align_b_bytes(K, N, esz);
+  const size_t copy = base + align_b_bytes(K, N, esz) + (plan && plan->mode == BSP_PLAN_PROTO ? col_stats_bytes(N) : 0);
   if (copy > *bytes) *bytes = copy;
   return BSP_OK;
 }

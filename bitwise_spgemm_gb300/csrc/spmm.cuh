@@ -69,6 +69,23 @@ struct SpmmArgs {
   int64_t n_list;
 };
 
+// Sizes of the values of B [R][N] by column (col_stats.cu), in col_stats_bytes(N)
+// of workspace: the largest biased FP32 exponent of every column and, with
+// octaves >= 0, its nonzero values and the sum of their exponents.  *flag
+// becomes nonzero if a value is not finite or at least 2^100, or if a column's
+// largest exponent is more than `octaves` above the mean one of its nonzeros.
+constexpr int kStatTop = 127 + 100;
+constexpr int64_t kStatMaxRows = (int64_t)1 << 22;  // (sums of exponents in 32 bits)
+struct ColStats {
+  int* flag;
+  int* max_exp;        // [N]
+  unsigned* done;      // [ceil(N/32)] blocks that have reported
+  unsigned* nonzeros;  // [N]
+  unsigned* exp_sum;   // [N]
+};
+size_t col_stats_bytes(int64_t N);
+int launch_col_stats(const void* B, int bdt, int64_t R, int64_t N, int64_t ldb, void* ws, int octaves, ColStats* st,
+                     cudaStream_t s);
 // B [K][N] (row stride ldb, any alignment) -> out [K][Nb], columns N..Nb-1 zero
 int launch_align_b(const void* B, int bdt, int64_t K, int64_t N, int64_t ldb, void* out, int64_t Nb, cudaStream_t s);
 // vec = B's layout allows 16-byte vector access (else lane-per-column path)

@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
   } else if (warp == kSchedWarp) {
     // ---------------- items and their lists ----------------
     uint32_t x = blockIdx.x, y = blockIdx.y, z = blockIdx.z;
-    [[maybe_unused]] const uint32_t row_blocks = BAT ? 0u : (uint32_t)(((TR ? a.K : a.M) + kRows - 1) / kRows);
+    [[maybe_unused]] const uint32_t row_blocks = BAT ? 1u : (uint32_t)(((TR ? a.K : a.M) + kRows - 1) / kRows);
     // the grid's x runs over row blocks, then over column blocks (gridDim.y is 1)
     auto place = [&]() {
       if (BAT) return;

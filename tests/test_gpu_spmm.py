@@ -544,3 +544,34 @@ def test_row_slot_order_does_not_change_results(tmp_path):
         assert r.returncode == 0, r.stderr[-2000:]
         outs.append(np.load(out))
     assert np.array_equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("kind", ["f32", "bf16"])
+@pytest.mark.parametrize("M,K,N", [(300, 500, 33), (1000, 2048, 65), (700, 3000, 250)])
+def test_prototype_plan_without_16_byte_rows(kind, M, K, N):
+    """Rows without 16-byte access under a prototype plan: a value that is not
+    finite reaches only the rows that hold its column, and one that would push
+    the others out of a prototype's sum leaves their values as the walk forms
+    them (the same bits); without either the plan's own sums stay exact on
+    integers."""
+    A, _, _ = W.clustered_bits(M, K, n_proto=4, p_proto=0.1, p_flip=0.01, seed_proto=M, seed_rows=K)
+    wd = words_dev(W.pack_bits(A))
+    plan = ops.Plan(wd, K, mode=capi.PLAN_PROTO)
+    assert plan.info()["mode"] == capi.PLAN_PROTO
+    dt = torch.float32 if kind == "f32" else torch.bfloat16
+    rng = np.random.default_rng(N)
+    # a column that most rows of a prototype hold, and some do not
+    share = A.mean(0)
+    k = int(np.argmax(np.where(A[0] & (share < 1), share, -1)))
+    B = torch.from_numpy(rng.integers(-8, 9, (K, N)).astype(np.float32)).cuda().to(dt)
+    out = torch.full((M, N + 2), 7.0, device="cuda")
+    ops.spmm(wd, K, B, plan=plan, out=out[:, :N])
+    assert np.array_equal(out[:, :N].cpu().numpy().astype(np.float64), O.spmm_f64(W.pack_bits(A), K, B.float().cpu().numpy()))
+    assert torch.all(out[:, N:] == 7.0)
+    for bad in (float("inf"), float("nan"), 1e30):
+        X = torch.from_numpy(rng.standard_normal((K, N)).astype(np.float32)).cuda().to(dt)
+        X[k, N // 2] = bad
+        got, want = ops.spmm(wd, K, X, plan=plan), ops.spmm(wd, K, X)
+        assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+        assert torch.isfinite(got[~torch.from_numpy(A[:, k]).cuda()]).all()
+    assert capi.device_status() == 0
