@@ -444,7 +444,8 @@ int bsp_spmm_workspace(const bsp_plan* plan, int64_t N, size_t* bytes) {
   return BSP_OK;
 }
 
-int bsp_spmm_workspace_preferred(const bsp_plan* plan, int64_t N, size_t* bytes) {
+// The preferred workspace for B of b_dtype, or of any type (-1).
+static int preferred_workspace(const bsp_plan* plan, int64_t N, int b_dtype, size_t* bytes) {
   BSP_TRY(bsp_spmm_workspace(plan, N, bytes));
   if (plan) {
     // an odd width needs the aligned copy of B behind the prototype sums, and
@@ -453,16 +454,20 @@ int bsp_spmm_workspace_preferred(const bsp_plan* plan, int64_t N, size_t* bytes)
       *bytes += align_b_bytes(plan->K, N, N % 4 != 0 ? 4 : 2);
       if (plan->mode == BSP_PLAN_PROTO) *bytes += col_stats_bytes(N);
     }
-    const size_t tc = tc_preferred_bytes(plan->M, N, plan->K);
+    const size_t tc = tc_preferred_bytes(plan->M, N, plan->K, b_dtype != BSP_F32);
     if (tc > *bytes) *bytes = tc;
   }
   return BSP_OK;
 }
 
+int bsp_spmm_workspace_preferred(const bsp_plan* plan, int64_t N, size_t* bytes) {
+  return preferred_workspace(plan, N, -1, bytes);
+}
+
 int bsp_spmm_workspace_layout(const bsp_plan* plan, int64_t K, int64_t N, const void* B, int b_dtype, int64_t ldb,
                               size_t* bytes) {
   if (K < 0 || (b_dtype != BSP_F32 && b_dtype != BSP_BF16 && b_dtype != BSP_F16)) return BSP_ERR_INVALID_ARG;
-  BSP_TRY(bsp_spmm_workspace_preferred(plan, N, bytes));
+  BSP_TRY(preferred_workspace(plan, N, b_dtype, bytes));
   const int esz = dtype_size(b_dtype);
   if (plan && b_dtype == BSP_F32 && N > 0 && use_tensor_cores(plan, N, esz, true)) {
     const size_t parts = tc_parts_bytes(plan->M, N, plan->K);
@@ -512,8 +517,10 @@ static int prepare_spmm(const uint32_t* A_words, int64_t M, int64_t K, const voi
   a->Nb = N;
   a->c_vec = is_aligned(C, 16) && ldc % 4 == 0 && N % 4 == 0;
   // 16-bit B by TMA boxes, or copied into tile order where its rows take none
+  // (and no row is long enough for the walk to sum it with compensation)
   *tc_ok = plan && b_dtype != BSP_F32 && plan->K <= tc_max_reduction() &&
-           (*vec || (workspace && workspace_bytes >= tc_tiled_b_bytes(K, N) && N <= ts_max_cols()));
+           (*vec || (workspace && workspace_bytes >= tc_tiled_b_bytes(K, N) && N <= ts_max_cols() &&
+                     plan->long_rows == 0));
   // FP32 as parts, where there is room for them
   if (plan && b_dtype == BSP_F32 && K <= kPartsMaxReduction && N <= (int64_t)1 << 21)
     *tc_ok = workspace && workspace_bytes >= tc_parts_bytes(M, N, K);

@@ -508,6 +508,7 @@ __global__ void __launch_bounds__(256) k_finalize_rows(
     cluster[row] = c;
     delta_cnt[row] = c >= 0 ? d : 0;
     atomicAdd(stats + 0, (unsigned long long)n);                  // nnz
+    if (n > kCompThreshold) atomicAdd(stats + 8, 1ull);           // rows that the walk sums with compensation
     if (c >= 0) {
       atomicAdd(stats + 1, (unsigned long long)d);                // delta entries
       atomicAdd(order_hist + (d < kOrderBuckets - 1 ? d : kOrderBuckets - 1), 1);
@@ -883,8 +884,8 @@ int plan_build(const uint32_t* words, int64_t M, int64_t K, const bsp_plan_param
   const size_t o_cid = take(sizeof(int32_t) * (M + 1));
   const size_t o_coff = take(sizeof(int32_t) * (M + 1));
   const size_t o_scan = take(scan_workspace_bytes(M + 1));
-  // stats[8], then the row-slot order's bucket counts and cursors
-  const size_t o_stats = take(sizeof(unsigned long long) * 8 + sizeof(int32_t) * 2 * kOrderBuckets);
+  // stats[9], then the row-slot order's bucket counts and cursors
+  const size_t o_stats = take(sizeof(unsigned long long) * 9 + sizeof(int32_t) * 2 * kOrderBuckets);
   const size_t o_dcnt = take(sizeof(int32_t) * M);
   DevBuf tmp;
   BSP_TRY(tmp.alloc(off, s));
@@ -900,11 +901,11 @@ int plan_build(const uint32_t* words, int64_t M, int64_t K, const bsp_plan_param
   int32_t* coff = (int32_t*)(T + o_coff);
   void* scanws = T + o_scan;
   unsigned long long* stats = (unsigned long long*)(T + o_stats);
-  int32_t* order_hist = (int32_t*)(stats + 8);
+  int32_t* order_hist = (int32_t*)(stats + 9);
   int32_t* dcnt = (int32_t*)(T + o_dcnt);
 
   BSP_TRY(launch_fill4(Fill{keys, tsize, kEmpty}, Fill{(uint32_t*)cnt, tsize, 0u},
-                       Fill{(uint32_t*)lead, tsize, 0x7f7f7f7fu}, Fill{(uint32_t*)stats, 16 + 2 * kOrderBuckets, 0u}, s));
+                       Fill{(uint32_t*)lead, tsize, 0x7f7f7f7fu}, Fill{(uint32_t*)stats, 18 + 2 * kOrderBuckets, 0u}, s));
 
   // ---- tensor-core structures: occupancy bitmaps and A's words by column
   // (the producers then load the words of 32 consecutive rows or columns as
@@ -1008,7 +1009,7 @@ int plan_build(const uint32_t* words, int64_t M, int64_t K, const bsp_plan_param
     BSP_LAUNCHED();
   }
   BSP_TRY(launch_scan_i32(dcnt, M, plan->delta_ptr, scanws, s));
-  unsigned long long st[8];
+  unsigned long long st[9];
   BSP_TRY(tc.join());
   BSP_CUDA(cudaMemcpyAsync(st, stats, sizeof(st), cudaMemcpyDeviceToHost, s));
   BSP_CUDA(cudaStreamSynchronize(s));
@@ -1020,6 +1021,7 @@ int plan_build(const uint32_t* words, int64_t M, int64_t K, const bsp_plan_param
   plan->occ_tiles = (int64_t)st[5];
   plan->occT_tiles = (int64_t)st[6];
   plan->proto_max_nnz = (int64_t)st[7];
+  plan->long_rows = (int64_t)st[8];
   if (plan->delta_nnz >= INT_MAX) return BSP_ERR_CAPACITY;
 
   // Cost model in gathered rows of B: direct = nnz; proto = prototype bits +

@@ -286,6 +286,14 @@ __device__ __forceinline__ void tma_store_3d(const void* map, int x, int y, int 
                : "memory");
 }
 
+// The same, added to the FP32 values that are there (rounded to nearest).
+__device__ __forceinline__ void tma_add_3d(const void* map, int x, int y, int z, const void* src_smem) {
+  asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(
+                   map),
+               "r"(x), "r"(y), "r"(z), "r"(smem_addr(src_smem))
+               : "memory");
+}
+
 // Acquire a tensor map that was written through the generic proxy (here: by
 // the host, into global memory) before TMA reads it.
 __device__ __forceinline__ void tensormap_acquire(const void* map) {

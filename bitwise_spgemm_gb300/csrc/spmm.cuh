@@ -6,6 +6,8 @@
 
 namespace bsp {
 
+constexpr int kCompThreshold = 4096;  // set bits above which rows use TwoSum
+
 // One problem of the batched form on the tensor cores: B's tensor map (64x32
 // boxes, 128-byte swizzle; first, so the record keeps the map's alignment), A
 // and C.
@@ -139,9 +141,10 @@ int tc_split_count(int64_t out_rows, int64_t out_cols, int64_t red_tiles);
 size_t tc_split_bytes(int64_t out_rows, int64_t out_cols, int64_t red_tiles);
 // B (fwd) / G (trans) copied into tile order for one bulk copy per tile: the
 // workspace it takes, and the workspace with which the tensor-core launch
-// both splits the reduction (when it would) and tiles B.
+// both splits the reduction (when it would) and tiles B; any_layout: and, where
+// the output's rows cannot start on 16 bytes, keeps its sums in rows that do.
 size_t tc_tiled_b_bytes(int64_t red_rows, int64_t cols);
-size_t tc_preferred_bytes(int64_t out_rows, int64_t out_cols, int64_t red_rows);
+size_t tc_preferred_bytes(int64_t out_rows, int64_t out_cols, int64_t red_rows, bool any_layout = false);
 // FP32 B (any layout) on the tensor cores as three exact BF16 parts: C = A·B, or
 // dX = Aᵀ·G with occT; the workspace must hold tc_parts_bytes(output rows, N,
 // reduction rows).  *skipped: a device flag, nonzero when C was left to the

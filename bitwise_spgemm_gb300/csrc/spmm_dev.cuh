@@ -7,7 +7,6 @@
 namespace bsp {
 namespace {
 
-constexpr int kCompThreshold = 4096;  // set bits above which rows use TwoSum
 
 // ---- vector loads of B ----------------------------------------------------
 template <typename BT> struct Vec;

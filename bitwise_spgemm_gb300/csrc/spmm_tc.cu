@@ -516,11 +516,12 @@ __global__ void __launch_bounds__(tc_threads(TPS), 1) k_spmm_tc(TcArgs a, const 
 // One thread per 16-byte chunk: a warp reads 512 contiguous bytes of one row
 // and writes four 128-byte runs.  VEC: B's rows take 16-byte loads; otherwise
 // the elements are read one by one, and `flag` is set if any of them is an
-// infinity or a NaN (exp_mask: the type's exponent bits).
+// infinity or a NaN (exp_mask: the type's exponent bits) or is nonzero with
+// less than the exponent bits exp_min.
 template <bool VEC>
 __global__ void __launch_bounds__(256) k_tile_b(const uint8_t* __restrict__ B, int64_t R, int64_t N, int64_t ldb,
                                                 int64_t ntiles, int64_t ncb, uint4* __restrict__ bt, uint32_t exp_mask,
-                                                int* flag) {
+                                                uint32_t exp_min, int* flag) {
   const int64_t total = ntiles * ncb * (kBTile / 16);
   bool bad = false;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
@@ -538,7 +539,8 @@ __global__ void __launch_bounds__(256) k_tile_b(const uint8_t* __restrict__ B, i
 #pragma unroll
       for (int i = 0; i < 8; i++) {
         w[i] = col + i < N ? (uint32_t)__ldg(p + i) : 0u;
-        bad |= (w[i] & exp_mask) == exp_mask;
+        const uint32_t e = w[i] & exp_mask;
+        bad |= e == exp_mask || (e < exp_min && (w[i] & 0x7fffu) != 0u);
       }
       v = make_uint4(w[0] | (w[1] << 16), w[2] | (w[3] << 16), w[4] | (w[5] << 16), w[6] | (w[7] << 16));
     }
@@ -896,11 +898,27 @@ constexpr int64_t kTiledMinRowBlocks = 16;
 // 18.7 us, x1024 41.3 and 37.6, x4096 144.9 and 131.7).
 constexpr double kTiledMinWork = 6e9;  // rows x columns x reduction
 
+// Stages (of four K tiles) between two additions in FP32 where a product that
+// the walk would form, rounded to nearest, goes to the tensor cores, whose sums
+// are cut off after every 16 products.  Errors against FP64 (Frobenius norm,
+// FP16 normals; walk, no segments, segments by this rule) and times without and
+// with segments: 16384x1024x1000 at 20 % 2.1e-8, 2.8e-8, 2.1e-8, 72 and 82 us;
+// 4096x4096x512 at 24 % 5.5e-8, 6.1e-8, 4.7e-8, 42 and 44; 8192x8192x1000 7.9e-8,
+// 2.1e-7, 6.0e-8, 123 and 154.  Four stages there 6.3e-8 and 193 us, eight at
+// K = 1024 2.8e-8 (one segment): the short form up to 2048 only.
+int seg_stages(int64_t red_tiles) { return red_tiles <= 64 ? 4 : 8; }
+
 bool tc_tiles_b(int64_t out_rows) { return ceil_div(out_rows, ts_item_rows()) >= kTiledMinRowBlocks; }
 
-size_t tc_preferred_bytes(int64_t out_rows, int64_t out_cols, int64_t red_rows) {
-  return tc_split_bytes(out_rows, out_cols, ceil_div(red_rows, kTcK)) +
-         (tc_tiles_b(out_rows) || out_cols % 8 != 0 ? tc_tiled_b_bytes(red_rows, out_cols) : 0);
+// FP32 output with 16-byte rows.
+static size_t one_part_bytes(int64_t rows, int64_t cols) {
+  return (size_t)rows * (size_t)(ceil_div(cols, 4) * 4) * sizeof(float) + 256;
+}
+
+size_t tc_preferred_bytes(int64_t out_rows, int64_t out_cols, int64_t red_rows, bool any_layout) {
+  size_t sums = tc_split_bytes(out_rows, out_cols, ceil_div(red_rows, kTcK));
+  if (sums == 0 && any_layout && out_cols % 4 != 0) sums = one_part_bytes(out_rows, out_cols);
+  return sums + (tc_tiles_b(out_rows) || out_cols % 8 != 0 ? tc_tiled_b_bytes(red_rows, out_cols) : 0);
 }
 
 namespace {
@@ -940,6 +958,19 @@ int launch_product(TsArgs a, const void* B, int64_t ldb, bool vec, bool trans, c
       used = bytes;
     }
   }
+  if (!vec) {
+    a.seg_stages = seg_stages(ceil_div(red_rows, kTcK));
+    // Sums of segments leave by TMA, which adds 16 bytes at a time: where C's rows
+    // do not start on 16 bytes, to a copy that does, as far as there is room
+    // (8192x8192x1001: 338 us by single additions to C).
+    const size_t bytes = one_part_bytes(rows, cols);
+    if (splits == 1 && !a.c_vec && ws && ws_bytes >= bytes + tiled_bytes) {
+      a.part = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(ws) + 255) & ~(uintptr_t)255);
+      a.ldp = ceil_div(cols, 4) * 4;
+      a.part_stride = rows * a.ldp;
+      used = bytes;
+    }
+  }
   // B in tile order when the rest of the workspace holds it (else tensor boxes)
   const bool room = ws && ws_bytes >= used + tiled_bytes;
   const bool tiled = !vec || (room && (form.tiled >= 0 ? form.tiled == 1
@@ -959,11 +990,12 @@ int launch_product(TsArgs a, const void* B, int64_t ldb, bool vec, bool trans, c
     const unsigned grid = (unsigned)(ceil_div(work, 256) < cap ? ceil_div(work, 256) : cap);
     if (vec) {
       k_tile_b<true><<<grid, 256, 0, s>>>(static_cast<const uint8_t*>(B), red_rows, cols, ldb, ntiles, ncb,
-                                          reinterpret_cast<uint4*>(bt), 0u, nullptr);
+                                          reinterpret_cast<uint4*>(bt), 0u, 0u, nullptr);
     } else {
       BSP_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), s));
       k_tile_b<false><<<grid, 256, 0, s>>>(static_cast<const uint8_t*>(B), red_rows, cols, ldb, ntiles, ncb,
-                                           reinterpret_cast<uint4*>(bt), a.bdt == BSP_BF16 ? 0x7f80u : 0x7c00u, flag);
+                                           reinterpret_cast<uint4*>(bt), a.bdt == BSP_BF16 ? 0x7f80u : 0x7c00u,
+                                           a.bdt == BSP_BF16 ? (127u - 100u) << 7 : 0u, flag);
       a.skip_if = flag;
       *skipped = flag;
     }
@@ -975,7 +1007,7 @@ int launch_product(TsArgs a, const void* B, int64_t ldb, bool vec, bool trans, c
     BSP_TRY(make_map(&map, B, a.bdt, red_rows, a.N, ldb, kBoxCols, kTcK, CU_TENSOR_MAP_SWIZZLE_128B));
   }
   BSP_TRY(launch_ts(a, map, trans, splits, s));
-  if (splits > 1) {
+  if (a.part) {
     const int64_t work = rows * ceil_div(cols, 4);
     const int64_t cap = (int64_t)num_sms() * 8;
     k_split_reduce<<<(unsigned)(ceil_div(work, 256) < cap ? ceil_div(work, 256) : cap), 256, 0, s>>>(

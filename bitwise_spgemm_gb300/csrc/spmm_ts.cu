@@ -75,6 +75,7 @@ constexpr int kItemUsers = kProdWarps + 3 + kEpiWarps;  // arrivals that free an
 constexpr int kAhead = 2;                       // tiles of its own a group loads A words ahead
 constexpr int kListPad = kTps * (kAhead + 1);   // entries past the list that may be read
 constexpr int kListMax = 4096;                  // K tiles of an item
+constexpr int kSegMax = 32 / kTps;              // stages of a segment: a lane for each of its tiles
 constexpr int kEpiCols = 64;                    // columns of an epilogue warp
 constexpr int kEpiBox = 32 * 32 * 4;            // its staging: two boxes of 32 rows x 32 columns (128-byte swizzle)
 constexpr int kErr = 5;
@@ -135,7 +136,8 @@ struct Transpose32 {
   }
 };
 
-constexpr int kModeBits = 0, kModeTrans = 1, kModeBatch = 2, kModeBatchTrans = 3, kModeI8 = 4;
+constexpr int kModeBits = 0, kModeTrans = 1, kModeBatch = 2, kModeBatchTrans = 3, kModeI8 = 4, kModeBitsSeg = 5,
+              kModeTransSeg = 6;
 
 // Two FP32 sums rounded to the 16-bit type.
 template <typename BT>
@@ -186,13 +188,17 @@ __device__ __forceinline__ void i8_pairs(const uint4& q, uint32_t* v) {  // 16 v
 // 29 us to stack B, 57 to multiply, 6 to reduce; values 19 in all).  Bound by
 // the producers' loads and conversions (4096^3: 132 us, 1.04 PFLOP/s).
 // TR: dX[K][N] = Aᵀ·G (output rows: columns of A, K tiles: 32 rows of A).
+// kSeg: the accumulators are handed over every a.seg_stages stages (TsArgs);
+// a kernel of its own, for the others' registers are full.
 // BAT: CTA x of the grid is work item x of a batch (problem, 256-row block,
 // 128-column block, K tiles), all of whose tiles are multiplied (a batch has
 // no occupancy plan) and whose words come from A's rows.
 template <typename BT, int MODE>
 __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_constant__ CUtensorMap mapB,
                                                          const __grid_constant__ CUtensorMap mapC) {
-  constexpr bool TR = MODE == kModeTrans || MODE == kModeBatchTrans, BAT = MODE == kModeBatch || MODE == kModeBatchTrans;
+  constexpr bool TR = MODE == kModeTrans || MODE == kModeBatchTrans || MODE == kModeTransSeg;
+  constexpr bool BAT = MODE == kModeBatch || MODE == kModeBatchTrans;
+  constexpr bool kSeg = MODE == kModeBitsSeg || MODE == kModeTransSeg;
   constexpr bool I8 = MODE == kModeI8;
   constexpr float kScale = I8 ? 1.f : tc::kTwoScale;  // a set bit is expanded to 2.0
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -407,8 +413,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
     const uint32_t ab = std::is_same<BT, __nv_bfloat16>::value ? 1u : 0u;
     const uint64_t bdesc = ptx::smem_desc_noswizzle_u32(ptx::smem_addr(sm.b), kBox, 1024) |
                            ((uint64_t)tc::kLayoutSw128 << 61);
-    uint32_t g = 0, s = 0, ph = 0;
-    for (int j = 0;; j++) {
+    uint32_t g = 0, s = 0, ph = 0, tq = 0;  // tq: segments handed over
+    for (int j = 0;; j++, tq++) {
       const int qs = j & (kItems - 1);
       if (!ptx::mbar_wait_warp(&sm.qfull[qs], (uint32_t)(j / kItems) & 1u)) {
         if (leader) fail();
@@ -422,13 +428,23 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
       // which of a stage's tiles have bits in this half, read before its wait
       const uint32_t bit = 0x1000u << h, bits = bit | (bit << 16);
       uint2 next = *reinterpret_cast<const uint2*>(lst);
-      bool ok = ptx::mbar_wait_warp(&sm.tempty[h], ((uint32_t)j & 1u) ^ 1u);
+      bool ok = ptx::mbar_wait_warp(&sm.tempty[h], (tq & 1u) ^ 1u);
       ptx::tc_fence_after_sync();
+      int left = a.seg_stages;              // stages until the accumulator is handed over
       bool started = false, whole = false;  // whole: every tile of the stage has bits in this half
       bool ready = false;                   // the stage's barrier was seen complete
       for (int k0 = 0; ok && k0 < n; k0 += kTps, g++) {
         const uint2 cur = next;
         next = *reinterpret_cast<const uint2*>(lst + k0 + kTps);
+        if (kSeg && left-- == 0) {  // a new segment, on an accumulator that the epilogue has read
+          if (leader) ptx::tc_commit(&sm.tfull[h]);
+          __syncwarp();
+          tq++;
+          ok = ptx::mbar_wait_warp(&sm.tempty[h], (tq & 1u) ^ 1u);
+          if (!ok) break;
+          started = whole = false;
+          left = a.seg_stages - 1;
+        }
         if (!ready) ok = ptx::mbar_wait_warp(&sm.full[s], ph);
         if (!ok) break;
         ptx::tc_fence_after_sync();
@@ -606,6 +622,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
       ptx::bar_sync(1 + kTps, kEpiWarps * 32);
       return !*(volatile int*)&sm.gave_up;
     };
+    uint32_t tq = 0;  // segments taken over
     for (int j = 0;; j++) {
       const int qs = j & (kItems - 1);
       if (!epi_wait(&sm.qfull[qs], (uint32_t)(j / kItems) & 1u)) {
@@ -625,72 +642,92 @@ __global__ void __launch_bounds__(kThreads, 1) k_spmm_ts(TsArgs a, const __grid_
       const int64_t gcol = (int64_t)it.y * kN + cw;
       const int cols = (int)max((int64_t)0, min((int64_t)kEpiCols, a.N - gcol));  // live columns of this warp
       bool ok = true;
-      for (int h = 0; h < 2; h++) {
-        if (!epi_wait(&sm.tfull[h], (uint32_t)j & 1u)) {
-          if (lane == 0) fail();
-          ok = false;
-          break;
+      int seg = 0, seen = it.seen;
+      do {
+        if (kSeg) {  // the halves with tiles in this segment
+          const int k = seg * kTps * a.seg_stages + lane;
+          if (it.n > 0)
+            seen = __reduce_or_sync(kFull, lane < kTps * a.seg_stages && k < it.n ? sm.list[qs][k] >> 12 : 0);
         }
-        ptx::tc_fence_after_sync();
-        const int64_t rbase = (int64_t)it.x * kRows + h * kM + q * 32;  // the warp's first row
-        const bool have = (it.seen >> h) & 1;
-        const bool live = rbase < out_rows && cols > 0;
-        if (leader) ptx::bulk_wait_read();  // the half before has left the boxes
-        __syncwarp();
-        // FP32 rows of 32 columns, or 16-bit rows of 64: 128 bytes either way.
-        // (dX in 16 bits from here instead of a pass that reads and casts it:
-        // training step 4096x4096x8192 BF16 624 -> 594 us.)
-        const bool half_out = MODE == kModeTrans && a.out16;
-        if (live) {
-          const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + h * kN + (uint32_t)cw;
-#pragma unroll
-          for (int c = 0; c < 2; c++) {
-            uint32_t v[32];
-            if (have) {
-              ptx::tmem_ld_32x32b_x32(tb + (uint32_t)(c * 32), v);
-              ptx::tmem_wait_ld();
-            }
-            if (half_out) {
-#pragma unroll
-              for (int u = 0; u < 4; u++) {
-                uint32_t p[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++)
-                  p[i] = have ? pack2<BT>(__uint_as_float(v[8 * u + 2 * i]) * kScale,
-                                          __uint_as_float(v[8 * u + 2 * i + 1]) * kScale)
-                              : 0u;
-                *reinterpret_cast<uint4*>(mine + (((c * 4 + u) ^ (mr & 7)) << 4)) = make_uint4(p[0], p[1], p[2], p[3]);
-              }
-              continue;
-            }
-#pragma unroll
-            for (int u = 0; u < 8; u++)
-              *reinterpret_cast<float4*>(mine + c * kEpiBox + ((u ^ (mr & 7)) << 4)) =
-                  have ? make_float4(__uint_as_float(v[4 * u]) * kScale, __uint_as_float(v[4 * u + 1]) * kScale,
-                                     __uint_as_float(v[4 * u + 2]) * kScale, __uint_as_float(v[4 * u + 3]) * kScale)
-                       : make_float4(0.f, 0.f, 0.f, 0.f);
+        const bool add = kSeg && seg > 0;  // to what the segments before left in the output
+        for (int h = 0; h < 2; h++) {
+          if (!epi_wait(&sm.tfull[h], tq & 1u)) {
+            if (lane == 0) fail();
+            ok = false;
+            break;
           }
-        }
-        ptx::tc_fence_before_sync();
-        ptx::fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&sm.tempty[h]);
-        if (!live) continue;
-        if (BAT || a.c_map) {  // rows and columns past the output are clipped
+          ptx::tc_fence_after_sync();
+          const int64_t rbase = (int64_t)it.x * kRows + h * kM + q * 32;  // the warp's first row
+          const bool have = (seen >> h) & 1;
+          const bool live = rbase < out_rows && cols > 0 && (have || !add);
           if (leader) {
-            for (int c = 0; c * (half_out ? 64 : 32) < cols; c++)
-              ptx::tma_store_3d(cmap, (int)gcol + c * 32, (int)rbase, BAT ? 0 : it.z, box + c * kEpiBox);
-            ptx::bulk_commit();
+            if (add) ptx::bulk_wait_all();  // the segment before is in the output
+            else ptx::bulk_wait_read();     // the half before has left the boxes
           }
-        } else {
-          const int nr = (int)min((int64_t)32, out_rows - rbase);
-          for (int r = 0; r < nr; r++)
-            for (int c = lane; c < cols; c += 32)
-              a.C[(rbase + r) * a.ldc + gcol + c] = *reinterpret_cast<const float*>(
-                  box + (c >> 5) * kEpiBox + r * 128 + ((((c & 31) >> 2) ^ (r & 7)) << 4) + (c & 3) * 4);
           __syncwarp();
+          // FP32 rows of 32 columns, or 16-bit rows of 64: 128 bytes either way.
+          // (dX in 16 bits from here instead of a pass that reads and casts it:
+          // training step 4096x4096x8192 BF16 624 -> 594 us.)
+          const bool half_out = MODE == kModeTrans && a.out16;
+          if (live) {
+            const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + h * kN + (uint32_t)cw;
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+              uint32_t v[32];
+              if (have) {
+                ptx::tmem_ld_32x32b_x32(tb + (uint32_t)(c * 32), v);
+                ptx::tmem_wait_ld();
+              }
+              if (half_out) {
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                  uint32_t p[4];
+#pragma unroll
+                  for (int i = 0; i < 4; i++)
+                    p[i] = have ? pack2<BT>(__uint_as_float(v[8 * u + 2 * i]) * kScale,
+                                            __uint_as_float(v[8 * u + 2 * i + 1]) * kScale)
+                                : 0u;
+                  *reinterpret_cast<uint4*>(mine + (((c * 4 + u) ^ (mr & 7)) << 4)) = make_uint4(p[0], p[1], p[2], p[3]);
+                }
+                continue;
+              }
+#pragma unroll
+              for (int u = 0; u < 8; u++)
+                *reinterpret_cast<float4*>(mine + c * kEpiBox + ((u ^ (mr & 7)) << 4)) =
+                    have ? make_float4(__uint_as_float(v[4 * u]) * kScale, __uint_as_float(v[4 * u + 1]) * kScale,
+                                       __uint_as_float(v[4 * u + 2]) * kScale, __uint_as_float(v[4 * u + 3]) * kScale)
+                         : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+          }
+          ptx::tc_fence_before_sync();
+          ptx::fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&sm.tempty[h]);
+          if (!live) continue;
+          if (BAT || a.c_map) {  // rows and columns past the output are clipped
+            if (leader) {
+              for (int c = 0; c * (half_out ? 64 : 32) < cols; c++) {
+                if (add) ptx::tma_add_3d(cmap, (int)gcol + c * 32, (int)rbase, it.z, box + c * kEpiBox);
+                else ptx::tma_store_3d(cmap, (int)gcol + c * 32, (int)rbase, BAT ? 0 : it.z, box + c * kEpiBox);
+              }
+              ptx::bulk_commit();
+            }
+          } else {
+            const int nr = (int)min((int64_t)32, out_rows - rbase);
+            for (int r = 0; r < nr; r++)
+              for (int c = lane; c < cols; c += 32) {
+                const float x = *reinterpret_cast<const float*>(
+                    box + (c >> 5) * kEpiBox + r * 128 + ((((c & 31) >> 2) ^ (r & 7)) << 4) + (c & 3) * 4);
+                float* o = a.C + (rbase + r) * a.ldc + gcol + c;
+                if (add) atomicAdd(o, x);  // (the thread that wrote it: in order)
+                else *o = x;
+              }
+            __syncwarp();
+          }
         }
-      }
+        tq++;
+        seg++;
+      } while (ok && kSeg && seg * kTps * a.seg_stages < it.n);
       if (!ok) break;
       if (lane == 0) ptx::mbar_arrive(&sm.qempty[qs]);
     }
@@ -735,11 +772,12 @@ int launch_ts(TsArgs a, const CUtensorMap& map, bool trans, int splits, cudaStre
   CUtensorMap mapc;
   memset(&mapc, 0, sizeof(mapc));
   const int64_t rows = trans ? a.K : a.M;
+  if (a.seg_stages < 0 || a.seg_stages > kSegMax) return BSP_ERR_INTERNAL;
   if (a.out16) {
-    if (splits > 1 || !trans || a.tiles) return BSP_ERR_UNSUPPORTED;
+    if (splits > 1 || !trans || a.tiles || a.seg_stages) return BSP_ERR_UNSUPPORTED;
     BSP_TRY(make_out_map16(&mapc, a.C, a.bdt, rows, a.N, a.ldc));
     a.c_map = true;
-  } else if (splits > 1) {
+  } else if (a.part) {
     BSP_TRY(make_out_map(&mapc, a.part, rows, a.N, a.ldp, splits, a.part_stride));
     a.c_map = true;
   } else if (a.c_vec) {
@@ -749,6 +787,13 @@ int launch_ts(TsArgs a, const CUtensorMap& map, bool trans, int splits, cudaStre
   if (a.tiles) {
     if (a.bdt == BSP_BF16) return launch_t<__nv_bfloat16, kModeI8>(a, map, mapc, grid, s);
     if (a.bdt == BSP_F16) return launch_t<__half, kModeI8>(a, map, mapc, grid, s);
+    return BSP_ERR_UNSUPPORTED;
+  }
+  if (a.seg_stages) {
+    if (a.bdt == BSP_BF16)
+      return trans ? launch_t<__nv_bfloat16, kModeTransSeg>(a, map, mapc, grid, s)
+                   : launch_t<__nv_bfloat16, kModeBitsSeg>(a, map, mapc, grid, s);
+    if (a.bdt == BSP_F16 && !trans) return launch_t<__half, kModeBitsSeg>(a, map, mapc, grid, s);
     return BSP_ERR_UNSUPPORTED;
   }
   if (a.bdt == BSP_BF16)

@@ -215,8 +215,11 @@ int bsp_spmm_workspace(const bsp_plan* plan, int64_t N, size_t* bytes);
  * CTAs and their FP32 partials (kept in the workspace) are added in a fixed
  * order; and (2) copies B into tile order first (ceil(K/32)·ceil(N/256)
  * blocks of 16 KB), so that each tile reaches shared memory as one bulk
- * copy.  A smaller workspace only turns these off (results are identical).
- * bsp_spmm_t uses its own workspace the same way when it is large enough. */
+ * copy; and (3), where C's rows cannot start on 16 bytes (N no multiple of 4),
+ * keeps the sums of the reduction's segments in rows that do.  A smaller
+ * workspace only turns these off (products whose sums are exact in FP32 are
+ * identical; the split adds the others in another order).  bsp_spmm_t uses its
+ * own workspace the same way when it is large enough.                       */
 int bsp_spmm_workspace_preferred(const bsp_plan* plan, int64_t N, size_t* bytes);
 
 /* Workspace for these operands: the above and, where B's rows do not take

@@ -348,3 +348,76 @@ def test_widths_past_65535_column_blocks(force_tc):
     os.environ["BSP_TC"] = "1"
     assert torch.equal(out, A @ Bf)
     assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("kind", ["bf16", "f16"])
+@pytest.mark.parametrize("M,K,N", [(130, 512, 132), (300, 2600, 264), (2100, 1700, 1296), (257, 8192, 8)])
+def test_tc_segments(force_tc, kind, M, K, N):
+    """Column slices of a wider B (tile order, sums handed over every 16 K
+    tiles): segments without tiles, halves with tiles in some segments only,
+    with and without split-K, C by TMA and by plain stores; exact on integers."""
+    rng = np.random.default_rng(M + K + N)
+    bits = rng.random((M, K)) < 0.2
+    bits[:128, 256:1100] = False
+    bits[128:, 600:900] = False
+    bits[256:, :300] = False
+    words = W.pack_bits(bits)
+    wd = words_dev(words)
+    plan = ops.Plan(wd, K)
+    wide, exact = _b16(rng.integers(-8, 9, (K, N + 5)).astype(np.float32), kind)
+    ref = O.spmm_f64(words, K, np.ascontiguousarray(exact[:, 3:N + 3]))
+    ws = torch.empty(plan.workspace_bytes(N + 1) + (1 << 24), dtype=torch.uint8, device="cuda")
+    for pad in (0, 4, 3):
+        out = torch.full((M, N + pad), 7.0, device="cuda")
+        ops.spmm(wd, K, wide[:, 3:N + 3], plan=plan, out=out[:, :N], workspace=ws)
+        assert np.array_equal(out[:, :N].cpu().numpy().astype(np.float64), ref)
+        assert torch.all(out[:, N:] == 7.0)
+    assert capi.device_status() == 0
+
+
+def test_tc_unaligned_columns_of_tiny_values(force_tc):
+    """BF16 values below 2^-100, whose sums may be subnormal: the walk's bits."""
+    rng = np.random.default_rng(4)
+    M, K, N = 300, 1500, 67
+    wd = words_dev(W.pack_bits(rng.random((M, K)) < 0.2))
+    B = torch.from_numpy((rng.standard_normal((K, N)) * 2.0 ** -128).astype(np.float32)).cuda().bfloat16()
+    C = ops.spmm(wd, K, B, plan=ops.Plan(wd, K))
+    assert torch.equal(C.view(torch.int32), ops.spmm(wd, K, B).view(torch.int32)) and bool((C != 0).any())
+
+
+def _frobenius(C, want):
+    return float((C.double() - want).norm() / want.norm())
+
+
+@pytest.mark.parametrize("kind", ["bf16", "f16"])
+@pytest.mark.parametrize("M,K,N,p", [(2048, 8192, 1281, 0.24), (3000, 4096, 901, 0.1), (8200, 2048, 301, 0.2)])
+def test_tc_unaligned_columns_lose_no_precision(force_tc, kind, M, K, N, p):
+    """Widths without 16-byte rows: N(0,1) products no further from FP64 than
+    the walk's sums (the outputs are wide enough to run without split-K)."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    A = torch.rand((M, K), device="cuda", generator=g) < p
+    wd = ops.pack_rows(A.to(torch.uint8))
+    plan = ops.Plan(wd, K)
+    B = torch.randn((K, N), device="cuda", generator=g).to(torch.bfloat16 if kind == "bf16" else torch.float16)
+    want = A.double() @ B.double()
+    C = ops.spmm(wd, K, B, plan=plan)
+    os.environ["BSP_TC"] = "0"
+    walk = ops.spmm(wd, K, B, plan=plan)
+    os.environ["BSP_TC"] = "1"
+    assert not torch.equal(C, walk)  # the tensor cores did run
+    assert _frobenius(C, want) <= _frobenius(walk, want)
+
+
+def test_tc_unaligned_columns_with_compensated_rows(force_tc):
+    """A row of more than 4096 set bits: the walk's compensated sums."""
+    g = torch.Generator(device="cuda").manual_seed(8)
+    M, K, N = 300, 12000, 129
+    A = torch.rand((M, K), device="cuda", generator=g) < 0.3
+    A[17] = torch.rand(K, device="cuda", generator=g) < 0.6
+    wd = ops.pack_rows(A.to(torch.uint8))
+    B = torch.randn((K, N), device="cuda", generator=g).half()
+    C = ops.spmm(wd, K, B, plan=ops.Plan(wd, K))
+    assert torch.equal(C, ops.spmm(wd, K, B))
+    # rounded once, and a compensated sum's 2^-24 of the error terms
+    want = A[17].double() @ B.double()
+    assert float((C[17].double() - want).abs().max()) <= 2.0 ** -23 * float(want.abs().max())
