@@ -233,12 +233,11 @@ static int64_t proto_ldp(int64_t N) { return (N + 7) / 8 * 8; }
 // FP32 B goes there as three BF16 parts, exact in B, where the dense products
 // cost less than the walk's gathers at their 17 TB/s and the parts' traffic
 // (10 bytes per value of B, 32 of C) and launches (walk and parts in us:
-// 512x512x256 at 10 % 4.7 and 21.5, 1024x1024x1024 at 5 % 19.6 and 28,
-// 2048x2048x256 at 10 % 29 and 27, 2048x2048x1024 at 2 % 31 and 48, at 5 % 57
-// and 49, at 10 % 97 and 49; the rule picks the smaller one each time).  B
-// whose values span too many octaves is left to the walk on the device
-// (k_split_b), and so is a reduction of more than 4096 rows: the walk sums
-// longer rows with compensation.
+// 512x512x256 at 10 % 4.7 and 24, 1024x1024x1024 at 5 % 19.6 and 30,
+// 2048x2048x1024 at 10 % 97 and 53, 4096x4096x512 at 10 % 181 and 81).  B with
+// columns of values too unequal for exact sums, or out of range, is left to the
+// walk on the device (k_split_b), and so is a reduction of more than 4096 rows:
+// the walk sums longer rows with compensation.
 constexpr int64_t kPartsMaxReduction = 4096;
 constexpr size_t kPartsMaxBytes = (size_t)4 << 30;
 static bool parts_pay(double tiles, double gathers, int64_t out_rows, int64_t N, int64_t red_rows) {
@@ -248,24 +247,25 @@ static bool parts_pay(double tiles, double gathers, int64_t out_rows, int64_t N,
   if (e) return e[0] == '1';
   const double n = (double)N;
   const double tc = tiles * 8192.0 * 3.0 * n / 1.2e15 + ((double)red_rows * 10.0 + (double)out_rows * 32.0) * n / 8e12;
-  return tc + 12e-6 < gathers * n * 4.0 / 17e12;
+  return tc + 16e-6 < gathers * n * 4.0 / 17e12;
 }
 
+// The walk that stands by for the parts sums every row from A: not behind a
+// plan whose prototypes save it a fifth of that, or its longer chains of sums.
+static double plan_gathers(const bsp_plan* plan) {
+  if (plan->mode != BSP_PLAN_PROTO) return (double)plan->nnz;
+  return (double)(plan->proto_nnz + plan->delta_nnz + plan->direct_nnz + plan->M);
+}
+static bool parts_apply(const bsp_plan* plan) { return (double)plan->nnz <= 1.25 * plan_gathers(plan); }
+
 static bool use_tensor_cores(const bsp_plan* plan, int64_t N, int esize, bool vec) {
-  if (esize == 4) {
-    double g = (double)plan->nnz;
-    if (plan->mode == BSP_PLAN_PROTO)
-      g = (double)(plan->proto_nnz + plan->delta_nnz + plan->direct_nnz + plan->M);
-    return parts_pay((double)plan->occ_tiles, g, plan->M, N, plan->K);
-  }
+  if (esize == 4)
+    return parts_apply(plan) && parts_pay((double)plan->occ_tiles, plan_gathers(plan), plan->M, N, plan->K);
   if (plan->K > tc_max_reduction()) return false;
   const char* e = getenv("BSP_TC");
   if (e) return e[0] == '1';
   const double tc = (double)plan->occ_tiles * 128.0 * 32.0 * (double)N * 2.0 / 1.2e15 + (vec ? 0.0 : 8e-6);
-  double gathers = (double)plan->nnz;
-  if (plan->mode == BSP_PLAN_PROTO)
-    gathers = (double)(plan->proto_nnz + plan->delta_nnz + plan->direct_nnz + plan->M);
-  const double cc = gathers * (double)N * (double)esize / 8e12;
+  const double cc = plan_gathers(plan) * (double)N * (double)esize / 8e12;
   return tc < cc;
 }
 
@@ -353,8 +353,8 @@ static int run_spmm(SpmmArgs a, const bsp_plan* plan, bool vec, const TuneSched&
   if (sc.engine == 1) {
     const int* skipped = nullptr;
     if (a.bdt == BSP_F32) {
-      BSP_TRY(launch_spmm_parts(a.A, a.M, a.K, plan->occ, plan->wordsT, static_cast<const float*>(a.B), a.ldb, a.N,
-                                a.C, a.ldc, false, s, workspace, workspace_bytes, &skipped));
+      BSP_TRY(launch_spmm_parts(a.A, a.M, a.K, plan->occ, plan->wordsT, plan->nnz, static_cast<const float*>(a.B),
+                                a.ldb, a.N, a.C, a.ldc, false, s, workspace, workspace_bytes, &skipped));
       a.run_if = skipped;
       return launch_spmm_rows(a, vec, s);
     }
@@ -523,7 +523,7 @@ static int prepare_spmm(const uint32_t* A_words, int64_t M, int64_t K, const voi
                      plan->long_rows == 0));
   // FP32 as parts, where there is room for them
   if (plan && b_dtype == BSP_F32 && K <= kPartsMaxReduction && N <= (int64_t)1 << 21)
-    *tc_ok = workspace && workspace_bytes >= tc_parts_bytes(M, N, K);
+    *tc_ok = parts_apply(plan) && workspace && workspace_bytes >= tc_parts_bytes(M, N, K);
   *esz_out = esz;
   return BSP_OK;
 }
@@ -952,8 +952,8 @@ int bsp_spmm_t(const uint32_t* A_words, int64_t M, int64_t K, const void* G, int
   const int* skipped = nullptr;
   if (plan && g_dtype == BSP_F32 && parts_pay((double)plan->occT_tiles, (double)plan->nnz, K, N, M) &&
       workspace_bytes >= need + tc_parts_bytes(K, N, M))
-    BSP_TRY(launch_spmm_parts(A_words, M, K, plan->occT, plan->wordsT, static_cast<const float*>(G), ldg, N, dX, lddx,
-                              true, s, static_cast<char*>(workspace) + need, workspace_bytes - need, &skipped));
+    BSP_TRY(launch_spmm_parts(A_words, M, K, plan->occT, plan->wordsT, plan->nnz, static_cast<const float*>(G), ldg, N,
+                              dX, lddx, true, s, static_cast<char*>(workspace) + need, workspace_bytes - need, &skipped));
   BSP_TRY(launch_transpose_bits(A_words, M, K, At, s, skipped));
   SpmmArgs a = {};
   a.A = At;

@@ -71,23 +71,33 @@ struct SpmmArgs {
   int64_t n_list;
 };
 
-// Sizes of the values of B [R][N] by column (col_stats.cu), in col_stats_bytes(N)
-// of workspace: the largest biased FP32 exponent of every column and, with
-// octaves >= 0, its nonzero values and the sum of their exponents.  *flag
-// becomes nonzero if a value is not finite or at least 2^100, or if a column's
-// largest exponent is more than `octaves` above the mean one of its nonzeros.
+// Sizes of the values of B [R][N] by column (col_stats.cu).
 constexpr int kStatTop = 127 + 100;
 constexpr int64_t kStatMaxRows = (int64_t)1 << 22;  // (sums of exponents in 32 bits)
 struct ColStats {
-  int* flag;
-  int* max_exp;        // [N]
+  int* flag;           // nonzero: the values do not pass
+  int* max_exp;        // [N] largest biased exponent (of FP32)
   unsigned* done;      // [ceil(N/32)] blocks that have reported
   unsigned* nonzeros;  // [N]
-  unsigned* exp_sum;   // [N]
+  unsigned* exp_sum;   // [N] of the nonzero values
+  // of a product in parts (spmm_tc.cu)
+  int* low;            // [N + 8] exponent below which a value's first part loses bits in the sums
+  unsigned* limit;     // [N] how many such values may be
+  unsigned* count;     // [N] how many there are
 };
+// *flag becomes nonzero if a value is not finite or at least 2^100, or if a
+// column's largest exponent is more than `octaves` above the mean one of its
+// nonzeros.  In col_stats_bytes(N) of workspace.
 size_t col_stats_bytes(int64_t N);
 int launch_col_stats(const void* B, int bdt, int64_t R, int64_t N, int64_t ldb, void* ws, int octaves, ColStats* st,
                      cudaStream_t s);
+// low and limit for sums of about `addends` values of a column (see k_split_b);
+// *flag as above, but for the octaves.
+constexpr int kPartsLow = 16;
+constexpr float kPartsLimit = 0.7f;
+size_t parts_stats_bytes(int64_t N);
+int launch_parts_stats(const float* B, int64_t R, int64_t N, int64_t ldb, void* ws, float addends, ColStats* st,
+                       cudaStream_t s);
 // B [K][N] (row stride ldb, any alignment) -> out [K][Nb], columns N..Nb-1 zero
 int launch_align_b(const void* B, int bdt, int64_t K, int64_t N, int64_t ldb, void* out, int64_t Nb, cudaStream_t s);
 // vec = B's layout allows 16-byte vector access (else lane-per-column path)
@@ -147,12 +157,12 @@ size_t tc_tiled_b_bytes(int64_t red_rows, int64_t cols);
 size_t tc_preferred_bytes(int64_t out_rows, int64_t out_cols, int64_t red_rows, bool any_layout = false);
 // FP32 B (any layout) on the tensor cores as three exact BF16 parts: C = A·B, or
 // dX = Aᵀ·G with occT; the workspace must hold tc_parts_bytes(output rows, N,
-// reduction rows).  *skipped: a device flag, nonzero when C was left to the
-// walking kernels (values outside the parts' range).
+// reduction rows), nnz are A's set bits.  *skipped: a device flag, nonzero when C was left to the
+// walking kernels (values outside the parts' range, or too unequal for exact sums).
 size_t tc_parts_bytes(int64_t out_rows, int64_t N, int64_t red_rows);
-int launch_spmm_parts(const uint32_t* A, int64_t M, int64_t K, const uint32_t* occ, const uint32_t* At, const float* B,
-                      int64_t ldb, int64_t N, float* C, int64_t ldc, bool trans, cudaStream_t s, void* ws,
-                      size_t ws_bytes, const int** skipped);
+int launch_spmm_parts(const uint32_t* A, int64_t M, int64_t K, const uint32_t* occ, const uint32_t* At, int64_t nnz,
+                      const float* B, int64_t ldb, int64_t N, float* C, int64_t ldc, bool trans, cudaStream_t s,
+                      void* ws, size_t ws_bytes, const int** skipped);
 // dX[K][N] = Aᵀ·G on the tensor cores, Aᵀ read from A's row words
 int launch_spmm_t_tc(const uint32_t* A, int64_t M, int64_t K, const void* G, int gdt, int64_t ldg, int64_t N,
                      void* dX, bool out16, int64_t lddx, const uint32_t* occT, const uint32_t* At, cudaStream_t s,

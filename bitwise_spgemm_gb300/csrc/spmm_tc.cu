@@ -550,34 +550,42 @@ __global__ void __launch_bounds__(256) k_tile_b(const uint8_t* __restrict__ B, i
 }
 
 // FP32 B [R][N] as three BF16 parts in tile order: part p of column c is column
-// p*Np + c of the tiles (Np = N rounded up to 8).  x = h + m + l exactly: each
-// part takes the next 8 bits of the significand, rounded, and what is left of
+// p*Np + c of the tiles (Np = N rounded up to 8).  x = h + m + l exactly (the
+// split of Henry, Tang and Heinecke, Leveraging the bfloat16 Artificial
+// Intelligence Datatype For Higher-Precision Computations, ARITH 2019): each part
+// takes the next 8 bits of the significand, rounded, and what is left of
 // 24 bits after two of them fits the third, as long as no part leaves BF16's
-// normal range.  The flag is set by any x that is not 0 or in [2^-100, 2^100),
-// infinities and NaN among them, and where the largest exponent is more than
-// kPartsOctaves above the mean one: the tensor cores' sums truncate, which
-// costs nothing while the first parts' 8 bits add up exactly in 24, as they do
-// for values of about one size (normal values: 3.5 octaves).  Rows past R are
-// zero; columns past 3 Np stay as they are (each column of a product depends
-// on its own alone).  Bound by memory: 4 bytes in, 6 out per value.
-constexpr int kPartsOctaves = 6;
-struct PartsStats {  // zeroed before the kernel
-  int flag, max_exp;
-  unsigned blocks_done, pad;
-  unsigned long long nonzeros, exp_sum;
-};
+// normal range: the flag is set by any x that is not 0 or in [2^-100, 2^100),
+// infinities and NaN among them.
+//
+// The tensor cores' sums are cut off towards zero at 24 bits, after every 16
+// products.  That costs nothing while the first parts' 8 bits add up exactly,
+// that is for values of at least 2^(E - 16), 2^E being where the sums are
+// (ColStats::low); each smaller one costs up to a unit of the last place, always
+// towards zero, where the walk rounds every addend to nearest.  The walk's
+// error grows with the square root of the addends, so the product keeps below it
+// while a column has at most 0.7 of that root of such values in a sum
+// (ColStats::limit); one column with more of them leaves the product to the
+// walk.  (Values in [1,2), a fraction of them times 2^-9 to 2^-18, all positive,
+// six sizes from 512x512 to 2048x4096 at 10 to 95 %: just inside the limit the
+// errors against FP64 are 0.12 to 1.0 of the walk's, normal values 0.05 to 0.2.)
+//
+// Rows past R are zero; columns past 3 Np stay as they are (each column of a
+// product depends on its own alone).  Bound by memory: 4 bytes in, 6 out per
+// value.
 template <bool VEC>
 __global__ void __launch_bounds__(256) k_split_b(const float* __restrict__ B, int64_t R, int64_t N, int64_t ldb,
                                                  int64_t ntiles, int64_t ncb, uint4* __restrict__ bt,
-                                                 PartsStats* st) {
+                                                 ColStats st) {
   const uint32_t q = (uint32_t)((N + 7) / 8);
   const int64_t rows = ntiles * kTcK;
   bool bad = false;
-  int top = 0;
-  unsigned long long nonzeros = 0, exps = 0;
-  for (int64_t row = blockIdx.y; row < rows; row += gridDim.y) {
-    for (uint32_t c8 = blockIdx.x * blockDim.x + threadIdx.x; c8 < q; c8 += gridDim.x * blockDim.x) {
-      const int64_t col = (int64_t)c8 * 8;
+  for (uint32_t c8 = blockIdx.x * blockDim.x + threadIdx.x; c8 < q && !bad; c8 += gridDim.x * blockDim.x) {
+    const int64_t col = (int64_t)c8 * 8;
+    const int4 l0 = __ldg(reinterpret_cast<const int4*>(st.low + col));
+    const int4 l1 = __ldg(reinterpret_cast<const int4*>(st.low + col) + 1);
+    const int low[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+    for (int64_t row = blockIdx.y; row < rows && !bad; row += gridDim.y) {
       float x[8];
 #pragma unroll
       for (int i = 0; i < 8; i++) x[i] = 0.f;
@@ -593,13 +601,14 @@ __global__ void __launch_bounds__(256) k_split_b(const float* __restrict__ B, in
             if (col + i < N) x[i] = __ldg(p + i);
         }
       }
+      if (row < R) {
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
-        const uint32_t e = (__float_as_uint(x[i]) >> 23) & 255u;
-        bad |= x[i] != 0.f && (e < 27u || e >= 227u);
-        top = max(top, (int)e);
-        nonzeros += x[i] != 0.f;
-        exps += e;
+        for (int i = 0; i < 8; i++) {
+          if (col + i >= N || x[i] == 0.f) continue;
+          const int e = (int)((__float_as_uint(x[i]) >> 23) & 255u);
+          bad |= e < 27;
+          if (e < low[i] && atomicAdd(st.count + col + i, 1u) >= __ldg(st.limit + col + i)) bad = true;
+        }
       }
 #pragma unroll
       for (int part = 0; part < 3; part++) {
@@ -617,35 +626,7 @@ __global__ void __launch_bounds__(256) k_split_b(const float* __restrict__ B, in
       }
     }
   }
-  // the block's figures, and the verdict by the block that comes last
-  __shared__ unsigned long long s_n[8], s_e[8];
-  __shared__ int s_top[8];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    nonzeros += __shfl_xor_sync(kFull, nonzeros, o);
-    exps += __shfl_xor_sync(kFull, exps, o);
-  }
-  top = __reduce_max_sync(kFull, top);
-  if (lane == 0) s_n[warp] = nonzeros, s_e[warp] = exps, s_top[warp] = top;
-  bad = __syncthreads_or(bad);
-  if (threadIdx.x != 0) return;
-  for (unsigned w = 1; w < blockDim.x / 32; w++) {
-    nonzeros += s_n[w];
-    exps += s_e[w];
-    top = max(top, s_top[w]);
-  }
-  if (bad) atomicExch(&st->flag, 1);
-  atomicMax(&st->max_exp, top);
-  atomicAdd(&st->nonzeros, nonzeros);
-  atomicAdd(&st->exp_sum, exps);
-  __threadfence();
-  if (atomicAdd(&st->blocks_done, 1u) + 1u == gridDim.x * gridDim.y) {
-    __threadfence();
-    const unsigned long long n = atomicAdd(&st->nonzeros, 0ull), e = atomicAdd(&st->exp_sum, 0ull);
-    const unsigned long long m = (unsigned long long)atomicMax(&st->max_exp, 0);
-    if (m * n > e + (unsigned long long)kPartsOctaves * n) atomicExch(&st->flag, 1);
-  }
+  if (bad) atomicExch(st.flag, 1);
 }
 
 // C = (Σ_z l + Σ_z m) + Σ_z h over the splits z (ascending), from the three
@@ -1023,7 +1004,8 @@ static int64_t parts_cols(int64_t N) { return ceil_div(N, 8) * 8; }
 size_t tc_parts_bytes(int64_t out_rows, int64_t N, int64_t red_rows) {
   const int64_t n3 = 3 * parts_cols(N);
   const int S = tc_split_count(out_rows, n3, ceil_div(red_rows, kTcK));
-  return (size_t)S * (size_t)out_rows * (size_t)n3 * sizeof(float) + 256 + tc_tiled_b_bytes(red_rows, n3);
+  return (size_t)S * (size_t)out_rows * (size_t)n3 * sizeof(float) + 256 + parts_stats_bytes(N) +
+         tc_tiled_b_bytes(red_rows, n3);
 }
 
 // C = A·B (trans: dX = Aᵀ·G) for FP32 B on the tensor cores, exact in B: its
@@ -1035,7 +1017,7 @@ size_t tc_parts_bytes(int64_t out_rows, int64_t N, int64_t red_rows) {
 // normal values 2.6e-7 and 2.7e-8, their magnitudes 2.2e-7 and 3.5e-8
 // (512x512x256 9.7e-8 and 2.5e-8, 1024x4096x512 3.7e-7 and 2.8e-8): the first
 // part's 8 bits add up nearly exactly.
-static int launch_parts(TsArgs a, const float* B, int64_t ldb, int64_t N, float* C, int64_t ldc, bool trans,
+static int launch_parts(TsArgs a, int64_t nnz, const float* B, int64_t ldb, int64_t N, float* C, int64_t ldc, bool trans,
                         cudaStream_t s, void* ws, size_t ws_bytes, const int** skipped) {
   const int64_t rows = trans ? a.K : a.M, red_rows = trans ? a.M : a.K;
   if (a.M > INT32_MAX || a.K > INT32_MAX || N > INT32_MAX / 4) return BSP_ERR_CAPACITY;
@@ -1044,11 +1026,21 @@ static int launch_parts(TsArgs a, const float* B, int64_t ldb, int64_t N, float*
   const int64_t Np = parts_cols(N), n3 = 3 * Np, ntiles = ceil_div(red_rows, kTcK), ncb = ceil_div(n3, kTcN);
   const int splits = tc_split_count(rows, n3, ntiles);
   float* part = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(ws) + 255) & ~(uintptr_t)255);
+  float* stats_ws = part + (int64_t)splits * rows * n3;
   uint8_t* bt = reinterpret_cast<uint8_t*>(
-      (reinterpret_cast<uintptr_t>(part + (int64_t)splits * rows * n3) + 256 + 1023) & ~(uintptr_t)1023);
-  PartsStats* stats = reinterpret_cast<PartsStats*>(bt - 256);
-  int* flag = &stats->flag;
-  BSP_CUDA(cudaMemsetAsync(stats, 0, sizeof(PartsStats), s));
+      (reinterpret_cast<uintptr_t>(stats_ws) + parts_stats_bytes(N) + 1023) & ~(uintptr_t)1023);
+  // Segments only where sums are long: normal values pass the columns' limits up
+  // to some 1500 addends.  A sum has an average row's bits of a slice or a segment,
+  // and a quarter more.  (3000x4096x1000 at 50 %: 85 us and 3.3e-7 for magnitudes
+  // of normals without segments, 120 and 5.5e-8 with them, the walk 990 and 6.5e-7.)
+  const double bits = (double)nnz / (double)rows;
+  a.seg_stages = bits <= 1024.0 ? 0 : bits > 0.55 * (double)red_rows ? 4 : 8;
+  double slice = (double)red_rows / splits;
+  if (a.seg_stages && slice > a.seg_stages * 4.0 * kTcK) slice = a.seg_stages * 4.0 * kTcK;
+  const double addends = 1.25 * bits * slice / (double)red_rows;
+  ColStats stats = {};
+  BSP_TRY(launch_parts_stats(B, red_rows, N, ldb, stats_ws, (float)(addends > 1.0 ? addends : 1.0), &stats, s));
+  int* flag = stats.flag;
   const int64_t q = Np / 8;
   const unsigned t = q >= 256 ? 256 : (unsigned)(ceil_div(q, 32) * 32);
   const unsigned gx = (unsigned)(ceil_div(q, t) < 1024 ? ceil_div(q, t) : 1024);
@@ -1083,9 +1075,9 @@ static int launch_parts(TsArgs a, const float* B, int64_t ldb, int64_t N, float*
   return BSP_OK;
 }
 
-int launch_spmm_parts(const uint32_t* A, int64_t M, int64_t K, const uint32_t* occ, const uint32_t* At, const float* B,
-                      int64_t ldb, int64_t N, float* C, int64_t ldc, bool trans, cudaStream_t s, void* ws,
-                      size_t ws_bytes, const int** skipped) {
+int launch_spmm_parts(const uint32_t* A, int64_t M, int64_t K, const uint32_t* occ, const uint32_t* At, int64_t nnz,
+                      const float* B, int64_t ldb, int64_t N, float* C, int64_t ldc, bool trans, cudaStream_t s,
+                      void* ws, size_t ws_bytes, const int** skipped) {
   TsArgs a = {};
   a.At = At;
   a.A = A;
@@ -1094,7 +1086,7 @@ int launch_spmm_parts(const uint32_t* A, int64_t M, int64_t K, const uint32_t* o
   a.Kw = ceil_div(K, 32);
   a.occ = occ;
   a.occ_words = trans ? tc_occupancy_t_words(M) : tc_occupancy_words(K);
-  return launch_parts(a, B, ldb, N, C, ldc, trans, s, ws, ws_bytes, skipped);
+  return launch_parts(a, nnz, B, ldb, N, C, ldc, trans, s, ws, ws_bytes, skipped);
 }
 
 int launch_spmm_tc(const SpmmArgs& sa, const uint32_t* occ, const uint32_t* At, bool vec, cudaStream_t s, void* ws,

@@ -421,3 +421,74 @@ def test_tc_unaligned_columns_with_compensated_rows(force_tc):
     # rounded once, and a compensated sum's 2^-24 of the error terms
     want = A[17].double() @ B.double()
     assert float((C[17].double() - want).abs().max()) <= 2.0 ** -23 * float(want.abs().max())
+
+
+def _columns(kind, K, N, g):
+    """FP32 values [K, N] of a kind, and whether the tensor cores' sums are exact enough for them."""
+    rnd = lambda: torch.rand((K, N), device="cuda", generator=g)
+    z = torch.randn((K, N), device="cuda", generator=g)
+    two = lambda f, d: torch.where(rnd() < f, 2.0 ** -d, 1.0) * (1 + rnd())
+    if kind == "normal":
+        return z, True
+    if kind == "lognormal":
+        return torch.exp(z), True
+    if kind == "outliers":
+        z[K // 3, ::7] = 100.0
+        return z, True
+    if kind == "half 2^-11":
+        return two(0.5, 11), None
+    if kind == "two per cent 2^-14":
+        return two(0.02, 14), None
+    if kind == "half 2^-16":
+        return two(0.5, 16), False
+    if kind == "softmax gradient":
+        p = torch.softmax(2 * z, 0)
+        p[0] -= 1
+        return p, False
+    z[:, N // 2] = two(0.3, 16)[:, 0] * 2.0 ** -10  # one column of unequal values below the others
+    return z, False
+
+
+@pytest.mark.parametrize("kind", ["normal", "lognormal", "outliers", "half 2^-11", "two per cent 2^-14", "half 2^-16",
+                                  "softmax gradient", "one column"])
+@pytest.mark.parametrize("M,K,N,p", [(600, 512, 256, 0.1), (1500, 4096, 256, 0.1), (512, 4096, 1800, 0.95)])
+def test_f32_parts_lose_no_precision(force_tc, kind, M, K, N, p):
+    """FP32 products on the tensor cores: no further from FP64 than the walk's
+    (its rounding is random, so by 3 %), whatever the values; the walk's bits where
+    a column's values are too unequal."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    A = torch.rand((M, K), device="cuda", generator=g) < p
+    wd = ops.pack_rows(A.to(torch.uint8))
+    plan = ops.Plan(wd, K, mode=capi.PLAN_DIRECT)
+    B, exact = _columns(kind, K, N, g)
+    G, exact_t = _columns(kind, M, N, g)
+    Ad = A.double()
+    got = ops.spmm(wd, K, B, plan=plan), ops.spmm_t(wd, M, K, G, plan=plan)
+    os.environ["BSP_TC"] = "0"
+    walk = ops.spmm(wd, K, B, plan=plan), ops.spmm_t(wd, M, K, G, plan=plan)
+    os.environ["BSP_TC"] = "1"
+    for c, w, want, ex in zip(got, walk, (Ad @ B.double(), Ad.T @ G.double()), (exact, exact_t)):
+        assert _frobenius(c, want) <= 1.03 * _frobenius(w, want)
+        if ex is not None:
+            assert torch.equal(c, w) == (not ex)
+    assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("M,K,N", [(300, 4096, 64), (64, 500, 257), (3000, 96, 40)])
+def test_f32_parts_of_long_integers(force_tc, M, K, N):
+    """Integers of 22 bits, which take all three parts, at most three a sum: exact."""
+    rng = np.random.default_rng(M + K)
+    bits = np.zeros((M, K), dtype=bool)
+    for i in range(M):
+        bits[i, rng.choice(K, 3, replace=False)] = True
+    words = W.pack_bits(bits)
+    wd = words_dev(words)
+    B = rng.integers(-(1 << 22), 1 << 22, (K, N)).astype(np.float32)
+    C = ops.spmm(wd, K, torch.from_numpy(B).cuda(), plan=ops.Plan(wd, K, mode=capi.PLAN_DIRECT))
+    assert np.array_equal(C.cpu().numpy().astype(np.float64), O.spmm_f64(words, K, B))
+    cols = W.pack_bits(np.ascontiguousarray(bits.T))
+    G = rng.integers(-(1 << 22), 1 << 22, (K, N)).astype(np.float32)
+    wt = words_dev(cols)
+    dX = ops.spmm_t(wt, K, M, torch.from_numpy(G).cuda(), plan=ops.Plan(wt, M, mode=capi.PLAN_DIRECT))
+    assert np.array_equal(dX.cpu().numpy().astype(np.float64), O.spmm_f64(words, K, G))
+    assert capi.device_status() == 0
