@@ -775,7 +775,7 @@ int bsp_i8_tiles(const int8_t* A, int64_t M, int64_t K, int64_t lda, int8_t* til
 
 int bsp_spmm_i8_tiles_workspace(int64_t M, int64_t K, int64_t N, size_t* bytes) {
   if (!bytes || M < 0 || K < 0 || N < 0) return BSP_ERR_INVALID_ARG;
-  *bytes = tc_preferred_bytes(M, N, K);
+  *bytes = tc_i8_bytes(M, N, K);
   return BSP_OK;
 }
 

@@ -168,7 +168,9 @@ int launch_spmm_t_tc(const uint32_t* A, int64_t M, int64_t K, const void* G, int
                      void* dX, bool out16, int64_t lddx, const uint32_t* occT, const uint32_t* At, cudaStream_t s,
                      void* ws, size_t ws_bytes);
 // C = A·B for int8 A in the order of launch_i8_tiles (values [ceil(K/32)][M][32], then a bit per 128 x 32
-// tile with a nonzero), 16-bit B, vector layouts
+// tile with a nonzero), 16-bit B, vector layouts; with tc_i8_bytes of workspace B goes there in two parts
+// (k_split16_b), with less as it is
+size_t tc_i8_bytes(int64_t M, int64_t N, int64_t K);
 size_t i8_values_bytes(int64_t M, int64_t K);
 size_t i8_tiles_bytes(int64_t M, int64_t K);
 int launch_spmm_i8_tc(const void* tiles, int64_t M, int64_t K, const void* B, int bdt, int64_t ldb, int64_t N, float* C,

@@ -185,8 +185,9 @@ __device__ __forceinline__ void i8_pairs(const uint4& q, uint32_t* v) {  // 16 v
 // I8: A is int8, [K tile][row][32] (bsp_i8_tiles), its values the MMA's operand
 // (exact in 16 bits): one product over K where the planes' bits take eight,
 // with weighted copies of B stacked first (4096x4096x256 BF16, 5 %: planes
-// 29 us to stack B, 57 to multiply, 6 to reduce; values 19 in all).  Bound by
-// the producers' loads and conversions (4096^3: 132 us, 1.04 PFLOP/s).
+// 29 us to stack B, 57 to multiply, 6 to reduce; values 19 in all, 32 with B in
+// two parts, see k_split16_b).  Bound by the producers' loads and conversions
+// (4096^3: 132 us, 1.04 PFLOP/s).
 // TR: dX[K][N] = Aᵀ·G (output rows: columns of A, K tiles: 32 rows of A).
 // kSeg: the accumulators are handed over every a.seg_stages stages (TsArgs);
 // a kernel of its own, for the others' registers are full.

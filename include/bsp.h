@@ -487,8 +487,9 @@ int bsp_stack_planes_b(const void* B, int b_dtype, int64_t ldb, int64_t K,
  * nonzero behind it (bsp_i8_tiles_bytes in all, 16-byte aligned);
  * bsp_spmm_i8_tiles is C = A·B in FP32 from it, for B and C rows that take
  * 16-byte access and N a multiple of 8 (BSP_ERR_ALIGNMENT), K up to 131072 and
- * N up to 65535 x 256 (BSP_ERR_CAPACITY); the workspace (may be smaller or NULL) only speeds it
- * up.  Same reference product as bsp_bitplane_spmm.                          */
+ * N up to 65535 x 256 (BSP_ERR_CAPACITY).  The workspace holds B in two parts
+ * (x = h + l), which keeps the sums as exact as the planes'; it may be smaller
+ * or NULL: B is multiplied as it is then.  Same reference product as bsp_bitplane_spmm.                          */
 int bsp_i8_tiles_bytes(int64_t M, int64_t K, size_t* bytes);
 int bsp_i8_tiles(const int8_t* A, int64_t M, int64_t K, int64_t lda, int8_t* tiles, bsp_stream_t stream);
 int bsp_spmm_i8_tiles_workspace(int64_t M, int64_t K, int64_t N, size_t* bytes);

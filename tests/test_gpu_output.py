@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import oracle as O
-from bitwise_spgemm_gb300 import ops
+from bitwise_spgemm_gb300 import capi, ops
 from bitwise_spgemm_gb300 import workloads as W
 from gpu_util import dev, words_dev, words_host
 
@@ -203,3 +203,47 @@ def test_int8_values_on_tensor_cores(M, K, N, dt):
     want = A.astype(np.float64) @ B.astype(np.float64)
     assert np.array_equal(got, want) and np.array_equal(out[:, :N].cpu().numpy(), want)
     assert (out[:, N:] == 7.0).all() and np.array_equal(planes, want)
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,K,N,p", [(256, 256, 16, 0.05), (256, 4096, 256, 0.02), (4096, 1024, 64, 0.03),
+                                     (4096, 4096, 256, 0.05), (4096, 4096, 2048, 0.05), (700, 3000, 200, 0.04)])
+def test_int8_values_lose_no_precision(M, K, N, p, dt):
+    """The values' product, B in two parts, is no further from FP64 than the
+    planes' (whose stacked operand is asked for)."""
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    hit = torch.rand((M, K), device="cuda", generator=g) < p
+    v = torch.randint(-128, 128, (M, K), device="cuda", generator=g)
+    A = torch.where(hit, v, torch.zeros_like(v)).to(torch.int8)
+    B = torch.randn((K, N), device="cuda", generator=g).to(dt)
+    m = ops.Int8Matrix(A)
+    assert m.tiles is not None
+    want = A.double() @ B.double()
+    err = lambda C: float((C.double() - want).norm() / want.norm())
+    stacked = torch.empty((m.Kc, N), dtype=dt, device="cuda")
+    # (errors of 1e-9, where nearly every sum is exact, vary by a few per cent)
+    assert err(m.matmul(B)) <= 1.03 * err(m.matmul(B, B_stacked=stacked))
+    assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+def test_int8_values_of_extreme_operands(dt):
+    """Infinities, NaN, the largest and the smallest values of B's type through
+    its two parts: dense positive A, so that every row holds every column."""
+    M, K, N = 200, 96, 40
+    rng = np.random.default_rng(6)
+    A = rng.integers(1, 128, (M, K)).astype(np.int8)
+    fin = torch.finfo(dt)
+    B = torch.from_numpy(rng.integers(-8, 9, (K, N)).astype(np.float32)).cuda().to(dt)
+    B[3, 1], B[4, 2], B[5, 3] = float("inf"), float("-inf"), float("nan")
+    B[:, 4] = 0
+    B[7, 4] = fin.max / 256 if dt == torch.bfloat16 else fin.max
+    B[:, 5] = 0
+    B[8, 5] = fin.tiny * 1.5
+    m = ops.Int8Matrix(torch.from_numpy(A).cuda())
+    assert m.tiles is not None
+    C = m.matmul(B).cpu().numpy()
+    want = A.astype(np.float64) @ B.double().cpu().numpy()
+    assert np.all(C[:, 1] == np.inf) and np.all(C[:, 2] == -np.inf) and np.all(np.isnan(C[:, 3]))
+    rest = [j for j in range(N) if j not in (1, 2, 3)]
+    assert np.array_equal(C[:, rest].astype(np.float64), want[:, rest])
