@@ -109,6 +109,39 @@ __global__ void __launch_bounds__(256) k_pack_rows_v16(const typename Elem<DT>::
   }
 }
 
+// Rows of up to kNarrowWords words: a warp takes 8 words one after the other,
+// over the rows' ends, 8 loads in flight.  (A warp per row, as below, has one
+// to three: 1048576x32 U8 194 us, here 45; 1048576x64 195 and 86.)
+constexpr int64_t kNarrowWords = 3;
+template <int DT>
+__global__ void __launch_bounds__(256) k_pack_rows_narrow(const typename Elem<DT>::T* __restrict__ dense, int64_t M,
+                                                          int64_t K, int64_t ld, uint32_t* __restrict__ words,
+                                                          int64_t Kw, int msb) {
+  using E = Elem<DT>;
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int64_t total = M * Kw;
+  for (int64_t base = warp * 8; base < total; base += nwarps * 8) {
+    int64_t r = base / Kw;
+    int w = (int)(base - r * Kw);
+    bool nz[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const int64_t c = w * 32 + lane;
+      nz[j] = r < M && c < K ? E::nz(dense[r * ld + c]) : false;
+      if (++w == (int)Kw) w = 0, r++;
+    }
+    uint32_t mine = 0;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const uint32_t b = __ballot_sync(kFull, nz[j]);
+      if (lane == j) mine = b;
+    }
+    if (lane < 8 && base + lane < total) words[base + lane] = msb ? __brev(mine) : mine;
+  }
+}
+
 // Any alignment: a warp takes 32 words of a row, one coalesced load of 32
 // columns and one ballot per word, 8 loads in flight; lane j keeps word j.
 template <int DT>
@@ -326,6 +359,8 @@ static void pack_rows_t(const void* dense, int64_t M, int64_t K, int64_t ld, uin
   if (is_aligned(dense, 16) && (ld * (int64_t)sizeof(T)) % 16 == 0 && K >= 32 * V::VEC)
     k_pack_rows_v16<DT><<<grid_for(M * ceil_div(Kw, V::VEC * V::U)), 256, 0, s>>>((const T*)dense, M, K, ld, words, Kw,
                                                                                msb);
+  else if (Kw <= kNarrowWords)
+    k_pack_rows_narrow<DT><<<grid_for(ceil_div(M * Kw, 8)), 256, 0, s>>>((const T*)dense, M, K, ld, words, Kw, msb);
   else
     k_pack_rows<DT><<<grid_for(M * ceil_div(Kw, 32)), 256, 0, s>>>((const T*)dense, M, K, ld, words, Kw, msb);
 }

@@ -106,3 +106,22 @@ def test_bitplanes_vector_path(M, K, LD):
     for planes, order in ((8, capi.LSB_FIRST), (3, capi.LSB_FIRST), (8, capi.MSB_FIRST)):
         got = ops.bitplanes(t, planes=planes, bit_order=order).cpu().numpy().view(np.uint32)
         assert np.array_equal(got, O.bitplanes(np.ascontiguousarray(v), planes, msb_first=order == capi.MSB_FIRST))
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.float16, torch.bfloat16, torch.uint8, torch.int8])
+@pytest.mark.parametrize("M,K,LD", [(1, 1, 1), (9, 31, 31), (100, 32, 32), (1000, 33, 40), (77, 64, 64), (555, 65, 67),
+                                    (20000, 96, 96), (64, 97, 97), (70000, 3, 5)])
+def test_pack_rows_of_few_words(M, K, LD, dt):
+    # up to three words a row: a warp's 8 words run over the rows' ends
+    rng = np.random.default_rng(M + K)
+    full = (rng.random((M, LD)) < 0.3).astype(np.uint8)
+    t = dev(full).to(dt)[:, :K]
+    for order in (capi.LSB_FIRST, capi.MSB_FIRST):
+        want = W.pack_bits(np.ascontiguousarray(full[:, :K]).astype(bool))
+        if order == capi.MSB_FIRST:
+            want = np.array([int("{:032b}".format(int(x))[::-1], 2) for x in want.reshape(-1)[:3000]], dtype=np.uint32)
+        got = ops.pack_rows(t, bit_order=order).cpu().numpy().view(np.uint32)
+        if order == capi.MSB_FIRST:
+            assert np.array_equal(got.reshape(-1)[:3000], want)
+        else:
+            assert np.array_equal(got, want)
