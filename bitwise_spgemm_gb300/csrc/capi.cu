@@ -515,6 +515,7 @@ static int prepare_spmm(const uint32_t* A_words, int64_t M, int64_t K, const voi
   a->C = C;
   a->ldc = ldc;
   a->Nb = N;
+  a->no_long_rows = plan && plan->long_rows == 0;
   a->c_vec = is_aligned(C, 16) && ldc % 4 == 0 && N % 4 == 0;
   // 16-bit B by TMA boxes, or copied into tile order where its rows take none
   // (and no row is long enough for the walk to sum it with compensation)

@@ -16,6 +16,8 @@
 // k_proto_sums (K split across the warps of a CTA, fixed-order reduction).
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
 #include "ptx.cuh"
 #include "spmm_dev.cuh"
 
@@ -36,15 +38,21 @@ namespace {
 // bit at a time from the words (find first set, shuffle, branch) between the
 // gathers spent about twenty dependent instructions per bit and cut every
 // round at a word: 1024x1024x256 FP32 at 10 %, 22.4 us against 9.7 now;
-// 2048x2048x1024, 155 us against 96 (17.9 TB/s of gathers, the L2 roof).  Rows with more than
+// 2048x2048x1024, 155 us against 85 (20 TB/s of gathers).  Rows with more than
 // kCompThreshold set bits, where there can be any, are summed with TwoSum one
 // vector at a time.
 constexpr int kListStep = 128;                 // entries wanted before a round of gathers
 constexpr int kListCap = kListStep + 32 * 32;  // one more group of 32 words
 
-template <typename V, int VPL, int D>
-__global__ void __launch_bounds__(256) k_spmm_list(SpmmArgs a) {
+//
+// FAST: no row has more than kCompThreshold set bits (K, or the plan, says so)
+// and B's element offsets fit in 32 bits; without the TwoSum walk and the 64-bit
+// row addresses, and with 4 gathers in flight, four blocks (MINB) run on an SM
+// instead of two.
+template <typename V, int VPL, int D, bool FAST, int MINB>
+__global__ void __launch_bounds__(256, MINB) k_spmm_list(SpmmArgs a) {
   using BT = typename V::T;
+  using Off = typename std::conditional<FAST, uint32_t, int64_t>::type;
   constexpr int COLS = V::COLS;
   constexpr int CW = 32 * VPL * COLS;
   constexpr int GROUPS = 4;  // word groups (of 32) loaded at a time
@@ -63,7 +71,8 @@ __global__ void __launch_bounds__(256) k_spmm_list(SpmmArgs a) {
   const BT* __restrict__ B = static_cast<const BT*>(a.B);
   const uint32_t* arow = a.A + row * a.Kw;
   const int Kw = (int)a.Kw;
-  const bool comp = a.K > kCompThreshold && row_popcount(arow, Kw, lane) > kCompThreshold;
+  const bool comp = !FAST && a.K > kCompThreshold && row_popcount(arow, Kw, lane) > kCompThreshold;
+  const Off ldb = (Off)a.ldb;
   for (int64_t n0 = (int64_t)blockIdx.y * CW; n0 < a.N; n0 += (int64_t)gridDim.y * CW) {
     int col[VPL];
     bool cvalid[VPL];
@@ -74,7 +83,7 @@ __global__ void __launch_bounds__(256) k_spmm_list(SpmmArgs a) {
       col[v] = cvalid[v] ? (int)c : 0;
     }
     float* crow = a.C + row * a.ldc;
-    if (comp) {
+    if (!FAST && comp) {
       for (int v = 0; v < VPL; v++) {
         BitWalker wk;
         wk.init(arow, 0, Kw, lane);
@@ -102,7 +111,7 @@ __global__ void __launch_bounds__(256) k_spmm_list(SpmmArgs a) {
       typename V::Raw raw[D][VPL];
 #pragma unroll
       for (int s = 0; s < D; s++) {
-        const BT* brow = B + (int64_t)idx[s] * a.ldb;
+        const BT* brow = B + (Off)idx[s] * ldb;
 #pragma unroll
         for (int v = 0; v < VPL; v++)
           if (s < n && cvalid[v]) raw[s][v] = V::load(brow + col[v]);
@@ -510,10 +519,15 @@ __global__ void __cluster_dims__(kSumCluster, 1, 1) __launch_bounds__(256) k_pro
   cluster.sync();
 }
 
-template <typename V, int VPL, int D>
+bool list_fast(const SpmmArgs& a) {
+  return (a.K <= kCompThreshold || a.no_long_rows) && a.K * a.ldb < ((int64_t)1 << 31);
+}
+
+template <typename V, int VPL, int D, bool FAST = false, int MINB = 0>
 int launch_list_s(const SpmmArgs& a, int64_t rows, cudaStream_t s) {
   const int64_t gy = ceil_div(a.N, 32 * VPL * V::COLS);
-  k_spmm_list<V, VPL, D><<<dim3((unsigned)ceil_div(rows, 8), (unsigned)(gy < 65535 ? gy : 65535)), 256, 0, s>>>(a);
+  k_spmm_list<V, VPL, D, FAST, MINB>
+      <<<dim3((unsigned)ceil_div(rows, 8), (unsigned)(gy < 65535 ? gy : 65535)), 256, 0, s>>>(a);
   BSP_LAUNCHED();
   return BSP_OK;
 }
@@ -556,13 +570,30 @@ int launch_rows_t(const SpmmArgs& a, cudaStream_t s) {
   // that runs (one row, 8192 columns at 5 %, N = 512: 9.1 us against 15.2;
   // from a few hundred tasks on the two are equal, 117 rows 21.5 and 20.0).
   if (tasks <= sms && a.K >= 1024 && chunks <= 65535) return launch_coop_s<V, VPL>(a, rows, s);
-  // One vector per lane: more warps beat wider slices at every size measured
-  // (2048x2048x1024 FP32, 10 %: 96 us, two vectors 106, four 112).  With 12
-  // or more warps an SM, 8 gathers in flight each (1024x1024x256: 9.7 us, 16
-  // in flight 11.2; 2048x2048x1024: 96 and 123); with fewer, 16 (300x4000x512
-  // at 2 %: 6.7 us, 8 in flight 7.7; 512x512x64: 4.3 and 5.2).
-  if (V::COLS == 1 || tasks >= 12 * sms) return launch_list_s<V, VPL, 8>(a, rows, s);
-  return launch_list_s<V, VPL, 16>(a, rows, s);
+  if constexpr (V::COLS == 1) {
+    // No more columns a lane than there are: 100000x32x8 FP32 170 us with four a
+    // lane, 29 with one; 4096x4096x12 BF16 at 5 % 107 and 23.
+    if (a.N <= 32) return list_fast(a) ? launch_list_s<V, 1, 4, true, 6>(a, rows, s) : launch_list_s<V, 1, 8>(a, rows, s);
+    if (a.N <= 64) return list_fast(a) ? launch_list_s<V, 2, 8, true>(a, rows, s) : launch_list_s<V, 2, 8>(a, rows, s);
+    return launch_list_s<V, VPL, 8>(a, rows, s);
+  } else {
+    // Many more warps than run at once: 4 gathers in flight each, four blocks an SM
+    // (2048x2048x1024 FP32 at 10 % 86 us, 8 in flight and two blocks 99;
+    // 4096x4096x512 BF16 at 5 % 67 and 76; 4000x400x2000 FP32 at 10 % 85 and 107),
+    // of FP32 two vectors a lane where they are nearly filled (one vector, two, 8 in
+    // flight: 4000x100x2000 at 10 % 45, 37, 56; 4096x4096x256 at 0.1 % 10.5, 8.4,
+    // 11.6; 2048x2048x1024 86, 85, 99; but 2000x3001x336 36, 38, 37).
+    // Not for FP16, whose conversions take the place (4096x4096x512 at 5 % 81 and 77).
+    if (!std::is_same<typename V::T, __half>::value && tasks >= 32 * sms && list_fast(a)) {
+      if (V::COLS == 4 && ceil_div(a.N, 256) * 256 * 10 <= a.N * 11) return launch_list_s<V, 2, 4, true>(a, rows, s);
+      return launch_list_s<V, 1, 4, true, 4>(a, rows, s);
+    }
+    // With 12 or more warps an SM, 8 gathers in flight each (1024x1024x256: 9.7 us,
+    // 16 in flight 11.2, 4 11.7; 2048x2048x1024: 96 and 123); with fewer, 16
+    // (300x4000x512 at 2 %: 6.7 us, 8 in flight 7.7; 512x512x64: 4.3 and 5.2).
+    if (tasks >= 12 * sms) return launch_list_s<V, VPL, 8>(a, rows, s);
+    return launch_list_s<V, VPL, 16>(a, rows, s);
+  }
 }
 
 template <typename BT>

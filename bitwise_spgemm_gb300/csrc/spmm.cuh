@@ -51,6 +51,7 @@ struct SpmmArgs {
   float* C;           // [M][ldc]
   int64_t ldc;
   bool c_vec;         // C's rows take 16-byte stores (else element by element)
+  bool no_long_rows;  // a plan says that no row has more than kCompThreshold set bits
   const int* run_if;  // device flag: zero = do nothing (walking kernels only); null = run
   // prototype mode (plan)
   const int32_t* row_cluster;  // [M], -1 = walk A's row

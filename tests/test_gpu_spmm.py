@@ -575,3 +575,39 @@ def test_prototype_plan_without_16_byte_rows(kind, M, K, N):
         assert torch.equal(got.view(torch.int32), want.view(torch.int32))
         assert torch.isfinite(got[~torch.from_numpy(A[:, k]).cuda()]).all()
     assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("kind", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("M,K,N,p,plan", [(5000, 70, 1, 0.2, False), (300, 1000, 32, 0.1, False), (300, 1000, 33, 0.1, False),
+                                          (700, 4099, 64, 0.03, False), (100, 500, 65, 0.1, False), (4900, 40, 128, 0.2, False),
+                                          (2500, 300, 256, 0.05, False), (2500, 4200, 512, 0.002, True),
+                                          (5000, 33, 264, 0.3, False), (20, 5000, 9, 0.9, False)])
+def test_walked_rows_forms(M, K, N, p, plan, kind):
+    """The walk's forms by width, number of warps, longest possible row and type:
+    a row's values are added in ascending order whatever the form, bit for bit."""
+    rng = np.random.default_rng(M + K + N)
+    bits = rng.random((M, K)) < p
+    if M > 100:
+        bits[M // 2] = True   # one full row, one empty
+        bits[M // 3] = False
+    words = W.pack_bits(bits)
+    wd = words_dev(words)
+    dt = {"f32": torch.float32, "bf16": torch.bfloat16, "f16": torch.float16}[kind]
+    Bt = torch.from_numpy(rng.standard_normal((K, N)).astype(np.float32)).cuda().to(dt)
+    pl = ops.Plan(wd, K, mode=capi.PLAN_DIRECT) if plan else None
+    import os
+    old = os.environ.get("BSP_TC")
+    os.environ["BSP_TC"] = "0"
+    try:
+        out = torch.full((M, N + 4), 7.0, device="cuda")
+        ops.spmm(wd, K, Bt, plan=pl, out=out[:, :N])
+    finally:
+        if old is None:
+            del os.environ["BSP_TC"]
+        else:
+            os.environ["BSP_TC"] = old
+    got, ref = out[:, :N].cpu().numpy(), O.spmm_f32(words, K, Bt.float().cpu().numpy())
+    long_rows = bits.sum(1) > 4096
+    assert np.array_equal(got[~long_rows], ref[~long_rows])
+    _check_f64(got, words, K, Bt.float().cpu().numpy())
+    assert torch.all(out[:, N:] == 7.0)
