@@ -4,7 +4,8 @@
 // (B's tensor map, encoded once on the host, and A, C, sizes) and a work list
 // with one item per (problem, 256-row block, 128-column block), sorted by
 // reduction length, longest first.  bsp_batched_spmm runs the list in one
-// launch of the persistent tensor-core kernel (spmm_ts.cu), with no host
+// launch of the persistent tensor-core kernel (spmm_ts.cu; batches wider than
+// 128 columns as 256x256 blocks of spmm_tc.cu where that is faster), with no host
 // synchronisation and no allocation; it reads the item's problem from its
 // record, runs every K tile of its rows (a batch has no occupancy plan) and
 // streams B by TMA through the problem's own tensor map.  dX of a gradient
@@ -29,7 +30,7 @@
 
 namespace bsp {
 
-// Kept for bsp_device_status: the tensor-core kernel reports its own waits.
+// The SDDMM's waits that ran out (the products report their own).
 __device__ int g_batch_error;
 
 int batched_device_error(int* out, bool clear) {
@@ -418,7 +419,8 @@ struct bsp_batch {
   void* dev = nullptr;  // records, items, the work-queue counter
   bsp::BatchProblemTc* probs = nullptr;    // forward, or Aᵀ·G (map = G)
   bsp::BatchProblemTc* probs_s = nullptr;  // SDDMM (map = G, map2 = X)
-  int4* items = nullptr;     // 256x256 blocks
+  int4* items = nullptr;     // 256x256 blocks (where they may run)
+  bool blocks = false;       // a forward batch that is faster in these blocks
   int4* items_ts = nullptr;  // the same output in 256x128 blocks, for the persistent kernel
   int n_items_ts = 0;
   int4* items_s = nullptr;
@@ -472,6 +474,56 @@ int batch_upload(bsp_batch* b, const std::vector<bsp::BatchProblemTc>& p1, const
   return BSP_OK;
 }
 
+bool env_is(const char* name, char v) {
+  const char* e = getenv(name);
+  return e && e[0] == v;
+}
+
+// Time (us) until the last of `sms` SMs, each taking the next item when it is
+// done, has finished a list of costs (of more than four rounds: what they add up
+// to, and half an item).
+double list_time(const std::vector<double>& cost, int sms) {
+  if (cost.size() > 4 * (size_t)sms) {
+    double sum = 0.0;
+    for (const double c : cost) sum += c;
+    return sum / sms + 0.5 * sum / (double)cost.size();
+  }
+  std::vector<double> busy((size_t)sms, 0.0);  // a heap, the first to be free on top
+  double last = 0.0;
+  for (const double c : cost) {
+    const double t = busy[0] + c;
+    last = std::max(last, t);
+    size_t i = 0;
+    for (size_t k = 1; k < busy.size(); k = 2 * i + 1) {
+      if (k + 1 < busy.size() && busy[k + 1] < busy[k]) k++;
+      if (busy[k] >= t) break;
+      busy[i] = busy[k];
+      i = k;
+    }
+    busy[i] = t;
+  }
+  return last;
+}
+
+// Forward batches wider than one 128-column item: a CTA per 256x256 block
+// (k_spmm_tc, whose expanded A serves 256 columns) or the persistent kernel's
+// 256x128 items, whichever finishes first by both lists' times; the figures are
+// fitted to 54 batches of 3 to 512 problems, N = 136 to 1024, where the rule
+// costs at most 1.13 of the better form and 1.01 on average (8 problems of 2048
+// to 4096 rows and columns, N = 136: 46 us and 59 persistent, N = 1024: 129 and
+// 163; 64 of 64 to 1024, N = 1024: 71 and 61; 3 of 4096, N = 256: 56 and 39).
+bool blocks_are_faster(const std::vector<int4>& blocks, const std::vector<int4>& items, int64_t N) {
+  std::vector<double> tb, ti;
+  tb.reserve(blocks.size());
+  ti.reserve(items.size());
+  for (const int4& b : blocks) {
+    const int64_t boxes = std::min<int64_t>(4, bsp::ceil_div(N - (int64_t)b.z * bsp::kItemCols, 64));
+    tb.push_back(9.0 + (double)b.w * (0.27 + 0.025 * (double)boxes));
+  }
+  for (const int4& i : items) ti.push_back(1.9 + (double)i.w * 0.285);
+  return list_time(tb, bsp::num_sms()) < 7.4 + list_time(ti, bsp::num_sms());
+}
+
 // longest reduction first (LPT), ties by problem order: stable
 void sort_items(std::vector<int4>& items) {
   std::stable_sort(items.begin(), items.end(), [](const int4& x, const int4& y) { return x.w > y.w; });
@@ -492,6 +544,7 @@ int bsp_batch_create(const bsp_problem* problems, int n, int64_t N, int b_dtype,
   if (N % 8 != 0) return BSP_ERR_ALIGNMENT;
   std::vector<BatchProblemTc> hp((size_t)n);
   std::vector<int4> items, ts;
+  const bool blocks = N > ts_item_cols() || env_is("BSP_BATCH_PERSIST", '0');
   for (int i = 0; i < n; i++) {
     const bsp_problem& p = problems[i];
     if (p.M < 0 || p.K < 0 || p.M > INT32_MAX || p.K > ((int64_t)1 << 30)) return BSP_ERR_INVALID_ARG;
@@ -513,7 +566,7 @@ int bsp_batch_create(const bsp_problem* problems, int n, int64_t N, int b_dtype,
     r.C = p.C;
     r.ldc = p.ldc;
     if (p.M > 0 && N > 0) BSP_TRY(make_out_map(&r.map2, p.C, p.M, N, p.ldc, 1, p.M * p.ldc));
-    for (int64_t rb = 0; rb < ceil_div(p.M, kItemRows); rb++)
+    for (int64_t rb = 0; blocks && rb < ceil_div(p.M, kItemRows); rb++)
       for (int64_t nb = 0; nb < ceil_div(N, kItemCols); nb++) items.push_back(make_int4(i, (int)rb, (int)nb, (int)Kw));
     for (int64_t rb = 0; rb < ceil_div(p.M, ts_item_rows()); rb++)
       for (int64_t nb = 0; nb < ceil_div(N, ts_item_cols()); nb++) ts.push_back(make_int4(i, (int)rb, (int)nb, (int)Kw));
@@ -526,6 +579,7 @@ int bsp_batch_create(const bsp_problem* problems, int n, int64_t N, int b_dtype,
   b->n = n;
   b->N = N;
   b->bdt = b_dtype;
+  b->blocks = !items.empty() && blocks_are_faster(items, ts, N);
   cudaGetDevice(&b->device);
   const int st = batch_upload(b, hp, items, {}, {}, (cudaStream_t)stream, ts);
   if (st != BSP_OK) {
@@ -548,6 +602,7 @@ int bsp_batch_grad_create(const bsp_problem_grad* problems, int n, int64_t N, in
   if (N % 8 != 0) return BSP_ERR_ALIGNMENT;
   std::vector<BatchProblemTc> pt, ps;
   std::vector<int4> it, is, isp, ts;
+  const bool blocks = env_is("BSP_BATCH_PERSIST", '0'), blocks_s = env_is("BSP_BATCH_SDDMM_PERSIST", '0');
   for (int i = 0; i < n; i++) {
     const bsp_problem_grad& p = problems[i];
     if (p.M < 0 || p.K < 0 || p.M > INT32_MAX || p.K > INT32_MAX) return BSP_ERR_INVALID_ARG;
@@ -575,7 +630,7 @@ int bsp_batch_grad_create(const bsp_problem_grad* problems, int n, int64_t N, in
       if (N > 0) BSP_TRY(make_out_map(&r.map2, p.dX, p.K, N, p.lddx, 1, p.K * p.lddx));
       const int idx = (int)pt.size();
       pt.push_back(r);
-      for (int64_t rb = 0; rb < ceil_div(p.K, kItemRows); rb++)
+      for (int64_t rb = 0; blocks && rb < ceil_div(p.K, kItemRows); rb++)
         for (int64_t nb = 0; nb < ceil_div(N, kItemCols); nb++)
           it.push_back(make_int4(idx, (int)rb, (int)nb, (int)ceil_div(p.M, 32)));
       for (int64_t rb = 0; rb < ceil_div(p.K, ts_item_rows()); rb++)
@@ -600,7 +655,7 @@ int bsp_batch_grad_create(const bsp_problem_grad* problems, int n, int64_t N, in
       r.ldc = p.ldda;
       const int idx = (int)ps.size();
       ps.push_back(r);
-      for (int64_t rb = 0; rb < ceil_div(p.M, kItemRows); rb++)
+      for (int64_t rb = 0; blocks_s && rb < ceil_div(p.M, kItemRows); rb++)
         for (int64_t kb = 0; kb < ceil_div(p.K, kItemCols); kb++)
           is.push_back(make_int4(idx, (int)rb, (int)kb, (int)ceil_div(N, 64)));
       for (int64_t rb = 0; rb < ceil_div(p.M, (int64_t)kSdRows); rb++)
@@ -643,12 +698,12 @@ int bsp_batched_spmm(const bsp_batch* b, bsp_stream_t stream) {
   int dev = -1;
   cudaGetDevice(&dev);
   if (dev != b->device) return BSP_ERR_INVALID_ARG;
-  if (b->n_items == 0 || b->N == 0) return BSP_OK;
+  if (b->n_items_ts == 0 || b->N == 0) return BSP_OK;
   const cudaStream_t s = (cudaStream_t)stream;
-  // the persistent kernel; BSP_BATCH_PERSIST=0 selects a CTA per 256x256 block,
-  // for comparisons
-  const char* e = getenv("BSP_BATCH_PERSIST");
-  if (!(e && e[0] == '0')) return launch_ts_batch(b->probs, b->items_ts, b->n_items_ts, b->N, b->bdt, false, s);
+  // (BSP_BATCH_PERSIST, for comparisons: 1 = the persistent kernel, 0 = a CTA per
+  // 256x256 block where the batch was created with it or is wider than 128)
+  const bool blocks = b->n_items > 0 && !env_is("BSP_BATCH_PERSIST", '1') && (b->blocks || env_is("BSP_BATCH_PERSIST", '0'));
+  if (!blocks) return launch_ts_batch(b->probs, b->items_ts, b->n_items_ts, b->N, b->bdt, false, s);
   return launch_batched_tc(b->probs, b->items, b->n_items, b->N, b->bdt, s);
 }
 
@@ -690,20 +745,21 @@ int bsp_batched_spmm_grad(const bsp_batch* b, bsp_stream_t stream) {
   if (dev != b->device) return BSP_ERR_INVALID_ARG;
   if (b->N == 0) return BSP_OK;
   const cudaStream_t s = (cudaStream_t)stream;
-  // dX = Aᵀ·G: the persistent kernel in its transposed form (BSP_BATCH_PERSIST=0
-  // selects a CTA per 256x256 block, for comparisons).  dA neither reads nor
+  // dX = Aᵀ·G: the persistent kernel in its transposed form.  dA neither reads nor
   // writes what dX does, and all that came before dX's launch is complete when
   // dX starts: as its programmatic dependent the persistent SDDMM takes the SMs
   // that dX's last items leave idle (128 problems of 64..2048 rows and columns, N
   // = 96, forward and both gradients: 111 -> 99 us).  Its counter is
   // reset before both, so that nothing stands between the two launches.
-  const char* ep = getenv("BSP_BATCH_PERSIST");
-  const char* e = getenv("BSP_BATCH_SDDMM_PERSIST");  // 0: a CTA per 256x256 block
-  const bool ts = !(ep && ep[0] == '0') && b->n_items_ts > 0, sd = !(e && e[0] == '0') && b->n_items_sp > 0;
+  // (BSP_BATCH_PERSIST=0, BSP_BATCH_SDDMM_PERSIST=0, set when the batch is created
+  // and when it runs: a CTA per 256x256 block)
+  const bool ts = b->n_items_ts > 0 && !(env_is("BSP_BATCH_PERSIST", '0') && b->n_items > 0);
+  const bool blocks_s = env_is("BSP_BATCH_SDDMM_PERSIST", '0') && b->n_items_s > 0;
+  const bool sd = !blocks_s && b->n_items_sp > 0;
   if (sd) BSP_CUDA(cudaMemsetAsync(b->counter, 0, sizeof(int), s));
   if (ts) BSP_TRY(launch_ts_batch(b->probs, b->items_ts, b->n_items_ts, b->N, b->bdt, true, s));
   else BSP_TRY(launch_batched_tc(b->probs, b->items, b->n_items, b->N, b->bdt, s, 1));
-  if (!(e && e[0] == '0')) {
+  if (!blocks_s) {
     if (!sd) return BSP_OK;
     if (b->bdt == BSP_BF16)
       return launch_sddmm_persist_t<__nv_bfloat16>(b->probs_s, b->items_sp, b->n_items_sp, b->counter, b->N, ts, s);

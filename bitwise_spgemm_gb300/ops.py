@@ -473,7 +473,8 @@ def csr_to_tiled(row_ptr, col_idx, M, K, tile_rows, tile_cols, values=None):
 class Batch:
     """Many independent C_i = A_i·B_i (16-bit B, shared N) in one tensor-core
     launch of the persistent kernel (a CTA per SM, items of 256 rows x 128
-    columns).  Runs of one batch must not overlap on the GPU (they share the
+    columns) or, wider than 128 columns, of a CTA per 256x256 block where that is
+    faster.  Runs of one batch must not overlap on the GPU (they share the
     C buffers).  ``problems``: list of (words, K, B, C) tensors; the
     tensors are referenced by the batch and must outlive it."""
 

@@ -266,8 +266,8 @@ typedef struct bsp_batch bsp_batch;
 
 /* Prepare a batch of n independent problems sharing N (multiple of 8) and a
  * 16-bit B type: encodes every problem's B tensor map and uploads them with
- * a work list of (problem, 256-row block, 256-column block) items sorted
- * longest reduction first; synchronises the stream once.  The problems'
+ * a work list of (problem, 256-row block, 128-column block) items (wider than 128:
+ * and of 256-column blocks) sorted longest reduction first; synchronises the stream once.  The problems'
  * buffers are referenced, not copied — they must outlive the batch.  Limit:
  * K ≤ 131072 per problem (BSP_ERR_CAPACITY).  No reference counterpart (the
  * reference runs one fixed-size problem per launch).                       */
@@ -276,8 +276,9 @@ int bsp_batch_create(const bsp_problem* problems, int n, int64_t N,
 int bsp_batch_destroy(bsp_batch* batch);
 /* Every problem of the batch in one tensor-core launch, with no host
  * synchronisation and no allocation; it can be captured in a CUDA graph.
- * The launch is persistent: a CTA per SM takes over the items of CTAs that
- * have not started.  Runs of one batch must not overlap on the GPU: they
+ * For N ≤ 128 the launch is persistent: a CTA per SM takes over the items of
+ * CTAs that have not started; for wider N it is that or a CTA per 256x256 block,
+ * by an estimate made when the batch is created.  Runs of one batch must not overlap on the GPU: they
  * share the C buffers.                                                      */
 int bsp_batched_spmm(const bsp_batch* batch, bsp_stream_t stream);
 /* Times the batch — once to warm up, then three runs — and returns the index
@@ -309,7 +310,7 @@ typedef struct bsp_problem_grad {
 
 /* Prepare a gradient batch: n problems sharing N (multiple of 8) and the
  * 16-bit type of X and G.  Encodes the G and X tensor maps, uploads them
- * with the work lists — (problem, 256-row block of dX, 256-column block)
+ * with the work lists — (problem, 256-row block of dX, 128-column block)
  * and (problem, 128-row block of dA, 256-column block of dA) — sorted
  * longest reduction first; synchronises the stream once.  Buffers are
  * referenced and must outlive the batch; bsp_batch_destroy releases it.

@@ -259,3 +259,38 @@ def test_batch_tune_keeps_results_exact():
     dev = _run(probs, 200)
     batch = ops.Batch(dev)
     assert batch.tune()[0] == 0
+
+
+@pytest.mark.parametrize("N,count,lo,hi", [(136, 8, 30, 60), (512, 3, 40, 41), (264, 60, 1, 12), (136, 2, 1, 2),
+                                           (1024, 12, 4, 30)])
+def test_wide_batches_in_both_forms(N, count, lo, hi):
+    """Batches wider than 128 columns: 256x256 blocks or 256x128 items, whichever
+    the estimate picks, and each asked for: exact on integers (uneven problems,
+    ragged rows, one without bits)."""
+    import os
+    rng = np.random.default_rng(N + count)
+    dev, want = [], []
+    for i in range(count):
+        M, K = 32 * int(rng.integers(lo, hi)) + (i % 3), 32 * int(rng.integers(lo, hi)) + 5 * (i % 2)
+        bits = rng.random((M, K)) < (0.0 if i == 2 else 0.1)
+        words = W.pack_bits(bits)
+        B = torch.from_numpy(rng.integers(-8, 9, (K, N)).astype(np.float32)).cuda()
+        wd = torch.from_numpy(words.view(np.int32)).cuda()
+        dev.append((wd, K, B.bfloat16(), torch.empty((M, N), device="cuda")))
+        want.append(torch.from_numpy(bits.astype(np.float32)).cuda() @ B)
+    batch = ops.Batch(dev)
+    old = os.environ.pop("BSP_BATCH_PERSIST", None)
+    try:
+        for form in (None, "0", "1"):
+            if form is not None:
+                os.environ["BSP_BATCH_PERSIST"] = form
+            for *_, C in dev:
+                C.fill_(float("nan"))
+            batch.run()
+            for (*_, C), w in zip(dev, want):
+                assert torch.equal(C, w), form
+    finally:
+        os.environ.pop("BSP_BATCH_PERSIST", None)
+        if old is not None:
+            os.environ["BSP_BATCH_PERSIST"] = old
+    assert capi.device_status() == 0
