@@ -247,3 +247,26 @@ def test_int8_values_of_extreme_operands(dt):
     assert np.all(C[:, 1] == np.inf) and np.all(C[:, 2] == -np.inf) and np.all(np.isnan(C[:, 3]))
     rest = [j for j in range(N) if j not in (1, 2, 3)]
     assert np.array_equal(C[:, rest].astype(np.float64), want[:, rest])
+
+
+@pytest.mark.parametrize("M,K,pad", [(1, 1, 0), (128, 1024, 0), (129, 1025, 0), (300, 2080, 4), (127, 33, 3), (640, 95, 1)])
+def test_int8_tile_order(M, K, pad):
+    """The values' order and the bit per 128 x 32 tile with a nonzero, at the
+    edges of tiles and of blocks, with and without 4-byte rows."""
+    import ctypes
+    rng = np.random.default_rng(M + K)
+    full = rng.integers(-128, 128, (M, K + pad)).astype(np.int8)
+    keep = rng.random((-(-M // 128), -(-K // 32))) < 0.5
+    full[:, :K] *= keep.repeat(128, 0).repeat(32, 1)[:M, :K]
+    A = dev(full)
+    n = ctypes.c_size_t()
+    capi.call("bsp_i8_tiles_bytes", M, K, ctypes.byref(n))
+    tiles = torch.full((n.value,), 77, dtype=torch.int8, device="cuda")
+    capi.call("bsp_i8_tiles", A.data_ptr(), M, K, K + pad, tiles.data_ptr(), None)
+    got, Kt = tiles.cpu().numpy(), -(-K // 32)
+    want = np.zeros((M, Kt * 32), dtype=np.int8)
+    want[:, :K] = full[:, :K]
+    assert np.array_equal(got[:M * Kt * 32].reshape(Kt, M, 32), want.reshape(M, Kt, 32).transpose(1, 0, 2))
+    bits = np.unpackbits(got[M * Kt * 32:].view(np.uint8), bitorder="little").reshape(-(-M // 128), -1)
+    hold = np.pad(want, ((0, -M % 128), (0, 0))).reshape(-(-M // 128), 128, Kt, 32).any((1, 3))
+    assert np.array_equal(bits[:, :Kt].astype(bool), hold) and not bits[:, Kt:].any()
