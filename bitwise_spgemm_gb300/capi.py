@@ -99,6 +99,7 @@ SIGNATURES = {
     "bsp_spmm_workspace_layout": [_P, _I64, _I64, _P, _I, _I64, C.POINTER(_SZ)],
     "bsp_spmm_workspace_preferred": [_P, _I64, C.POINTER(_SZ)],
     "bsp_spmm_t_as": [_P, _I64, _I64, _P, _I, _I64, _I64, _P, _I, _I64, _P, _P, _SZ, _P],
+    "bsp_spmm_t_as_workspace": [_P, _I64, _I64, _P, _I, _I64, _I64, _I, C.POINTER(_SZ)],
     "bsp_spmm_t_workspace_layout": [_P, _I64, _I64, _I64, _I, C.POINTER(_SZ)],
     "bsp_spmm_t_workspace_preferred": [_I64, _I64, _I64, C.POINTER(_SZ)],
     "bsp_tune": [_P, _I64, _I64, _P, _I, _I64, _I64, _P, _I64, _P, _P, _SZ, _P, C.POINTER(Schedule)],

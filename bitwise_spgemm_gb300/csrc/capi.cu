@@ -345,6 +345,12 @@ static bool align_operands(SpmmArgs* a, const bsp_plan* plan, void* workspace, s
   return true;
 }
 
+// 16-bit B in tile order, whatever its layout: not beyond the kernel's limits, nor
+// with a row that the walk sums with compensation.
+static bool unaligned_on_tensor_cores(const bsp_plan* plan, int64_t N) {
+  return plan->K <= tc_max_reduction() && N <= ts_max_cols() && plan->long_rows == 0;
+}
+
 // Runs the SpMM with a given schedule (arguments already validated).
 static int run_spmm(SpmmArgs a, const bsp_plan* plan, bool vec, const TuneSched& sc, void* workspace,
                     size_t workspace_bytes, cudaStream_t s) {
@@ -467,17 +473,29 @@ int bsp_spmm_workspace_preferred(const bsp_plan* plan, int64_t N, size_t* bytes)
 int bsp_spmm_workspace_layout(const bsp_plan* plan, int64_t K, int64_t N, const void* B, int b_dtype, int64_t ldb,
                               size_t* bytes) {
   if (K < 0 || (b_dtype != BSP_F32 && b_dtype != BSP_BF16 && b_dtype != BSP_F16)) return BSP_ERR_INVALID_ARG;
-  BSP_TRY(preferred_workspace(plan, N, b_dtype, bytes));
   const int esz = dtype_size(b_dtype);
-  if (plan && b_dtype == BSP_F32 && N > 0 && use_tensor_cores(plan, N, esz, true)) {
-    const size_t parts = tc_parts_bytes(plan->M, N, plan->K);
-    if (parts > *bytes) *bytes = parts;
+  const bool rows16 = is_aligned(B, 16) && (ldb * esz) % 16 == 0 && (N * esz) % 16 == 0;
+  const bool parts = plan && b_dtype == BSP_F32 && N > 0 && use_tensor_cores(plan, N, esz, true);
+  if (rows16) {
+    BSP_TRY(preferred_workspace(plan, N, b_dtype, bytes));
+    if (parts && tc_parts_bytes(plan->M, N, plan->K) > *bytes) *bytes = tc_parts_bytes(plan->M, N, plan->K);
+    return BSP_OK;
   }
-  if (is_aligned(B, 16) && (ldb * esz) % 16 == 0 && (N * esz) % 16 == 0) return BSP_OK;
-  size_t base = 0;
-  BSP_TRY(bsp_spmm_workspace(plan, N, &base));
-  const size_t copy = base + align_b_bytes(K, N, esz) + (plan && plan->mode == BSP_PLAN_PROTO ? col_stats_bytes(N) : 0);
-  if (copy > *bytes) *bytes = copy;
+  // what the product of these rows will use: B in tile order and room for sums, B's
+  // parts, or a copy with 16-byte rows where that pays (nothing for small calls)
+  BSP_TRY(bsp_spmm_workspace(plan, N, bytes));
+  if (N == 0) return BSP_OK;
+  size_t need = 0;
+  if (parts) {
+    need = tc_parts_bytes(plan->M, N, plan->K);
+  } else if (plan && esz == 2 && unaligned_on_tensor_cores(plan, N) && use_tensor_cores(plan, N, esz, false)) {
+    need = tc_unaligned_bytes(plan->M, N, plan->K);
+  } else {
+    need = *bytes;
+    if (plan && plan->mode == BSP_PLAN_PROTO) need += col_stats_bytes(N);
+    if (!plan || align_pays(plan, plan->M, K, N, esz)) need += align_b_bytes(K, N, esz);
+  }
+  if (need > *bytes) *bytes = need;
   return BSP_OK;
 }
 
@@ -520,8 +538,7 @@ static int prepare_spmm(const uint32_t* A_words, int64_t M, int64_t K, const voi
   // 16-bit B by TMA boxes, or copied into tile order where its rows take none
   // (and no row is long enough for the walk to sum it with compensation)
   *tc_ok = plan && b_dtype != BSP_F32 && plan->K <= tc_max_reduction() &&
-           (*vec || (workspace && workspace_bytes >= tc_tiled_b_bytes(K, N) && N <= ts_max_cols() &&
-                     plan->long_rows == 0));
+           (*vec || (workspace && workspace_bytes >= tc_tiled_b_bytes(K, N) && unaligned_on_tensor_cores(plan, N)));
   // FP32 as parts, where there is room for them
   if (plan && b_dtype == BSP_F32 && K <= kPartsMaxReduction && N <= (int64_t)1 << 21)
     *tc_ok = parts_apply(plan) && workspace && workspace_bytes >= tc_parts_bytes(M, N, K);
@@ -900,6 +917,21 @@ static bool trans_on_tensor_cores(const bsp_plan* plan, int64_t N) {
   return tc < cc;
 }
 
+// dX in G's 16-bit type: rounded in the epilogue of one pass over the whole
+// reduction, or not here.
+static bool trans_in_16_bits(const bsp_plan* plan, int64_t M, int64_t K, const void* G, int g_dtype, int64_t ldg,
+                             int64_t N, int dx_dtype) {
+  return plan && g_dtype != BSP_F32 && dx_dtype == g_dtype && M > 0 && K > 0 && N > 0 && M <= tc_max_reduction() &&
+         tc_split_count(K, N, ceil_div(M, 32)) == 1 && trans_on_tensor_cores(plan, N) && layout16(G, ldg, 2, N, 8);
+}
+
+int bsp_spmm_t_as_workspace(const bsp_plan* plan, int64_t M, int64_t K, const void* G, int g_dtype, int64_t ldg,
+                            int64_t N, int dx_dtype, size_t* bytes) {
+  if (!bytes || M < 0 || K < 0 || N < 0) return BSP_ERR_INVALID_ARG;
+  if (!trans_in_16_bits(plan, M, K, G, g_dtype, ldg, N, dx_dtype)) return BSP_ERR_UNSUPPORTED;
+  return bsp_spmm_t_workspace_preferred(M, K, N, bytes);
+}
+
 int bsp_spmm_t_as(const uint32_t* A_words, int64_t M, int64_t K, const void* G, int g_dtype, int64_t ldg, int64_t N,
                   void* dX, int dx_dtype, int64_t lddx, const bsp_plan* plan, void* workspace, size_t workspace_bytes,
                   bsp_stream_t stream) {
@@ -909,13 +941,10 @@ int bsp_spmm_t_as(const uint32_t* A_words, int64_t M, int64_t K, const void* G, 
   BSP_TRY(check_dims(M, K));
   if (N < 0 || N > kMaxCols || ldg < N || lddx < N) return BSP_ERR_INVALID_ARG;
   if (plan && (plan->M != M || plan->K != K || plan->device != current_device())) return BSP_ERR_INVALID_ARG;
-  // rounded in the epilogue of one pass over the whole reduction, or not here
-  if (!plan || g_dtype == BSP_F32 || dx_dtype != g_dtype || M == 0 || K == 0 || N == 0 || M > tc_max_reduction() ||
-      tc_split_count(K, N, ceil_div(M, 32)) > 1 || !trans_on_tensor_cores(plan, N))
-    return BSP_ERR_UNSUPPORTED;
+  if (!trans_in_16_bits(plan, M, K, G, g_dtype, ldg, N, dx_dtype)) return BSP_ERR_UNSUPPORTED;
   if (!dX || !A_words || !G) return BSP_ERR_INVALID_ARG;
   if (!is_aligned(A_words, 4)) return BSP_ERR_ALIGNMENT;
-  if (!layout16(G, ldg, 2, N, 8) || !layout16(dX, lddx, 2, N, 8)) return BSP_ERR_UNSUPPORTED;
+  if (!layout16(dX, lddx, 2, N, 8)) return BSP_ERR_UNSUPPORTED;
   return launch_spmm_t_tc(A_words, M, K, G, g_dtype, ldg, N, dX, true, lddx, plan->occT, plan->wordsT,
                           (cudaStream_t)stream, workspace, workspace_bytes);
 }

@@ -156,6 +156,8 @@ size_t tc_split_bytes(int64_t out_rows, int64_t out_cols, int64_t red_tiles);
 // the output's rows cannot start on 16 bytes, keeps its sums in rows that do.
 size_t tc_tiled_b_bytes(int64_t red_rows, int64_t cols);
 size_t tc_preferred_bytes(int64_t out_rows, int64_t out_cols, int64_t red_rows, bool any_layout = false);
+// ... of a 16-bit B without 16-byte rows: in tile order always
+size_t tc_unaligned_bytes(int64_t out_rows, int64_t out_cols, int64_t red_rows);
 // FP32 B (any layout) on the tensor cores as three exact BF16 parts: C = A·B, or
 // dX = Aᵀ·G with occT; the workspace must hold tc_parts_bytes(output rows, N,
 // reduction rows), nnz are A's set bits.  *skipped: a device flag, nonzero when C was left to the

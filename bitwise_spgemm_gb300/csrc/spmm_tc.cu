@@ -945,6 +945,12 @@ size_t tc_preferred_bytes(int64_t out_rows, int64_t out_cols, int64_t red_rows, 
   return sums + (tc_tiles_b(out_rows) || out_cols % 8 != 0 ? tc_tiled_b_bytes(red_rows, out_cols) : 0);
 }
 
+size_t tc_unaligned_bytes(int64_t out_rows, int64_t out_cols, int64_t red_rows) {
+  size_t sums = tc_split_bytes(out_rows, out_cols, ceil_div(red_rows, kTcK));
+  if (sums == 0 && out_cols % 4 != 0) sums = one_part_bytes(out_rows, out_cols);
+  return sums + tc_tiled_b_bytes(red_rows, out_cols);
+}
+
 namespace {
 
 // BSP_TC_TILED_B=0 keeps B on tensor boxes even with room for the tiled copy.

@@ -209,13 +209,14 @@ def spmm_t(words, M, K, G, plan=None, out=None, workspace=None, dtype=torch.floa
         return dX if dX is not None else spmm_t(words, M, K, G, plan, None, workspace).to(dtype)
     if out is None:
         out = torch.empty((K, N), dtype=torch.float32, device=G.device)
-    n_min, n_pref = C.c_size_t(), C.c_size_t()
-    call("bsp_spmm_t_workspace", M, K, C.byref(n_min))
-    call("bsp_spmm_t_workspace_layout", plan.handle if plan is not None else None, M, K, N, _DT[G.dtype],
-         C.byref(n_pref))
     # a caller's workspace is used if it holds the minimum; else the preferred size
-    if workspace is None or workspace.numel() * workspace.element_size() < n_min.value:
-        workspace = torch.empty(n_pref.value, dtype=torch.uint8, device=G.device)
+    n = C.c_size_t()
+    if workspace is not None:
+        call("bsp_spmm_t_workspace", M, K, C.byref(n))
+    if workspace is None or workspace.numel() * workspace.element_size() < n.value:
+        call("bsp_spmm_t_workspace_layout", plan.handle if plan is not None else None, M, K, N, _DT[G.dtype],
+             C.byref(n))
+        workspace = torch.empty(n.value, dtype=torch.uint8, device=G.device)
     call("bsp_spmm_t", _p(words), M, K, _p(G), _DT[G.dtype], ldg, N, _p(out), out.stride(0),
          plan.handle if plan is not None else None, _p(workspace),
          workspace.numel() * workspace.element_size(), _stream())
@@ -224,10 +225,12 @@ def spmm_t(words, M, K, G, plan=None, out=None, workspace=None, dtype=torch.floa
 
 def _spmm_t_as(words, M, K, G, plan, workspace, dtype):
     """dX in G's 16-bit type from the product's own epilogue, or None where
-    the library has no such pass."""
+    the library has no such pass (asked before anything is allocated)."""
     N = G.shape[1]
     n = C.c_size_t()
-    call("bsp_spmm_t_workspace_preferred", M, K, N, C.byref(n))
+    if capi.lib().bsp_spmm_t_as_workspace(plan.handle, M, K, _p(G), _DT[G.dtype], G.stride(0), N, _DT[dtype],
+                                          C.byref(n)) != capi.BSP_OK:
+        return None
     if workspace is None or workspace.numel() * workspace.element_size() < n.value:
         workspace = torch.empty(n.value, dtype=torch.uint8, device=G.device)
     out = torch.empty((K, N), dtype=dtype, device=G.device)

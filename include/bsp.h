@@ -222,9 +222,10 @@ int bsp_spmm_workspace(const bsp_plan* plan, int64_t N, size_t* bytes);
  * own workspace the same way when it is large enough.                       */
 int bsp_spmm_workspace_preferred(const bsp_plan* plan, int64_t N, size_t* bytes);
 
-/* Workspace for these operands: the above and, where B's rows do not take
- * 16-byte loads (B, ldb or N not a multiple of 16 bytes; plan may be NULL),
- * room for a copy of B that does; for FP32 B whose product is cheaper on the
+/* Workspace for these operands: the above or, where B's rows do not take
+ * 16-byte loads (B, ldb or N not a multiple of 16 bytes; plan may be NULL), what
+ * the product will use of it: room for B in tile order, or for a copy of B that
+ * takes them where it pays; for FP32 B whose product is cheaper on the
  * tensor cores, room for its three BF16 parts (exact: x = h + m + l) and their
  * products.  A smaller workspace only turns these off (the copy changes no
  * result, the parts change the order of the FP32 sums).  B is looked at as an
@@ -397,6 +398,9 @@ int bsp_spmm_t(const uint32_t* A_words, int64_t M, int64_t K, const void* G,
  * rounded once where it leaves the tensor cores.  BSP_ERR_UNSUPPORTED, with
  * nothing launched, where the 16-bit form has no such pass (no plan, another
  * engine, a split reduction, rows without 16-byte access): take dX in FP32.  */
+int bsp_spmm_t_as_workspace(const bsp_plan* plan, int64_t M, int64_t K, const void* G,
+                            int g_dtype, int64_t ldg, int64_t N, int dx_dtype,
+                            size_t* bytes);  /* its workspace, or BSP_ERR_UNSUPPORTED (dX with 16-byte rows taken for granted) */
 int bsp_spmm_t_as(const uint32_t* A_words, int64_t M, int64_t K, const void* G,
                   int g_dtype, int64_t ldg, int64_t N, void* dX, int dx_dtype,
                   int64_t lddx, const bsp_plan* plan, void* workspace,

@@ -492,3 +492,49 @@ def test_f32_parts_of_long_integers(force_tc, M, K, N):
     dX = ops.spmm_t(wt, K, M, torch.from_numpy(G).cuda(), plan=ops.Plan(wt, M, mode=capi.PLAN_DIRECT))
     assert np.array_equal(dX.cpu().numpy().astype(np.float64), O.spmm_f64(words, K, G))
     assert capi.device_status() == 0
+
+
+def test_workspace_of_column_slices():
+    """Rows of B off the 16-byte grid, N a multiple of 8: the workspace that is
+    asked for lets a dense product use the tensor cores, and is empty for a small
+    one, which uses none."""
+    import ctypes
+    g = torch.Generator(device="cuda").manual_seed(2)
+
+    def layout(plan, K, N, B):
+        n = ctypes.c_size_t()
+        capi.call("bsp_spmm_workspace_layout", plan.handle, K, N, B.data_ptr(),
+                  capi.F32 if B.dtype == torch.float32 else capi.BF16, B.stride(0), ctypes.byref(n))
+        return n.value
+
+    for M, K, N in [(600, 2048, 512), (2600, 2048, 1024)]:  # with a split reduction, and without
+        A = torch.rand((M, K), device="cuda", generator=g) < 0.3
+        wd = ops.pack_rows(A.to(torch.uint8))
+        plan = ops.Plan(wd, K, mode=capi.PLAN_DIRECT)
+        B = torch.randn((K, N + 5), device="cuda", generator=g).bfloat16()[:, 3:N + 3]
+        C = ops.spmm(wd, K, B, plan=plan)
+        assert not torch.equal(C, ops.spmm(wd, K, B))  # not the walk's sums
+        assert float((C - A.float() @ B.float()).abs().max()) <= 1e-3
+    A = torch.rand((64, 96), device="cuda", generator=g) < 0.1
+    wd = ops.pack_rows(A.to(torch.uint8))
+    plan = ops.Plan(wd, 96, mode=capi.PLAN_DIRECT)
+    for B in (torch.randn((96, 21), device="cuda").bfloat16()[:, 3:19], torch.randn((96, 17), device="cuda")):
+        assert layout(plan, 96, B.shape[1], B) == 0
+        assert torch.equal(ops.spmm(wd, 96, B, plan=plan), ops.spmm(wd, 96, B))
+
+
+def test_spmm_t_in_16_bits_asks_before_it_allocates(force_tc, monkeypatch):
+    """Where the library has no 16-bit pass (a split reduction, rows off the
+    grid) nothing is allocated for it."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    cases = []
+    for M, K, N in [(2000, 500, 200), (300, 2600, 1001)]:
+        wd = ops.pack_rows((torch.rand((M, K), device="cuda", generator=g) < 0.1).to(torch.uint8))
+        cases.append((wd, M, K, torch.randn((M, N), device="cuda", generator=g).bfloat16(), ops.Plan(wd, K)))
+
+    def refuse(*a, **k):
+        raise AssertionError("allocated")
+
+    monkeypatch.setattr(torch, "empty", refuse)
+    for wd, M, K, G, plan in cases:
+        assert ops._spmm_t_as(wd, M, K, G, plan, None, G.dtype) is None
