@@ -374,8 +374,11 @@ static int run_spmm(SpmmArgs a, const bsp_plan* plan, bool vec, const TuneSched&
   int path = sc.proto_path;
   bool proto = plan && plan->mode == BSP_PLAN_PROTO;
   size_t need = 0;
-  ColStats stats = {};
   const bool plain = vec;
+  const void* B0 = a.B;
+  const int64_t ldb0 = a.ldb;
+  void* stats_ws = nullptr;
+  SpmmArgs walk = a;
   if (proto) {
     bsp_spmm_workspace(plan, N, &need);
     const bool room = workspace && workspace_bytes >= need;
@@ -390,16 +393,13 @@ static int run_spmm(SpmmArgs a, const bsp_plan* plan, bool vec, const TuneSched&
       proto = workspace && workspace_bytes >= need + col_stats_bytes(N) && N <= (int64_t)65535 * 32 &&
               K <= kStatMaxRows;
       if (proto) {
-        BSP_TRY(launch_col_stats(a.B, a.bdt, K, N, a.ldb, static_cast<char*>(workspace) + need, kProtoOctaves, &stats,
-                                 s));
+        stats_ws = static_cast<char*>(workspace) + need;
         need += col_stats_bytes(N);
       } else {
         need = 0;
       }
     }
   }
-  SpmmArgs walk = a;
-  walk.run_if = stats.flag;
   if (!vec) {
     path = 0;  // the staged rows copy whole slices: natural layouts only
     vec = align_operands(&a, plan, workspace, workspace_bytes, need, s);
@@ -433,7 +433,10 @@ static int run_spmm(SpmmArgs a, const bsp_plan* plan, bool vec, const TuneSched&
         d.n_list = plan->direct_rows;
         BSP_TRY(launch_spmm_rows(d, vec, s));
       }
-      return plain ? BSP_OK : launch_spmm_rows(walk, vec, s);
+      if (plain) return BSP_OK;
+      BSP_TRY(launch_col_stats(B0, a.bdt, K, N, ldb0, stats_ws, kProtoOctaves, &walk.run_if, &walk.run_if_n, s));
+      walk.run_if_late = walk.run_if_n > 1;
+      return launch_spmm_rows(walk, vec, s);
     }
     BSP_TRY(launch_proto_sums(a, vec, s));
     return launch_spmm_rows_wide(a, s);

@@ -26,6 +26,15 @@ namespace cg = cooperative_groups;
 namespace bsp {
 namespace {
 
+// A product that stands by for another one and is not asked for (whole block).
+__device__ __forceinline__ bool stands_by(const SpmmArgs& a) {
+  if (!a.run_if) return false;
+  if (a.run_if_late) ptx::griddep_wait();
+  int any = 0;
+  for (int i = threadIdx.x; i < max(a.run_if_n, 1); i += blockDim.x) any |= __ldcg(a.run_if + i);
+  return !__syncthreads_or(any);
+}
+
 // Walking kernel: one warp per (row, column chunk of 32*VPL*COLS).  The warp
 // first writes the columns of its row's set bits to a list in shared memory,
 // 128 words at a time (a prefix sum of the lanes' bit counts gives every lane
@@ -60,7 +69,7 @@ __global__ void __launch_bounds__(256, MINB) k_spmm_list(SpmmArgs a) {
   __shared__ __align__(16) uint32_t lists[8][kListCap];
   const int lane = threadIdx.x & 31;
   uint32_t* list = lists[threadIdx.x >> 5];
-  if (a.run_if && !__ldg(a.run_if)) return;
+  if (stands_by(a)) return;
   int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (a.row_list) {
     if (row >= a.n_list) return;
@@ -208,7 +217,7 @@ __global__ void __launch_bounds__(256) k_spmm_coop(SpmmArgs a) {
   extern __shared__ __align__(16) uint8_t coop_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(coop_raw);
   ptx::griddep_launch_dependents();
-  if (a.run_if && !__ldg(a.run_if)) return;  // (never with a row list)
+  if (stands_by(a)) return;  // (never with a row list)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t row = a.row_list ? (int64_t)__ldg(a.row_list + blockIdx.x) : (int64_t)blockIdx.x;
   const BT* __restrict__ B = static_cast<const BT*>(a.B);
@@ -526,9 +535,22 @@ bool list_fast(const SpmmArgs& a) {
 template <typename V, int VPL, int D, bool FAST = false, int MINB = 0>
 int launch_list_s(const SpmmArgs& a, int64_t rows, cudaStream_t s) {
   const int64_t gy = ceil_div(a.N, 32 * VPL * V::COLS);
-  k_spmm_list<V, VPL, D, FAST, MINB>
-      <<<dim3((unsigned)ceil_div(rows, 8), (unsigned)(gy < 65535 ? gy : 65535)), 256, 0, s>>>(a);
-  BSP_LAUNCHED();
+  const dim3 g((unsigned)ceil_div(rows, 8), (unsigned)(gy < 65535 ? gy : 65535));
+  if (!a.run_if_late) {
+    k_spmm_list<V, VPL, D, FAST, MINB><<<g, 256, 0, s>>>(a);
+    BSP_LAUNCHED();
+    return BSP_OK;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = g;
+  cfg.blockDim = dim3(256);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  BSP_CUDA(cudaLaunchKernelEx(&cfg, k_spmm_list<V, VPL, D, FAST, MINB>, a));
   return BSP_OK;
 }
 
@@ -555,7 +577,7 @@ int launch_coop_s(const SpmmArgs& a, int64_t rows, cudaStream_t s) {
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = a.row_list ? 1 : 0;
+  cfg.numAttrs = a.row_list || a.run_if_late ? 1 : 0;
   BSP_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
   return BSP_OK;
 }

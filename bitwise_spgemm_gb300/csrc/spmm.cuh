@@ -52,7 +52,9 @@ struct SpmmArgs {
   int64_t ldc;
   bool c_vec;         // C's rows take 16-byte stores (else element by element)
   bool no_long_rows;  // a plan says that no row has more than kCompThreshold set bits
-  const int* run_if;  // device flag: zero = do nothing (walking kernels only); null = run
+  const int* run_if;  // device flags: all zero = do nothing (walking kernels only); null = run
+  int run_if_n;       // how many (0 = one)
+  bool run_if_late;   // the kernel before sets them: launched as its programmatic dependent
   // prototype mode (plan)
   const int32_t* row_cluster;  // [M], -1 = walk A's row
   const int32_t* delta_ptr;    // [M+1]
@@ -74,30 +76,26 @@ struct SpmmArgs {
 
 // Sizes of the values of B [R][N] by column (col_stats.cu).
 constexpr int kStatTop = 127 + 100;
-constexpr int64_t kStatMaxRows = (int64_t)1 << 22;  // (sums of exponents in 32 bits)
-struct ColStats {
-  int* flag;           // nonzero: the values do not pass
-  int* max_exp;        // [N] largest biased exponent (of FP32)
-  unsigned* done;      // [ceil(N/32)] blocks that have reported
-  unsigned* nonzeros;  // [N]
-  unsigned* exp_sum;   // [N] of the nonzero values
-  // of a product in parts (spmm_tc.cu)
-  int* low;            // [N + 8] exponent below which a value's first part loses bits in the sums
-  unsigned* limit;     // [N] how many such values may be
-  unsigned* count;     // [N] how many there are
-};
-// *flag becomes nonzero if a value is not finite or at least 2^100, or if a
-// column's largest exponent is more than `octaves` above the mean one of its
-// nonzeros.  In col_stats_bytes(N) of workspace.
+constexpr int64_t kStatMaxRows = 65536;  // (a block reads all of them)
+constexpr int kStatCols = 8;             // columns of a block
+// n_flags device flags, at most 512, one of them nonzero if a value is not finite
+// or at least 2^100, or if a column's largest exponent is more than `octaves`
+// above the mean one of its nonzeros; runs beside the kernels before it.  In
+// col_stats_bytes(N) of workspace.
 size_t col_stats_bytes(int64_t N);
-int launch_col_stats(const void* B, int bdt, int64_t R, int64_t N, int64_t ldb, void* ws, int octaves, ColStats* st,
-                     cudaStream_t s);
-// low and limit for sums of about `addends` values of a column (see k_split_b);
-// *flag as above, but for the octaves.
+int launch_col_stats(const void* B, int bdt, int64_t R, int64_t N, int64_t ldb, void* ws, int octaves,
+                     const int** flags, int* n_flags, cudaStream_t s);
+// The values of a product in parts (spmm_tc.cu), R up to 4096: bad[b] = 1 if
+// columns 8b to 8b+7 do not pass (see k_split_b, which sets flag then).
+constexpr int kStatBottom = 127 - 100;
 constexpr int kPartsLow = 16;
 constexpr float kPartsLimit = 0.7f;
+struct PartsStats {
+  int* flag;
+  int* bad;
+};
 size_t parts_stats_bytes(int64_t N);
-int launch_parts_stats(const float* B, int64_t R, int64_t N, int64_t ldb, void* ws, float addends, ColStats* st,
+int launch_parts_stats(const float* B, int64_t R, int64_t N, int64_t ldb, void* ws, float addends, PartsStats* st,
                        cudaStream_t s);
 // B [K][N] (row stride ldb, any alignment) -> out [K][Nb], columns N..Nb-1 zero
 int launch_align_b(const void* B, int bdt, int64_t K, int64_t N, int64_t ldb, void* out, int64_t Nb, cudaStream_t s);

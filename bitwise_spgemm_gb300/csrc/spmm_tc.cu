@@ -555,20 +555,20 @@ __global__ void __launch_bounds__(256) k_tile_b(const uint8_t* __restrict__ B, i
 // Intelligence Datatype For Higher-Precision Computations, ARITH 2019): each part
 // takes the next 8 bits of the significand, rounded, and what is left of
 // 24 bits after two of them fits the third, as long as no part leaves BF16's
-// normal range: the flag is set by any x that is not 0 or in [2^-100, 2^100),
-// infinities and NaN among them.
+// normal range: a column with an x that is not 0 or in [2^-100, 2^100), an infinity
+// or a NaN does not pass (k_parts_stats).
 //
 // The tensor cores' sums are cut off towards zero at 24 bits, after every 16
 // products.  That costs nothing while the first parts' 8 bits add up exactly,
-// that is for values of at least 2^(E - 16), 2^E being where the sums are
-// (ColStats::low); each smaller one costs up to a unit of the last place, always
-// towards zero, where the walk rounds every addend to nearest.  The walk's
-// error grows with the square root of the addends, so the product keeps below it
-// while a column has at most 0.7 of that root of such values in a sum
-// (ColStats::limit); one column with more of them leaves the product to the
-// walk.  (Values in [1,2), a fraction of them times 2^-9 to 2^-18, all positive,
-// six sizes from 512x512 to 2048x4096 at 10 to 95 %: just inside the limit the
-// errors against FP64 are 0.12 to 1.0 of the walk's, normal values 0.05 to 0.2.)
+// that is for values of at least 2^(E - 16), 2^E being where the sums are; each
+// smaller one costs up to a unit of the last place, always towards zero, where
+// the walk rounds every addend to nearest.  The walk's error grows with the square
+// root of the addends, so the product keeps below it while a column has at most
+// 0.7 of that root of such values in a sum; one column with more of them leaves
+// the product to the walk.  (Values in [1,2), a fraction of them times 2^-9 to
+// 2^-18, all positive, six sizes from 512x512 to 2048x4096 at 10 to 95 %: just
+// inside the limit the errors against FP64 are 0.12 to 1.0 of the walk's, normal
+// values 0.05 to 0.2.)
 //
 // Rows past R are zero; columns past 3 Np stay as they are (each column of a
 // product depends on its own alone).  Bound by memory: 4 bytes in, 6 out per
@@ -576,16 +576,16 @@ __global__ void __launch_bounds__(256) k_tile_b(const uint8_t* __restrict__ B, i
 template <bool VEC>
 __global__ void __launch_bounds__(256) k_split_b(const float* __restrict__ B, int64_t R, int64_t N, int64_t ldb,
                                                  int64_t ntiles, int64_t ncb, uint4* __restrict__ bt,
-                                                 ColStats st) {
+                                                 PartsStats st) {
   const uint32_t q = (uint32_t)((N + 7) / 8);
   const int64_t rows = ntiles * kTcK;
-  bool bad = false;
-  for (uint32_t c8 = blockIdx.x * blockDim.x + threadIdx.x; c8 < q && !bad; c8 += gridDim.x * blockDim.x) {
+  for (uint32_t c8 = blockIdx.x * blockDim.x + threadIdx.x; c8 < q; c8 += gridDim.x * blockDim.x) {
     const int64_t col = (int64_t)c8 * 8;
-    const int4 l0 = __ldg(reinterpret_cast<const int4*>(st.low + col));
-    const int4 l1 = __ldg(reinterpret_cast<const int4*>(st.low + col) + 1);
-    const int low[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
-    for (int64_t row = blockIdx.y; row < rows && !bad; row += gridDim.y) {
+    if (__ldg(st.bad + c8)) {
+      *st.flag = 1;
+      return;
+    }
+    for (int64_t row = blockIdx.y; row < rows; row += gridDim.y) {
       float x[8];
 #pragma unroll
       for (int i = 0; i < 8; i++) x[i] = 0.f;
@@ -599,15 +599,6 @@ __global__ void __launch_bounds__(256) k_split_b(const float* __restrict__ B, in
 #pragma unroll
           for (int i = 0; i < 8; i++)
             if (col + i < N) x[i] = __ldg(p + i);
-        }
-      }
-      if (row < R) {
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-          if (col + i >= N || x[i] == 0.f) continue;
-          const int e = (int)((__float_as_uint(x[i]) >> 23) & 255u);
-          bad |= e < 27;
-          if (e < low[i] && atomicAdd(st.count + col + i, 1u) >= __ldg(st.limit + col + i)) bad = true;
         }
       }
 #pragma unroll
@@ -626,7 +617,6 @@ __global__ void __launch_bounds__(256) k_split_b(const float* __restrict__ B, in
       }
     }
   }
-  if (bad) atomicExch(st.flag, 1);
 }
 
 // 16-bit B [R][N] (16-byte rows, N a multiple of 8) as two parts in tile order,
@@ -1100,7 +1090,7 @@ static int launch_parts(TsArgs a, int64_t nnz, const float* B, int64_t ldb, int6
   double slice = (double)red_rows / splits;
   if (a.seg_stages && slice > a.seg_stages * 4.0 * kTcK) slice = a.seg_stages * 4.0 * kTcK;
   const double addends = 1.25 * bits * slice / (double)red_rows;
-  ColStats stats = {};
+  PartsStats stats = {};
   BSP_TRY(launch_parts_stats(B, red_rows, N, ldb, stats_ws, (float)(addends > 1.0 ? addends : 1.0), &stats, s));
   int* flag = stats.flag;
   const int64_t q = Np / 8;
