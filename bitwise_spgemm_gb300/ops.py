@@ -26,6 +26,20 @@ def _p(t):
     return t.data_ptr() if t is not None else None
 
 
+def _scratch(device, *sizes):
+    """A workspace of the first of ``sizes`` bytes, largest first, that there is
+    memory for (None for 0): on a nearly full GPU a product takes its smaller
+    form instead of failing."""
+    for i, n in enumerate(sizes):
+        if n == 0:
+            return None
+        try:
+            return torch.empty(n, dtype=torch.uint8, device=device)
+        except torch.OutOfMemoryError:
+            if i + 1 == len(sizes):
+                raise
+
+
 def _rowmajor(t, name):
     if t.dim() != 2 or t.stride(1) != 1:
         raise ValueError("%s must be a 2-D tensor with unit column stride" % name)
@@ -190,8 +204,10 @@ def spmm(words, K, B, plan=None, out=None, workspace=None):
     if not fits:
         n = C.c_size_t()
         call("bsp_spmm_workspace_layout", h, K, N, _p(B), _DT[B.dtype], ldb, C.byref(n))
-        workspace = torch.empty(n.value, dtype=torch.uint8, device=B.device) if n.value else None
-        have = n.value
+        workspace = None
+        if n.value:
+            workspace = _scratch(B.device, n.value, plan.workspace_bytes(N, preferred=False) if plan is not None else 0)
+        have = workspace.numel() if workspace is not None else 0
     if workspace is not None:
         ws_ptr, ws_n = _p(workspace), have
     call("bsp_spmm", _p(words), M, K, _p(B), _DT[B.dtype], ldb, N, _p(out), ldc, h, ws_ptr, ws_n,
@@ -216,7 +232,9 @@ def spmm_t(words, M, K, G, plan=None, out=None, workspace=None, dtype=torch.floa
     if workspace is None or workspace.numel() * workspace.element_size() < n.value:
         call("bsp_spmm_t_workspace_layout", plan.handle if plan is not None else None, M, K, N, _DT[G.dtype],
              C.byref(n))
-        workspace = torch.empty(n.value, dtype=torch.uint8, device=G.device)
+        most = n.value
+        call("bsp_spmm_t_workspace", M, K, C.byref(n))
+        workspace = _scratch(G.device, most, n.value)
     call("bsp_spmm_t", _p(words), M, K, _p(G), _DT[G.dtype], ldg, N, _p(out), out.stride(0),
          plan.handle if plan is not None else None, _p(workspace),
          workspace.numel() * workspace.element_size(), _stream())
@@ -232,11 +250,12 @@ def _spmm_t_as(words, M, K, G, plan, workspace, dtype):
                                           C.byref(n)) != capi.BSP_OK:
         return None
     if workspace is None or workspace.numel() * workspace.element_size() < n.value:
-        workspace = torch.empty(n.value, dtype=torch.uint8, device=G.device)
+        workspace = _scratch(G.device, n.value, 0)
     out = torch.empty((K, N), dtype=dtype, device=G.device)
     st = capi.lib().bsp_spmm_t_as(_p(words), M, K, _p(G), _DT[G.dtype], G.stride(0), N, _p(out), _DT[dtype],
                                   out.stride(0), plan.handle, _p(workspace),
-                                  workspace.numel() * workspace.element_size(), _stream())
+                                  workspace.numel() * workspace.element_size() if workspace is not None else 0,
+                                  _stream())
     if st == capi.BSP_ERR_UNSUPPORTED:
         return None
     if st != capi.BSP_OK:
@@ -274,7 +293,7 @@ def tune(words, K, B, plan, out=None, workspace=None):
     if workspace is None or workspace.numel() * workspace.element_size() < need:
         n = C.c_size_t()
         call("bsp_spmm_workspace_layout", plan.handle, K, N, _p(B), _DT[B.dtype], ldb, C.byref(n))
-        workspace = torch.empty(max(n.value, 1), dtype=torch.uint8, device=B.device)
+        workspace = _scratch(B.device, max(n.value, need, 1), max(need, 1))
     best = capi.Schedule()
     call("bsp_tune", _p(words), M, K, _p(B), _DT[B.dtype], ldb, N, _p(out), out.stride(0), plan.handle,
          _p(workspace), workspace.numel() * workspace.element_size(), _stream(), C.byref(best))
@@ -410,15 +429,21 @@ class Int8Matrix:
                 out = torch.empty((self.M, N), dtype=torch.float32, device=B.device)
             n = C.c_size_t()
             call("bsp_spmm_i8_tiles_workspace", self.M, self.K, N, C.byref(n))
-            ws = torch.empty(max(n.value, 1), dtype=torch.uint8, device=B.device)
-            call("bsp_spmm_i8_tiles", _p(self.tiles), self.M, self.K, _p(B), _DT[B.dtype], B.stride(0), N, _p(out),
-                 out.stride(0), _p(ws), n.value, _stream())
-            return out
+            try:
+                ws = _scratch(B.device, n.value)
+            except torch.OutOfMemoryError:
+                ws = None
+            if ws is not None:
+                call("bsp_spmm_i8_tiles", _p(self.tiles), self.M, self.K, _p(B), _DT[B.dtype], B.stride(0), N, _p(out),
+                     out.stride(0), _p(ws), n.value, _stream())
+                return out
+            # no room for B in two parts: the planes, whose sums are as exact
         Bs = stack_planes_b(B, self.K, 8, True, out=B_stacked)
         return spmm(self.words, self.Kc, Bs, plan=self.plan, out=out)
 
     def close(self):
         self.plan.close()
+        self.tiles = None
 
 
 def _ws(fn, *args, device):

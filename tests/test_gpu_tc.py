@@ -538,3 +538,37 @@ def test_spmm_t_in_16_bits_asks_before_it_allocates(force_tc, monkeypatch):
     monkeypatch.setattr(torch, "empty", refuse)
     for wd, M, K, G, plan in cases:
         assert ops._spmm_t_as(wd, M, K, G, plan, None, G.dtype) is None
+
+
+def test_products_on_a_nearly_full_gpu(monkeypatch):
+    """Where the preferred workspace cannot be had, the products run in the
+    minimum: as they did before they knew of parts, copies and splits."""
+    g = torch.Generator(device="cuda").manual_seed(4)
+    M, K, N = 1024, 2048, 512
+    A = torch.rand((M, K), device="cuda", generator=g) < 0.2
+    wd = ops.pack_rows(A.to(torch.uint8))
+    plan = ops.Plan(wd, K, mode=capi.PLAN_DIRECT)
+    real = torch.empty
+
+    def empty(*size, **kw):
+        if kw.get("dtype") == torch.uint8 and size[0] > 1 << 20:
+            raise torch.OutOfMemoryError("full")
+        return real(*size, **kw)
+
+    for dt, width in ((torch.float32, N), (torch.bfloat16, N), (torch.bfloat16, N + 1)):
+        B = torch.randint(-8, 9, (K, width), device="cuda", generator=g).to(dt)
+        G = torch.randint(-8, 9, (M, width), device="cuda", generator=g).to(dt)
+        with monkeypatch.context() as m:
+            m.setattr(torch, "empty", empty)
+            C, dX = ops.spmm(wd, K, B, plan=plan), ops.spmm_t(wd, M, K, G, plan=plan)
+            dX16 = ops.spmm_t(wd, M, K, G, plan=plan, dtype=dt)
+        assert torch.equal(C, A.float() @ B.float()) and torch.equal(dX, A.float().T @ G.float())
+        assert torch.equal(dX16, dX.to(dt))
+    W8 = torch.randint(-8, 9, (M, K), device="cuda", generator=g).to(torch.int8)
+    mat = ops.Int8Matrix(W8)
+    B = torch.randint(-8, 9, (K, N), device="cuda", generator=g).bfloat16()
+    with monkeypatch.context() as m:
+        m.setattr(torch, "empty", empty)
+        C = mat.matmul(B)
+    assert torch.equal(C, W8.float() @ B.float())
+    assert capi.device_status() == 0
