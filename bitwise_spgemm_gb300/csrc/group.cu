@@ -48,8 +48,13 @@ __global__ void __launch_bounds__(256) k_group_rows(const uint32_t* __restrict__
       const uint32_t my = next;
       next = c0 + 32 + lane < nr ? __ldg(col + (int64_t)(c0 + 32 + lane) * Kw) : 0u;
       int myg = 0;
-      bool fits = false;
-      for (int g = 0; g < G; g++) fits |= (__shfl_sync(kFull, gm, g) & my) == 0u;
+      // settling takes G steps, the chain one per row: only for more rows than groups
+      // (4096x128 words, 32 groups, 1 % set: 198 us with it always, 177 so)
+      bool fits = true;
+      if (__popc(__ballot_sync(kFull, my != 0u)) > G) {
+        fits = my == 0u;
+        for (int g = 0; g < G; g++) fits |= (__shfl_sync(kFull, gm, g) & my) == 0u;
+      }
       uint32_t spilled = __ballot_sync(kFull, !fits);  // (a zero word fits)
       uint32_t pending = __ballot_sync(kFull, fits && my != 0u);
       while (pending) {
