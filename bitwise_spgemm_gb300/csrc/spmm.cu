@@ -30,8 +30,9 @@ namespace {
 __device__ __forceinline__ bool stands_by(const SpmmArgs& a) {
   if (!a.run_if) return false;
   if (a.run_if_late) ptx::griddep_wait();
+  if (a.run_if_n <= 1) return !__ldcg(a.run_if);
   int any = 0;
-  for (int i = threadIdx.x; i < max(a.run_if_n, 1); i += blockDim.x) any |= __ldcg(a.run_if + i);
+  for (int i = threadIdx.x; i < a.run_if_n; i += blockDim.x) any |= __ldcg(a.run_if + i);
   return !__syncthreads_or(any);
 }
 
