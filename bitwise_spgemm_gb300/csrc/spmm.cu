@@ -59,7 +59,12 @@ constexpr int kListCap = kListStep + 32 * 32;  // one more group of 32 words
 // and B's element offsets fit in 32 bits; without the TwoSum walk and the 64-bit
 // row addresses, and with 4 gathers in flight, four blocks (MINB) run on an SM
 // instead of two.
-template <typename V, int VPL, int D, bool FAST, int MINB>
+//
+// LOOP: a walk that stands by; blocks for a few rounds go through all rows, so that
+// the usual case, in which it is not asked for, does not start one for every
+// eight rows (4096x4096x2048 BF16, single elements: 8192 blocks that end at once
+// 22 us, now 4).
+template <typename V, int VPL, int D, bool FAST, int MINB, bool LOOP>
 __global__ void __launch_bounds__(256, MINB) k_spmm_list(SpmmArgs a) {
   using BT = typename V::T;
   using Off = typename std::conditional<FAST, uint32_t, int64_t>::type;
@@ -71,124 +76,124 @@ __global__ void __launch_bounds__(256, MINB) k_spmm_list(SpmmArgs a) {
   const int lane = threadIdx.x & 31;
   uint32_t* list = lists[threadIdx.x >> 5];
   if (stands_by(a)) return;
-  int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (a.row_list) {
-    if (row >= a.n_list) return;
-    row = __ldg(a.row_list + row);
-  } else if (row >= a.M) {
-    return;
-  }
-  const BT* __restrict__ B = static_cast<const BT*>(a.B);
-  const uint32_t* arow = a.A + row * a.Kw;
-  const int Kw = (int)a.Kw;
-  const bool comp = !FAST && a.K > kCompThreshold && row_popcount(arow, Kw, lane) > kCompThreshold;
-  const Off ldb = (Off)a.ldb;
-  for (int64_t n0 = (int64_t)blockIdx.y * CW; n0 < a.N; n0 += (int64_t)gridDim.y * CW) {
-    int col[VPL];
-    bool cvalid[VPL];
+  const int64_t rows = a.row_list ? a.n_list : a.M;
+  int64_t at = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (at >= rows) return;
+  do {
+    const int64_t row = a.row_list ? (int64_t)__ldg(a.row_list + at) : at;
+    const BT* __restrict__ B = static_cast<const BT*>(a.B);
+    const uint32_t* arow = a.A + row * a.Kw;
+    const int Kw = (int)a.Kw;
+    const bool comp = !FAST && a.K > kCompThreshold && row_popcount(arow, Kw, lane) > kCompThreshold;
+    const Off ldb = (Off)a.ldb;
+    for (int64_t n0 = (int64_t)blockIdx.y * CW; n0 < a.N; n0 += (int64_t)gridDim.y * CW) {
+      int col[VPL];
+      bool cvalid[VPL];
 #pragma unroll
-    for (int v = 0; v < VPL; v++) {
-      const int64_t c = n0 + (v * 32 + lane) * COLS;
-      cvalid[v] = c < a.Nb;
-      col[v] = cvalid[v] ? (int)c : 0;
-    }
-    float* crow = a.C + row * a.ldc;
-    if (!FAST && comp) {
       for (int v = 0; v < VPL; v++) {
-        BitWalker wk;
-        wk.init(arow, 0, Kw, lane);
-        Acc<1, COLS, true> acc;
-        acc.zero();
-        int c1[1] = {col[v]};
-        bool ok[1] = {cvalid[v]};
-        accumulate_walk<V, 1, 4, true>(wk, B, a.ldb, c1, ok, acc);
-        store_vecs<1, COLS, true>(crow, c1, ok, acc, nullptr, a.c_vec, a.N);
+        const int64_t c = n0 + (v * 32 + lane) * COLS;
+        cvalid[v] = c < a.Nb;
+        col[v] = cvalid[v] ? (int)c : 0;
       }
-      continue;
-    }
-    Acc<VPL, COLS, false> acc;
-    acc.zero();
-    auto gather = [&](int i, int n) {  // list entries [i, i + n), n <= D (uniform)
-      uint32_t idx[D];
-#pragma unroll
-      for (int s = 0; s < D; s += 4) {
-        const uint4 q = *reinterpret_cast<const uint4*>(list + i + s);
-        idx[s] = q.x;
-        idx[s + 1] = q.y;
-        idx[s + 2] = q.z;
-        idx[s + 3] = q.w;
-      }
-      typename V::Raw raw[D][VPL];
-#pragma unroll
-      for (int s = 0; s < D; s++) {
-        const BT* brow = B + (Off)idx[s] * ldb;
-#pragma unroll
-        for (int v = 0; v < VPL; v++)
-          if (s < n && cvalid[v]) raw[s][v] = V::load(brow + col[v]);
-      }
-#pragma unroll
-      for (int s = 0; s < D; s++) {
-        if (s >= n) break;
-#pragma unroll
+      float* crow = a.C + row * a.ldc;
+      if (!FAST && comp) {
         for (int v = 0; v < VPL; v++) {
-          if (!cvalid[v]) continue;
-          float f[COLS];
-          V::cvt(raw[s][v], f);
-#pragma unroll
-          for (int j = 0; j < COLS; j++) acc.add(v, j, f[j]);
+          BitWalker wk;
+          wk.init(arow, 0, Kw, lane);
+          Acc<1, COLS, true> acc;
+          acc.zero();
+          int c1[1] = {col[v]};
+          bool ok[1] = {cvalid[v]};
+          accumulate_walk<V, 1, 4, true>(wk, B, a.ldb, c1, ok, acc);
+          store_vecs<1, COLS, true>(crow, c1, ok, acc, nullptr, a.c_vec, a.N);
         }
+        continue;
       }
-    };
-    uint32_t wx[GROUPS];
+      Acc<VPL, COLS, false> acc;
+      acc.zero();
+      auto gather = [&](int i, int n) {  // list entries [i, i + n), n <= D (uniform)
+        uint32_t idx[D];
 #pragma unroll
-    for (int g = 0; g < GROUPS; g++) wx[g] = g * 32 + lane < Kw ? __ldg(arow + g * 32 + lane) : 0u;
-    int n = 0;  // entries in the list
-    for (int w0 = 0; w0 < Kw; w0 += GROUPS * 32) {
-      uint32_t wn[GROUPS];
-#pragma unroll
-      for (int g = 0; g < GROUPS; g++) {
-        const int w = w0 + (GROUPS + g) * 32 + lane;
-        wn[g] = w < Kw ? __ldg(arow + w) : 0u;
-      }
-#pragma unroll
-      for (int g = 0; g < GROUPS; g++) {
-        if (w0 + g * 32 >= Kw) break;
-        uint32_t x = wx[g];
-        const int c = __popc(x);
-        int incl = c;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int y = __shfl_up_sync(kFull, incl, o);
-          if (lane >= o) incl += y;
+        for (int s = 0; s < D; s += 4) {
+          const uint4 q = *reinterpret_cast<const uint4*>(list + i + s);
+          idx[s] = q.x;
+          idx[s + 1] = q.y;
+          idx[s + 2] = q.z;
+          idx[s + 3] = q.w;
         }
-        int pos = n + incl - c;
-        const uint32_t k0 = (uint32_t)(w0 + g * 32 + lane) * 32u;
-        while (x) {
-          list[pos++] = k0 + (uint32_t)(__ffs(x) - 1);
-          x &= x - 1;
+        typename V::Raw raw[D][VPL];
+#pragma unroll
+        for (int s = 0; s < D; s++) {
+          const BT* brow = B + (Off)idx[s] * ldb;
+#pragma unroll
+          for (int v = 0; v < VPL; v++)
+            if (s < n && cvalid[v]) raw[s][v] = V::load(brow + col[v]);
         }
-        n += __shfl_sync(kFull, incl, 31);
-        const bool last = w0 + (g + 1) * 32 >= Kw;
-        if (n < kListStep && !last) continue;
-        __syncwarp();
-        int i = 0;
-        for (; i + D <= n; i += D) gather(i, D);
-        n -= i;
-        if (last) {
-          if (n > 0) gather(i, n);
-        } else if (i > 0) {  // the rest (less than D entries) starts the next round
-          const uint32_t rest = lane < n ? list[i + lane] : 0u;
+#pragma unroll
+        for (int s = 0; s < D; s++) {
+          if (s >= n) break;
+#pragma unroll
+          for (int v = 0; v < VPL; v++) {
+            if (!cvalid[v]) continue;
+            float f[COLS];
+            V::cvt(raw[s][v], f);
+#pragma unroll
+            for (int j = 0; j < COLS; j++) acc.add(v, j, f[j]);
+          }
+        }
+      };
+      uint32_t wx[GROUPS];
+#pragma unroll
+      for (int g = 0; g < GROUPS; g++) wx[g] = g * 32 + lane < Kw ? __ldg(arow + g * 32 + lane) : 0u;
+      int n = 0;  // entries in the list
+      for (int w0 = 0; w0 < Kw; w0 += GROUPS * 32) {
+        uint32_t wn[GROUPS];
+#pragma unroll
+        for (int g = 0; g < GROUPS; g++) {
+          const int w = w0 + (GROUPS + g) * 32 + lane;
+          wn[g] = w < Kw ? __ldg(arow + w) : 0u;
+        }
+#pragma unroll
+        for (int g = 0; g < GROUPS; g++) {
+          if (w0 + g * 32 >= Kw) break;
+          uint32_t x = wx[g];
+          const int c = __popc(x);
+          int incl = c;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += y;
+          }
+          int pos = n + incl - c;
+          const uint32_t k0 = (uint32_t)(w0 + g * 32 + lane) * 32u;
+          while (x) {
+            list[pos++] = k0 + (uint32_t)(__ffs(x) - 1);
+            x &= x - 1;
+          }
+          n += __shfl_sync(kFull, incl, 31);
+          const bool last = w0 + (g + 1) * 32 >= Kw;
+          if (n < kListStep && !last) continue;
           __syncwarp();
-          if (lane < n) list[lane] = rest;
+          int i = 0;
+          for (; i + D <= n; i += D) gather(i, D);
+          n -= i;
+          if (last) {
+            if (n > 0) gather(i, n);
+          } else if (i > 0) {  // the rest (less than D entries) starts the next round
+            const uint32_t rest = lane < n ? list[i + lane] : 0u;
+            __syncwarp();
+            if (lane < n) list[lane] = rest;
+          }
+          __syncwarp();
         }
-        __syncwarp();
-      }
 #pragma unroll
-      for (int g = 0; g < GROUPS; g++) wx[g] = wn[g];
+        for (int g = 0; g < GROUPS; g++) wx[g] = wn[g];
+      }
+      store_vecs<VPL, COLS, false>(crow, col, cvalid, acc, nullptr, a.c_vec, a.N);
+      __syncwarp();
     }
-    store_vecs<VPL, COLS, false>(crow, col, cvalid, acc, nullptr, a.c_vec, a.N);
-    __syncwarp();
-  }
+    at += (int64_t)gridDim.x * (blockDim.x >> 5);
+  } while (LOOP && at < rows);
 }
 
 // A few long rows: a CTA per (row, column chunk).  Its 8 warps write the row's
@@ -536,22 +541,29 @@ bool list_fast(const SpmmArgs& a) {
 template <typename V, int VPL, int D, bool FAST = false, int MINB = 0>
 int launch_list_s(const SpmmArgs& a, int64_t rows, cudaStream_t s) {
   const int64_t gy = ceil_div(a.N, 32 * VPL * V::COLS);
-  const dim3 g((unsigned)ceil_div(rows, 8), (unsigned)(gy < 65535 ? gy : 65535));
-  if (!a.run_if_late) {
-    k_spmm_list<V, VPL, D, FAST, MINB><<<g, 256, 0, s>>>(a);
-    BSP_LAUNCHED();
-    return BSP_OK;
-  }
+  k_spmm_list<V, VPL, D, FAST, MINB, false>
+      <<<dim3((unsigned)ceil_div(rows, 8), (unsigned)(gy < 65535 ? gy : 65535)), 256, 0, s>>>(a);
+  BSP_LAUNCHED();
+  return BSP_OK;
+}
+
+// ... of a walk that stands by: 4 blocks an SM at most.
+template <typename V, int VPL, int D, bool FAST, int MINB>
+int launch_standby_s(const SpmmArgs& a, int64_t rows, cudaStream_t s) {
+  const int64_t most = (int64_t)num_sms() * 4;
+  int64_t gy = ceil_div(a.N, 32 * VPL * V::COLS), gx = ceil_div(rows, 8);
+  if (gy > most) gy = most;
+  if (gx * gy > most) gx = most / gy > 0 ? most / gy : 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = g;
+  cfg.gridDim = dim3((unsigned)gx, (unsigned)gy);
   cfg.blockDim = dim3(256);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  BSP_CUDA(cudaLaunchKernelEx(&cfg, k_spmm_list<V, VPL, D, FAST, MINB>, a));
+  cfg.numAttrs = a.run_if_late ? 1 : 0;
+  BSP_CUDA(cudaLaunchKernelEx(&cfg, k_spmm_list<V, VPL, D, FAST, MINB, true>, a));
   return BSP_OK;
 }
 
@@ -593,6 +605,12 @@ int launch_rows_t(const SpmmArgs& a, cudaStream_t s) {
   // that runs (one row, 8192 columns at 5 %, N = 512: 9.1 us against 15.2;
   // from a few hundred tasks on the two are equal, 117 rows 21.5 and 20.0).
   if (tasks <= sms && a.K >= 1024 && chunks <= 65535) return launch_coop_s<V, VPL>(a, rows, s);
+  if (a.run_if) {
+    if constexpr (V::COLS != 1) {  // (as below)
+      if (tasks >= 32 * sms && list_fast(a)) return launch_standby_s<V, VPL, 4, true, 4>(a, rows, s);
+    }
+    return launch_standby_s<V, VPL, 8, false, 0>(a, rows, s);
+  }
   if constexpr (V::COLS == 1) {
     // No more columns a lane than there are: 100000x32x8 FP32 170 us with four a
     // lane, 29 with one; 4096x4096x12 BF16 at 5 % 107 and 23.

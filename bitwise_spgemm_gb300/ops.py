@@ -26,18 +26,18 @@ def _p(t):
     return t.data_ptr() if t is not None else None
 
 
-def _scratch(device, *sizes):
-    """A workspace of the first of ``sizes`` bytes, largest first, that there is
-    memory for (None for 0): on a nearly full GPU a product takes its smaller
-    form instead of failing."""
-    for i, n in enumerate(sizes):
-        if n == 0:
-            return None
+def _scratch(device, n, least):
+    """A workspace of ``n`` bytes (None for 0) or, where there is no memory for
+    it, of the ``least()`` that the product runs in: on a nearly full GPU it takes
+    its smaller form instead of failing."""
+    if n:
         try:
             return torch.empty(n, dtype=torch.uint8, device=device)
         except torch.OutOfMemoryError:
-            if i + 1 == len(sizes):
+            small = least()
+            if small >= n:
                 raise
+            return torch.empty(small, dtype=torch.uint8, device=device) if small else None
 
 
 def _rowmajor(t, name):
@@ -204,9 +204,8 @@ def spmm(words, K, B, plan=None, out=None, workspace=None):
     if not fits:
         n = C.c_size_t()
         call("bsp_spmm_workspace_layout", h, K, N, _p(B), _DT[B.dtype], ldb, C.byref(n))
-        workspace = None
-        if n.value:
-            workspace = _scratch(B.device, n.value, plan.workspace_bytes(N, preferred=False) if plan is not None else 0)
+        workspace = _scratch(B.device, n.value,
+                             lambda: plan.workspace_bytes(N, preferred=False) if plan is not None else 0)
         have = workspace.numel() if workspace is not None else 0
     if workspace is not None:
         ws_ptr, ws_n = _p(workspace), have
@@ -232,9 +231,7 @@ def spmm_t(words, M, K, G, plan=None, out=None, workspace=None, dtype=torch.floa
     if workspace is None or workspace.numel() * workspace.element_size() < n.value:
         call("bsp_spmm_t_workspace_layout", plan.handle if plan is not None else None, M, K, N, _DT[G.dtype],
              C.byref(n))
-        most = n.value
-        call("bsp_spmm_t_workspace", M, K, C.byref(n))
-        workspace = _scratch(G.device, most, n.value)
+        workspace = _scratch(G.device, n.value, lambda: _size("bsp_spmm_t_workspace", M, K))
     call("bsp_spmm_t", _p(words), M, K, _p(G), _DT[G.dtype], ldg, N, _p(out), out.stride(0),
          plan.handle if plan is not None else None, _p(workspace),
          workspace.numel() * workspace.element_size(), _stream())
@@ -250,7 +247,7 @@ def _spmm_t_as(words, M, K, G, plan, workspace, dtype):
                                           C.byref(n)) != capi.BSP_OK:
         return None
     if workspace is None or workspace.numel() * workspace.element_size() < n.value:
-        workspace = _scratch(G.device, n.value, 0)
+        workspace = _scratch(G.device, n.value, lambda: 0)
     out = torch.empty((K, N), dtype=dtype, device=G.device)
     st = capi.lib().bsp_spmm_t_as(_p(words), M, K, _p(G), _DT[G.dtype], G.stride(0), N, _p(out), _DT[dtype],
                                   out.stride(0), plan.handle, _p(workspace),
@@ -293,7 +290,7 @@ def tune(words, K, B, plan, out=None, workspace=None):
     if workspace is None or workspace.numel() * workspace.element_size() < need:
         n = C.c_size_t()
         call("bsp_spmm_workspace_layout", plan.handle, K, N, _p(B), _DT[B.dtype], ldb, C.byref(n))
-        workspace = _scratch(B.device, max(n.value, need, 1), max(need, 1))
+        workspace = _scratch(B.device, max(n.value, need, 1), lambda: max(need, 1))
     best = capi.Schedule()
     call("bsp_tune", _p(words), M, K, _p(B), _DT[B.dtype], ldb, N, _p(out), out.stride(0), plan.handle,
          _p(workspace), workspace.numel() * workspace.element_size(), _stream(), C.byref(best))
@@ -429,10 +426,7 @@ class Int8Matrix:
                 out = torch.empty((self.M, N), dtype=torch.float32, device=B.device)
             n = C.c_size_t()
             call("bsp_spmm_i8_tiles_workspace", self.M, self.K, N, C.byref(n))
-            try:
-                ws = _scratch(B.device, n.value)
-            except torch.OutOfMemoryError:
-                ws = None
+            ws = _scratch(B.device, n.value, lambda: 0)
             if ws is not None:
                 call("bsp_spmm_i8_tiles", _p(self.tiles), self.M, self.K, _p(B), _DT[B.dtype], B.stride(0), N, _p(out),
                      out.stride(0), _p(ws), n.value, _stream())
@@ -446,10 +440,14 @@ class Int8Matrix:
         self.tiles = None
 
 
-def _ws(fn, *args, device):
+def _size(fn, *args):
     need = C.c_size_t(0)
     call(fn, *args, C.byref(need))
-    return torch.empty(max(need.value, 1), dtype=torch.uint8, device=device)
+    return need.value
+
+
+def _ws(fn, *args, device):
+    return torch.empty(max(_size(fn, *args), 1), dtype=torch.uint8, device=device)
 
 
 def rows_to_tiles8(words, K):
