@@ -699,7 +699,7 @@ def run_batched(args, emit=True):
            "ms_per_step": ms, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
            "dtype": "bf16", "data": "synthetic (seeded numpy, seed 7+i per problem)",
            "config": {"workload": "batched_512_N128_bf16", "problems": len(probs), "N": N,
-                      "nnz": nnz, "graph": "one persistent launch (a CTA per SM taking 256-row items from a device work queue), graph-captured",
+                      "nnz": nnz, "graph": "one persistent launch (256-row items, taken over by cluster launch control), graph-captured",
                       "kernel_shape": {"index": shape, "tuned_ms": tune_ms,
                                        "by": "bsp_batch_tune (one form is built)"}},
            "aggregate_gbs": ws * comp / (ms * 1e-3) / 1e9,

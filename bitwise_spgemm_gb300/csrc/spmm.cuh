@@ -133,9 +133,9 @@ int launch_occupancy(const uint32_t* A, int64_t M, int64_t K, uint32_t* occ, uin
 // order (used when the rest holds tc_tiled_b_bytes(...)); else ignored.
 // At (optional): A's words column by column ([Kw][M], launch_transpose_words)
 // for coalesced word loads; null = loads from the rows.
-// form: the tile form a tuned schedule fixes (0 / -1 fields = the rule):
-// K tiles per stage (2 or 3), B pre-tiled (1) or by TMA boxes (0), split-K
-// allowed (-1) or not (0).
+// form: the tile form a tuned schedule fixes (-1 = the rule): B pre-tiled (1)
+// or by TMA boxes (0), split-K allowed (-1) or not (0).  tps, once the K tiles
+// of a stage, chooses nothing: one stage form is built.
 struct TcForm {
   int tps = 0, tiled = -1, split = -1;
 };

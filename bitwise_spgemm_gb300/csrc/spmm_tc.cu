@@ -2,8 +2,8 @@
 // (tcgen05, TMEM accumulators) and the host side of the tensor-core products.
 //
 // k_spmm_tc runs the SDDMM dA = (G·Xᵀ) ⊙ A, dense over N with a masked store,
-// and the CTA-per-item forms of the batched products (forward, Aᵀ·G and
-// SDDMM).  The single forward product and Aᵀ·G run on the persistent kernel of
+// and the CTA-per-item forms of the batched products (forward, which wide
+// batches take where it finishes first; Aᵀ·G and SDDMM on request).  The single forward product and Aᵀ·G run on the persistent kernel of
 // spmm_ts.cu, launched from here.
 //
 // CTA tile: 256 rows x 256 columns of C as two 128-row halves, each with its
@@ -1062,9 +1062,9 @@ static int launch_join(const float* part, int64_t Np, int64_t stride, int splits
 
 // C = A·B (trans: dX = Aᵀ·G) for FP32 B on the tensor cores, exact in B: its
 // three BF16 parts are multiplied as 3N columns, each with accumulators of its
-// own, and joined afterwards.  2048x2048x1024 at 10 %: walk 97 us, here 49
-// (Aᵀ·G 99 and 51); 4096x4096x2048 at 5 % 389 and 188.  Bound there by the
-// tensor kernel's producers, below about 1024x1024x1024 by its five launches.
+// own, and joined afterwards.  2048x2048x1024 at 10 %: walk 85 us, here 56, two
+// of them to look at the columns.  Bound there by the tensor kernel's producers,
+// below about 1024x1024x1024 by its launches.
 // Errors against FP64, relative in the Frobenius norm, walk and here:
 // normal values 2.6e-7 and 2.7e-8, their magnitudes 2.2e-7 and 3.5e-8
 // (512x512x256 9.7e-8 and 2.5e-8, 1024x4096x512 3.7e-7 and 2.8e-8): the first

@@ -22,11 +22,7 @@ constexpr uint32_t kLbo = 128, kSbo = 512;
 //     (1024 B, rows 128 B apart, 16-byte chunk q of row r stored at chunk
 //     q ^ (r & 7)); SBO = distance between 8-row groups along the reduction,
 //     LBO = distance between 64-element atoms along M / N.
-//   K-major, 64-byte swizzle: atoms of 8 rows x 32 reduction elements (512 B,
-//     chunk q of row r at q ^ ((r >> 1) & 3)); SBO = distance between 8-row
-//     groups, LBO unused; the second K=16 half starts 32 bytes in.
-constexpr uint32_t kLayoutSw128 = 2, kLayoutSw64 = 4;
-constexpr uint32_t kSw128Atom = 1024, kSw64Atom = 512;
+constexpr uint32_t kLayoutSw128 = 2;
 
 // Instruction descriptor for kind::f16: D f32 (bits 4-5), A and B of the
 // same 16-bit type (bits 7-9, 10-12: bf16 = 1, f16 = 0), A / B major (bits
@@ -71,15 +67,6 @@ __device__ __forceinline__ void expand32_two(uint32_t w, uint4 (&o)[4]) {
   expand_pairs(unshuffle32(w), v);
 #pragma unroll
   for (int c = 0; c < 4; c++) o[c] = make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
-}
-
-// 8 bits of a word → 8 16-bit values 0 / one, packed little-endian.
-__device__ __forceinline__ uint4 expand8(uint32_t byte, uint32_t one) {
-  uint32_t w[4];
-#pragma unroll
-  for (int j = 0; j < 4; j++)
-    w[j] = (((byte >> (2 * j)) & 1u) ? one : 0u) | ((((byte >> (2 * j + 1)) & 1u) ? one : 0u) << 16);
-  return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
 }  // namespace tc

@@ -2,7 +2,7 @@
 //
 // A schedule says which engine runs the SpMM (tensor cores or CUDA cores —
 // the tensor-core density threshold of the bucket), on the tensor cores
-// which tile form (K tiles per stage, B by TMA boxes or pre-tiled, split-K
+// which tile form (B by TMA boxes or pre-tiled, split-K
 // or not), and on the CUDA cores which prototype-row kernel (register
 // gathers or TMA-staged slices) and which of its shapes.  bsp_tune (capi.cu) times the
 // candidates on the caller's data and stores the fastest here under a bucket

@@ -14,7 +14,7 @@ struct TuneSched {
   int proto_variant = 4;  // kernel shape of that path
   double ms = 0.0;        // measured time of the schedule
   // tensor cores: the tile form (0 / -1 = the launcher's own rule)
-  int tc_tps = 0;         // K tiles per pipeline stage: 2 (three stages) or 3 (two stages)
+  int tc_tps = 0;         // kept for files that hold it (0, 2 or 3); one stage form is built
   int tc_tiled = -1;      // B by TMA boxes (0) or copied into tile order first (1)
   int tc_split = -1;      // split-K over the reduction when the output grid is small: 0 = never
 };

@@ -267,9 +267,10 @@ typedef struct bsp_batch bsp_batch;
 
 /* Prepare a batch of n independent problems sharing N (multiple of 8) and a
  * 16-bit B type: encodes every problem's B tensor map and uploads them with
- * a work list of (problem, 256-row block, 128-column block) items (wider than 128:
- * and of 256-column blocks) sorted longest reduction first; synchronises the stream once.  The problems'
- * buffers are referenced, not copied — they must outlive the batch.  Limit:
+ * a work list of (problem, 256-row block, 128-column block) items — for N above
+ * 128 also one of 256-column blocks — sorted longest reduction first;
+ * synchronises the stream once.  The problems' buffers are referenced, not
+ * copied — they must outlive the batch.  Limit:
  * K ≤ 131072 per problem (BSP_ERR_CAPACITY).  No reference counterpart (the
  * reference runs one fixed-size problem per launch).                       */
 int bsp_batch_create(const bsp_problem* problems, int n, int64_t N,
@@ -335,7 +336,7 @@ int bsp_batched_spmm_grad(const bsp_batch* batch, bsp_stream_t stream);
 
 /* A measured SpMM schedule: engine 1 = tensor cores, 2 = CUDA cores (per
  * shape bucket, this is the tensor-core density threshold); on the tensor
- * cores the tile form (K tiles per stage, B pre-tiled or by TMA boxes,
+ * cores the tile form (B pre-tiled or by TMA boxes,
  * split-K or not); on the CUDA cores with a prototype plan, proto_path 0 =
  * register gathers / 1 = TMA-staged slices and proto_variant = that
  * kernel's shape (columns per warp, gathers in flight, CTAs per SM); ms =
@@ -345,13 +346,13 @@ typedef struct bsp_schedule {
   int proto_path;
   int proto_variant;
   float ms;
-  int tc_stage_tiles;  /* tensor cores: K tiles per stage (2 or 3; 0 = rule) */
+  int tc_stage_tiles;  /* tensor cores: reported (2), chooses nothing: one stage form is built */
   int tc_tiled_b;      /* tensor cores: B copied into tile order (1), TMA boxes (0), rule (-1) */
   int tc_split;        /* tensor cores: split-K by the rule (-1) or never (0) */
 } bsp_schedule;
 
 /* Times every candidate schedule of bsp_spmm for this plan and these
- * operands (the tensor cores in 8 tile forms when allowed; each
+ * operands (the tensor cores in 4 tile forms when allowed, FP32 B in 1; each
  * prototype-kernel shape on both paths; 2 warm-up + 5 timed runs each, CUDA
  * events on `stream`, which it synchronises), leaves C holding the fastest one's result, returns it in
  * *best and caches it for the shape bucket (log2 of M, K, N; density in half
@@ -494,7 +495,8 @@ int bsp_stack_planes_b(const void* B, int b_dtype, int64_t ldb, int64_t K,
  * 16-byte access and N a multiple of 8 (BSP_ERR_ALIGNMENT), K up to 131072 and
  * N up to 65535 x 256 (BSP_ERR_CAPACITY).  The workspace holds B in two parts
  * (x = h + l), which keeps the sums as exact as the planes'; it may be smaller
- * or NULL: B is multiplied as it is then.  Same reference product as bsp_bitplane_spmm.                          */
+ * or NULL: B is multiplied as it is then.  Same reference product as
+ * bsp_bitplane_spmm.                                                       */
 int bsp_i8_tiles_bytes(int64_t M, int64_t K, size_t* bytes);
 int bsp_i8_tiles(const int8_t* A, int64_t M, int64_t K, int64_t lda, int8_t* tiles, bsp_stream_t stream);
 int bsp_spmm_i8_tiles_workspace(int64_t M, int64_t K, int64_t N, size_t* bytes);
@@ -560,9 +562,10 @@ int bsp_csr_to_tiled(const int32_t* row_ptr, const int32_t* col_idx,
  * device memory belongs to another allocator).  It runs bsp_spmm with, as
  * workspace, a static device array of 8 MiB inside the library, held on
  * every GPU that loads the library until the process exits: the array holds
- * the prototype sums and, for 16-bit B on the tensor cores, the split-K
- * partials and the tiled copy of B whenever they fit in it (the same route
- * bsp_spmm takes with an 8 MiB workspace, whatever the plan).
+ * the prototype sums and, whenever they fit in it, the scratch of the tensor
+ * cores (split-K partials, the tiled copy of B, sums in aligned rows, FP32 B's
+ * three parts) or an aligned copy of B (the same route bsp_spmm takes with an
+ * 8 MiB workspace, whatever the plan).
  * Limit: bsp_spmm_workspace(plan, N) must be ≤ 8 MiB (≈ n_proto * N * 4
  * bytes), else BSP_ERR_CAPACITY.  The first call on a device looks the
  * array's address up (cudaGetSymbolAddress) and keeps it: make that first
@@ -589,8 +592,11 @@ int bsp_probe_gather(const void* buf, int64_t rows, int64_t row_bytes,
                      const uint32_t* row_idx, int64_t n_warps, int64_t per_warp,
                      int slice_bytes, float* sink, bsp_stream_t stream);
 
-/* Device-side status of the asynchronous kernels (0 = none; 1 = a bounded
- * mbarrier wait of the TMA-staged SpMM expired and its output is invalid).
+/* Device-side status of the asynchronous kernels: 0 = none, else a bounded
+ * mbarrier wait expired and the output of that kernel is invalid — 1 the
+ * TMA-staged prototype rows, 2 the prototype sums, 3 the 16-bit SDDMM and the
+ * batches' launches of a CTA per item, 4 the batched SDDMM, 5 the tensor-core
+ * product (bits, int8 values, batches), 6 the staged FP32 SDDMM.
  * Synchronises the device; clear != 0 resets the word.  No reference
  * counterpart (the reference has no device-side error reporting).         */
 int bsp_device_status(int* status, int clear);
