@@ -279,7 +279,8 @@ def tune(words, K, B, plan, out=None, workspace=None):
     """Time every SpMM schedule for this plan and operands (bsp_tune), keep
     the fastest in the library's per-shape-bucket cache and return it as a
     dict (engine 1 = tensor cores, 2 = CUDA cores; the tensor-core tile form:
-    B pre-tiled or by boxes, split-K; the prototype path and shape; ms).  ``out`` ends holding the product."""
+    B pre-tiled or by boxes, split-K; the prototype path and shape; ms).
+    ``out`` ends holding the product."""
     M = words.shape[0]
     ldb = _rowmajor(B, "B")
     N = B.shape[1]
