@@ -294,3 +294,33 @@ def test_wide_batches_in_both_forms(N, count, lo, hi):
         if old is not None:
             os.environ["BSP_BATCH_PERSIST"] = old
     assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("switch", ["BSP_BATCH_PERSIST", "BSP_BATCH_SDDMM_PERSIST"])
+@pytest.mark.parametrize("N", [24, 264])
+def test_gradient_batches_a_block_at_a_time(N, switch, monkeypatch):
+    """The launches of a CTA per 256x256 block, whose lists a gradient batch builds
+    when the switch is set: exact on integers, as the persistent ones; without
+    the switch at creation the batch has the persistent form alone."""
+    probs = _grad_problems(9, N, seed=N + 7, integer=True)
+    dev, want = [], []
+    for A, words, K, X16, G16 in probs:
+        M = words.shape[0]
+        wd = torch.from_numpy(np.ascontiguousarray(words).view(np.int32)).cuda()
+        X, G = bf16_dev(X16), bf16_dev(G16)
+        dev.append((wd, K, X, G, torch.empty((K, N), device="cuda"), torch.empty((M, K), device="cuda")))
+        Ad = torch.from_numpy(A.astype(np.float32)).cuda()
+        want.append((Ad.T.double() @ G.double(), (G.double() @ X.double().T) * Ad.double()))
+    plain = ops.BatchGrad(dev)
+    monkeypatch.setenv(switch, "0")
+    blocks = ops.BatchGrad(dev)
+    for batch in (blocks, plain):
+        for *_, dX, dA in dev:
+            dX.fill_(float("nan"))
+            dA.fill_(float("nan"))
+        batch.run()
+        torch.cuda.synchronize()
+        for (*_, dX, dA), (wX, wA) in zip(dev, want):
+            assert torch.equal(dX.double(), wX) and torch.equal(dA.double(), wA)
+        batch.close()
+    assert capi.device_status() == 0
